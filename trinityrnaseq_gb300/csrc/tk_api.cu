@@ -326,12 +326,19 @@ int tk_ctx_create(int device, tk_ctx **out) {
         uint64_t thr = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
-    if (cudaMalloc(&c->d_err, DE_COUNT * sizeof(uint32_t)) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&c->h_wait_err, sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
         cudaStreamDestroy(c->stream);
         delete c;
         return TK_E_OOM;
     }
-    cudaMemset(c->d_err, 0, DE_COUNT * sizeof(uint32_t));
+    *c->h_wait_err = 0;
+    if (cudaMalloc(&c->d_err, (DE_COUNT + 1) * sizeof(uint32_t)) != cudaSuccess) {
+        cudaFreeHost(c->h_wait_err);
+        cudaStreamDestroy(c->stream);
+        delete c;
+        return TK_E_OOM;
+    }
+    cudaMemset(c->d_err, 0, (DE_COUNT + 1) * sizeof(uint32_t));
     *out = c;
     return TK_OK;
 }
@@ -364,6 +371,7 @@ static void ctx_release_now(tk_ctx *c) {
     for (auto e : c->free_events) cudaEventDestroy(e);
     if (c->bins_exec) cudaGraphExecDestroy(c->bins_exec);
     cudaFree(c->d_err);
+    cudaFreeHost(c->h_wait_err);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, c->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);
@@ -839,6 +847,7 @@ int tk_table_dump(tk_table *t, uint32_t min_count, int where, uint64_t *keys, ui
     dfree(c, dk);
     dfree(c, dc);
     if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "dump sync");
+    if (!e) e = wait_status(c);
     return e;
 }
 

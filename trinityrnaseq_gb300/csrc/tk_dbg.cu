@@ -282,6 +282,8 @@ int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id
     int rbits = 1;
     while ((1ULL << rbits) < n_rec) rbits++;
     TK_TRY(radix_sort_pairs(c, rec, idx, M, rbits, rec2, idx2, &in_tmp));
+    TK_CUDA(c, cudaStreamSynchronize(c->stream));
+    TK_TRY(wait_status(c));   // the sorted values index arrays below
     const uint64_t *srec = in_tmp ? rec2 : rec;
     const uint32_t *sidx = in_tmp ? idx2 : idx;
     uint32_t *head = nullptr;
@@ -310,6 +312,8 @@ int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id
     int pbits = 1;
     while ((1ULL << pbits) < n_pos) pbits++;
     TK_TRY(radix_sort_pairs(c, node_first, node_g, G, pbits, node_first2, node_g2, &in_tmp));
+    TK_CUDA(c, cudaStreamSynchronize(c->stream));
+    TK_TRY(wait_status(c));
     const uint64_t *ofirst = in_tmp ? node_first2 : node_first;
     const uint32_t *og = in_tmp ? node_g2 : node_g;
     uint32_t *rank_of = nullptr, *rec_first = nullptr;

@@ -207,7 +207,8 @@ struct tk_ctx {
     // host <-> device copies that overlap the work on `stream` (created on
     // first use; tk_ctx_synchronize waits for both streams)
     cudaStream_t copy_stream = nullptr;
-    uint32_t *d_err = nullptr;             // tk::DE_COUNT words
+    uint32_t *d_err = nullptr;             // tk::DE_COUNT words, then the sorts' wait error
+    uint32_t *h_wait_err = nullptr;        // page-locked: set when a sort's bounded wait ran out (wait_status)
     std::string last_error;
     // profiling (CUDA events on `stream` around the hot kernels)
     bool prof = false;
@@ -367,6 +368,7 @@ int scan_excl_u32_to_u64(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t 
 // K4 formatting of sorted (key, count) pairs (tk_table.cu)
 int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n, int k, char **text, uint64_t *len,
                 uint64_t **offs_out = nullptr);
+int wait_status(tk_ctx *c);
 int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits,
                      uint64_t *tmp_keys, uint32_t *tmp_vals, bool *result_in_tmp, int first_bit = 0);
 int table_alloc(tk_table *t, uint64_t capacity);

@@ -1102,6 +1102,7 @@ static int sort_side(tk_ctx *c, NormSide &s) {
     TK_TRY(sc.get((void **)&tperm, n * 4, "sort order"));
     TK_TRY(sc.get((void **)&d_u32, 16, "sort scalars"));
     TK_TRY(sc.get((void **)&orand, 16, "sort key bits"));
+    TK_CUDA(c, cudaMemsetAsync(tperm, 0, n * 4, c->stream));   // whatever a sort leaves there indexes a read
     TK_CUDA(c, cudaMemsetAsync(d_u32, 0, 16, c->stream));
     k_name_maxlen<<<(unsigned)std::min<uint64_t>(nm_grid(n), (uint64_t)c->sm_count * 8), NM_THREADS, 0, c->stream>>>(
         s.nlen, n, d_u32);
@@ -1163,6 +1164,7 @@ static int sort_side(tk_ctx *c, NormSide &s) {
         for (int ch = (int)nch - 1; ch >= 0; ch--) TK_TRY(pass(0, (uint32_t)ch));
         TK_TRY(gather());
     }
+    TK_TRY(wait_status(c));   // the sorts before the last synchronisation
     if (perm != s.perm) {
         TK_CUDA(c, cudaMemcpyAsync(s.perm, perm, n * 4, cudaMemcpyDeviceToDevice, c->stream));
     }
