@@ -1,6 +1,7 @@
 """FASTQ -> FASTA read prep on the GPU (tk_reads_to_fasta, bin/seqtk-trinity)
 against util/support_scripts/fastQ_to_fastA.pl's own output (golden fixtures)
 and the oracle's restatement of it, byte for byte."""
+import random
 import subprocess
 
 import pytest
@@ -38,6 +39,30 @@ def test_prep_parity_200k_pairs(ctx, oracle, append, rev, if_missing):
     flags = (oracle.FA_REV if rev else 0) | (oracle.FA_IF_MISSING if if_missing else 0)
     want = oracle.fastq_to_fasta(text, append, flags)
     assert ReadSet(ctx, text).to_fasta(append, revcomp=rev, if_missing=if_missing) == want
+
+
+@pytest.mark.parametrize("crlf", [False, True])
+@pytest.mark.parametrize("append,rev", [(1, False), (12, True)])
+def test_prep_record_shapes(ctx, oracle, crlf, append, rev):
+    """Headers with and without further fields, names of 0 to 40 bytes, sequences of 0 to 70, qualities of another
+    length or blank, '+' lines that repeat the name, and a last record without a newline; with CRs (the set's lines
+    are then searched) and without."""
+    rng = random.Random(7)
+    recs = []
+    for i in range(1500):
+        name = "".join(rng.choice("abcXYZ019:/_") for _ in range(rng.choice([0, 1, 2, 13, 40]))) + rng.choice(["", "/1", "/2"])
+        rest = rng.choice(["", "", " 1:N:0:ATC", " 2:Y:0", "\t1:", " x 1:", "  "])
+        n = rng.choice([0, 1, 15, 16, 17, 33, 70])
+        seq = "0" if n == 1 and rng.random() < 0.3 else "".join(rng.choice("ACGTNacgtRYKM") for _ in range(n))
+        q = "I" * (n + rng.choice([0, 0, 0, 0, 1])) if rng.random() < 0.95 else " " * n
+        recs.append(f"@{name}{rest}\n{seq}\n+{rng.choice(['', name])}\n{q}\n")
+    text = "".join(recs + ["@last\nACGTAC\n+\nIIIIII"])
+    if crlf:
+        text = text.replace("\n", "\r\n")
+    text = text.encode()
+    flags = oracle.FA_IGNORE_DIRTY | (oracle.FA_REV if rev else 0)
+    want = oracle.fastq_to_fasta(text, append, flags)
+    assert ReadSet(ctx, text).to_fasta(append, revcomp=rev, ignore_dirty=True) == want
 
 
 def test_prep_rejects_fasta_input(ctx, golden):

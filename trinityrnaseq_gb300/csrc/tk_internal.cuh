@@ -248,6 +248,7 @@ struct tk_reads {
     uint64_t *d_rd_off = nullptr;           // n_reads + 1
     uint64_t *d_name_off = nullptr;         // n_reads
     uint32_t *d_name_len = nullptr;         // n_reads
+    bool plain_seq = false;                 // FASTQ whose sequence lines hold no whitespace (a line = its read)
     char *d_fasta = nullptr;                // last FASTA conversion (tk_reads_to_fasta)
     uint64_t fasta_len = 0;
     int fasta_append = 0, fasta_flags = -1;
