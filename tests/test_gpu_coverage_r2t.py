@@ -116,6 +116,21 @@ def test_stats_narrow_read_sets(ctx, oracle, longest, ds):
     assert_stats(got, oracle.cov_values(text, keys, counts, 25, ds))
 
 
+@pytest.mark.parametrize("k,top", [(25, 200), (31, 70_000), (17, 0xFFFFFFF0), (25, 1)])
+@pytest.mark.parametrize("ds", [True, False])
+def test_stats_reads_past_the_register_classes(ctx, oracle, k, top, ds):
+    """257 to 1024 windows (values in shared memory, histogram select) and the first lengths past it, with counts of
+    one, two and four bytes; a fifth of the k-mers are absent from the catalogue."""
+    text = window_class_reads(k + 50, k, 4, [256, 257, 287, 288, 289, 400, 511, 512, 513, 1023, 1024, 1025, 1500])
+    keys, _ = oracle.count(text, k, ds)
+    rnd = np.random.default_rng(k)
+    keys = keys[rnd.random(keys.size) < 0.8]
+    counts = rnd.integers(1, top + 1, keys.size).astype(np.uint32)
+    t = KmerTable(ctx, k, ds)
+    t.load_pairs(keys, counts)
+    assert_stats(coverage_stats(t, ReadSet(ctx, text)), oracle.cov_values(text, keys, counts, k, ds))
+
+
 def test_stats_parity_1M_reads(ctx, oracle):
     text = synth.transcriptome_reads(seed=1, n_reads=1_000_000).tobytes()
     keys, counts = oracle.count(text, 25, True)

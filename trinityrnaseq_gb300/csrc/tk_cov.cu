@@ -9,8 +9,10 @@
 // mean and stdev come from exact integer sums (see finish_stats).
 //
 // Reads with at most 256 windows: one warp per read, values in registers,
-// median by a warp radix select (tk_warp.cuh).  Longer reads: one block per
-// read, values in a global scratch slab, block bitonic sort.
+// median by a warp radix select (tk_warp.cuh).  Up to 1024 windows: one warp
+// per read, values in shared memory, median by a histogram select.  Longer
+// reads: one block per read, values in a global scratch slab, block bitonic
+// sort.
 //
 // Coverage cache.  The reads whose coverage is asked for are, in Trinity's
 // use, the reads that were counted (insilico_read_normalization.pl counts
@@ -359,6 +361,148 @@ __global__ void __launch_bounds__(CV_THREADS, MAXS <= 4 ? 8 : 6) k_coverage(CovC
                                     long_n, held + (threadIdx.x & ~31u));
 }
 
+// Reads with more windows than the registers of a warp hold, up to CV_MID_MAX:
+// a warp per read, the lookups of four windows per lane issued together, the
+// values kept in the warp's shared memory, the median by counting them in a
+// 256-bin histogram per byte of the largest count.  A warp takes `per` reads
+// of the list and finishes their floating-point part in one pass; reads with
+// more windows go to `rest`.  Bound by the table's random access (4.2 TB/s of
+// DRAM reads, issue slots 31% busy): 1.78 ms for 124,000
+// reads of 257-570 windows, k = 31; a block per read with a bitonic sort in
+// global memory took 10.7 ms.
+constexpr uint32_t CV_MID_MAX = 1024;
+
+// shared memory of one block: per warp the values, the histogram, the sums
+static inline size_t mid_smem(uint32_t cap) { return (size_t)(CV_THREADS / 32) * (cap * 4 + 1024 + 32 * sizeof(ReadSums)); }
+
+// Element m (0-based, ascending) of the n values that are not PAD_VAL; mx is
+// the largest of them.
+__device__ __forceinline__ uint32_t warp_hist_select(const uint32_t *vals, uint32_t n, uint32_t m, uint32_t mx,
+                                                     uint32_t *hist) {
+    const unsigned lane = lane_id();
+    uint32_t prefix = 0;
+    for (int shift = mx ? (31 - __clz((int)mx)) & ~7 : 0; shift >= 0; shift -= 8) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) hist[i * 32 + lane] = 0;
+        __syncwarp();
+        for (uint32_t i = lane; i < n; i += 32) {
+            const uint32_t v = vals[i];
+            if (v != PAD_VAL && ((uint64_t)v >> (shift + 8)) == ((uint64_t)prefix >> (shift + 8)))
+                atomicAdd(&hist[(v >> shift) & 255u], 1u);
+        }
+        __syncwarp();
+        uint32_t sum = 0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) sum += hist[lane * 8 + i];
+        const uint32_t incl = warp_incl_scan(sum);
+        const unsigned owner = __ffs((int)__ballot_sync(0xffffffffu, incl > m)) - 1;   // its bins hold element m
+        uint32_t bin = 0, left = 0;
+        if (lane == owner) {
+            left = m - (incl - sum);
+            bin = lane * 8;
+            while (left >= hist[bin]) left -= hist[bin++];
+        }
+        bin = __shfl_sync(0xffffffffu, bin, (int)owner);
+        m = __shfl_sync(0xffffffffu, left, (int)owner);
+        prefix |= bin << shift;
+        __syncwarp();
+    }
+    return prefix;
+}
+
+template <bool CANON>
+__global__ void __launch_bounds__(CV_THREADS) k_coverage_mid(CovCache cc, DevTable t, const uint64_t *__restrict__ codes,
+                                                            const uint32_t *__restrict__ inv,
+                                                            const uint64_t *__restrict__ rd_off,
+                                                            const uint32_t *__restrict__ list, uint64_t n_list, int per,
+                                                            uint32_t cap, int k, uint32_t *__restrict__ median,
+                                                            float *__restrict__ mean, float *__restrict__ stdev,
+                                                            uint32_t *__restrict__ rest,
+                                                            unsigned long long *__restrict__ rest_n) {
+    extern __shared__ __align__(16) unsigned char mid_mem[];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    ReadSums *held = reinterpret_cast<ReadSums *>(mid_mem) + warp * 32;
+    uint32_t *hist = reinterpret_cast<uint32_t *>(mid_mem + (CV_THREADS / 32) * 32 * sizeof(ReadSums)) + warp * 256;
+    uint32_t *vals = reinterpret_cast<uint32_t *>(mid_mem + (CV_THREADS / 32) * (32 * sizeof(ReadSums) + 1024)) + warp * cap;
+    const uint64_t i0 = ((uint64_t)blockIdx.x * (CV_THREADS / 32) + warp) * (uint64_t)per;
+    const uint32_t nr = i0 >= n_list ? 0u : (uint32_t)min((uint64_t)per, n_list - i0);
+    for (uint32_t i = 0; i < nr; i++) {
+        const uint32_t r = list[i0 + i];
+        const uint64_t start = rd_off[r];
+        const uint64_t nwin = rd_off[r + 1] - start - 1 - (k - 1);
+        ReadSums rs{};
+        if (nwin > cap) {   // left to the block-per-read pass
+            rs.cnt = LONG_READ;
+            if (lane == 0) {
+                rest[atomicAdd(rest_n, 1ULL)] = r;
+                held[i] = rs;
+            }
+            continue;
+        }
+        uint32_t cnt = 0, mx = 0;
+        uint64_t sum = 0, hi = 0, lo = 0;
+        for (uint32_t w0 = 0; w0 < nwin; w0 += 128) {
+            uint64_t key[4];
+            uint32_t v[4], in = 0, need = 0;
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t w = w0 + u * 32 + lane;
+                key[u] = 0;
+                v[u] = PAD_VAL;
+                if (w < nwin && window_at<CANON>(codes, inv, start + w + (uint64_t)k - 1, k, key[u])) in |= 1u << u;
+            }
+            need = in;
+            if (cc.ent) {
+#pragma unroll
+                for (int u = 0; u < 4; u++)
+                    if ((in >> u) & 1u) {
+                        uint32_t tag;
+                        const uint64_t *b = cache_bucket(cc, key[u], &tag);
+                        const uint32_t c = cache_match(b, tag);
+                        if (c) {
+                            v[u] = c;
+                            need &= ~(1u << u);
+                        }
+                    }
+            }
+            tbl_get_many<4>(t, key, need, 1u, v);
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t w = w0 + u * 32 + lane;
+                if (w < nwin) vals[w] = v[u];
+                if (v[u] != PAD_VAL) {
+                    cnt++;
+                    mx = max(mx, v[u]);
+                    sum += v[u];
+                    const uint64_t sq = (uint64_t)v[u] * v[u], nlo = lo + sq;
+                    hi += nlo < lo;
+                    lo = nlo;
+                }
+            }
+        }
+        __syncwarp();
+        rs.cnt = __reduce_add_sync(0xffffffffu, cnt);
+        mx = __reduce_max_sync(0xffffffffu, mx);
+        rs.sum = warp_sum(sum);
+        warp_sum_u128(hi, lo);
+        rs.hi = hi;
+        rs.lo = lo;
+        rs.med = rs.cnt ? warp_hist_select(vals, (uint32_t)nwin, rs.cnt / 2, mx, hist) : 0u;
+        if (lane == 0) held[i] = rs;
+        __syncwarp();
+    }
+    __syncwarp();
+    if (lane < nr && held[lane].cnt != LONG_READ) {
+        const ReadSums mine = held[lane];
+        const uint32_t r = list[i0 + lane];
+        float m, sd;
+        finish_stats(mine.cnt, mine.sum, mine.hi, mine.lo, &m, &sd);
+        median[r] = mine.med;
+        mean[r] = m;
+        stdev[r] = sd;
+    }
+}
+
 // long reads: one block per read, `slab` = this block's scratch (n2max values)
 template <bool CANON>
 __global__ void __launch_bounds__(CV_THREADS) k_coverage_long(CovCache cc, DevTable t, const uint8_t *__restrict__ seq,
@@ -489,6 +633,40 @@ int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d
         e = cuda_check(c, cudaMemcpyAsync(&hl, long_n, 8, cudaMemcpyDeviceToHost, c->stream), "long n");
         if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "long sync");
     }
+    uint32_t *rest = nullptr;
+    const uint32_t *list = long_list;
+    if (!e && hl) {
+        const uint64_t max_win = rd->max_len - k + 1;
+        const uint32_t cap = (uint32_t)std::min<uint64_t>((max_win + 31) & ~31ULL, CV_MID_MAX);
+        const size_t smem = mid_smem(cap);
+        const bool more = max_win > cap;   // some reads may be left to the block-per-read pass
+        if (more) e = dmalloc(c, (void **)&rest, hl * 4, "long-read rest");
+        if (!e) e = cuda_check(c, cudaMemsetAsync(long_n, 0, 8, c->stream), "long reset");
+        const void *fn = t->canonical ? (const void *)k_coverage_mid<true> : (const void *)k_coverage_mid<false>;
+        if (!e) e = cuda_check(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)mid_smem(CV_MID_MAX)),
+                               "coverage mid smem");
+        if (!e) {
+            // reads per warp: as many as leave every resident warp some
+            const uint64_t resident = (uint64_t)c->sm_count * (CV_THREADS / 32) * std::max<uint64_t>(1, 220 * 1024 / smem);
+            const int per = (int)std::max<uint64_t>(1, std::min<uint64_t>(32, hl / (2 * resident)));
+            const uint64_t per_block = (uint64_t)per * (CV_THREADS / 32);
+            const unsigned grid = (unsigned)((hl + per_block - 1) / per_block);
+            if (t->canonical)
+                k_coverage_mid<true><<<grid, CV_THREADS, smem, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, long_list,
+                                                                            hl, per, cap, k, d_median, d_mean, d_stdev, rest, long_n);
+            else
+                k_coverage_mid<false><<<grid, CV_THREADS, smem, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, long_list,
+                                                                             hl, per, cap, k, d_median, d_mean, d_stdev, rest, long_n);
+            c->launches++;
+            e = check_launch(c, "coverage mid");
+        }
+        list = rest;
+        hl = 0;
+        if (!e && more) {
+            e = cuda_check(c, cudaMemcpyAsync(&hl, long_n, 8, cudaMemcpyDeviceToHost, c->stream), "rest n");
+            if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "rest sync");
+        }
+    }
     if (!e && hl) {
         uint64_t n2max = 1;
         while (n2max < (uint64_t)(rd->max_len - k + 1)) n2max <<= 1;
@@ -498,15 +676,16 @@ int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d
         if (!e) {
             if (t->canonical)
                 k_coverage_long<true><<<(unsigned)grid, CV_THREADS, 0, c->stream>>>(
-                    cc, dt, rd->d_seq, rd->d_rd_off, long_list, hl, k, scratch, n2max, d_median, d_mean, d_stdev);
+                    cc, dt, rd->d_seq, rd->d_rd_off, list, hl, k, scratch, n2max, d_median, d_mean, d_stdev);
             else
                 k_coverage_long<false><<<(unsigned)grid, CV_THREADS, 0, c->stream>>>(
-                    cc, dt, rd->d_seq, rd->d_rd_off, long_list, hl, k, scratch, n2max, d_median, d_mean, d_stdev);
+                    cc, dt, rd->d_seq, rd->d_rd_off, list, hl, k, scratch, n2max, d_median, d_mean, d_stdev);
             c->launches++;
             e = check_launch(c, "coverage long");
             dfree(c, scratch);
         }
     }
+    if (rest) dfree(c, rest);
     if (long_list) dfree(c, long_list);
     dfree(c, long_n);
     if (empty) dfree(c, empty);

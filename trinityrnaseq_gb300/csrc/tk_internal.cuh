@@ -139,6 +139,45 @@ __device__ __forceinline__ uint32_t tbl_get(DevTable t, uint64_t key, uint32_t m
     return miss;
 }
 
+// Both slots of the 32-byte sector holding slot s, in one load.
+__device__ __forceinline__ void tbl_load_pair(const DevTable &t, uint64_t s, ulonglong2 &a, ulonglong2 &b) {
+    asm("ld.global.L1::no_allocate.v4.u64 {%0,%1,%2,%3}, [%4];"
+        : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
+        : "l"(t.slots + (s & ~1ULL)));
+}
+
+// key's value in the sector (a, b) its probe reached at slot s: true when the
+// probe ends there.  (The slot before an odd s is not on the probe's way, but
+// a key found there is the key all the same.)
+__device__ __forceinline__ bool tbl_in_pair(uint64_t key, uint64_t s, const ulonglong2 &a, const ulonglong2 &b,
+                                            uint32_t miss, uint32_t &v) {
+    const bool ha = a.x == key, hb = b.x == key;
+    v = ha ? (uint32_t)a.y : hb ? (uint32_t)b.y : miss;
+    return ha || hb || b.x == EMPTY_KEY || (a.x == EMPTY_KEY && !(s & 1));
+}
+
+// tbl_get for U keys at once: the first sector of every key in `need` is
+// loaded before any is looked at, and a probe takes a sector (two slots) per
+// step.  Keys not in `need` keep their v.
+template <int U>
+__device__ __forceinline__ void tbl_get_many(const DevTable &t, const uint64_t (&key)[U], uint32_t need, uint32_t miss,
+                                             uint32_t (&v)[U]) {
+    ulonglong2 a[U], b[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+        if ((need >> u) & 1u) tbl_load_pair(t, tbl_home(t, mix64(key[u])), a[u], b[u]);
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+        if (!((need >> u) & 1u)) continue;
+        uint64_t s = tbl_home(t, mix64(key[u]));
+        for (uint64_t i = 0; i <= t.lmask; i += 2) {
+            if (i) tbl_load_pair(t, s, a[u], b[u]);
+            if (tbl_in_pair(key[u], s, a[u], b[u], miss, v[u])) break;
+            s = tbl_next(t, s | 1);
+        }
+    }
+}
+
 // one-slot-pair table every lookup misses in (an empty catalogue)
 __host__ __device__ __forceinline__ DevTable tbl_empty(Slot *two_slots) {
     DevTable t;

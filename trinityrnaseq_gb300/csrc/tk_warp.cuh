@@ -179,6 +179,24 @@ __device__ __forceinline__ void lane_windows_codes(const uint64_t *__restrict__ 
     }
 }
 
+// The window ending at position e of the read set's 2-bit codes (see
+// lane_windows_codes): its key, and whether all its positions are A/C/G/T.
+template <bool CANON>
+__device__ __forceinline__ bool window_at(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv, uint64_t e,
+                                          int k, uint64_t &key) {
+    const int64_t q = (int64_t)(e >> 5);
+    const int i = (int)(e & 31), s = 62 - 2 * i;
+    const uint64_t hi = __ldg(codes + q - 1), lo = __ldg(codes + q);
+    const uint64_t m = ((uint64_t)__ldg(inv + q - 1) << 32) | __ldg(inv + q);
+    const uint64_t fw = (s ? ((lo >> s) | (hi << (64 - s))) : lo) & ((1ULL << (2 * k)) - 1);
+    key = fw;
+    if (CANON) {
+        const uint64_t rc = kmer_revcomp(fw, k);
+        key = rc < fw ? rc : fw;
+    }
+    return ((m >> (31 - i)) & ((1ULL << k) - 1)) == 0;
+}
+
 // Element m (0-based, ascending) of the warp's valid values -- value v[j] of a
 // lane counts when bit j of its vm is set -- by a bit-serial radix select from
 // the top bit of the largest value: per bit, the values still in the running
