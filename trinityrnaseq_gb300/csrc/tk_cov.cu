@@ -36,6 +36,7 @@
 #include "tk_warp.cuh"
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <mutex>
 #include <string>
@@ -200,7 +201,12 @@ constexpr uint32_t LONG_READ = 0xFFFFFFFFu;   // cnt of a read left to the long-
 // statistics.  The lookups of a stage are independent loads issued together.
 // (Pipelining two reads -- the next read's cache answers and table prefetches
 // before the current read's statistics -- was 2.4x slower on GB300: the
-// registers it holds across stages spill.)
+// registers it holds across stages spill.  Issuing the first sector of all of
+// a lane's table lookups together, as the mid-length pass does, needs 64
+// registers: at 4 blocks per SM 15.9 ms against 14.2 for 5M pairs.  A table
+// probe of a sector per step instead of a slot, the sectors first to leave L2,
+// took them from 15.6 ms: random sectors come from HBM at 38 G/s on GB300
+// whatever their size up to 128 bytes, so what counts is their number.)
 template <int S, bool CANON>
 __device__ __forceinline__ void cov_stage1(const CovCache &cc, const uint64_t *__restrict__ codes,
                                            const uint32_t *__restrict__ inv, uint64_t start, uint32_t nwin, int k,
@@ -223,10 +229,11 @@ __device__ __forceinline__ void cov_stage1(const CovCache &cc, const uint64_t *_
 }
 
 template <int S>
-__device__ __forceinline__ void cov_stage2(DevTable t, const uint64_t (&key)[S], uint32_t (&v)[S], uint32_t vm) {
+__device__ __forceinline__ void cov_stage2(DevTable t, bool stream, const uint64_t (&key)[S], uint32_t (&v)[S],
+                                           uint32_t vm) {
 #pragma unroll
     for (int j = 0; j < S; j++)
-        if (((vm >> j) & 1u) && v[j] == 0) v[j] = tbl_get(t, key[j], 1u);
+        if (((vm >> j) & 1u) && v[j] == 0) v[j] = tbl_get2(t, key[j], stream, 1u);
 }
 
 template <int S>
@@ -283,15 +290,15 @@ __device__ __forceinline__ ReadSums cov_warp_read(const CovCache &cc, DevTable t
     uint64_t key[S];
     uint32_t v[S], vm;
     cov_stage1<S, CANON>(cc, codes, inv, start, nwin, k, key, v, vm);
-    cov_stage2<S>(t, key, v, vm);
+    cov_stage2<S>(t, cc.ent != nullptr, key, v, vm);
     return cov_stage3<S>(v, vm);
 }
 
-// One warp, 32 consecutive reads [r0, r0 + 32): the warp computes each read's
-// sums in turn and lane i keeps read r0 + i's; then every lane finishes its own
-// read.  The floating-point finish runs on the FP64 pipe, whose cost is per
-// warp instruction whatever the number of active lanes, so finishing 32 reads
-// in one pass costs what one read alone would.  Reads with more than
+// One warp, `per` (at most 32) consecutive reads from r0 on: the warp computes
+// each read's sums in turn and lane i keeps read r0 + i's; then every lane
+// finishes its own read.  The floating-point finish runs on the FP64 pipe,
+// whose cost is per warp instruction whatever the number of active lanes, so
+// finishing 32 reads in one pass costs what one read alone would.  Reads with more than
 // CV_WARP_MAX windows are appended to long_list (or, with no list, left to a
 // separate pass) and not written here.  MAXS = the largest window class
 // compiled in (windows per lane); a read set whose reads all have at most
@@ -299,12 +306,12 @@ __device__ __forceinline__ ReadSums cov_warp_read(const CovCache &cc, DevTable t
 template <bool CANON, int MAXS = 8>
 __device__ __forceinline__ void cov_warp_chunk(const CovCache &cc, DevTable t, const uint64_t *__restrict__ codes,
                                                const uint32_t *__restrict__ inv,
-                                               const uint64_t *__restrict__ rd_off, uint64_t n_reads, int k, uint64_t r0,
-                                               uint32_t *__restrict__ median, float *__restrict__ mean,
+                                               const uint64_t *__restrict__ rd_off, uint64_t n_reads, uint32_t per, int k,
+                                               uint64_t r0, uint32_t *__restrict__ median, float *__restrict__ mean,
                                                float *__restrict__ stdev, uint32_t *__restrict__ long_list,
                                                unsigned long long *__restrict__ long_n, ReadSums *__restrict__ held) {
     const unsigned lane = lane_id();
-    const uint32_t nr = n_reads - r0 < 32 ? (uint32_t)(n_reads - r0) : 32u;
+    const uint32_t nr = n_reads - r0 < per ? (uint32_t)(n_reads - r0) : per;
     // lane i holds the start of read r0 + i; the end of the last is one more load
     const uint64_t my_start = rd_off[r0 + (lane < nr ? lane : nr)];
     const uint64_t last_end = __shfl_sync(0xffffffffu, my_start, (int)(nr < 32 ? nr : 31));
@@ -349,16 +356,24 @@ __device__ __forceinline__ void cov_warp_chunk(const CovCache &cc, DevTable t, c
 template <bool CANON, int MAXS>
 __global__ void __launch_bounds__(CV_THREADS, MAXS <= 4 ? 8 : 6) k_coverage(CovCache cc, DevTable t, const uint64_t *__restrict__ codes,
                                                         const uint32_t *__restrict__ inv,
-                                                        const uint64_t *__restrict__ rd_off, uint64_t n_reads, int k,
+                                                        const uint64_t *__restrict__ rd_off, uint64_t n_reads,
+                                                        uint32_t per, int k,
                                                         uint32_t *__restrict__ median, float *__restrict__ mean,
                                                         float *__restrict__ stdev, uint32_t *__restrict__ long_list,
                                                         unsigned long long *__restrict__ long_n) {
     __shared__ ReadSums held[CV_THREADS];
     const uint64_t warps = (uint64_t)gridDim.x * (CV_THREADS / 32);
-    const uint64_t chunks = (n_reads + 31) / 32;
+    const uint64_t chunks = (n_reads + per - 1) / per;
     for (uint64_t ch = (uint64_t)blockIdx.x * (CV_THREADS / 32) + (threadIdx.x >> 5); ch < chunks; ch += warps)
-        cov_warp_chunk<CANON, MAXS>(cc, t, codes, inv, rd_off, n_reads, k, ch * 32, median, mean, stdev, long_list,
+        cov_warp_chunk<CANON, MAXS>(cc, t, codes, inv, rd_off, n_reads, per, k, ch * per, median, mean, stdev, long_list,
                                     long_n, held + (threadIdx.x & ~31u));
+}
+
+// Reads per warp and turn.  A warp's turn costs about 9 us per read (its chain
+// of lookups) and one FP64 finish, 1.2 us of its SM's pipe whatever the number
+// of reads; the sum of the two is least at sqrt(n / 1200) reads, up to 32.
+static uint32_t reads_per_turn(uint64_t n) {
+    return (uint32_t)std::max(1.0, std::min(32.0, std::sqrt((double)n / 1200.0)));
 }
 
 // Reads with more windows than the registers of a warp hold, up to CV_MID_MAX:
@@ -465,7 +480,7 @@ __global__ void __launch_bounds__(CV_THREADS) k_coverage_mid(CovCache cc, DevTab
                         }
                     }
             }
-            tbl_get_many<4>(t, key, need, 1u, v);
+            tbl_get_many<4>(t, key, need, cc.ent != nullptr, 1u, v);
 #pragma unroll
             for (int u = 0; u < 4; u++) {
                 const uint32_t w = w0 + u * 32 + lane;
@@ -588,8 +603,8 @@ int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d
     CovCache cc{};
     if (!e && t->capacity) e = cache_get_or_build(t, &cc);
     if (!e) {
-        // one wave of resident blocks, each warp striding over the 32-read
-        // chunks (a grid of several partial waves leaves SMs idle at its end)
+        // one wave of resident blocks, each warp striding over the chunks of
+        // `per` reads (a grid of several partial waves leaves SMs idle at its end);
         // the narrowest kernel that holds the longest read's windows
         static int per_sm[6] = {0, 0, 0, 0, 0, 0};
         const uint64_t max_win = rd->max_len >= (uint32_t)k ? rd->max_len - k + 1 : 0;
@@ -606,14 +621,15 @@ int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d
             }
             per_sm[ci] = std::max(1, b);
         }
-        const uint64_t chunks = (n + 31) / 32;
+        const uint32_t per = reads_per_turn(n);
+        const uint64_t chunks = (n + per - 1) / per;
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((chunks + CV_THREADS / 32 - 1) / (CV_THREADS / 32),
                                   (uint64_t)c->sm_count * (uint64_t)per_sm[ci]));
         cudaEvent_t ev;
         prof_begin(c, TK_KID_COVERAGE, &ev);
 #define TK_COV_LAUNCH(C, M)                                                                                   \
-    k_coverage<C, M><<<grid, CV_THREADS, 0, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, n, k, d_median, \
+    k_coverage<C, M><<<grid, CV_THREADS, 0, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, n, per, k, d_median, \
                                                          d_mean, d_stdev, long_list, long_n)
         switch (ci) {
         case 0: TK_COV_LAUNCH(false, 8); break;
@@ -714,7 +730,7 @@ constexpr uint64_t NOALLOC_SLAB = NOALLOC_SCRATCH_BYTES / 4 / NOALLOC_BLOCKS;   
 constexpr int NOALLOC_MAX_DEVICES = 64;
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_SCRATCH_BYTES / 4];
-static __device__ __align__(16) Slot g_noalloc_empty[2] = {{EMPTY_KEY, 0u, 0u}, {EMPTY_KEY, 0u, 0u}};
+static __device__ __align__(32) Slot g_noalloc_empty[2] = {{EMPTY_KEY, 0u, 0u}, {EMPTY_KEY, 0u, 0u}};
 
 // short reads only (<= 256 windows); longer reads are left to k_coverage_long_slab
 template <bool CANON>
@@ -728,7 +744,7 @@ __global__ void __launch_bounds__(CV_THREADS, 4) k_coverage_short(DevTable t, co
     const uint64_t chunks = (n_reads + 31) / 32;
     const CovCache none{};
     for (uint64_t ch = (uint64_t)blockIdx.x * (CV_THREADS / 32) + (threadIdx.x >> 5); ch < chunks; ch += warps)
-        cov_warp_chunk<CANON>(none, t, codes, inv, rd_off, n_reads, k, ch * 32, median, mean, stdev, nullptr, nullptr,
+        cov_warp_chunk<CANON>(none, t, codes, inv, rd_off, n_reads, 32, k, ch * 32, median, mean, stdev, nullptr, nullptr,
                               held + (threadIdx.x & ~31u));
 }
 

@@ -139,11 +139,19 @@ __device__ __forceinline__ uint32_t tbl_get(DevTable t, uint64_t key, uint32_t m
     return miss;
 }
 
-// Both slots of the 32-byte sector holding slot s, in one load.
-__device__ __forceinline__ void tbl_load_pair(const DevTable &t, uint64_t s, ulonglong2 &a, ulonglong2 &b) {
-    asm("ld.global.L1::no_allocate.v4.u64 {%0,%1,%2,%3}, [%4];"
-        : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
-        : "l"(t.slots + (s & ~1ULL)));
+// Both slots of the 32-byte sector holding slot s, in one load.  `stream`: the
+// sector is the first to leave L2 (lookups into a table far larger than L2,
+// beside something that is to stay there).
+__device__ __forceinline__ void tbl_load_pair(const DevTable &t, uint64_t s, bool stream, ulonglong2 &a, ulonglong2 &b) {
+    const Slot *p = t.slots + (s & ~1ULL);
+    if (stream)
+        asm("ld.global.L1::no_allocate.L2::evict_first.v4.u64 {%0,%1,%2,%3}, [%4];"
+            : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
+            : "l"(p));
+    else
+        asm("ld.global.L1::no_allocate.v4.u64 {%0,%1,%2,%3}, [%4];"
+            : "=l"(a.x), "=l"(a.y), "=l"(b.x), "=l"(b.y)
+            : "l"(p));
 }
 
 // key's value in the sector (a, b) its probe reached at slot s: true when the
@@ -156,22 +164,34 @@ __device__ __forceinline__ bool tbl_in_pair(uint64_t key, uint64_t s, const ulon
     return ha || hb || b.x == EMPTY_KEY || (a.x == EMPTY_KEY && !(s & 1));
 }
 
-// tbl_get for U keys at once: the first sector of every key in `need` is
-// loaded before any is looked at, and a probe takes a sector (two slots) per
-// step.  Keys not in `need` keep their v.
+// key's value, or miss: a sector (two slots) per probe step.
+__device__ __forceinline__ uint32_t tbl_get2(const DevTable &t, uint64_t key, bool stream, uint32_t miss) {
+    uint64_t s = tbl_home(t, mix64(key));
+    uint32_t v = miss;
+    for (uint64_t i = 0; i <= t.lmask; i += 2) {
+        ulonglong2 a, b;
+        tbl_load_pair(t, s, stream, a, b);
+        if (tbl_in_pair(key, s, a, b, miss, v)) break;
+        s = tbl_next(t, s | 1);
+    }
+    return v;
+}
+
+// tbl_get2 for U keys at once: the first sector of every key in `need` is
+// loaded before any is looked at.  Keys not in `need` keep their v.
 template <int U>
-__device__ __forceinline__ void tbl_get_many(const DevTable &t, const uint64_t (&key)[U], uint32_t need, uint32_t miss,
-                                             uint32_t (&v)[U]) {
+__device__ __forceinline__ void tbl_get_many(const DevTable &t, const uint64_t (&key)[U], uint32_t need, bool stream,
+                                             uint32_t miss, uint32_t (&v)[U]) {
     ulonglong2 a[U], b[U];
 #pragma unroll
     for (int u = 0; u < U; u++)
-        if ((need >> u) & 1u) tbl_load_pair(t, tbl_home(t, mix64(key[u])), a[u], b[u]);
+        if ((need >> u) & 1u) tbl_load_pair(t, tbl_home(t, mix64(key[u])), stream, a[u], b[u]);
 #pragma unroll
     for (int u = 0; u < U; u++) {
         if (!((need >> u) & 1u)) continue;
         uint64_t s = tbl_home(t, mix64(key[u]));
         for (uint64_t i = 0; i <= t.lmask; i += 2) {
-            if (i) tbl_load_pair(t, s, a[u], b[u]);
+            if (i) tbl_load_pair(t, s, stream, a[u], b[u]);
             if (tbl_in_pair(key[u], s, a[u], b[u], miss, v[u])) break;
             s = tbl_next(t, s | 1);
         }
