@@ -169,6 +169,59 @@ def test_r2t_parity_medium_and_long(ctx, oracle):
             oracle.r2t(r, b, 25, False, p)
 
 
+def r2t_shapes(seed, k, n_reads):
+    """A bundle whose records share stretches, on both strands and inside one record, with contigs as short as a
+    window, N and X breaks; and reads cut from it across errors, breaks, ends and two records, of every length the
+    alignment path takes and a few past it."""
+    rnd = np.random.default_rng(seed)
+    acgt = np.frombuffer(b"ACGT", dtype=np.uint8)
+    comp = bytes.maketrans(b"ACGT", b"TGCA")
+    rc = lambda s: s.translate(comp)[::-1]
+    contigs, recs = [], []
+    for i in range(60):
+        cs = []
+        for _ in range(rnd.integers(1, 5)):
+            c = rnd.choice(acgt, rnd.integers(k, 400)).tobytes()
+            if contigs and rnd.random() < 0.6:
+                o = contigs[rnd.integers(len(contigs))]
+                a = rnd.integers(0, max(1, len(o) - k))
+                piece = o[a:a + rnd.integers(k, 200)]
+                c = c[:100] + (rc(piece) if rnd.random() < 0.5 else piece) + c[100:]
+            if rnd.random() < 0.2:
+                c = c[:50] + b"N" + c[51:]
+            cs.append(c)
+            contigs.append(c)
+        recs.append(b">s_%d\n" % (1000 - i) + b"X".join(cs) + b"\n")
+    reads = []
+    for i in range(n_reads):
+        c = contigs[rnd.integers(len(contigs))]
+        L = int(rnd.choice([k - 1, k, k + 1, 33, 64, 76, 100, 127 + k, 128 + k, 150, 300]))
+        a = int(rnd.integers(0, max(1, len(c) - 10)))
+        s = bytearray(c[a:a + L])
+        if rnd.random() < 0.2:
+            s += contigs[rnd.integers(len(contigs))][:L - len(s)]
+        for _ in range(rnd.integers(0, 4)):
+            if s:
+                s[rnd.integers(len(s))] = rnd.choice(np.frombuffer(b"ACGTN", dtype=np.uint8))
+        s = bytes(s) or b"A"
+        reads.append(b">q%d\n" % i + (rc(s) if rnd.random() < 0.5 else s) + b"\n")
+    return b"".join(recs), b"".join(reads)
+
+
+@pytest.mark.parametrize("k", [7, 24, 25, 31])
+@pytest.mark.parametrize("strand", [False, True])
+def test_r2t_alignment_path(ctx, oracle, k, strand):
+    """A read set larger than its bundle is aligned, a small one voted per window; both give the oracle's records."""
+    b, r = r2t_shapes(k, k, 4000)
+    small = b"".join(r.split(b">q")[0:1] + [b">q" + x for x in r.split(b">q")[1:40]])
+    z = ReadsToTranscripts(ctx, b, k, strand)
+    for text in (small, r, small):
+        for g, w in zip(z.assign(ReadSet(ctx, text)), oracle.r2t_values(text, b, k, strand)):
+            np.testing.assert_array_equal(g, w)
+    keys, _ = oracle.count(b.replace(b"X", b"N"), k, not strand)
+    assert z.n_kmers == keys.size
+
+
 def test_r2t_first_record_owns_shared_kmer(ctx):
     shared = b"ACGTTGCAAGCTTAGCATCGATCGGATCCAGT"
     b = b">s_7\n" + shared + b"X" + b"T" * 30 + b"\n>s_3\n" + b"G" * 10 + shared + b"\n"

@@ -20,7 +20,8 @@ int table_sorted_pairs(tk_table *t, uint32_t min_count, uint64_t **keys, uint32_
 int table_insert_pairs(tk_table *t, const uint64_t *d_keys, const uint32_t *d_cnt, uint64_t n);
 int table_load_dump_reads(tk_table *t, const tk_reads *r);
 int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d_mean, float *d_stdev);
-int r2t_build(tk_r2t *z, const tk_reads *b);
+int r2t_build(tk_r2t *z, tk_reads *b);
+void r2t_release(tk_r2t *z);
 int r2t_assign(tk_r2t *z, const tk_reads *rd, int32_t *d_rec, uint32_t *d_hits, uint32_t *d_nwin);
 
 int set_err(tk_ctx *c, int code, const std::string &msg) {
@@ -1093,6 +1094,7 @@ void tk_r2t_free(tk_r2t *z) {
     if (!z) return;
     tk_ctx *c = z->ctx;
     if (z->table) tk_table_free(z->table);
+    r2t_release(z);
     delete z;
     ctx_release(c);
 }

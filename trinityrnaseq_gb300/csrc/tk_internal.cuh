@@ -114,13 +114,34 @@ __device__ __forceinline__ bool tbl_add(DevTable t, uint64_t key, uint32_t inc, 
     return false;
 }
 
-// Keeps the minimum value per key (ReadsToTranscripts ownership).
-__device__ __forceinline__ bool tbl_min(DevTable t, uint64_t key, uint32_t v, int max_probes) {
+// Claims an empty slot (key EMPTY_KEY, value words `empty`) for (key, v) in one
+// 128-bit CAS; returns what the slot held.  For keys that are mostly new: a
+// CAS of the key and a second atomic on the value cost two random accesses
+// (13.6M bundle windows 1.13 ms with a 64-bit minimum, 0.68 with a 32-bit one;
+// 0.55 this way).
+__device__ __forceinline__ ulonglong2 slot_claim(Slot *slot, uint64_t empty, uint64_t key, uint64_t v) {
+    ulonglong2 r;
+    asm volatile("{\n\t.reg .b128 d, e, n;\n\tmov.b128 e, {%3, %4};\n\tmov.b128 n, {%5, %6};\n\t"
+                 "atom.global.cas.b128 d, [%2], e, n;\n\tmov.b128 {%0, %1}, d;\n\t}"
+                 : "=l"(r.x), "=l"(r.y)
+                 : "l"(slot), "l"(EMPTY_KEY), "l"(empty), "l"(key), "l"(v)
+                 : "memory");
+    return r;
+}
+
+// Keeps the minimum 64-bit value per key, in the slot's val (low half) and pad
+// (ReadsToTranscripts: the record in the low half, a position in the high
+// one; empty slots hold ~0).  *added counts the keys inserted.
+__device__ __forceinline__ bool tbl_min(DevTable t, uint64_t key, uint64_t v, int max_probes, uint32_t *added) {
     uint64_t s = tbl_home(t, mix64(key));
     for (int i = 0; i < max_probes; i++) {
-        unsigned long long cur = tbl_claim(&t.slots[s], key);
-        if (cur == key) {
-            atomicMin(&t.slots[s].val, v);
+        const ulonglong2 was = slot_claim(&t.slots[s], ~0ULL, key, v);
+        if (was.x == EMPTY_KEY) {
+            *added += 1;
+            return true;
+        }
+        if (was.x == key) {
+            if (was.y > v) atomicMin(reinterpret_cast<unsigned long long *>(&t.slots[s].val), (unsigned long long)v);
             return true;
         }
         s = tbl_next(t, s);
@@ -157,17 +178,19 @@ __device__ __forceinline__ void tbl_load_pair(const DevTable &t, uint64_t s, boo
 // key's value in the sector (a, b) its probe reached at slot s: true when the
 // probe ends there.  (The slot before an odd s is not on the probe's way, but
 // a key found there is the key all the same.)
-__device__ __forceinline__ bool tbl_in_pair(uint64_t key, uint64_t s, const ulonglong2 &a, const ulonglong2 &b,
-                                            uint32_t miss, uint32_t &v) {
+template <typename V>
+__device__ __forceinline__ bool tbl_in_pair(uint64_t key, uint64_t s, const ulonglong2 &a, const ulonglong2 &b, V miss,
+                                            V &v) {
     const bool ha = a.x == key, hb = b.x == key;
-    v = ha ? (uint32_t)a.y : hb ? (uint32_t)b.y : miss;
+    v = ha ? (V)a.y : hb ? (V)b.y : miss;
     return ha || hb || b.x == EMPTY_KEY || (a.x == EMPTY_KEY && !(s & 1));
 }
 
 // key's value, or miss: a sector (two slots) per probe step.
-__device__ __forceinline__ uint32_t tbl_get2(const DevTable &t, uint64_t key, bool stream, uint32_t miss) {
+template <typename V>
+__device__ __forceinline__ V tbl_get2(const DevTable &t, uint64_t key, bool stream, V miss) {
     uint64_t s = tbl_home(t, mix64(key));
-    uint32_t v = miss;
+    V v = miss;
     for (uint64_t i = 0; i <= t.lmask; i += 2) {
         ulonglong2 a, b;
         tbl_load_pair(t, s, stream, a, b);
@@ -351,6 +374,16 @@ struct tk_r2t {
     tk_table *table = nullptr;              // key -> bundle record index
     uint64_t n_records = 0;
     std::vector<uint64_t> comp_id;          // per bundle record
+    // the bundle's 2-bit form (kept from its parse) and the index over it that
+    // the first large enough read set builds (tk_r2t.cu)
+    uint64_t seq_len = 0, n_bases = 0;
+    uint64_t *d_pack_alloc = nullptr;
+    const uint64_t *d_codes = nullptr;
+    const uint32_t *d_inv = nullptr;
+    uint64_t *d_rd_off = nullptr;
+    uint32_t *d_foreign = nullptr;          // bit per window end: an earlier record owns its k-mer (word 1 = word 0 of inv)
+    unsigned long long *d_filter = nullptr; // two bits per k-mer of the bundle in a 64-bit word
+    uint64_t filter_mask = 0;
 };
 
 // per-record de Bruijn k-mer graphs of a bundle (tk_dbg.cu)
@@ -432,7 +465,7 @@ int wait_status(tk_ctx *c);
 int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits,
                      uint64_t *tmp_keys, uint32_t *tmp_vals, bool *result_in_tmp, int first_bit = 0);
 int table_alloc(tk_table *t, uint64_t capacity);
-int table_alloc_init(tk_table *t, uint64_t capacity, uint32_t init_val);
+int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val);
 int table_rehash(tk_table *t, uint64_t new_capacity);
 int table_count_seq(tk_table *t, const tk_reads *r);
 int reads_fasta(tk_reads *r, int append, int flags, char **d_text, uint64_t *text_len);

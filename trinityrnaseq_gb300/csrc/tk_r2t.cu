@@ -4,13 +4,28 @@
 // Build: the bundle (one '>s_<component>' record per component, contigs
 // joined by 'X', util/support_scripts/add_LR_reads_to_iworm_bundle.pl:19-47)
 // is parsed like reads; every window of k A/C/G/T bases is inserted with
-// value = its record index through atomicMin, so a k-mer held by several
-// records belongs to the first of them whatever the insertion order.
-// Assign: one warp per read packs the read's bases 2 bits each into shared
-// memory, cuts each lane's windows out of it, looks them up, sorts the record
-// indices in registers and takes the longest run: the record with most votes,
-// ties to the smaller index.  Reads with more than 256 windows use one block
-// and a global scratch slab.
+// value = (its end position, its record index) through a 64-bit atomicMin, so
+// a k-mer held by several records belongs to the first of them whatever the
+// insertion order, and the table also says where it first occurs.
+//
+// Assign, by alignment (k_r2t_align): one thread per read.  A lookup of the
+// read's first open window gives the place of its k-mer in the bundle; from
+// there read and bundle are compared 32 bases at a time, and every window up
+// to the first difference has the same owner, as long as no earlier record
+// owns the bundle's k-mer there (a bit per bundle position).  Windows over a
+// sequencing error mostly hold k-mers the bundle does not have: a small filter
+// of the bundle's k-mers that stays in L2 answers for them.  A read of 100
+// bases then costs two or three random table accesses instead of 76.  Reads
+// whose windows belong to more than one record, or with more than 128
+// windows, are left to the per-window kernel.  The bits and the filter are
+// built by the first read set that has as many bases as the bundle.
+//
+// Assign, per window (k_r2t_assign): one warp per read packs the read's bases
+// 2 bits each into shared memory, cuts each lane's windows out of it, looks
+// them up, sorts the record indices in registers and takes the longest run:
+// the record with most votes, ties to the smaller index.  Reads with more than
+// 256 windows use one block and a global scratch slab.
+#include "tk_windows.cuh"
 #include "tk_warp.cuh"
 
 #include <algorithm>
@@ -22,45 +37,225 @@ constexpr int RT_SPAN = 32;
 constexpr uint32_t RT_WARP_MAX = 256;
 
 int parse_reads(tk_ctx *c, tk_reads *r);
-int table_alloc_init(tk_table *t, uint64_t capacity, uint32_t init_val);
+int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val);
 
+// the record holding position p: the largest r with rd_off[r] <= p
+__device__ __forceinline__ uint64_t r2t_record_of(const uint64_t *__restrict__ rd_off, uint64_t n_rec, uint64_t p) {
+    uint64_t lo = 0, hi = n_rec;
+    while (hi - lo > 1) {
+        const uint64_t mid = (lo + hi) >> 1;
+        if (__ldg(rd_off + mid) <= p) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// Calls f(key, end position, record) for every window of the bundle ending in
+// the thread's 32 positions.
+template <bool CANON, typename F>
+__device__ __forceinline__ void bundle_windows(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv,
+                                               uint64_t w, uint64_t n, const uint64_t *__restrict__ rd_off, uint64_t n_rec,
+                                               int k, F &&f) {
+    const uint64_t p0 = w * RT_SPAN;
+    uint64_t rec = 0, next = 0;
+    if (p0 < n) {
+        rec = r2t_record_of(rd_off, n_rec, p0);
+        next = __ldg(rd_off + rec + 1);
+    }
+    thread_windows<CANON>(codes, inv, w, p0 < n, k, [&](uint64_t key, int i) {
+        while (p0 + i >= next && rec + 1 < n_rec) next = __ldg(rd_off + ++rec + 1);
+        f(key, p0 + i, (uint32_t)rec);
+    });
+}
+
+// Bound by the atomics into a table larger than L2: one CAS per window, 23 G/s
+// on GB300 (13.6M windows 0.55 ms).
 template <bool CANON>
-__global__ void __launch_bounds__(RT_THREADS) k_r2t_build(const uint8_t *__restrict__ seq, uint64_t n,
+__global__ void __launch_bounds__(RT_THREADS) k_r2t_build(const uint64_t *__restrict__ codes,
+                                                         const uint32_t *__restrict__ inv, uint64_t n,
                                                          const uint64_t *__restrict__ rd_off, uint64_t n_rec, int k,
-                                                         DevTable t, int max_probes, uint32_t *__restrict__ err) {
-    const uint64_t kmask = (1ULL << (2 * k)) - 1;
-    const int shift = 2 * (k - 1);
-    const uint64_t stride = (uint64_t)gridDim.x * RT_THREADS * RT_SPAN;
-    for (uint64_t p0 = ((uint64_t)blockIdx.x * RT_THREADS + threadIdx.x) * RT_SPAN; p0 < n; p0 += stride) {
-        // record holding position p0: largest r with rd_off[r] <= p0
-        uint64_t lo = 0, hi = n_rec;
-        while (hi - lo > 1) {
-            uint64_t mid = (lo + hi) >> 1;
-            if (rd_off[mid] <= p0) lo = mid; else hi = mid;
+                                                         DevTable t, int max_probes, uint32_t *__restrict__ err,
+                                                         unsigned long long *__restrict__ distinct) {
+    const uint64_t w = (uint64_t)blockIdx.x * RT_THREADS + threadIdx.x;
+    uint32_t added = 0;
+    bundle_windows<CANON>(codes, inv, w, n, rd_off, n_rec, k, [&](uint64_t key, uint64_t e, uint32_t rec) {
+        // positions past 2^32 - 2 only order the records (no index is built over such a bundle)
+        const uint64_t pos = e < 0xFFFFFFFEull ? e : 0xFFFFFFFEull;
+        if (!tbl_min(t, key, pos << 32 | rec, max_probes, &added)) atomicExch(&err[DE_OVERFLOW], 1u);
+    });
+    added = warp_sum(added);
+    if (lane_id() == 0 && added) atomicAdd(distinct, (unsigned long long)added);
+}
+
+// ---- the index of the alignment path
+
+__device__ __forceinline__ unsigned long long filter_bits(uint64_t h) { return (1ULL << (h & 63)) | (1ULL << ((h >> 6) & 63)); }
+__device__ __forceinline__ uint64_t filter_word(uint64_t h, uint64_t mask) { return (h >> 32) & mask; }
+
+// foreign[j] bit 31-i: an earlier record owns the k-mer of the window ending
+// at 32j + i; and the filter's bits of every k-mer.
+template <bool CANON>
+__global__ void __launch_bounds__(RT_THREADS) k_r2t_index(const uint64_t *__restrict__ codes,
+                                                         const uint32_t *__restrict__ inv, uint64_t n,
+                                                         const uint64_t *__restrict__ rd_off, uint64_t n_rec, int k,
+                                                         DevTable t, uint32_t *__restrict__ foreign,
+                                                         unsigned long long *__restrict__ filter, uint64_t filter_mask) {
+    const uint64_t w = (uint64_t)blockIdx.x * RT_THREADS + threadIdx.x;
+    uint32_t bits = 0;
+    bundle_windows<CANON>(codes, inv, w, n, rd_off, n_rec, k, [&](uint64_t key, uint64_t e, uint32_t rec) {
+        if (tbl_get2<uint32_t>(t, key, false, PAD_VAL) != rec) bits |= 0x80000000u >> (e & 31);
+        const uint64_t h = mix64(key);
+        atomicOr(&filter[filter_word(h, filter_mask)], filter_bits(h));
+    });
+    if (w * RT_SPAN < n) foreign[w] = bits;
+}
+
+// 32 positions from p on, the first in the top bits (p >= -32)
+__device__ __forceinline__ uint64_t codes_at(const uint64_t *__restrict__ codes, int64_t p) {
+    const int64_t q = p >> 5;
+    const int s = 2 * (int)(p & 31);
+    const uint64_t hi = __ldg(codes + q);
+    return s ? (hi << s) | (__ldg(codes + q + 1) >> (64 - s)) : hi;
+}
+__device__ __forceinline__ uint32_t bits_at(const uint32_t *__restrict__ w, int64_t p) {
+    const int64_t q = p >> 5;
+    return __funnelshift_l(__ldg(w + q + 1), __ldg(w + q), (uint32_t)(p & 31));
+}
+
+struct R2tIndex {
+    const uint64_t *codes;
+    const uint32_t *inv, *foreign;
+    const unsigned long long *filter;
+    uint64_t filter_mask;
+};
+constexpr uint32_t RT_ALIGN_MAX = 128;   // windows of a read the alignment path takes (two 64-bit masks)
+
+// A read's open windows as a bit mask.
+struct WinMask {
+    uint64_t a, b;
+    __device__ __forceinline__ uint32_t first() const { return a ? (uint32_t)__ffsll((long long)a) - 1 : 63u + (uint32_t)__ffsll((long long)b); }
+    // drops windows [lo, hi]; how many of them were open
+    __device__ __forceinline__ uint32_t drop(uint32_t lo, uint32_t hi) {
+        const uint64_t ma = lo < 64 ? (~0ULL << lo) & (~0ULL >> (63 - min(hi, 63u))) : 0ULL;
+        const uint64_t mb = hi >= 64 ? (~0ULL >> (127 - hi)) & (lo > 64 ? ~0ULL << (lo - 64) : ~0ULL) : 0ULL;
+        const uint32_t c = __popcll(a & ma) + __popcll(b & mb);
+        a &= ~ma;
+        b &= ~mb;
+        return c;
+    }
+};
+
+// The windows [0, nwin) of the read at `start` that hold A/C/G/T only.
+__device__ __forceinline__ WinMask read_windows(const uint32_t *__restrict__ inv, uint64_t start, uint32_t nwin, int k) {
+    // invalid positions of the read, position j at bit j of m0, m1, m2
+    uint64_t m0, m1, m2;
+    {
+        const int64_t p = (int64_t)start;
+        m0 = (uint64_t)__brev(bits_at(inv, p));
+        m1 = m2 = 0;
+        const uint32_t L = nwin + (uint32_t)k - 1;   // nothing past the read is asked for
+        if (L > 32) m0 |= (uint64_t)__brev(bits_at(inv, p + 32)) << 32;
+        if (L > 64) m1 = (uint64_t)__brev(bits_at(inv, p + 64));
+        if (L > 96) m1 |= (uint64_t)__brev(bits_at(inv, p + 96)) << 32;
+        if (L > 128) m2 = (uint64_t)__brev(bits_at(inv, p + 128));
+    }
+    uint64_t b0 = 0, b1 = 0;   // window w covers an invalid position
+    int sh = 0;
+#pragma unroll
+    for (int l = 0; l < 5; l++) {
+        if (k & (1 << l)) {
+            b0 |= sh ? (m0 >> sh) | (m1 << (64 - sh)) : m0;
+            b1 |= sh ? (m1 >> sh) | (m2 << (64 - sh)) : m1;
+            sh += 1 << l;
         }
-        uint64_t rec = lo;
-        uint64_t next = rd_off[rec + 1];
-        uint64_t fw = 0, rc = 0;
-        int run = 0;
-        const uint8_t *p = seq + p0 - 32;
-#pragma unroll 4
-        for (int j = 0; j < 64; j++) {
-            uint32_t c = base_code(p[j]);
-            if (c > 3) {
-                run = 0;
-            } else {
-                fw = ((fw << 2) | c) & kmask;
-                rc = (rc >> 2) | ((uint64_t)(3u - c) << shift);
-                run++;
+        const int d = 1 << l;
+        m0 |= (m0 >> d) | (m1 << (64 - d));
+        m1 |= (m1 >> d) | (m2 << (64 - d));
+        m2 |= m2 >> d;
+    }
+    WinMask u;
+    u.a = ~b0 & (nwin >= 64 ? ~0ULL : (1ULL << nwin) - 1);
+    u.b = nwin > 64 ? ~b1 & (~0ULL >> (128 - nwin)) : 0ULL;
+    return u;
+}
+
+// A thread per read (see the head of the file).  3M reads of 100 nt against
+// 13.6M bundle k-mers: 1.44 ms (ALU 90% busy: a lane whose read has errors keeps
+// its warp), and 0.10 for the reads left over; the per-window kernel takes
+// 7.68 ms, bound by its 76 random accesses per read at 38-44 G/s.
+template <bool CANON>
+__global__ void __launch_bounds__(RT_THREADS) k_r2t_align(R2tIndex ix, DevTable t, const uint64_t *__restrict__ codes,
+                                                         const uint32_t *__restrict__ inv,
+                                                         const uint64_t *__restrict__ rd_off, uint64_t n_reads, int k,
+                                                         int32_t *__restrict__ rec, uint32_t *__restrict__ hits,
+                                                         uint32_t *__restrict__ nwin_out, uint32_t *__restrict__ rest,
+                                                         unsigned long long *__restrict__ rest_n) {
+    const uint64_t r = (uint64_t)blockIdx.x * RT_THREADS + threadIdx.x;
+    if (r >= n_reads) return;
+    const uint64_t start = rd_off[r];
+    const uint64_t L = rd_off[r + 1] - start - 1;
+    const uint64_t nw = L >= (uint64_t)k ? L - k + 1 : 0;
+    nwin_out[r] = (uint32_t)nw;
+    if (nw > RT_ALIGN_MAX) {
+        rest[atomicAdd(rest_n, 1ULL)] = (uint32_t)r;
+        return;
+    }
+    const uint32_t nwin = (uint32_t)nw;
+    uint32_t owner = PAD_VAL, votes = 0;
+    if (nwin) {
+        WinMask open = read_windows(inv, start, nwin, k);
+        const uint64_t kmask = (1ULL << (2 * k)) - 1;
+        while (open.a | open.b) {
+            const uint32_t w = open.first();
+            const uint64_t fw = codes_at(codes, (int64_t)(start + w)) >> (64 - 2 * k);
+            uint64_t key = fw;
+            if (CANON) {
+                const uint64_t rc = kmer_revcomp(fw, k);
+                key = rc < fw ? rc : fw;
             }
-            if (j >= 32 && run >= k) {
-                uint64_t e = p0 - 32 + j;
-                while (e >= next && rec + 1 < n_rec) { rec++; next = rd_off[rec + 1]; }
-                uint64_t key = (CANON && rc < fw) ? rc : fw;
-                if (!tbl_min(t, key, (uint32_t)rec, max_probes)) atomicExch(&err[DE_OVERFLOW], 1u);
+            const uint64_t h = mix64(key);
+            const unsigned long long fb = filter_bits(h);
+            uint64_t hit = ~0ULL;
+            if ((__ldg(ix.filter + filter_word(h, ix.filter_mask)) & fb) == fb) hit = tbl_get2<uint64_t>(t, key, true, ~0ULL);
+            if (hit == ~0ULL) {
+                open.drop(w, w);
+                continue;
             }
+            const uint32_t own = (uint32_t)hit;
+            const int64_t e = (int64_t)(hit >> 32), s0 = e - k + 1;   // the bundle's window: positions s0 .. e
+            const bool forward = !CANON || (codes_at(ix.codes, s0) >> (64 - 2 * k) & kmask) == fw;
+            // t further windows: the read's bases after this window against the
+            // bundle's after e, or the complements of those before s0
+            const uint32_t most = nwin - 1 - w;
+            uint32_t ext = 0;
+            while (ext < most) {
+                const uint64_t rw = codes_at(codes, (int64_t)(start + w + k) + ext);
+                uint64_t bw;
+                uint32_t stop;
+                if (forward) {
+                    bw = codes_at(ix.codes, e + 1 + ext);
+                    stop = bits_at(ix.inv, e + 1 + ext) | bits_at(ix.foreign, e + 1 + ext);
+                } else {
+                    bw = kmer_revcomp(codes_at(ix.codes, s0 - 32 - (int64_t)ext), 32);
+                    stop = __brev(bits_at(ix.inv, s0 - 32 - (int64_t)ext) | bits_at(ix.foreign, e - 32 - (int64_t)ext));
+                }
+                const uint64_t x = rw ^ bw;
+                const uint32_t same = min(x ? (uint32_t)__clzll((long long)x) >> 1 : 32u, (uint32_t)__clz((int)stop));
+                ext += same;
+                if (same < 32) break;
+            }
+            ext = min(ext, most);
+            const uint32_t c = open.drop(w, w + ext);
+            if (owner == PAD_VAL) {
+                owner = own;
+            } else if (owner != own) {
+                rest[atomicAdd(rest_n, 1ULL)] = (uint32_t)r;   // more than one record: votes are counted per window
+                return;
+            }
+            votes += c;
         }
     }
+    rec[r] = votes ? (int32_t)owner : -1;
+    hits[r] = votes;
 }
 
 template <int S, bool CANON>
@@ -70,7 +265,7 @@ __device__ __forceinline__ void r2t_warp_read(DevTable t, const uint8_t *__restr
     const unsigned lane = lane_id();
     const uint32_t span = (nwin + 31) / 32;
     uint32_t v[S];
-    auto body = [&](int j, bool valid, uint64_t key) { v[j] = valid ? tbl_get(t, key, PAD_VAL) : PAD_VAL; };
+    auto body = [&](int j, bool valid, uint64_t key) { v[j] = valid ? tbl_get2<uint32_t>(t, key, false, PAD_VAL) : PAD_VAL; };
     // k-mers cut from the read packed in shared memory; reads with another
     // character take the byte path
     if (!lane_windows_packed<S, CANON>(seq, start, nwin, span, k, words, body))
@@ -123,12 +318,14 @@ __global__ void __launch_bounds__(RT_THREADS, 6) k_r2t_assign(DevTable t, const 
                                                              const uint64_t *__restrict__ rd_off, uint64_t n_reads,
                                                              int k, int32_t *__restrict__ rec,
                                                              uint32_t *__restrict__ hits, uint32_t *__restrict__ nwin_out,
+                                                             const uint32_t *__restrict__ list,
                                                              uint32_t *__restrict__ long_list,
                                                              unsigned long long *__restrict__ long_n) {
     __shared__ uint64_t words[RT_THREADS / 32][12];
     uint64_t *w = words[threadIdx.x >> 5];
     const uint64_t warps = (uint64_t)gridDim.x * (RT_THREADS / 32);
-    for (uint64_t r = (uint64_t)blockIdx.x * (RT_THREADS / 32) + (threadIdx.x >> 5); r < n_reads; r += warps) {
+    for (uint64_t i = (uint64_t)blockIdx.x * (RT_THREADS / 32) + (threadIdx.x >> 5); i < n_reads; i += warps) {
+        const uint64_t r = list ? list[i] : i;   // n_reads = the list's length, with a list
         const uint64_t start = rd_off[r];
         const uint64_t L = rd_off[r + 1] - start - 1;
         const uint32_t nwin = L >= (uint64_t)k ? (uint32_t)(L - k + 1) : 0u;
@@ -154,7 +351,7 @@ __global__ void __launch_bounds__(RT_THREADS) k_r2t_long(DevTable t, const uint8
         const uint32_t nwin = (uint32_t)(rd_off[r + 1] - start - 1 - (k - 1));
         uint32_t n2 = 1;
         while (n2 < nwin) n2 <<= 1;
-        block_window_values<CANON>(seq, start, nwin, n2, k, slab, [&](uint64_t key) { return tbl_get(t, key, PAD_VAL); });
+        block_window_values<CANON>(seq, start, nwin, n2, k, slab, [&](uint64_t key) { return tbl_get2<uint32_t>(t, key, false, PAD_VAL); });
         block_bitonic_sort(slab, n2);
         if (threadIdx.x == 0) {
             uint32_t best_len = 0, best_v = PAD_VAL;
@@ -171,33 +368,101 @@ __global__ void __launch_bounds__(RT_THREADS) k_r2t_long(DevTable t, const uint8
     }
 }
 
-int r2t_build(tk_r2t *z, const tk_reads *b) {
+int r2t_build(tk_r2t *z, tk_reads *b) {
     tk_ctx *c = z->ctx;
     tk_table *t = z->table;
     uint64_t want = 1024;
     while (want < 2 * std::max<uint64_t>(b->n_bases, 1)) want <<= 1;
-    TK_TRY(table_alloc_init(t, want, PAD_VAL));
+    TK_TRY(table_alloc_init(t, want, ~0ULL));
+    t->distinct = 0;
+    t->distinct_valid = true;
     if (b->n_reads == 0 || b->seq_len == 0) return TK_OK;
     TK_CUDA(c, cudaMemsetAsync(c->d_err, 0, DE_COUNT * 4, c->stream));
-    const uint64_t n = b->seq_len;
-    const unsigned grid = (unsigned)std::max<uint64_t>(
-        1, std::min<uint64_t>((n + RT_THREADS * RT_SPAN - 1) / (RT_THREADS * RT_SPAN), (uint64_t)c->sm_count * 16));
+    TK_CUDA(c, cudaMemsetAsync(t->d_counters, 0, 8, c->stream));
+    const uint64_t n = b->seq_len, per_block = (uint64_t)RT_THREADS * RT_SPAN;
+    const unsigned grid = (unsigned)((n + per_block - 1) / per_block);
     cudaEvent_t ev;
     prof_begin(c, TK_KID_R2T_BUILD, &ev);
     if (!z->strand)
-        k_r2t_build<true><<<grid, RT_THREADS, 0, c->stream>>>(b->d_seq, n, b->d_rd_off, b->n_reads, z->k, t->t,
-                                                              c->max_probes, c->d_err);
+        k_r2t_build<true><<<grid, RT_THREADS, 0, c->stream>>>(b->d_codes, b->d_inv, n, b->d_rd_off, b->n_reads, z->k, t->t,
+                                                              c->max_probes, c->d_err, t->d_counters);
     else
-        k_r2t_build<false><<<grid, RT_THREADS, 0, c->stream>>>(b->d_seq, n, b->d_rd_off, b->n_reads, z->k, t->t,
-                                                               c->max_probes, c->d_err);
+        k_r2t_build<false><<<grid, RT_THREADS, 0, c->stream>>>(b->d_codes, b->d_inv, n, b->d_rd_off, b->n_reads, z->k, t->t,
+                                                               c->max_probes, c->d_err, t->d_counters);
     c->launches++;
     prof_end(c, TK_KID_R2T_BUILD, ev, b->n_bases);
     TK_TRY(check_launch(c, "r2t build"));
     uint32_t herr[DE_COUNT];
+    unsigned long long distinct = 0;
     TK_CUDA(c, cudaMemcpyAsync(herr, c->d_err, sizeof(herr), cudaMemcpyDeviceToHost, c->stream));
+    TK_CUDA(c, cudaMemcpyAsync(&distinct, t->d_counters, 8, cudaMemcpyDeviceToHost, c->stream));
     TK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (herr[DE_OVERFLOW]) return set_err(c, TK_E_TABLE_FULL, "bundle k-mer table: probe limit reached");
-    t->distinct_valid = false;
+    t->distinct = distinct;
+    // the bundle's 2-bit form stays for the alignment path
+    z->seq_len = b->seq_len;
+    z->n_bases = b->n_bases;
+    z->n_records = b->n_reads;
+    z->d_pack_alloc = b->d_pack_alloc;
+    z->d_codes = b->d_codes;
+    z->d_inv = b->d_inv;
+    z->d_rd_off = b->d_rd_off;
+    b->d_pack_alloc = nullptr;
+    b->d_codes = nullptr;
+    b->d_inv = nullptr;
+    b->d_rd_off = nullptr;
+    return TK_OK;
+}
+
+void r2t_release(tk_r2t *z) {
+    void *p[] = {z->d_pack_alloc, z->d_rd_off, z->d_foreign, z->d_filter};
+    for (void *q : p)
+        if (q) dfree(z->ctx, q);
+}
+
+// The bits and the filter of the alignment path; *ready false when they cannot
+// be held (the per-window path then serves).
+static int r2t_index(tk_r2t *z, bool *ready) {
+    tk_ctx *c = z->ctx;
+    *ready = z->d_foreign != nullptr;
+    if (*ready || !z->d_codes || z->seq_len >= 0xFFFFFFFEull) return TK_OK;
+    uint64_t words = 1024;   // a word per 12 bundle bases or fewer
+    while (words * 12 < z->n_bases) words <<= 1;
+    const uint64_t n_words = (z->seq_len + 31) / 32 + 2;   // word -1 and one past the last, like inv
+    uint32_t *foreign = nullptr;
+    unsigned long long *filter = nullptr;
+    int e = dmalloc(c, (void **)&foreign, (n_words + 1) * 4, "bundle ownership bits");
+    if (!e) e = dmalloc(c, (void **)&filter, words * 8, "bundle k-mer filter");
+    if (e) {
+        if (foreign) dfree(c, foreign);
+        return TK_OK;
+    }
+    e = cuda_check(c, cudaMemsetAsync(foreign, 0, (n_words + 1) * 4, c->stream), "ownership bits reset");
+    if (!e) e = cuda_check(c, cudaMemsetAsync(filter, 0, words * 8, c->stream), "filter reset");
+    if (!e) {
+        const uint64_t per_block = (uint64_t)RT_THREADS * RT_SPAN;
+        const unsigned grid = (unsigned)((z->seq_len + per_block - 1) / per_block);
+        cudaEvent_t ev;
+        prof_begin(c, TK_KID_R2T_BUILD, &ev);
+        if (!z->strand)
+            k_r2t_index<true><<<grid, RT_THREADS, 0, c->stream>>>(z->d_codes, z->d_inv, z->seq_len, z->d_rd_off, z->n_records,
+                                                                  z->k, z->table->t, foreign + 1, filter, words - 1);
+        else
+            k_r2t_index<false><<<grid, RT_THREADS, 0, c->stream>>>(z->d_codes, z->d_inv, z->seq_len, z->d_rd_off, z->n_records,
+                                                                   z->k, z->table->t, foreign + 1, filter, words - 1);
+        c->launches++;
+        prof_end(c, TK_KID_R2T_BUILD, ev, z->n_bases);
+        e = check_launch(c, "r2t index");
+    }
+    if (e) {
+        dfree(c, foreign);
+        dfree(c, filter);
+        return e;
+    }
+    z->d_foreign = foreign;
+    z->d_filter = filter;
+    z->filter_mask = words - 1;
+    *ready = true;
     return TK_OK;
 }
 
@@ -213,19 +478,51 @@ int r2t_assign(tk_r2t *z, const tk_reads *rd, int32_t *d_rec, uint32_t *d_hits, 
     int e = TK_OK;
     if (may_long) e = dmalloc(c, (void **)&long_list, n * 4, "long-read list");
     if (!e) e = cuda_check(c, cudaMemsetAsync(long_n, 0, 8, c->stream), "long reset");
-    if (!e) {
-        const unsigned grid = (unsigned)std::max<uint64_t>(
-            1, std::min<uint64_t>((n + RT_THREADS / 32 - 1) / (RT_THREADS / 32), (uint64_t)c->sm_count * 16));
+    // The alignment path, for reads of at most 128 windows on average: from as
+    // many read bases as the bundle has on, building its index costs less than
+    // it saves (0.29 ms for 13.6M bundle bases against 7.7 -> 1.5 ms for 228M
+    // windows); once built, every such read set takes it.
+    bool align = rd->n_bases <= n * (uint64_t)(RT_ALIGN_MAX + k - 1);
+    uint32_t *rest = nullptr;
+    uint64_t n_rest = n;
+    if (!e && align) {
+        align = z->d_foreign != nullptr;
+        if (!align && rd->n_bases >= z->n_bases) e = r2t_index(z, &align);
+        if (!e && align && dmalloc(c, (void **)&rest, n * 4, "reads left to the per-window vote")) align = false;
+    }
+    if (!e && align) {
+        const R2tIndex ix{z->d_codes, z->d_inv, z->d_foreign + 1, z->d_filter, z->filter_mask};
+        const unsigned grid = (unsigned)((n + RT_THREADS - 1) / RT_THREADS);
         cudaEvent_t ev;
         prof_begin(c, TK_KID_R2T_ASSIGN, &ev);
         if (!z->strand)
-            k_r2t_assign<true><<<grid, RT_THREADS, 0, c->stream>>>(z->table->t, rd->d_seq, rd->d_rd_off, n, k, d_rec,
-                                                                   d_hits, d_nwin, long_list, long_n);
+            k_r2t_align<true><<<grid, RT_THREADS, 0, c->stream>>>(ix, z->table->t, rd->d_codes, rd->d_inv, rd->d_rd_off, n, k,
+                                                                  d_rec, d_hits, d_nwin, rest, long_n);
         else
-            k_r2t_assign<false><<<grid, RT_THREADS, 0, c->stream>>>(z->table->t, rd->d_seq, rd->d_rd_off, n, k, d_rec,
-                                                                    d_hits, d_nwin, long_list, long_n);
+            k_r2t_align<false><<<grid, RT_THREADS, 0, c->stream>>>(ix, z->table->t, rd->d_codes, rd->d_inv, rd->d_rd_off, n, k,
+                                                                   d_rec, d_hits, d_nwin, rest, long_n);
         c->launches++;
         prof_end(c, TK_KID_R2T_ASSIGN, ev, rd->n_bases);
+        e = check_launch(c, "r2t align");
+        unsigned long long hr = 0;
+        if (!e) e = cuda_check(c, cudaMemcpyAsync(&hr, long_n, 8, cudaMemcpyDeviceToHost, c->stream), "rest n");
+        if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "rest sync");
+        if (!e) e = cuda_check(c, cudaMemsetAsync(long_n, 0, 8, c->stream), "long reset");
+        n_rest = hr;
+    }
+    if (!e && n_rest) {
+        const unsigned grid = (unsigned)std::max<uint64_t>(
+            1, std::min<uint64_t>((n_rest + RT_THREADS / 32 - 1) / (RT_THREADS / 32), (uint64_t)c->sm_count * 16));
+        cudaEvent_t ev;
+        prof_begin(c, TK_KID_R2T_ASSIGN, &ev);
+        if (!z->strand)
+            k_r2t_assign<true><<<grid, RT_THREADS, 0, c->stream>>>(z->table->t, rd->d_seq, rd->d_rd_off, n_rest, k, d_rec,
+                                                                   d_hits, d_nwin, rest, long_list, long_n);
+        else
+            k_r2t_assign<false><<<grid, RT_THREADS, 0, c->stream>>>(z->table->t, rd->d_seq, rd->d_rd_off, n_rest, k, d_rec,
+                                                                    d_hits, d_nwin, rest, long_list, long_n);
+        c->launches++;
+        prof_end(c, TK_KID_R2T_ASSIGN, ev, align ? 0 : rd->n_bases);
         e = check_launch(c, "r2t assign");
     }
     unsigned long long hl = 0;
@@ -253,6 +550,7 @@ int r2t_assign(tk_r2t *z, const tk_reads *rd, int32_t *d_rec, uint32_t *d_hits, 
             dfree(c, scratch);
         }
     }
+    if (rest) dfree(c, rest);
     if (long_list) dfree(c, long_list);
     dfree(c, long_n);
     return e;

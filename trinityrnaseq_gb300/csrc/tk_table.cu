@@ -14,7 +14,7 @@
 // the leader adds the multiplicity with one atomic.  A key that finds no slot
 // within max_probes goes to an overflow list; the host then doubles the table
 // and re-inserts it, so no k-mer is ever dropped silently.
-#include "tk_internal.cuh"
+#include "tk_windows.cuh"
 
 #include <algorithm>
 #include <cmath>
@@ -38,57 +38,6 @@ static_assert((NBUCKETS / (SC_THREADS / 32)) % 2 == 0, "buckets are flushed in p
 constexpr size_t SC_SMEM = (size_t)NBUCKETS * SC_BUF * 8 + (size_t)NBUCKETS * 8 + (size_t)NBUCKETS * 4;
 constexpr uint64_t INS_CHUNK = (uint64_t)CT_THREADS * INS_PER_THREAD;
 enum NextMode { NEXT_NONE = 0, NEXT_FILL = 1, NEXT_PREFETCH = 2 };
-
-// Windows of the 2-bit code form of a packed read array.  A thread owns the
-// 32 window end positions [32w, 32w + 32); the 64 positions [32w - 32, 32w + 32)
-// (code words w-1 and w, invalid bits likewise) hold every base those windows
-// use (k <= 31).  Each window is cut out of the 128-bit code pair with one
-// funnel shift, its reverse complement out of the pair's reverse complement,
-// and it is valid when none of its k positions has its invalid bit set.
-// Calls f(key) for every valid window, in position order.
-template <bool CANON, typename F>
-__device__ __forceinline__ void thread_windows(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv,
-                                               uint64_t w, bool active, int k, F &&f) {
-    uint64_t hi = 0, lo = 0, m = ~0ULL;
-    if (active) {
-        hi = __ldg(codes + w - 1);
-        lo = __ldg(codes + w);
-        m = ((uint64_t)__ldg(inv + w - 1) << 32) | __ldg(inv + w);
-    }
-    // bit b of `bad`: some position among bits b .. b+k-1 of m (position
-    // 32w - 32 + x sits at bit 63 - x) is not A/C/G/T
-    uint64_t bad = 0, span = m;
-    int sh = 0;
-#pragma unroll
-    for (int l = 0; l < 5; l++) {
-        if (k & (1 << l)) {
-            bad |= span >> sh;
-            sh += 1 << l;
-        }
-        span |= span >> (1 << l);
-    }
-    // reverse complement of the 64 positions: complement, then reverse the
-    // order of the 2-bit groups
-    uint64_t rhi = __brevll(~lo), rlo = __brevll(~hi);
-    rhi = ((rhi >> 1) & 0x5555555555555555ULL) | ((rhi & 0x5555555555555555ULL) << 1);
-    rlo = ((rlo >> 1) & 0x5555555555555555ULL) | ((rlo & 0x5555555555555555ULL) << 1);
-    const uint64_t kmask = (1ULL << (2 * k)) - 1;
-#pragma unroll
-    for (int i = 0; i < 32; i++) {
-        if ((bad >> (31 - i)) & 1ULL) continue;
-        // forward: the window ends at position 32 + i of the 64
-        const int s = 62 - 2 * i;
-        const uint64_t fw = (s ? ((lo >> s) | (hi << (64 - s))) : lo) & kmask;
-        uint64_t key = fw;
-        if (CANON) {
-            // reverse complement: it ends where the window starts, 33 + i - k
-            const int r = 66 + 2 * i - 2 * k;   // 4 .. 126
-            const uint64_t rc = (r >= 64 ? (rhi >> (r - 64)) : ((rlo >> r) | (rhi << (64 - r)))) & kmask;
-            key = rc < fw ? rc : fw;
-        }
-        f(key);
-    }
-}
 
 // Pass 1a: k-mers per (hash bucket, column) and the HLL sketch of the batch.
 // hist is bucket-major with `cols` columns per bucket; the read set uses the
@@ -119,7 +68,7 @@ __global__ void __launch_bounds__(HIST_THREADS) k_part_hist(const uint64_t *__re
     for (uint64_t base = ((uint64_t)blockIdx.x + (uint64_t)half * gridDim.x) * tile; base < n;
          base += 2ull * gridDim.x * tile) {
         const uint64_t p0 = base + (uint64_t)t * CT_SPAN;
-        thread_windows<CANON>(codes, inv, p0 >> 5, p0 < n, k, [&](uint64_t key) {
+        thread_windows<CANON>(codes, inv, p0 >> 5, p0 < n, k, [&](uint64_t key, int) {
             uint64_t h = mix64(key);
             atomicAdd(&sh[h >> (64 - BUCKET_BITS)], 1u);
             uint32_t idx = (uint32_t)(h & (HLL_M - 1));
@@ -165,7 +114,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_part_scatter(const uint64_t *
     const uint64_t stride = (uint64_t)gridDim.x * SC_THREADS * CT_SPAN;
     for (uint64_t base = (uint64_t)blockIdx.x * SC_THREADS * CT_SPAN; base < n; base += stride) {
         const uint64_t p0 = base + (uint64_t)threadIdx.x * CT_SPAN;
-        thread_windows<CANON>(codes, inv, p0 >> 5, p0 < n, k, [&](uint64_t key) {
+        thread_windows<CANON>(codes, inv, p0 >> 5, p0 < n, k, [&](uint64_t key, int) {
             const uint32_t b = (uint32_t)(mix64(key) >> (64 - BUCKET_BITS));
             const uint32_t r = atomicAdd(&cnt[b], 1u);
             if (r < SC_BUF) buf[b * SC_BUF + r] = key;
@@ -639,7 +588,7 @@ __global__ void k_insert_pairs(const uint64_t *__restrict__ keys, const uint32_t
     }
 }
 
-__global__ void k_fill_empty(Slot *slots, uint64_t cap, uint32_t init_val) {
+__global__ void k_fill_empty(Slot *slots, uint64_t cap, uint64_t init_val) {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (uint64_t)gridDim.x * blockDim.x) {
         ulonglong2 v;
         v.x = EMPTY_KEY;
@@ -821,7 +770,7 @@ static unsigned stream_grid(tk_ctx *c, uint64_t n, int threads) {
 
 // fill = false leaves the slots unwritten: the partitioned count pass fills
 // each slice right before its inserts (a "fresh" table)
-static int table_alloc_geom(tk_table *t, uint64_t capacity, uint32_t init_val, bool fill) {
+static int table_alloc_geom(tk_table *t, uint64_t capacity, uint64_t init_val, bool fill) {
     tk_ctx *c = t->ctx;
     Slot *s = nullptr;
     TK_TRY(dmalloc(c, (void **)&s, capacity * sizeof(Slot), "k-mer table"));
@@ -842,7 +791,7 @@ static int table_alloc_geom(tk_table *t, uint64_t capacity, uint32_t init_val, b
     return check_launch(c, "table fill");
 }
 
-int table_alloc_init(tk_table *t, uint64_t capacity, uint32_t init_val) {
+int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val) {
     return table_alloc_geom(t, capacity, init_val, true);
 }
 
