@@ -12,7 +12,7 @@
 // and all before it) and, in the sort, bits 58-61 the pass it belongs to.
 // Every wait is bounded: past WAIT_POLLS polls the block sets the error word
 // and returns without storing, and the host reports it (wait_status).
-#include "tk_internal.cuh"
+#include "tk_emit.cuh"
 
 #include <algorithm>
 
@@ -47,14 +47,23 @@ __device__ __forceinline__ void load4(const uint64_t *in, uint64_t (&x)[4]) {
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
+// what the scan adds up for an input item
+struct ItemItself {
+    __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return x; }
+};
+struct RecordLength {   // ">COUNT\nKMER\n"
+    int k;
+    __device__ __forceinline__ uint64_t operator()(uint64_t count) const { return 3u + dec_digits((uint32_t)count) + (uint32_t)k; }
+};
+
 // A warp owns 512 consecutive items, four rounds of four per lane (16-byte
 // loads and stores of consecutive lanes adjoin).  Bound by memory: 12 bytes
 // an item for u32 input.  The three-kernel scan this replaces (reduce, one
 // block over the tile sums, and a pass whose threads each walked 16
 // consecutive items) took 10.5 us of kernels for 12,000 items and 45 us for 17M,
 // and read its input twice.
-template <typename Tin>
-__global__ void __launch_bounds__(SN_THREADS) k_scan(const Tin *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
+template <typename Tin, typename F>
+__global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
                                                     int vec, ScanHead *__restrict__ head, uint64_t *__restrict__ state) {
     __shared__ uint64_t s_warp[SN_WARPS], s_before;
     __shared__ uint32_t s_tile, s_fail;
@@ -76,6 +85,9 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(const Tin *__restrict__ in,
 #pragma unroll
             for (int j = 0; j < 4; j++) x[r][j] = i + j < n ? (uint64_t)in[i + j] : 0;
         }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+            if (i + j < n) x[r][j] = f(x[r][j]);
     }
 #pragma unroll
     for (int r = 0; r < SN_ROUNDS; r++) {
@@ -153,8 +165,8 @@ int wait_status(tk_ctx *c) {
     return set_err(c, TK_E_CUDA, "radix sort: the wait for an earlier tile ran out");
 }
 
-template <typename Tin>
-static int scan_impl(tk_ctx *c, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
+template <typename Tin, typename F>
+static int scan_impl(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
     *total_host = 0;
     if (n == 0) return TK_OK;
     const uint64_t nt = (n + SN_TILE - 1) / SN_TILE;
@@ -165,7 +177,7 @@ static int scan_impl(tk_ctx *c, const Tin *in, uint64_t *out, uint64_t n, uint64
     int e = cuda_check(c, cudaMemsetAsync(mem, 0, bytes, c->stream), "scan reset");
     if (!e) {
         const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
-        k_scan<Tin><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(in, out, n, vec, head,
+        k_scan<Tin, F><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, head,
                                                                reinterpret_cast<uint64_t *>(mem + sizeof(ScanHead)));
         c->launches++;
         e = check_launch(c, "scan");
@@ -181,11 +193,16 @@ static int scan_impl(tk_ctx *c, const Tin *in, uint64_t *out, uint64_t n, uint64
 }
 
 int scan_excl_u64(tk_ctx *c, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
-    return scan_impl<uint64_t>(c, in, out, n, total_host);
+    return scan_impl<uint64_t>(c, ItemItself{}, in, out, n, total_host);
 }
 
 int scan_excl_u32_to_u64(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
-    return scan_impl<uint32_t>(c, in, out, n, total_host);
+    return scan_impl<uint32_t>(c, ItemItself{}, in, out, n, total_host);
+}
+
+// Offsets of the dump records of n counts (k-mers of k bases).
+int scan_record_lengths(tk_ctx *c, const uint32_t *counts, uint64_t *out, uint64_t n, int k, uint64_t *total_host) {
+    return scan_impl<uint32_t>(c, RecordLength{k}, counts, out, n, total_host);
 }
 
 // ------------------------------------------------------------------ radix sort
