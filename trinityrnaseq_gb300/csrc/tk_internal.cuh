@@ -129,6 +129,25 @@ __device__ __forceinline__ ulonglong2 slot_claim(Slot *slot, uint64_t empty, uin
     return r;
 }
 
+// tbl_add for keys that are mostly new to the table: claims the slot with its
+// count in one CAS.  *added counts the keys inserted.
+__device__ __forceinline__ bool tbl_add_new(DevTable t, uint64_t key, uint32_t inc, int max_probes, uint32_t *added) {
+    uint64_t s = tbl_home(t, mix64(key));
+    for (int i = 0; i < max_probes; i++) {
+        const ulonglong2 was = slot_claim(&t.slots[s], 0, key, inc);
+        if (was.x == EMPTY_KEY) {
+            *added += 1;
+            return true;
+        }
+        if (was.x == key) {
+            atomicAdd(&t.slots[s].val, inc);
+            return true;
+        }
+        s = tbl_next(t, s);
+    }
+    return false;
+}
+
 // Keeps the minimum 64-bit value per key, in the slot's val (low half) and pad
 // (ReadsToTranscripts: the record in the low half, a position in the high
 // one; empty slots hold ~0).  *added counts the keys inserted.

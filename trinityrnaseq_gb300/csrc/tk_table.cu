@@ -235,31 +235,35 @@ __global__ void __launch_bounds__(CT_THREADS) k_part_step(const uint64_t *__rest
     }
 }
 
-// ---- pass 2 by ranges (slices of at least 2^SR_MIN_LBITS slots).  Per
-// partition p the keys are regrouped by the range of the slice their home slot
-// falls in (a slice is cut into SR_BUILD_PER_SM ranges per SM, so that the
-// build runs as one wave; k_sr_hist, k_sr_scatter), and one block per range then
-// builds that range in shared memory (k_sr_build): it loads the range (all
-// empty on a fresh table), inserts the range's keys with shared-memory CAS
-// and add, and writes the range back whole.  A key whose probe run reaches the
-// end of its range (its chain goes on into the next range, which another block
-// owns) is merged into a small per-block table and then appended with its
-// multiplicity to a deferred list that is inserted into the global table once
-// every range is written; the global probe order (home, home+1, ... wrapping
-// in the slice) is the one every reader uses, so the layout is an ordinary
-// linear-probing table.  Global atomics drop from two per occurrence to the
-// deferred keys alone, and a fresh slice needs no separate fill.
+// ---- pass 2 by ranges (slices of at least 2^SR_MIN_LBITS slots), a batch of
+// partitions at a time.  k_sr_group cuts each partition's keys into chunks and
+// sorts every chunk by the range of the slice its keys' home slots fall in (a
+// slice is cut into SR_BUILD_PER_SM ranges per SM); a chunk needs nothing from
+// the others, so the keys are read once and no totals are known beforehand.
+// k_sr_build then takes a block per range: it gathers the range's run of every
+// chunk, builds the range in shared memory (all empty at first) with
+// shared-memory CAS and add, and writes the range back whole.  A key whose
+// probe run reaches the end of its range (its chain goes on into the next
+// range, which another block owns) is merged into a small per-block table and
+// then appended with its multiplicity to a deferred list that is inserted into
+// the global table once every range is written; the global probe order (home,
+// home+1, ... wrapping in the slice) is the one every reader uses, so the
+// layout is an ordinary linear-probing table.  Global atomics drop from two
+// per occurrence to the deferred keys alone, and a fresh slice needs no
+// separate fill.
+//
+// A batch holds about SR_BATCH_KEYS keys: enough blocks per launch that one
+// block's loads, inserts and writes overlap another's, few enough that the
+// grouped keys are still in L2 when the build reads them.
 constexpr int SR_MIN_LBITS = 12;        // slices below 4096 slots keep the atomic path
-// Two build blocks of 1024 threads per SM (32 registers, 110 KB of shared
-// memory each) with ranges of up to 9200 slots: half the ranges per slice of
-// four 512-thread blocks with 4600, so the regrouping passes' per-range work
-// (counts, cursor atomics, runs) halves; 58.1 -> 50.9 ms per step at 20M pairs.
-constexpr int SR_BUILD_PER_SM = 2;      // build blocks resident per SM: the slice is cut into one wave of ranges
-constexpr int SR_MAX_SLOTS = 9200;      // slots of one range in shared memory (12 bytes each)
-constexpr int SR_THREADS = 1024;        // regrouping passes (2 blocks per SM: few per-block range counts)
+constexpr int SR_BUILD_PER_SM = 2;      // ranges per slice and SM
+constexpr int SR_MAX_SLOTS = 7168;      // slots of one range in shared memory (12 bytes each)
 constexpr int SR_BUILD_THREADS = 1024;
 constexpr int SR_MINI = 64;
-constexpr size_t SR_SMEM = (size_t)(SR_MAX_SLOTS + SR_MINI) * 12;
+constexpr int SG_THREADS = 512;
+constexpr int SG_KEYS = 12;             // keys per thread, in registers
+constexpr uint32_t SG_CHUNK = SG_THREADS * SG_KEYS;
+constexpr uint64_t SR_BATCH_KEYS = 6ull << 20;
 
 // A slice of 2^lbits slots is cut into nsub ranges: slot s belongs to range
 // floor(s * nsub / 2^lbits), so range r is [ceil(r 2^lbits / nsub),
@@ -332,124 +336,71 @@ __device__ __forceinline__ uint32_t seg_of(const SegView &v, uint64_t i) {
     return s;
 }
 
-// The partition's keys split evenly over the blocks.  Per block, keys per
-// range (counts[range * gridDim.x + block]) and, summed over blocks after
-// rounding each up to a multiple of 4, per range (totals, zeroed beforehand).
-__global__ void __launch_bounds__(SR_THREADS) k_sr_hist(const KeySeg *__restrict__ segs, uint32_t nseg,
-                                                       DevTable t, uint32_t nsub, uint32_t *__restrict__ counts,
-                                                       uint32_t *__restrict__ totals) {
-    extern __shared__ uint32_t sr_h[];
+// A partition's chunks in its batch's buffers.
+struct PartGeom {
+    uint32_t chunk0, chunks;
+};
+
+// Chunk blockIdx.x of the batch, sorted by range into out[blockIdx.x *
+// SG_CHUNK ...]; starts[blockIdx.x * (nsub + 1) + r] = where range r's run
+// begins (entry nsub: the chunk's keys without the EMPTY_KEY padding).
+__global__ void __launch_bounds__(SG_THREADS, 2) k_sr_group(const KeySeg *__restrict__ segs, uint32_t nseg,
+                                                           const PartGeom *__restrict__ parts, uint32_t n_parts,
+                                                           DevTable t, uint32_t nsub, uint64_t *__restrict__ out,
+                                                           uint16_t *__restrict__ starts) {
+    extern __shared__ __align__(16) unsigned char sg_smem[];
+    uint64_t *skeys = reinterpret_cast<uint64_t *>(sg_smem);               // [SG_CHUNK]
+    uint32_t *cnt = reinterpret_cast<uint32_t *>(skeys + SG_CHUNK);        // [nsub]
+    __shared__ uint32_t sm[SG_THREADS / 32 + 1];
     __shared__ SegView sv;
-    for (uint32_t i = threadIdx.x; i < nsub; i += SR_THREADS) sr_h[i] = 0;
-    seg_view_load(sv, segs, nseg);   // synchronises
-    const uint64_t n = sv.cum[sv.n];
-    const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const uint64_t lo = (uint64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
+    uint32_t lo = 0, hi = n_parts;   // the chunk's partition (partitions without chunks share a first one)
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (parts[mid].chunk0 <= blockIdx.x) lo = mid; else hi = mid;
+    }
+    for (uint32_t r = threadIdx.x; r < nsub; r += SG_THREADS) cnt[r] = 0;
+    seg_view_load(sv, segs + (uint64_t)lo * nseg, nseg);   // synchronises
+    const uint64_t n = sv.cum[sv.n], c0 = (uint64_t)(blockIdx.x - parts[lo].chunk0) * SG_CHUNK;
     SegCursor cur;
-    seg_cursor_at(sv, cur, seg_of(sv, lo));
-    for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += 4 * SR_THREADS) {
-        uint64_t k4[4];
+    seg_cursor_at(sv, cur, seg_of(sv, c0));
+    uint64_t key[SG_KEYS];
+    uint32_t at[SG_KEYS];   // (range << 16) | rank in the chunk's run of it
 #pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint64_t i = i0 + (uint64_t)u * SR_THREADS;   // ascending over u and over the loop
-            k4[u] = i < hi ? seg_key(sv, cur, i) : EMPTY_KEY;
-        }
+    for (int u = 0; u < SG_KEYS; u++) {
+        const uint64_t i = c0 + (uint64_t)u * SG_THREADS + threadIdx.x;   // ascending over u
+        key[u] = i < n ? seg_key(sv, cur, i) : EMPTY_KEY;
+    }
 #pragma unroll
-        for (int u = 0; u < 4; u++)
-            if (k4[u] != EMPTY_KEY) atomicAdd(&sr_h[key_range(t, k4[u], nsub)], 1u);
-    }
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nsub; i += SR_THREADS) {
-        counts[(uint64_t)i * gridDim.x + blockIdx.x] = sr_h[i];
-        if (sr_h[i]) atomicAdd(&totals[i], (sr_h[i] + 3u) & ~3u);   // each block's run padded to whole sectors
-    }
-}
-
-// exclusive prefix of totals[0..nsub) into out[0..nsub) (block-wide scan;
-// thread t sums a run of consecutive ranges)
-__device__ __forceinline__ void range_starts(const uint32_t *__restrict__ totals, uint32_t nsub, uint64_t *out) {
-    __shared__ uint64_t sm[SR_THREADS / 32 + 1];
-    const uint32_t per = (nsub + SR_THREADS - 1) / SR_THREADS;
-    const uint32_t lo = min(nsub, threadIdx.x * per), hi = min(nsub, lo + per);
-    uint64_t sum = 0;
-    for (uint32_t j = lo; j < hi; j++) sum += totals[j];
-    uint64_t tot;
-    uint64_t run = block_excl_scan<uint64_t>(sum, sm, &tot);
-    for (uint32_t j = lo; j < hi; j++) {
-        out[j] = run;
-        run += totals[j];
-    }
-    __syncthreads();
-}
-
-// The same keys into range order.  Each block reserves its share of every
-// range (rounded up to whole 32-byte sectors) with one atomic on the range's
-// cursor, counting-sorts its chunk by range in shared memory, and writes each
-// range's run as whole sectors, the rounding filled with EMPTY_KEY (the build
-// skips it).  Scattered single-key stores instead cost one L2 request per key.
-constexpr int SRS_MAX = 12288;   // keys of one block's chunk (the host sizes the grid to fit)
-static inline size_t SRS_SMEM(uint32_t nsub) { return (size_t)SRS_MAX * 8 + (size_t)nsub * 16; }
-
-__global__ void __launch_bounds__(SR_THREADS) k_sr_scatter(const KeySeg *__restrict__ segs, uint32_t nseg,
-                                                          DevTable t, uint32_t nsub, const uint32_t *__restrict__ counts,
-                                                          const uint32_t *__restrict__ totals,
-                                                          unsigned long long *__restrict__ cursor,
-                                                          uint64_t *__restrict__ range_keys) {
-    extern __shared__ __align__(16) unsigned char srs_smem[];
-    uint64_t *skeys = reinterpret_cast<uint64_t *>(srs_smem);                          // [SRS_MAX]
-    unsigned long long *gbase = reinterpret_cast<unsigned long long *>(skeys + SRS_MAX);  // [nsub]
-    uint32_t *lstart = reinterpret_cast<uint32_t *>(gbase + nsub);                      // [nsub]
-    uint32_t *lcur = lstart + nsub;                                                      // [nsub]
-    __shared__ uint32_t sm[SR_THREADS / 32 + 1];
-    __shared__ SegView sv;
-    seg_view_load(sv, segs, nseg);   // synchronises
-    range_starts(totals, nsub, reinterpret_cast<uint64_t *>(gbase));
-    // this block's run of every range, and where its keys sit in shared memory
-    const uint32_t per = (nsub + SR_THREADS - 1) / SR_THREADS;
-    const uint32_t lo_r = min(nsub, threadIdx.x * per), hi_r = min(nsub, lo_r + per);
-    uint32_t sum = 0;
-    for (uint32_t r = lo_r; r < hi_r; r++) {
-        const uint32_t mine = counts[(uint64_t)r * gridDim.x + blockIdx.x];
-        if (mine) gbase[r] += atomicAdd(&cursor[r], (unsigned long long)((mine + 3u) & ~3u));
-        lcur[r] = mine;
-        sum += mine;
-    }
-    uint32_t tot;
-    uint32_t run = block_excl_scan<uint32_t>(sum, sm, &tot);
-    for (uint32_t r = lo_r; r < hi_r; r++) {
-        lstart[r] = run;
-        run += lcur[r];
-        lcur[r] = 0;
-    }
-    __syncthreads();
-    const uint64_t n = sv.cum[sv.n];
-    const uint64_t chunk = (n + gridDim.x - 1) / gridDim.x;
-    const uint64_t lo = (uint64_t)blockIdx.x * chunk, hi = min(n, lo + chunk);
-    SegCursor cur;
-    seg_cursor_at(sv, cur, seg_of(sv, lo));
-    for (uint64_t i0 = lo + threadIdx.x; i0 < hi; i0 += 4 * SR_THREADS) {
-        uint64_t k4[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint64_t i = i0 + (uint64_t)u * SR_THREADS;   // ascending over u and over the loop
-            k4[u] = i < hi ? seg_key(sv, cur, i) : EMPTY_KEY;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            if (k4[u] == EMPTY_KEY) continue;
-            const uint32_t r = key_range(t, k4[u], nsub);
-            skeys[lstart[r] + atomicAdd(&lcur[r], 1u)] = k4[u];
+    for (int u = 0; u < SG_KEYS; u++) {
+        at[u] = 0;
+        if (key[u] != EMPTY_KEY) {
+            const uint32_t r = key_range(t, key[u], nsub);
+            at[u] = r << 16 | atomicAdd(&cnt[r], 1u);
         }
     }
     __syncthreads();
-    // one warp per range at a time: consecutive lanes store consecutive keys
-    const unsigned lane = lane_id();
-    for (uint32_t r = threadIdx.x >> 5; r < nsub; r += SR_THREADS / 32) {
-        const uint32_t n = lcur[r], n4 = (n + 3u) & ~3u;
-        const uint64_t g = gbase[r];
-        const uint32_t l0 = lstart[r];
-        for (uint32_t j = lane; j < n4; j += 32) range_keys[g + j] = j < n ? skeys[l0 + j] : EMPTY_KEY;
+    // counts -> starts (thread t sums a run of consecutive ranges)
+    const uint32_t per = (nsub + SG_THREADS - 1) / SG_THREADS;
+    const uint32_t r0 = min(nsub, threadIdx.x * per), r1 = min(nsub, r0 + per);
+    uint32_t sum = 0, m;
+    for (uint32_t r = r0; r < r1; r++) sum += cnt[r];
+    uint32_t run = block_excl_scan<uint32_t>(sum, sm, &m);
+    uint16_t *st = starts + (uint64_t)blockIdx.x * (nsub + 1);
+    for (uint32_t r = r0; r < r1; r++) {
+        const uint32_t c = cnt[r];
+        cnt[r] = run;
+        st[r] = (uint16_t)run;
+        run += c;
     }
+    if (threadIdx.x == 0) st[nsub] = (uint16_t)m;
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < SG_KEYS; u++)
+        if (key[u] != EMPTY_KEY) skeys[cnt[at[u] >> 16] + (at[u] & 0xFFFFu)] = key[u];
+    __syncthreads();
+    uint64_t *o = out + (uint64_t)blockIdx.x * SG_CHUNK;
+    for (uint32_t i = 2 * threadIdx.x; i < m; i += 2 * SG_THREADS)   // SG_CHUNK is even: the last pair stays inside
+        *reinterpret_cast<ulonglong2 *>(o + i) = *reinterpret_cast<const ulonglong2 *>(skeys + i);
 }
 
 // Shared-memory probe from `loc` up to `end` in a table kept as separate key
@@ -457,13 +408,15 @@ __global__ void __launch_bounds__(SR_THREADS) k_sr_scatter(const KeySeg *__restr
 // per slot as 16-byte slots would); adds `inc` where the key lives or lands.
 // A slot's key never changes once set, so a plain load that sees the key (most
 // occurrences repeat a key already placed) needs only the add; an empty slot
-// is claimed with CAS.  Returns false if the probe ran off the end.
+// is claimed with CAS (counted in `added`).  Returns false if the probe ran off
+// the end.
 __device__ __forceinline__ bool smem_add(unsigned long long *keys, uint32_t *vals, uint32_t loc, uint32_t end,
-                                         uint64_t key, uint32_t inc) {
+                                         uint64_t key, uint32_t inc, uint32_t &added) {
     for (; loc < end; loc++) {
         unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(&keys[loc]);
         if (cur == EMPTY_KEY) cur = atomicCAS(&keys[loc], EMPTY_KEY, (unsigned long long)key);
         if (cur == EMPTY_KEY || cur == key) {
+            added += cur == EMPTY_KEY;
             atomicAdd(&vals[loc], inc);
             return true;
         }
@@ -471,94 +424,110 @@ __device__ __forceinline__ bool smem_add(unsigned long long *keys, uint32_t *val
     return false;
 }
 
-__global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *__restrict__ range_keys,
-                                                        const uint32_t *__restrict__ totals, uint32_t nsub, int p,
-                                                        DevTable t, int fresh, uint32_t *__restrict__ next_totals,
-                                                        unsigned long long *__restrict__ next_cursor,
-                                                        uint64_t *__restrict__ defer_keys, uint32_t *__restrict__ defer_cnt,
-                                                        uint64_t defer_cap, unsigned long long *__restrict__ defer_n) {
+struct BuildSmem {
+    unsigned long long tkey[SR_MAX_SLOTS], mkey[SR_MINI];
+    uint32_t tval[SR_MAX_SLOTS], mval[SR_MINI];
+    uint32_t cum[SR_BUILD_THREADS + 1];      // keys of the range in the chunks before
+    uint32_t run[SR_BUILD_THREADS];          // where the chunk's run begins in the grouped keys
+    uint32_t scan[SR_BUILD_THREADS / 32 + 1];
+};
+
+// Range blockIdx.x % nsub of partition p0 + blockIdx.x / nsub.
+__global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *__restrict__ grouped,
+                                                        const uint16_t *__restrict__ starts,
+                                                        const PartGeom *__restrict__ parts, uint32_t nsub, int p0,
+                                                        DevTable t, uint64_t *__restrict__ defer_keys,
+                                                        uint32_t *__restrict__ defer_cnt, uint64_t defer_cap,
+                                                        unsigned long long *__restrict__ defer_n,
+                                                        unsigned long long *__restrict__ distinct) {
     extern __shared__ __align__(16) unsigned char sr_smem[];
-    unsigned long long *tkey = reinterpret_cast<unsigned long long *>(sr_smem);   // [SR_MAX_SLOTS]
-    unsigned long long *mkey = tkey + SR_MAX_SLOTS;                                // [SR_MINI]
-    uint32_t *tval = reinterpret_cast<uint32_t *>(mkey + SR_MINI);                 // [SR_MAX_SLOTS]
-    uint32_t *mval = tval + SR_MAX_SLOTS;                                          // [SR_MINI]
-    __shared__ uint64_t ab[2];
-    const uint32_t r = blockIdx.x;
+    BuildSmem &sm = *reinterpret_cast<BuildSmem *>(sr_smem);
+    const uint32_t pb = blockIdx.x / nsub, r = blockIdx.x % nsub;
+    const PartGeom part = parts[pb];
     const uint64_t r0 = range_first(t, r, nsub);
     const uint32_t len = (uint32_t)(range_first(t, r + 1, nsub) - r0);   // <= SR_MAX_SLOTS (host checks)
-    if (r == 0) {
-        // the next partition's range counters (their last users finished before this launch)
-        for (uint32_t i = threadIdx.x; i < nsub; i += SR_BUILD_THREADS) {
-            next_totals[i] = 0;
-            next_cursor[i] = 0;
-        }
-    }
-    {
-        // this range's keys: [start, start + total) of the range-ordered buffer
-        uint64_t sum = 0;
-        for (uint32_t i = threadIdx.x; i < r; i += SR_BUILD_THREADS) sum += totals[i];
-        sum = warp_sum(sum);
-        __shared__ uint64_t part[SR_BUILD_THREADS / 32];
-        if (lane_id() == 0) part[threadIdx.x >> 5] = sum;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            uint64_t a = 0;
-            for (int w = 0; w < SR_BUILD_THREADS / 32; w++) a += part[w];
-            ab[0] = a;
-            ab[1] = a + totals[r];
-        }
-    }
-    ulonglong2 *g = reinterpret_cast<ulonglong2 *>(t.slots + ((uint64_t)p << t.lbits) + r0);
     for (uint32_t i = threadIdx.x; i < len; i += SR_BUILD_THREADS) {
-        if (fresh) {
-            tkey[i] = EMPTY_KEY;
-            tval[i] = 0;
-        } else {
-            const ulonglong2 v = g[i];
-            tkey[i] = v.x;
-            tval[i] = (uint32_t)v.y;
-        }
+        sm.tkey[i] = EMPTY_KEY;
+        sm.tval[i] = 0;
     }
     for (int i = threadIdx.x; i < SR_MINI; i += SR_BUILD_THREADS) {
-        mkey[i] = EMPTY_KEY;
-        mval[i] = 0;
+        sm.mkey[i] = EMPTY_KEY;
+        sm.mval[i] = 0;
     }
-    __syncthreads();
-    const uint64_t a = ab[0], b = ab[1];
-    for (uint64_t i0 = a + threadIdx.x; i0 < b; i0 += 4 * SR_BUILD_THREADS) {
-        uint64_t k4[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint64_t i = i0 + (uint64_t)u * SR_BUILD_THREADS;
-            k4[u] = i < b ? __ldcs(range_keys + i) : EMPTY_KEY;
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    uint32_t added = 0, unused = 0;
+    for (uint32_t t0 = 0; t0 < part.chunks; t0 += SR_BUILD_THREADS) {
+        // the runs of up to SR_BUILD_THREADS chunks, taken as one sequence
+        const uint32_t c = t0 + threadIdx.x;
+        uint32_t n = 0, first = 0;
+        if (c < part.chunks) {
+            const uint16_t *st = starts + (uint64_t)(part.chunk0 + c) * (nsub + 1) + r;
+            const uint32_t a = st[0];
+            n = st[1] - a;
+            first = (part.chunk0 + c) * SG_CHUNK + a;
         }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-            const uint64_t key = k4[u];
-            if (key == EMPTY_KEY || smem_add(tkey, tval, (uint32_t)((mix64(key) & t.lmask) - r0), len, key, 1u)) continue;
-            // the probe left the range: count it in the per-block table, or defer it singly
-            const uint32_t m = (uint32_t)(mix64(key ^ 0x5851F42D4C957F2DULL) & (SR_MINI - 1));
-            if (smem_add(mkey, mval, m, SR_MINI, key, 1u) || (m && smem_add(mkey, mval, 0, m, key, 1u))) continue;
-            const unsigned long long j = atomicAdd(defer_n, 1ULL);
-            if (j < defer_cap) {
-                defer_keys[j] = key;
-                defer_cnt[j] = 1u;
+        uint32_t total;
+        sm.cum[threadIdx.x] = block_excl_scan<uint32_t>(n, sm.scan, &total);
+        sm.run[threadIdx.x] = first;
+        if (threadIdx.x == 0) sm.cum[SR_BUILD_THREADS] = total;
+        __syncthreads();
+        // a warp takes a stretch of the sequence; a lane walks its runs forward
+        const uint32_t per = (total + SR_BUILD_THREADS - 1) / SR_BUILD_THREADS * 32;
+        const uint32_t lo = warp * per, hi = min(total, lo + per);
+        uint32_t q = 0;
+        if (lo < hi) {
+            uint32_t e = SR_BUILD_THREADS;   // cum[q] <= lo < cum[e]
+            while (e - q > 1) {
+                const uint32_t mid = (q + e) >> 1;
+                if (sm.cum[mid] <= lo) q = mid; else e = mid;
             }
         }
+        for (uint32_t i0 = lo + lane; i0 < hi; i0 += 128) {
+            uint64_t k4[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint32_t i = i0 + u * 32;
+                k4[u] = EMPTY_KEY;
+                if (i < hi) {
+                    while (sm.cum[q + 1] <= i) q++;
+                    k4[u] = __ldcg(grouped + sm.run[q] + (i - sm.cum[q]));
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; u++) {
+                const uint64_t key = k4[u];
+                if (key == EMPTY_KEY || smem_add(sm.tkey, sm.tval, (uint32_t)((mix64(key) & t.lmask) - r0), len, key, 1u, added))
+                    continue;
+                // the probe left the range: count it in the per-block table, or defer it singly
+                const uint32_t m = (uint32_t)(mix64(key ^ 0x5851F42D4C957F2DULL) & (SR_MINI - 1));
+                if (smem_add(sm.mkey, sm.mval, m, SR_MINI, key, 1u, unused) ||
+                    (m && smem_add(sm.mkey, sm.mval, 0, m, key, 1u, unused)))
+                    continue;
+                const unsigned long long j = atomicAdd(defer_n, 1ULL);
+                if (j < defer_cap) {
+                    defer_keys[j] = key;
+                    defer_cnt[j] = 1u;
+                }
+            }
+        }
+        __syncthreads();
     }
     __syncthreads();
+    added = warp_sum(added);
+    if (lane == 0 && added) atomicAdd(distinct, (unsigned long long)added);
+    ulonglong2 *g = reinterpret_cast<ulonglong2 *>(t.slots + ((uint64_t)(p0 + pb) << t.lbits) + r0);
     for (uint32_t i = threadIdx.x; i < len; i += SR_BUILD_THREADS) {
         ulonglong2 v;
-        v.x = tkey[i];
-        v.y = tval[i];
+        v.x = sm.tkey[i];
+        v.y = sm.tval[i];
         g[i] = v;
     }
     for (int i = threadIdx.x; i < SR_MINI; i += SR_BUILD_THREADS) {
-        if (mkey[i] == EMPTY_KEY) continue;
+        if (sm.mkey[i] == EMPTY_KEY) continue;
         const unsigned long long j = atomicAdd(defer_n, 1ULL);
         if (j < defer_cap) {
-            defer_keys[j] = mkey[i];
-            defer_cnt[j] = mval[i];
+            defer_keys[j] = sm.mkey[i];
+            defer_cnt[j] = sm.mval[i];
         }
     }
 }
@@ -566,10 +535,11 @@ __global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *_
 __global__ void k_rehash(const Slot *__restrict__ old, uint64_t old_cap, DevTable t, int max_probes,
                          uint64_t *__restrict__ ovf_keys, uint32_t *__restrict__ ovf_cnt, uint64_t ovf_cap,
                          unsigned long long *__restrict__ counters) {
+    uint32_t added = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < old_cap; i += (uint64_t)gridDim.x * blockDim.x) {
         ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(&old[i]));
         if (v.x == EMPTY_KEY) continue;
-        if (!tbl_add(t, v.x, (uint32_t)v.y, max_probes)) {
+        if (!tbl_add_new(t, v.x, (uint32_t)v.y, max_probes, &added)) {
             unsigned long long j = atomicAdd(&counters[0], 1ULL);
             if (j < ovf_cap) { ovf_keys[j] = v.x; ovf_cnt[j] = (uint32_t)v.y; }
         }
@@ -578,14 +548,20 @@ __global__ void k_rehash(const Slot *__restrict__ old, uint64_t old_cap, DevTabl
 
 __global__ void k_insert_pairs(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ cnt, uint64_t n, DevTable t,
                                int max_probes, uint64_t *__restrict__ ovf_keys, uint32_t *__restrict__ ovf_cnt,
-                               uint64_t ovf_cap, unsigned long long *__restrict__ counters) {
+                               uint64_t ovf_cap, unsigned long long *__restrict__ counters,
+                               unsigned long long *__restrict__ distinct) {
+    uint32_t added = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t key = keys[i];
         uint32_t c = cnt ? cnt[i] : 1u;
-        if (!tbl_add(t, key, c, max_probes)) {
+        if (!tbl_add_new(t, key, c, max_probes, &added)) {
             unsigned long long j = atomicAdd(&counters[0], 1ULL);
             if (j < ovf_cap) { ovf_keys[j] = key; ovf_cnt[j] = c; }
         }
+    }
+    if (distinct) {
+        added = warp_sum(added);
+        if (lane_id() == 0 && added) atomicAdd(distinct, (unsigned long long)added);
     }
 }
 
@@ -827,6 +803,7 @@ static int drain_overflow(tk_table *t) {
         unsigned long long ovf = 0;
         TK_TRY(overflow_read(t, &ovf));
         if (ovf == 0) return TK_OK;
+        t->distinct_valid = false;
         if (ovf > t->ovf_cap)
             return set_err(c, TK_E_TABLE_FULL,
                            "table overflow list overran (" + std::to_string(ovf) + " keys); create the table with a larger capacity");
@@ -844,7 +821,7 @@ static int drain_overflow(tk_table *t) {
         if (!e) {
             k_insert_pairs<<<stream_grid(c, ovf, 256), 256, 0, c->stream>>>(pk, pc, ovf, t->t, c->max_probes, t->d_ovf,
                                                                              (uint32_t *)(t->d_ovf + t->ovf_cap), t->ovf_cap,
-                                                                             t->d_counters);
+                                                                             t->d_counters, nullptr);
             c->launches++;
             e = check_launch(c, "overflow insert");
         }
@@ -909,12 +886,12 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
     tk_ctx *c = t->ctx;
     *done = false;
     const int nparts = 1 << t->t.pbits;
-    // ranges per slice: one wave of SR_BUILD_PER_SM build blocks per SM, more if a range
-    // would not fit in shared memory
+    // ranges per slice: SR_BUILD_PER_SM per SM, more if a range would not fit in shared memory
     const uint64_t slice = 1ULL << t->t.lbits, wave = (uint64_t)c->sm_count * SR_BUILD_PER_SM;
     uint32_t nsub;
     if (slice / 1024 < wave) nsub = (uint32_t)(slice / 1024);   // a small slice: ranges of 1024 slots
-    else nsub = (uint32_t)(wave * ((slice + wave * SR_MAX_SLOTS - 1) / (wave * SR_MAX_SLOTS)));   // whole waves
+    else nsub = (uint32_t)(wave * ((slice + wave * SR_MAX_SLOTS - 1) / (wave * SR_MAX_SLOTS)));
+    if (nsub > 0xFFFF) return TK_OK;   // run starts and ranges are 16-bit
     const uint64_t bpp = (uint64_t)(NBUCKETS >> t->t.pbits);
     // partition boundaries on the host: the first offset of each partition's
     // buckets in each set's buffer; partition p's keys are one segment of each
@@ -926,7 +903,9 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
                                          cudaMemcpyDeviceToHost, c->stream));
     TK_CUDA(c, cudaStreamSynchronize(c->stream));
     std::vector<KeySeg> segs((size_t)nparts * nsets);
-    uint64_t max_part = 0, all_keys = 0;
+    std::vector<PartGeom> parts(nparts);
+    std::vector<int> batch{0};                 // first partition of every batch, then nparts
+    uint64_t all_keys = 0, batch_keys = 0, batch_chunks = 0, max_chunks = 0;
     for (int p = 0; p < nparts; p++) {
         uint64_t part = 0;
         for (uint32_t q = 0; q < nsets; q++) {
@@ -935,57 +914,63 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
             g.len = bk[q].keys ? pb[q][p + 1] - pb[q][p] : 0;
             part += g.len;
         }
-        max_part = std::max(max_part, part);
+        if (p > batch.back() && batch_keys + part > SR_BATCH_KEYS) {
+            batch.push_back(p);
+            batch_keys = batch_chunks = 0;
+        }
+        const uint64_t chunks = (part + SG_CHUNK - 1) / SG_CHUNK;
+        parts[p].chunk0 = (uint32_t)batch_chunks;
+        parts[p].chunks = (uint32_t)chunks;
+        batch_keys += part;
+        batch_chunks += chunks;
+        max_chunks = std::max(max_chunks, batch_chunks);
         all_keys += part;
     }
-    // blocks of the regrouping passes: two per SM, more if a block's chunk
-    // would not fit in the scatter's shared memory (rounding that up to whole
-    // waves of two blocks per SM was slower: 52.5 against 50.9 ms per step)
-    const unsigned G = (unsigned)std::max<uint64_t>((uint64_t)c->sm_count * 2, (max_part + SRS_MAX - 1) / SRS_MAX);
-    const uint64_t cells = (uint64_t)nsub * G;
+    batch.push_back(nparts);
+    if (max_chunks * SG_CHUNK > 0xFFFFFFFFull) return TK_OK;   // places in the grouped keys are 32-bit
     uint64_t defer_cap = std::max<uint64_t>(1u << 16, std::min<uint64_t>(all_keys / 64, 1u << 24));
     if (const char *v = getenv("TRINKMER_DEFER_CAP")) defer_cap = std::max<uint64_t>(1, strtoull(v, nullptr, 10));   // tests: force the fallback
-    uint64_t *range_keys = nullptr, *defer_keys = nullptr;
-    uint32_t *counts = nullptr, *defer_cnt = nullptr, *totals = nullptr;
-    unsigned long long *defer_n = nullptr, *cursor = nullptr;
+    uint64_t *grouped = nullptr, *defer_keys = nullptr;
+    uint32_t *defer_cnt = nullptr;
+    uint16_t *starts = nullptr;
+    unsigned long long *counters = nullptr;   // deferred keys, distinct keys
     KeySeg *d_segs = nullptr;
-    // a partition's keys plus the sector rounding of every (range, block) run
-    int e = dmalloc(c, (void **)&range_keys, (max_part + 3 * cells + 1) * 8, "range keys");
+    PartGeom *d_parts = nullptr;
+    int e = dmalloc(c, (void **)&grouped, max_chunks * SG_CHUNK * 8, "grouped keys");
+    if (!e) e = dmalloc(c, (void **)&starts, max_chunks * (nsub + 1) * 2, "group starts");
     if (!e) e = dmalloc(c, (void **)&d_segs, segs.size() * sizeof(KeySeg), "partition segments");
-    if (!e) e = cuda_check(c, cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(KeySeg), cudaMemcpyHostToDevice,
-                                              c->stream), "partition segments h2d");
-    if (!e) e = dmalloc(c, (void **)&counts, cells * 4, "range counts");
-    if (!e) e = dmalloc(c, (void **)&totals, 2ull * nsub * 4, "range totals");
-    if (!e) e = dmalloc(c, (void **)&cursor, 2ull * nsub * 8, "range cursors");
+    if (!e) e = dmalloc(c, (void **)&d_parts, parts.size() * sizeof(PartGeom), "partition chunks");
     if (!e) e = dmalloc(c, (void **)&defer_keys, defer_cap * 8, "deferred keys");
     if (!e) e = dmalloc(c, (void **)&defer_cnt, defer_cap * 4, "deferred counts");
-    if (!e) e = dmalloc(c, (void **)&defer_n, 8, "deferred count");
-    if (!e) e = cuda_check(c, cudaMemsetAsync(defer_n, 0, 8, c->stream), "defer reset");
-    if (!e) e = cuda_check(c, cudaMemsetAsync(totals, 0, 2ull * nsub * 4, c->stream), "totals reset");
-    if (!e) e = cuda_check(c, cudaMemsetAsync(cursor, 0, 2ull * nsub * 8, c->stream), "cursor reset");
-    if (!e) e = cuda_check(c, cudaFuncSetAttribute(k_sr_build, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SR_SMEM),
+    if (!e) e = dmalloc(c, (void **)&counters, 16, "count counters");
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(KeySeg), cudaMemcpyHostToDevice,
+                                              c->stream), "partition segments h2d");
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(d_parts, parts.data(), parts.size() * sizeof(PartGeom), cudaMemcpyHostToDevice,
+                                              c->stream), "partition chunks h2d");
+    if (!e) e = cuda_check(c, cudaMemsetAsync(counters, 0, 16, c->stream), "count counters reset");
+    const int group_smem = (int)(SG_CHUNK * 8 + nsub * 4), build_smem = (int)sizeof(BuildSmem);
+    if (!e) e = cuda_check(c, cudaFuncSetAttribute(k_sr_build, cudaFuncAttributeMaxDynamicSharedMemorySize, build_smem),
                            "range build smem");
-    if (!e) e = cuda_check(c, cudaFuncSetAttribute(k_sr_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                   (int)SRS_SMEM(nsub)), "range scatter smem");
-    for (int p = 0; !e && p < nparts; p++) {
-        uint64_t part = 0;
-        for (uint32_t q = 0; q < nsets; q++) part += segs[(size_t)p * nsets + q].len;
-        const KeySeg *ps = d_segs + (size_t)p * nsets;
-        uint32_t *tot = totals + (uint64_t)(p & 1) * nsub, *tot_next = totals + (uint64_t)((p + 1) & 1) * nsub;
-        unsigned long long *cur = cursor + (uint64_t)(p & 1) * nsub, *cur_next = cursor + (uint64_t)((p + 1) & 1) * nsub;
-        if (part) {
-            k_sr_hist<<<G, SR_THREADS, nsub * 4, c->stream>>>(ps, nsets, t->t, nsub, counts, tot);
-            k_sr_scatter<<<G, SR_THREADS, SRS_SMEM(nsub), c->stream>>>(ps, nsets, t->t, nsub, counts, tot, cur, range_keys);
-            c->launches += 2;
+    if (!e) e = cuda_check(c, cudaFuncSetAttribute(k_sr_group, cudaFuncAttributeMaxDynamicSharedMemorySize, group_smem),
+                           "range group smem");
+    for (size_t b = 0; !e && b + 1 < batch.size(); b++) {
+        const int p0 = batch[b], np = batch[b + 1] - p0;
+        const unsigned chunks = parts[p0 + np - 1].chunk0 + parts[p0 + np - 1].chunks;
+        if (chunks) {
+            k_sr_group<<<chunks, SG_THREADS, group_smem, c->stream>>>(d_segs + (size_t)p0 * nsets, nsets, d_parts + p0, np, t->t,
+                                                                     nsub, grouped, starts);
+            c->launches++;
         }
-        k_sr_build<<<nsub, SR_BUILD_THREADS, SR_SMEM, c->stream>>>(range_keys, tot, nsub, p, t->t, 1, tot_next, cur_next,
-                                                             defer_keys, defer_cnt, defer_cap, defer_n);
+        k_sr_build<<<nsub * np, SR_BUILD_THREADS, build_smem, c->stream>>>(grouped, starts, d_parts + p0, nsub, p0, t->t,
+                                                                          defer_keys, defer_cnt, defer_cap, counters,
+                                                                          counters + 1);
         c->launches++;
     }
-    unsigned long long nd = 0;
+    unsigned long long h[2] = {0, 0};
     if (!e) e = check_launch(c, "range build");
-    if (!e) e = cuda_check(c, cudaMemcpyAsync(&nd, defer_n, 8, cudaMemcpyDeviceToHost, c->stream), "defer d2h");
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(h, counters, 16, cudaMemcpyDeviceToHost, c->stream), "count counters d2h");
     if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "defer sync");
+    const unsigned long long nd = h[0];
     if (!e && nd > defer_cap) {
         // the deferred list overran: empty the table again and count with atomics
         k_fill_empty<<<stream_grid(c, t->capacity, 256), 256, 0, c->stream>>>(t->t.slots, t->capacity, 0);
@@ -997,20 +982,25 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
         if (nd) {
             k_insert_pairs<<<stream_grid(c, nd, 256), 256, 0, c->stream>>>(defer_keys, defer_cnt, nd, t->t, c->max_probes,
                                                                             t->d_ovf, (uint32_t *)(t->d_ovf + t->ovf_cap),
-                                                                            t->ovf_cap, t->d_counters);
+                                                                            t->ovf_cap, t->d_counters, counters + 1);
             c->launches++;
             e = check_launch(c, "deferred insert");
+            if (!e) e = cuda_check(c, cudaMemcpyAsync(h, counters, 16, cudaMemcpyDeviceToHost, c->stream), "count counters d2h");
+            if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "deferred insert sync");
         }
-        if (!e) *done = true;
+        if (!e) {
+            t->distinct = h[1];   // every key of the table was new to it once
+            t->distinct_valid = true;
+            *done = true;
+        }
     }
-    dfree(c, range_keys);
+    dfree(c, grouped);
+    if (starts) dfree(c, starts);
     if (d_segs) dfree(c, d_segs);
-    dfree(c, counts);
-    dfree(c, totals);
-    dfree(c, cursor);
-    dfree(c, defer_keys);
-    dfree(c, defer_cnt);
-    dfree(c, defer_n);
+    if (d_parts) dfree(c, d_parts);
+    if (defer_keys) dfree(c, defer_keys);
+    if (defer_cnt) dfree(c, defer_cnt);
+    if (counters) dfree(c, counters);
     return e;
 }
 
@@ -1107,6 +1097,7 @@ int table_count_buckets(tk_table *t, std::vector<BucketKeys> &bk) {
     cudaEvent_t ev;
     if (!e && windows) {
         e = overflow_reset(t);
+        t->distinct_valid = false;
         prof_begin(c, TK_KID_COUNT, &ev);
         bool done = false;
         if (!e && t->fresh && t->t.lbits >= SR_MIN_LBITS) e = count_by_ranges(t, bk, &done);
@@ -1130,7 +1121,6 @@ int table_count_buckets(tk_table *t, std::vector<BucketKeys> &bk) {
     }
     if (e) return e;
     t->total += windows;
-    t->distinct_valid = false;
     return drain_overflow(t);
 }
 
@@ -1331,7 +1321,7 @@ int table_insert_pairs(tk_table *t, const uint64_t *d_keys, const uint32_t *d_cn
     prof_begin(c, TK_KID_LOAD, &ev);
     k_insert_pairs<<<stream_grid(c, n, 256), 256, 0, c->stream>>>(d_keys, d_cnt, n, t->t, c->max_probes, t->d_ovf,
                                                                    (uint32_t *)(t->d_ovf + t->ovf_cap), t->ovf_cap,
-                                                                   t->d_counters);
+                                                                   t->d_counters, nullptr);
     c->launches++;
     prof_end(c, TK_KID_LOAD, ev, n);
     TK_TRY(check_launch(c, "insert pairs"));
