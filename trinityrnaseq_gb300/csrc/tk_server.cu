@@ -67,7 +67,7 @@ uint64_t job_estimate(const tk_job_spec &s) {
     switch (s.kind) {
     case TK_JOB_COUNT: return 32 * a + (64ULL << 20);
     case TK_JOB_NORMALIZE: return (s.max_cov >= 2 ? 40 : 32) * (a + b) + (64ULL << 20);
-    case TK_JOB_R2T: return 6 * a + 52 * b + (64ULL << 20);
+    case TK_JOB_R2T: return 6 * a + 48 * b + (64ULL << 20);
     default: return 64ULL << 20;
     }
 }

@@ -252,9 +252,17 @@ __global__ void __launch_bounds__(CT_THREADS) k_part_step(const uint64_t *__rest
 // per occurrence to the deferred keys alone, and a fresh slice needs no
 // separate fill.
 //
-// A batch holds about SR_BATCH_KEYS keys: enough blocks per launch that one
-// block's loads, inserts and writes overlap another's, few enough that the
-// grouped keys are still in L2 when the build reads them.
+// A batch holds about SR_BATCH_KEYS keys (256 MB of grouped keys): what counts
+// is that a launch has many blocks, whose loads, inserts and writes overlap, not
+// that the grouped keys are still in L2 when the build reads them.  5M pairs
+// (760M keys, 256 partitions), group + build: 6M keys a batch 3.9 + 8.0 ms, 12M
+// 3.4 + 6.1, 24M 3.2 + 5.7, 48M 3.1 + 5.5, 96M 3.1 + 5.4 (the histogram,
+// regrouping and build of one partition after another that this replaces: 2.7 +
+// 5.4 + 6.8).  The group is bound by memory and its shared-memory sort (3.9
+// TB/s), the build by its probes' instructions (180 per 32 keys).  Ranges of
+// half the size with 512-thread blocks 6.3, of twice the size 6.9, 768-thread
+// blocks 6.0 ms at 48M; chunks of 4096 (three blocks per SM) and 8192 keys
+// (one) 3.2 and 4.8.
 constexpr int SR_MIN_LBITS = 12;        // slices below 4096 slots keep the atomic path
 constexpr int SR_BUILD_PER_SM = 2;      // ranges per slice and SM
 constexpr int SR_MAX_SLOTS = 7168;      // slots of one range in shared memory (12 bytes each)
@@ -263,7 +271,7 @@ constexpr int SR_MINI = 64;
 constexpr int SG_THREADS = 512;
 constexpr int SG_KEYS = 12;             // keys per thread, in registers
 constexpr uint32_t SG_CHUNK = SG_THREADS * SG_KEYS;
-constexpr uint64_t SR_BATCH_KEYS = 6ull << 20;
+constexpr uint64_t SR_BATCH_KEYS = 32ull << 20;
 
 // A slice of 2^lbits slots is cut into nsub ranges: slot s belongs to range
 // floor(s * nsub / 2^lbits), so range r is [ceil(r 2^lbits / nsub),
@@ -408,24 +416,34 @@ __global__ void __launch_bounds__(SG_THREADS, 2) k_sr_group(const KeySeg *__rest
 // per slot as 16-byte slots would); adds `inc` where the key lives or lands.
 // A slot's key never changes once set, so a plain load that sees the key (most
 // occurrences repeat a key already placed) needs only the add; an empty slot
-// is claimed with CAS (counted in `added`).  Returns false if the probe ran off
-// the end.
+// is claimed with CAS (counted in `added`).  A step looks at an aligned pair of
+// slots (one 16-byte load; 6% of the build).  `keys` has an even number of
+// entries.  Returns false if the probe ran off the end.
 __device__ __forceinline__ bool smem_add(unsigned long long *keys, uint32_t *vals, uint32_t loc, uint32_t end,
                                          uint64_t key, uint32_t inc, uint32_t &added) {
-    for (; loc < end; loc++) {
-        unsigned long long cur = *reinterpret_cast<volatile unsigned long long *>(&keys[loc]);
+    while (loc < end) {
+        unsigned long long a, b;
+        asm volatile("ld.volatile.shared.v2.u64 {%0, %1}, [%2];"
+                     : "=l"(a), "=l"(b)
+                     : "r"((uint32_t)__cvta_generic_to_shared(&keys[loc & ~1u])));
+        unsigned long long cur = loc & 1u ? b : a;
+        if (!(loc & 1u) && cur != key && cur != EMPTY_KEY) {
+            cur = b;
+            if (++loc >= end) return false;
+        }
         if (cur == EMPTY_KEY) cur = atomicCAS(&keys[loc], EMPTY_KEY, (unsigned long long)key);
         if (cur == EMPTY_KEY || cur == key) {
             added += cur == EMPTY_KEY;
             atomicAdd(&vals[loc], inc);
             return true;
         }
+        loc++;
     }
     return false;
 }
 
-struct BuildSmem {
-    unsigned long long tkey[SR_MAX_SLOTS], mkey[SR_MINI];
+struct __align__(16) BuildSmem {
+    unsigned long long tkey[SR_MAX_SLOTS], mkey[SR_MINI];   // 16-byte aligned pairs
     uint32_t tval[SR_MAX_SLOTS], mval[SR_MINI];
     uint32_t cum[SR_BUILD_THREADS + 1];      // keys of the range in the chunks before
     uint32_t run[SR_BUILD_THREADS];          // where the chunk's run begins in the grouped keys
