@@ -63,6 +63,25 @@ def test_extract_matches_reference(ctx, golden):
     assert e.value.status == native.TK_E_PARSE
 
 
+@pytest.mark.parametrize("lo,hi", [(1, 3), (1, 40), (60, 120), (400, 900), (1, 6000)])
+def test_extract_record_sizes(ctx, oracle, lo, hi):
+    """Records shorter than the 16-byte chunks the copy writes, of ordinary size, and so long that a block's output
+    passes its chunk table; runs of records that are not selected between them, and a text without a last newline."""
+    rnd = np.random.default_rng(hi)
+    n = 1500
+    recs = []
+    for i in range(n):
+        L = int(rnd.integers(lo, hi + 1))
+        recs.append(b"@%d%s\n%s\n+\n%s\n" % (i, b"/1" if rnd.random() < 0.5 else b"", rnd.choice(
+            np.frombuffer(b"ACGT", np.uint8), L).tobytes(), b"I" * L))
+    text = b"".join(recs)[:-1]
+    rs = ReadSet(ctx, text)
+    med = np.where((np.arange(n) // 37) % 3 == 0, 200, 2).astype(np.uint32)   # a third mostly thinned out, in runs
+    nm = Normalization(ctx, rs, (med, med.astype(np.float32), np.ones(n, np.float32)), max_cov=20, min_cov=1, max_cv=10000)
+    assert 0 < nm.counts["selected"] < n
+    assert nm.extract(rs) == oracle.norm_extract(text, nm.accs())
+
+
 def test_extract_fasta(ctx, golden, oracle):
     """FASTA input: the name z\xc3z loses its high byte in Fasta_reader, so
     the full selection dies as the script does; without that pair the records
