@@ -190,6 +190,44 @@ def test_odd_names_take_the_repair_walk(ctx, oracle):
     assert single.accs() == a1
 
 
+NAME_STYLES = {
+    "numbers": lambda r, i: f"r{i:010d}",                                       # a few varying digits
+    "ragged": lambda r, i: f"r{i}",                                             # lengths differ
+    "sequencer": lambda r, i: f"HWI-ST0:7:C0AB:{r.randint(1, 8)}:{r.randint(1101, 2316)}:{r.randint(1000, 21000)}:{i}",
+    "letters": lambda r, i: "".join(r.choice("abcdefghijXYZ0189_-") for _ in range(r.randint(12, 20))),   # > 64 bits
+    "long": lambda r, i: "x" * 70 + f"{i:05d}",                                 # past the packed key's chunks
+    "wide": lambda r, i: f"{i % 7}" + "y" * 50 + f"{i // 7}",                   # varying bits far apart
+}
+
+
+@pytest.mark.parametrize("style", sorted(NAME_STYLES))
+@pytest.mark.parametrize("dups", [0, 200])
+def test_name_styles(ctx, oracle, style, dups):
+    """Sort keys packed from the bits that differ and sorts 8 bytes at a time, over merge chunks of 16 rows, with
+    duplicated names at their boundaries."""
+    rnd = random.Random(5)
+    cores = list(dict.fromkeys(NAME_STYLES[style](rnd, i) for i in range(3000)))
+    left = [c + "/1" for c in cores if rnd.random() < 0.95]
+    right = [c + "/2" for c in cores if rnd.random() < 0.95]
+    left += rnd.choices(left, k=dups)
+    right += rnd.choices(right, k=dups)
+    rnd.shuffle(left)
+    rnd.shuffle(right)
+
+    def side(names):
+        med = np.array([rnd.randint(0, 20) for _ in names], dtype=np.uint32)
+        mean = np.array([rnd.choice([1.5, 2.25, 7.0, 13.37]) for _ in names], dtype=np.float32)
+        sd = np.array([rnd.choice([0.0, 0.5, 1.25, 3.3]) for _ in names], dtype=np.float32)
+        fa = "".join(f">{n}\nACGT\n" for n in names).encode()
+        return ReadSet(ctx, fa), (med, mean, sd), format_stats([n.encode() for n in names], med, mean, sd)
+
+    lrs, ls, lt = side(left)
+    rrs, rs, rt = side(right)
+    nm = Normalization(ctx, lrs, ls, rrs, rs, 4, 1, 2)
+    table, accs, cnt = oracle.norm(lt, rt, 4, 1, 2)
+    assert nm.table() == table and nm.accs() == accs
+
+
 def test_empty_and_device_inputs(ctx, oracle):
     import torch
     empty = ReadSet(ctx, b"")

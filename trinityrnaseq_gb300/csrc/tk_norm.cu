@@ -30,16 +30,20 @@
 // exact operands.  The "%.1f" averages are carried as integers N (text N/10)
 // rounded the same way, and read back as N / 10.0.
 //
-// Sorting is an LSD radix sort of the names 8 bytes at a time (zero padded,
-// big-endian), skipping the bits every name shares.  Two names whose padded
+// Sorting is an LSD radix sort of the names (zero padded, big-endian).  The
+// bits in which some names of the side differ are packed into one 64-bit key
+// when they fit (names of up to 64 bytes that differ in a number do); otherwise
+// the names are sorted 8 bytes at a time, skipping the bits every name
+// shares.  Two names whose padded
 // bytes agree (equal names, or names differing only in trailing NUL bytes)
 // make the order depend on the rest of the line; when any exist the sort is
 // redone on the full key (suffix text, then name length, then name bytes).
 //
 // The merge is the scripts' sequential two-cursor walk, run speculatively in
-// chunks of MG_CHUNK left rows: chunk k starts at (k*C, the number of right
-// names below left name k*C) and walks until it stands exactly on the next
-// chunk's start.  The walk is deterministic, so a chunk that starts on the
+// chunks of about C left rows (merge_chunk): chunk k starts at (k*C, the number
+// of right names below left name k*C), or at the first of the next few left
+// rows whose core name is not the one before's, and walks until it stands
+// exactly on the next chunk's start.  The walk is deterministic, so a chunk that starts on the
 // true path and reaches the next start hands over to a chunk that is on the
 // true path too; the first chunk that overshoots is walked again, from its
 // (true) start to the end, by one thread.  For reads named <core>/1 and
@@ -57,7 +61,13 @@
 namespace tk {
 
 constexpr int NM_THREADS = 256;
-constexpr uint32_t MG_CHUNK = 256;          // left rows per speculative merge chunk
+// Left rows per speculative merge chunk: one thread walks a chunk, so small
+// sides take small chunks (a walk of 256 rows takes 0.22 ms whatever the number
+// of threads beside it).  About 64K chunks fill the GPU.
+constexpr uint32_t MG_SHIFT = 8;            // rows a chunk's start moves past equal core names at most
+static inline uint32_t merge_chunk(uint64_t rows) {
+    return (uint32_t)std::max<uint64_t>(16, std::min<uint64_t>(256, rows / 65536));
+}
 constexpr int SFX_SLOT = 48;                // bytes per read of "\t%u\t%g\t%g" (full-key sort)
 
 enum : uint32_t { NE_DOMAIN = 0, NE_DIV0 = 1, NE_HASH = 2, NE_WORDS = 4 };
@@ -305,18 +315,109 @@ __device__ __forceinline__ uint64_t slot_chunk(const uint8_t *__restrict__ slots
     return k;
 }
 
-__global__ void k_name_maxlen(const uint32_t *__restrict__ len, uint64_t n, uint32_t *__restrict__ out) {
-    __shared__ uint32_t sm[NM_THREADS / 32];
-    uint32_t v = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        v = max(v, len[i]);
-    v = __reduce_max_sync(0xffffffffu, v);
-    if (lane_id() == 0) sm[threadIdx.x >> 5] = v;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < NM_THREADS / 32; w++) v = max(v, sm[w]);
-        if (v) atomicMax(out, v);
+// What a side's names have in common: the longest, and per 8-byte chunk (up to
+// NAME_CHUNKS of them) the bits set in some name and in all.
+constexpr uint32_t NAME_CHUNKS = 8;
+struct NameStats {
+    unsigned long long some[NAME_CHUNKS], all[NAME_CHUNKS];
+    uint32_t max_len;
+};
+
+__global__ void __launch_bounds__(NM_THREADS) k_name_stats(const uint64_t *__restrict__ addr, const uint32_t *__restrict__ len,
+                                                           uint64_t n, NameStats *__restrict__ out) {
+    __shared__ unsigned long long s_some[NAME_CHUNKS], s_all[NAME_CHUNKS];
+    if (threadIdx.x < NAME_CHUNKS) {
+        s_some[threadIdx.x] = 0;
+        s_all[threadIdx.x] = ~0ULL;
     }
+    __syncthreads();
+    unsigned long long some[NAME_CHUNKS], all[NAME_CHUNKS];
+#pragma unroll
+    for (uint32_t c = 0; c < NAME_CHUNKS; c++) {
+        some[c] = 0;
+        all[c] = ~0ULL;
+    }
+    uint32_t ml = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t l = len[i];
+        ml = max(ml, l);
+        const char *nm = at(addr[i]);
+#pragma unroll
+        for (uint32_t c = 0; c < NAME_CHUNKS; c++) {
+            const uint64_t k = c * 8 < l ? name_chunk(nm, l, c) : 0ULL;
+            some[c] |= k;
+            all[c] &= k;
+        }
+    }
+    ml = __reduce_max_sync(0xffffffffu, ml);
+#pragma unroll
+    for (uint32_t c = 0; c < NAME_CHUNKS; c++) {
+        // the warp's or / and by 32-bit halves
+        const uint32_t oh = __reduce_or_sync(0xffffffffu, (uint32_t)(some[c] >> 32));
+        const uint32_t ol = __reduce_or_sync(0xffffffffu, (uint32_t)some[c]);
+        const uint32_t ah = __reduce_and_sync(0xffffffffu, (uint32_t)(all[c] >> 32));
+        const uint32_t al = __reduce_and_sync(0xffffffffu, (uint32_t)all[c]);
+        if (lane_id() == 0) {
+            atomicOr(&s_some[c], (unsigned long long)oh << 32 | ol);
+            atomicAnd(&s_all[c], (unsigned long long)ah << 32 | al);
+        }
+    }
+    if (lane_id() == 0 && ml) atomicMax(&out->max_len, ml);
+    __syncthreads();
+    if (threadIdx.x < NAME_CHUNKS) {
+        atomicOr(&out->some[threadIdx.x], s_some[threadIdx.x]);
+        atomicAnd(&out->all[threadIdx.x], s_all[threadIdx.x]);
+    }
+}
+
+// The bits of a name that make its sort key, most significant first: `width`
+// bits from bit `shift` up of chunk `chunk`.
+struct NameBits {
+    uint32_t n = 0, bits = 0;
+    uint8_t chunk[64], shift[64], width[64];
+};
+
+// The runs of differing bits of the first nch chunks; false when they are more than 64 bits.
+static bool name_bits(const NameStats &st, uint32_t nch, NameBits *nb) {
+    for (uint32_t c = 0; c < nch; c++) {
+        uint64_t diff = st.some[c] ^ st.all[c];
+        while (diff) {
+            const int hi = 63 - __builtin_clzll(diff);
+            int lo = hi;
+            while (lo > 0 && (diff >> (lo - 1)) & 1) lo--;
+            const uint32_t w = (uint32_t)(hi - lo + 1);
+            if (nb->bits + w > 64) return false;
+            nb->chunk[nb->n] = (uint8_t)c;
+            nb->shift[nb->n] = (uint8_t)lo;
+            nb->width[nb->n] = (uint8_t)w;
+            nb->n++;
+            nb->bits += w;
+            diff &= lo ? (1ULL << lo) - 1 : 0ULL;
+        }
+    }
+    return true;
+}
+
+// keys[i] = read i's packed key, perm[i] = i
+__global__ void k_pack_names(const uint64_t *__restrict__ addr, const uint32_t *__restrict__ len, uint64_t n, NameBits nb,
+                             uint64_t *__restrict__ keys, uint32_t *__restrict__ perm) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const char *nm = at(addr[i]);
+    const uint32_t l = len[i];
+    uint64_t key = 0, k = 0;
+    uint32_t have = ~0u;
+    for (uint32_t q = 0; q < nb.n; q++) {
+        if (nb.chunk[q] != have) {
+            have = nb.chunk[q];
+            k = name_chunk(nm, l, have);
+        }
+        const uint32_t w = nb.width[q];
+        const uint64_t part = k >> nb.shift[q];
+        key = w == 64 ? part : (key << w) | (part & ((1ULL << w) - 1));
+    }
+    keys[i] = key;
+    perm[i] = (uint32_t)i;
 }
 
 __global__ void k_iota(uint32_t *__restrict__ p, uint64_t n) {
@@ -452,13 +553,17 @@ __device__ bool sn_core_eq(const SNames &A, uint64_t i, const SNames &B, uint64_
     return true;
 }
 
-// chunk k's start: (k*C, number of right names below left name k*C); chunk 0 at (0, 0)
-__global__ void k_merge_starts(SNames L, uint64_t nL, SNames R, uint64_t nR, uint64_t nchunks,
-                               uint64_t *__restrict__ jstart) {
+// chunk k's start: the left row i = k*C, moved on while its core name is the
+// one before's (the walk pairs one of them only, so it does not stand between
+// them), and the number of right names below left name i; chunk 0 at (0, 0)
+__global__ void k_merge_starts(SNames L, uint64_t nL, SNames R, uint64_t nR, uint64_t nchunks, uint32_t chunk,
+                               uint64_t *__restrict__ istart, uint64_t *__restrict__ jstart) {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nchunks) return;
-    if (k == 0) { jstart[0] = 0; return; }
-    const uint64_t i = k * MG_CHUNK;
+    if (k == 0) { istart[0] = jstart[0] = 0; return; }
+    uint64_t i = k * chunk;
+    for (uint32_t q = 0; q < MG_SHIFT && i + 1 < nL && sn_core_eq(L, i, L, i - 1); q++) i++;
+    istart[k] = i;
     uint64_t lo = 0, hi = nR;
     while (lo < hi) {
         const uint64_t mid = (lo + hi) >> 1;
@@ -476,17 +581,18 @@ __device__ __forceinline__ bool merge_step(const SNames &L, const SNames &R, uin
     return false;
 }
 
-__global__ void k_merge_run(SNames L, uint64_t nL, SNames R, uint64_t nR, uint64_t nchunks,
-                            const uint64_t *__restrict__ jstart, uint2 *__restrict__ slots,
+__global__ void k_merge_run(SNames L, uint64_t nL, SNames R, uint64_t nR, uint64_t nchunks, uint32_t chunk,
+                            const uint64_t *__restrict__ istart, const uint64_t *__restrict__ jstart, uint2 *__restrict__ slots,
                             uint32_t *__restrict__ cnt, uint8_t *__restrict__ status) {
     const uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= nchunks) return;
     const bool last = k + 1 == nchunks;
-    const uint64_t ti = last ? nL : (k + 1) * MG_CHUNK, tj = last ? nR : jstart[k + 1];
-    uint64_t i = k * MG_CHUNK, j = jstart[k];
+    const uint64_t ti = last ? nL : istart[k + 1], tj = last ? nR : jstart[k + 1];
+    uint64_t i = istart[k], j = jstart[k];
     uint32_t c = 0;
     uint8_t st = MG_END;
-    uint2 *out = slots + k * (MG_CHUNK + 1);
+    const uint32_t room = chunk + MG_SHIFT;   // left rows of a chunk at most
+    uint2 *out = slots + k * (room + 1);
     while (i < nL && j < nR) {
         if (!last) {
             if (i == ti && j == tj) { st = MG_REACHED; break; }
@@ -494,11 +600,11 @@ __global__ void k_merge_run(SNames L, uint64_t nL, SNames R, uint64_t nR, uint64
         }
         const uint64_t i0 = i, j0 = j;
         if (merge_step(L, R, i, j)) {
-            if (c <= MG_CHUNK) out[c] = make_uint2((uint32_t)i0, (uint32_t)j0);
+            if (c <= room) out[c] = make_uint2((uint32_t)i0, (uint32_t)j0);
             c++;
         }
     }
-    if (c > MG_CHUNK + 1) st = MG_FAIL;
+    if (c > room + 1) st = MG_FAIL;
     cnt[k] = c;
     status[k] = st;
 }
@@ -522,12 +628,12 @@ __global__ void k_merge_repair(SNames L, uint64_t nL, SNames R, uint64_t nR, uin
 }
 
 __global__ void k_merge_compact(const uint2 *__restrict__ slots, const uint32_t *__restrict__ cnt,
-                                const uint64_t *__restrict__ offs, uint64_t nvalid, uint32_t *__restrict__ row_l,
-                                uint32_t *__restrict__ row_r) {
+                                const uint64_t *__restrict__ offs, uint64_t nvalid, uint32_t room,
+                                uint32_t *__restrict__ row_l, uint32_t *__restrict__ row_r) {
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    const uint64_t k = t / (MG_CHUNK + 1), s = t % (MG_CHUNK + 1);
+    const uint64_t k = t / (room + 1), s = t % (room + 1);
     if (k >= nvalid || s >= cnt[k]) return;
-    const uint2 p = slots[k * (MG_CHUNK + 1) + s];
+    const uint2 p = slots[k * (room + 1) + s];
     row_l[offs[k] + s] = p.x;
     row_r[offs[k] + s] = p.y;
 }
@@ -1147,16 +1253,21 @@ static int sort_side(tk_ctx *c, NormSide &s) {
     TK_TRY(sc.get((void **)&keys, n * 8, "sort keys"));
     TK_TRY(sc.get((void **)&tkeys, n * 8, "sort keys"));
     TK_TRY(sc.get((void **)&tperm, n * 4, "sort order"));
+    NameStats *d_stats = nullptr, stats;
     TK_TRY(sc.get((void **)&d_u32, 16, "sort scalars"));
+    TK_TRY(sc.get((void **)&d_stats, sizeof(NameStats), "name statistics"));
     TK_TRY(sc.get((void **)&orand, 16, "sort key bits"));
     TK_CUDA(c, cudaMemsetAsync(tperm, 0, n * 4, c->stream));   // whatever a sort leaves there indexes a read
-    TK_CUDA(c, cudaMemsetAsync(d_u32, 0, 16, c->stream));
-    k_name_maxlen<<<(unsigned)std::min<uint64_t>(nm_grid(n), (uint64_t)c->sm_count * 8), NM_THREADS, 0, c->stream>>>(
-        s.nlen, n, d_u32);
+    TK_CUDA(c, cudaMemsetAsync(tperm, 0, n * 4, c->stream));   // whatever a sort leaves there indexes a read
+    TK_CUDA(c, cudaMemsetAsync(d_stats, 0, sizeof(NameStats), c->stream));
+    TK_CUDA(c, cudaMemsetAsync(d_stats->all, 0xFF, sizeof stats.all, c->stream));
+    k_name_stats<<<(unsigned)std::min<uint64_t>(nm_grid(n), (uint64_t)c->sm_count * 8), NM_THREADS, 0, c->stream>>>(
+        s.addr, s.nlen, n, d_stats);
     c->launches++;
-    uint32_t maxlen = 0;
-    TK_CUDA(c, cudaMemcpyAsync(&maxlen, d_u32, 4, cudaMemcpyDeviceToHost, c->stream));
+    TK_TRY(check_launch(c, "name statistics"));
+    TK_CUDA(c, cudaMemcpyAsync(&stats, d_stats, sizeof stats, cudaMemcpyDeviceToHost, c->stream));
     TK_CUDA(c, cudaStreamSynchronize(c->stream));
+    const uint32_t maxlen = stats.max_len;
     const uint32_t nch = std::max<uint32_t>(1, (maxlen + 7) / 8);
     uint32_t *perm = s.perm;
     auto pass = [&](int mode, uint32_t ch) -> int {
@@ -1183,8 +1294,24 @@ static int sort_side(tk_ctx *c, NormSide &s) {
         k_iota<<<nm_grid(n), NM_THREADS, 0, c->stream>>>(perm, n);
         c->launches++;
     };
-    iota();
-    for (int ch = (int)nch - 1; ch >= 0; ch--) TK_TRY(pass(0, (uint32_t)ch));
+    NameBits nb;
+    if (nch <= NAME_CHUNKS && name_bits(stats, nch, &nb)) {
+        // one key of the bits that differ: 2M names of ten digits take one sort of
+        // 4 passes instead of two of 7 in all, and no gather of name bytes in
+        // sorted order between them
+        k_pack_names<<<nm_grid(n), NM_THREADS, 0, c->stream>>>(s.addr, s.nlen, n, nb, keys, perm);
+        c->launches++;
+        TK_TRY(check_launch(c, "name keys"));
+        bool in_tmp = false;
+        TK_TRY(radix_sort_pairs(c, keys, perm, n, (int)nb.bits, tkeys, tperm, &in_tmp));
+        if (in_tmp) {
+            std::swap(keys, tkeys);
+            std::swap(perm, tperm);
+        }
+    } else {
+        iota();
+        for (int ch = (int)nch - 1; ch >= 0; ch--) TK_TRY(pass(0, (uint32_t)ch));
+    }
     auto gather = [&]() -> int {
         k_sorted_names<<<nm_grid(n), NM_THREADS, 0, c->stream>>>(s.addr, s.nlen, perm, n, s.h0, s.h1, s.off, s.len,
                                                                   s.core);
@@ -1236,21 +1363,24 @@ static int merge_sides(tk_norm *nm) {
     nm->n_rows = 0;
     if (!nL || !nR) return TK_OK;
     const SNames L = snames(A), R = snames(B);
-    const uint64_t nchunks = (nL + MG_CHUNK - 1) / MG_CHUNK;
+    const uint32_t chunk = merge_chunk(nL);
+    const uint64_t nchunks = (nL + chunk - 1) / chunk;
     Scratch sc(c);
-    uint64_t *jstart = nullptr, *offs = nullptr;
+    uint64_t *istart = nullptr, *jstart = nullptr, *offs = nullptr;
+    const uint32_t room = chunk + MG_SHIFT;
     uint2 *slots = nullptr, *rep = nullptr;
     uint32_t *cnt = nullptr;
     uint8_t *status = nullptr;
     unsigned long long *d_first = nullptr;
+    TK_TRY(sc.get((void **)&istart, (nchunks + 1) * 8, "merge starts"));
     TK_TRY(sc.get((void **)&jstart, (nchunks + 1) * 8, "merge starts"));
-    TK_TRY(sc.get((void **)&slots, nchunks * (MG_CHUNK + 1) * sizeof(uint2), "merge rows"));
+    TK_TRY(sc.get((void **)&slots, nchunks * (room + 1) * sizeof(uint2), "merge rows"));
     TK_TRY(sc.get((void **)&cnt, nchunks * 4, "merge counts"));
     TK_TRY(sc.get((void **)&status, nchunks, "merge status"));
     TK_TRY(sc.get((void **)&d_first, 16, "merge first"));
-    k_merge_starts<<<nm_grid(nchunks), NM_THREADS, 0, c->stream>>>(L, nL, R, nR, nchunks, jstart);
+    k_merge_starts<<<nm_grid(nchunks), NM_THREADS, 0, c->stream>>>(L, nL, R, nR, nchunks, chunk, istart, jstart);
     c->launches++;
-    k_merge_run<<<nm_grid(nchunks, 128), 128, 0, c->stream>>>(L, nL, R, nR, nchunks, jstart, slots, cnt, status);
+    k_merge_run<<<nm_grid(nchunks, 128), 128, 0, c->stream>>>(L, nL, R, nR, nchunks, chunk, istart, jstart, slots, cnt, status);
     c->launches++;
     TK_TRY(check_launch(c, "merge"));
     const unsigned long long none = nchunks;
@@ -1263,7 +1393,8 @@ static int merge_sides(tk_norm *nm) {
     TK_CUDA(c, cudaStreamSynchronize(c->stream));
     if (first >= nchunks) return set_err(c, TK_E_INVAL, "pair merge: no chunk ends the walk");   // the last one always does
     TK_CUDA(c, cudaMemcpyAsync(&st, status + first, 1, cudaMemcpyDeviceToHost, c->stream));
-    uint64_t j_first = 0;
+    uint64_t i_first = 0, j_first = 0;
+    TK_CUDA(c, cudaMemcpyAsync(&i_first, istart + first, 8, cudaMemcpyDeviceToHost, c->stream));
     TK_CUDA(c, cudaMemcpyAsync(&j_first, jstart + first, 8, cudaMemcpyDeviceToHost, c->stream));
     TK_CUDA(c, cudaStreamSynchronize(c->stream));
     const uint64_t nvalid = st == MG_END ? first + 1 : first;
@@ -1272,7 +1403,7 @@ static int merge_sides(tk_norm *nm) {
     if (nvalid) TK_TRY(scan_excl_u32_to_u64(c, cnt, offs, nvalid, &n_main));
     unsigned long long n_rep = 0;
     if (st == MG_FAIL) {
-        const uint64_t i0 = first * MG_CHUNK;
+        const uint64_t i0 = i_first;
         const uint64_t cap = std::min(nL - i0, nR - std::min(nR, j_first)) + 1;
         unsigned long long *d_nrep = d_first + 1;
         TK_TRY(sc.get((void **)&rep, cap * sizeof(uint2), "merge repair rows"));
@@ -1286,7 +1417,7 @@ static int merge_sides(tk_norm *nm) {
     TK_TRY(dmalloc(c, (void **)&nm->row_l, nm->n_rows * 4 + 4, "merged rows"));
     TK_TRY(dmalloc(c, (void **)&nm->row_r, nm->n_rows * 4 + 4, "merged rows"));
     if (nvalid) {
-        k_merge_compact<<<nm_grid(nvalid * (MG_CHUNK + 1)), NM_THREADS, 0, c->stream>>>(slots, cnt, offs, nvalid,
+        k_merge_compact<<<nm_grid(nvalid * (room + 1)), NM_THREADS, 0, c->stream>>>(slots, cnt, offs, nvalid, room,
                                                                                         nm->row_l, nm->row_r);
         c->launches++;
     }
