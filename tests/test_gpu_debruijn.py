@@ -53,6 +53,22 @@ def test_edge_records(ctx, oracle, golden):
             assert gpu_text(ctx, b, K, ss) == oracle.debruijn(b, K, ss), (K, ss)
 
 
+@pytest.mark.parametrize("lo,hi,n", [(0, 40, 3000), (250, 262, 200), (8000, 20000, 3)])
+def test_record_sizes_around_a_block(ctx, oracle, lo, hi, n):
+    """Many records in the positions one block takes, records of about a block, and records of many blocks; each
+    with a stretch repeated inside it and shared with the record before."""
+    rnd = np.random.default_rng(hi)
+    recs, last = [], b""
+    for i in range(n):
+        s = rnd.choice(np.frombuffer(b"ACGTN" if i % 5 == 0 else b"ACGT", dtype=np.uint8), rnd.integers(lo, hi)).tobytes()
+        s = s[:len(s) // 2] + last[:30] + s[len(s) // 2:] + s[:30]
+        last = s
+        recs.append(b">s_%d\n%s\n" % (i, s))
+    b = b"".join(recs)
+    for ss in (False, True):
+        assert gpu_text(ctx, b, 24, ss) == oracle.debruijn(b, 24, ss)
+
+
 def test_empty_inputs(ctx, oracle):
     for b in (b"", b">s_1\n\n", b">s_1\nACGT\n>s_2\nNNNNNNNNNNNNNNNNNNNNNNNNNNNNNN\n"):
         assert gpu_text(ctx, b, 24) == oracle.debruijn(b, 24, False) == b""

@@ -11,17 +11,23 @@
 // then "<node>\t<prev>\t<count>\t<kmer>" per node; a record without any
 // window is left out.
 //
-// GPU plan, all over the record-concatenated bundle read set:
-//  1. one thread per position: the window starting there, cut from the 2-bit
-//     codes with its validity; the valid ones compacted (key, position);
-//  2. stable radix sorts by key, then by record: equal (record, key) runs
-//     with ascending positions, so a run's head is the node's first occurrence
-//     and its length the count; every window position is mapped to its node;
-//  3. nodes radix-sorted by first position = record order, then order of first
-//     occurrence; node id = rank - the record's first rank; prev through the
-//     position map of the window before;
-//  4. line lengths, a scan, and one thread per line writing it.
+// GPU plan, all over the record-concatenated bundle read set, a thread per
+// window end position throughout:
+//  1. every record gets a slice of a hash table (a power of two, at least 1.5
+//     times its bases); each window is inserted into its record's slice, which
+//     keeps its count and the first position it ends at, and the position
+//     keeps the slot;
+//  2. a position is a node when its slot's first position is its own: a bit per
+//     position, and the nodes in the 32 positions of every word scanned;
+//     node id = nodes before the position - nodes before the record;
+//  3. prev through the slot of the window before; line lengths, a scan, and one
+//     thread per line writing it.
+// Neighbouring threads work on neighbouring positions, so the slices in use at
+// any time are those of a short stretch of the bundle and stay in L2.  (Three
+// radix sorts -- by k-mer, by record, by first position -- and the passes that
+// joined their results took 3.0 of the 4.5 ms of 30,000 contigs.)
 #include "tk_emit.cuh"
+#include "tk_warp.cuh"
 
 #include <algorithm>
 #include <vector>
@@ -48,102 +54,90 @@ __device__ __forceinline__ char *dbg_put_dec(char *o, uint64_t v) {
     return o + n;
 }
 
-// record holding position p: the largest r with rd_off[r] <= p
-__device__ __forceinline__ uint32_t dbg_record_of(const uint64_t *__restrict__ rd_off, uint64_t n_rec, uint64_t p) {
-    uint64_t lo = 0, hi = n_rec;
-    while (hi - lo > 1) {
-        const uint64_t mid = (lo + hi) >> 1;
-        if (__ldg(rd_off + mid) <= p) lo = mid;
-        else hi = mid;
+constexpr int DBG_THREADS = 256;
+
+// The record holding this thread's position p: the record of the block's first
+// position is searched once, and the threads walk on from it.
+__device__ __forceinline__ uint32_t dbg_record(const uint64_t *__restrict__ rd_off, uint64_t n_rec, uint64_t p) {
+    __shared__ uint32_t s_rec;
+    if (threadIdx.x == 0) {
+        uint64_t lo = 0, hi = n_rec;   // the largest r with rd_off[r] <= p
+        while (hi - lo > 1) {
+            const uint64_t mid = (lo + hi) >> 1;
+            if (rd_off[mid] <= p) lo = mid;
+            else hi = mid;
+        }
+        s_rec = (uint32_t)lo;
     }
-    return (uint32_t)lo;
+    __syncthreads();
+    uint32_t r = s_rec;
+    while (r + 1 < n_rec && __ldg(rd_off + r + 1) <= p) r++;
+    return r;
 }
 
-// 1. window starting at p (positions p .. p+k1-1) from the code pair holding its end
+// 1. slots of each record's slice
+__global__ void k_dbg_slices(const uint64_t *__restrict__ rd_off, uint64_t n_rec, uint64_t *__restrict__ size) {
+    const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n_rec) return;
+    const uint64_t bases = rd_off[r + 1] - rd_off[r] - 1;
+    uint64_t s = 32;
+    while (2 * s < 3 * bases) s <<= 1;
+    size[r] = s;
+}
+
 template <bool CANON>
-__global__ void k_dbg_windows(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv, uint64_t n_pos,
-                              int k1, uint32_t *__restrict__ valid, uint64_t *__restrict__ keys) {
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_pos) return;
-    const uint64_t e = p + (uint64_t)k1 - 1;
-    const int64_t q = (int64_t)(e >> 5);
-    const int i = (int)(e & 31);
-    const uint64_t hi = __ldg(codes + q - 1), lo = __ldg(codes + q);
-    const uint64_t m = ((uint64_t)__ldg(inv + q - 1) << 32) | __ldg(inv + q);
-    const bool ok = ((m >> (31 - i)) & ((1ULL << k1) - 1)) == 0;
-    const int s = 62 - 2 * i;
-    const uint64_t fw = (s ? ((lo >> s) | (hi << (64 - s))) : lo) & ((1ULL << (2 * k1)) - 1);
-    uint64_t key = fw;
-    if (CANON) {
-        uint64_t x = __brevll(~fw);
-        x = ((x >> 1) & 0x5555555555555555ULL) | ((x & 0x5555555555555555ULL) << 1);
-        const uint64_t rc = x >> (64 - 2 * k1);
-        key = rc < fw ? rc : fw;
-    }
-    valid[p] = ok ? 1u : 0u;
-    keys[p] = key;
-}
-
-__global__ void k_dbg_compact(const uint32_t *__restrict__ valid, const uint64_t *__restrict__ keys,
-                              const uint64_t *__restrict__ off, uint64_t n_pos, uint64_t *__restrict__ okeys,
-                              uint32_t *__restrict__ opos) {
-    const uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n_pos || !valid[p]) return;
-    okeys[off[p]] = keys[p];
-    opos[off[p]] = (uint32_t)p;
-}
-
-// record of every (key-sorted) window, as the key of the second sort; the value
-// is the window's index in the key order
-__global__ void k_dbg_rec_keys(const uint32_t *__restrict__ pos, uint64_t n, const uint64_t *__restrict__ rd_off,
-                               uint64_t n_rec, uint64_t *__restrict__ rec, uint32_t *__restrict__ idx) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    rec[j] = dbg_record_of(rd_off, n_rec, pos[j]);
-    idx[j] = (uint32_t)j;
-}
-
-// 2. windows in (record, key, position) order: run heads, and the position map
-__global__ void k_dbg_heads(const uint64_t *__restrict__ rec, const uint32_t *__restrict__ idx,
-                            const uint64_t *__restrict__ keys, uint64_t n, uint32_t *__restrict__ head) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    head[j] = (j == 0 || rec[j] != rec[j - 1] || keys[idx[j]] != keys[idx[j - 1]]) ? 1u : 0u;
-}
-
-__global__ void k_dbg_nodes(const uint32_t *__restrict__ head, const uint64_t *__restrict__ hoff,
-                            const uint32_t *__restrict__ idx, const uint32_t *__restrict__ pos, uint64_t n,
-                            uint64_t n_nodes, uint32_t *__restrict__ node_start, uint64_t *__restrict__ node_first,
-                            uint32_t *__restrict__ node_g, uint32_t *__restrict__ pos_node) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j > n) return;
-    if (j == n) {
-        node_start[n_nodes] = (uint32_t)n;
+__global__ void __launch_bounds__(DBG_THREADS) k_dbg_insert(const uint64_t *__restrict__ codes,
+                                                            const uint32_t *__restrict__ inv, uint64_t n_pos, int k1,
+                                                            const uint64_t *__restrict__ rd_off, uint64_t n_rec,
+                                                            const uint64_t *__restrict__ base,
+                                                            const uint64_t *__restrict__ size, Slot *__restrict__ slots,
+                                                            uint32_t *__restrict__ slot_of) {
+    const uint64_t e = (uint64_t)blockIdx.x * DBG_THREADS + threadIdx.x;
+    const uint32_t r = dbg_record(rd_off, n_rec, e);
+    if (e >= n_pos) return;
+    uint64_t key;
+    if (!window_at<CANON>(codes, inv, e, k1, key)) {
+        slot_of[e] = NO_NODE;
         return;
     }
-    const uint32_t g = (uint32_t)(hoff[j] + head[j] - 1);
-    const uint32_t p = pos[idx[j]];
-    if (head[j]) {
-        node_start[g] = (uint32_t)j;
-        node_first[g] = p;
-        node_g[g] = g;
+    Slot *t = slots + base[r];
+    const uint32_t mask = (uint32_t)(size[r] - 1);
+    uint32_t s = (uint32_t)mix64(key) & mask;
+    const uint64_t mine = e << 32 | 1u;   // first position, count (the slice has room for every window of its record)
+    for (;; s = (s + 1) & mask) {
+        if (s == NO_NODE) continue;   // no position can name that slot
+        const ulonglong2 was = slot_claim(t + s, 0, key, mine);
+        if (was.x == EMPTY_KEY) break;
+        if (was.x == key) {
+            atomicAdd(&t[s].val, 1u);
+            if ((uint32_t)(was.y >> 32) > (uint32_t)e) atomicMin(&t[s].pad, (uint32_t)e);
+            break;
+        }
     }
-    pos_node[p] = g;
+    slot_of[e] = s;
 }
 
-// 3. per rank (nodes in first-position order): the rank of each node, and the
-// first rank of each record that has nodes
-__global__ void k_dbg_ranks(const uint64_t *__restrict__ first, const uint32_t *__restrict__ g_of, uint64_t n_nodes,
-                            const uint64_t *__restrict__ rd_off, uint64_t n_rec, uint32_t *__restrict__ rank_of,
-                            uint32_t *__restrict__ rec_first, unsigned long long *__restrict__ n_comp) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_nodes) return;
-    rank_of[g_of[j]] = (uint32_t)j;
-    const uint32_t r = dbg_record_of(rd_off, n_rec, first[j]);
-    if (j == 0 || dbg_record_of(rd_off, n_rec, first[j - 1]) != r) {
-        rec_first[r] = (uint32_t)j;
-        atomicAdd(n_comp, 1ULL);
+// 2. a bit per position (bit i of word j: position 32j + i) that is a node, and the nodes of each word
+__global__ void __launch_bounds__(DBG_THREADS) k_dbg_heads(uint64_t n_pos, const uint64_t *__restrict__ rd_off,
+                                                           uint64_t n_rec, const uint64_t *__restrict__ base,
+                                                           const Slot *__restrict__ slots,
+                                                           const uint32_t *__restrict__ slot_of,
+                                                           uint32_t *__restrict__ head, uint32_t *__restrict__ heads) {
+    const uint64_t e = (uint64_t)blockIdx.x * DBG_THREADS + threadIdx.x;
+    const uint32_t r = dbg_record(rd_off, n_rec, e);
+    const uint32_t s = e < n_pos ? slot_of[e] : NO_NODE;
+    const bool node = s != NO_NODE && slots[base[r] + s].pad == (uint32_t)e;
+    const uint32_t bits = __ballot_sync(0xffffffffu, node);
+    if (lane_id() == 0 && e < n_pos) {
+        head[e >> 5] = bits;
+        heads[e >> 5] = __popc(bits);
     }
+}
+
+// the nodes ending before position e
+__device__ __forceinline__ uint32_t dbg_rank(const uint32_t *__restrict__ head, const uint64_t *__restrict__ before,
+                                             uint64_t e) {
+    return (uint32_t)before[e >> 5] + __popc(head[e >> 5] & ((1u << (e & 31)) - 1u));
 }
 
 struct DbgLine {
@@ -153,30 +147,38 @@ struct DbgLine {
     uint32_t rec;      // record index; header line before the record's first node
 };
 
-__global__ void k_dbg_lines(const uint64_t *__restrict__ first, const uint32_t *__restrict__ g_of, uint64_t n_nodes,
-                            const uint64_t *__restrict__ rd_off, uint64_t n_rec,
-                            const uint32_t *__restrict__ rank_of, const uint32_t *__restrict__ rec_first,
-                            const uint32_t *__restrict__ node_start, const uint32_t *__restrict__ pos_node,
-                            const uint64_t *__restrict__ comp, int k1, DbgLine *__restrict__ line,
-                            uint64_t *__restrict__ len) {
-    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_nodes) return;
-    const uint64_t p = first[j];
-    const uint32_t g = g_of[j];
-    const uint32_t r = dbg_record_of(rd_off, n_rec, p);
-    const uint32_t r0 = rec_first[r];
+// 3. every node's line (in position order), its window's first position and its text length
+__global__ void __launch_bounds__(DBG_THREADS) k_dbg_lines(uint64_t n_pos, const uint64_t *__restrict__ rd_off,
+                                                           uint64_t n_rec, const uint64_t *__restrict__ base,
+                                                           const Slot *__restrict__ slots,
+                                                           const uint32_t *__restrict__ slot_of,
+                                                           const uint32_t *__restrict__ head,
+                                                           const uint64_t *__restrict__ before,
+                                                           const uint64_t *__restrict__ comp, int k1,
+                                                           DbgLine *__restrict__ line, uint64_t *__restrict__ first,
+                                                           uint32_t *__restrict__ len,
+                                                           unsigned long long *__restrict__ n_comp) {
+    const uint64_t e = (uint64_t)blockIdx.x * DBG_THREADS + threadIdx.x;
+    const uint32_t r = dbg_record(rd_off, n_rec, e);
+    if (e >= n_pos || !((head[e >> 5] >> (e & 31)) & 1u)) return;
+    const Slot *t = slots + base[r];
+    const uint32_t j = dbg_rank(head, before, e), r0 = dbg_rank(head, before, rd_off[r]);
     DbgLine L;
-    L.id = (uint32_t)j - r0;
-    L.count = node_start[g + 1] - node_start[g];
+    L.id = j - r0;
+    L.count = t[slot_of[e]].val;
     L.rec = r;
     // the window just before the first occurrence, when it is a valid window
     // (it then lies in the same contig of the same record)
-    const uint32_t pn = p > 0 ? pos_node[p - 1] : NO_NODE;
-    L.prev = pn == NO_NODE ? -1 : (int32_t)(rank_of[pn] - r0);
+    const uint32_t ps = e > 0 ? slot_of[e - 1] : NO_NODE;
+    L.prev = ps == NO_NODE ? -1 : (int32_t)(dbg_rank(head, before, t[ps].pad) - r0);
     line[j] = L;
-    uint64_t n = dbg_dec_len(L.id) + 1 + (L.prev < 0 ? 2 : dbg_dec_len((uint32_t)L.prev)) + 1 + dbg_dec_len(L.count) + 1 +
-                 (uint64_t)k1 + 1;
-    if (L.id == 0) n += 10 + dbg_dec_len(comp[r]) + 1;   // "Component " id "\n"
+    first[j] = e - (uint64_t)k1 + 1;
+    uint32_t n = dec_digits(L.id) + 1 + (L.prev < 0 ? 2 : dec_digits((uint32_t)L.prev)) + 1 + dec_digits(L.count) + 1 +
+                 (uint32_t)k1 + 1;
+    if (L.id == 0) {
+        n += 10 + dbg_dec_len(comp[r]) + 1;   // "Component " id "\n"
+        atomicAdd(n_comp, 1ULL);
+    }
     len[j] = n;
 }
 
@@ -185,7 +187,6 @@ __global__ void k_dbg_lines(const uint64_t *__restrict__ first, const uint32_t *
 // its line's bytes one by one took 2.24 ms).  The k-mer comes from the codes: a
 // window holds A/C/G/T only, in upper case in the read array.
 constexpr int DBG_LINE = 10 + 1 + 11 + 1 + 10 + 1 + MAX_K + 1;
-constexpr int DBG_THREADS = 256;
 constexpr int DBG_BYTES = (DBG_THREADS * (DBG_LINE + 10 + 20 + 1) + 16 + 15) & ~15;
 
 __global__ void __launch_bounds__(DBG_THREADS) k_dbg_write(const DbgLine *__restrict__ line,
@@ -255,107 +256,55 @@ int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id
     DbgScratch sc(c);
     cudaEvent_t ev;
     prof_begin(c, TK_KID_DBG, &ev);
-    // 1. windows, compacted
-    uint32_t *valid = nullptr;
-    uint64_t *keys = nullptr, *off = nullptr;
-    TK_TRY(sc.get((void **)&valid, n_pos * 4, "window flags"));
-    TK_TRY(sc.get((void **)&keys, n_pos * 8, "window keys"));
-    TK_TRY(sc.get((void **)&off, (n_pos + 1) * 8, "window offsets"));
-    const uint64_t n_win_pos = n_pos - (uint64_t)k1 + 1;   // window starts whose window ends inside the set
-    if (g->strand)
-        k_dbg_windows<false><<<dbg_grid(n_win_pos, 256), 256, 0, c->stream>>>(b->d_codes, b->d_inv, n_win_pos, k1,
-                                                                             valid, keys);
-    else
-        k_dbg_windows<true><<<dbg_grid(n_win_pos, 256), 256, 0, c->stream>>>(b->d_codes, b->d_inv, n_win_pos, k1,
-                                                                            valid, keys);
+    if (n_pos >= NO_NODE) return set_err(c, TK_E_RANGE, "FastaToDeBruijn: a bundle of 2^32 - 1 bytes or more");
+    const uint64_t n_words = (n_pos + 31) / 32;
+    uint32_t *slot_of = nullptr, *head = nullptr, *heads = nullptr;
+    uint64_t *size = nullptr, *base = nullptr, *before = nullptr, n_slots = 0, G = 0;
+    Slot *slots = nullptr;
+    TK_TRY(sc.get((void **)&size, n_rec * 8, "slice sizes"));
+    TK_TRY(sc.get((void **)&base, n_rec * 8, "slice starts"));
+    k_dbg_slices<<<dbg_grid(n_rec, 256), 256, 0, c->stream>>>(b->d_rd_off, n_rec, size);
     c->launches++;
+    TK_TRY(scan_excl_u64(c, size, base, n_rec, &n_slots));
+    TK_TRY(sc.get((void **)&slots, n_slots * sizeof(Slot), "k-mer slices"));
+    TK_TRY(sc.get((void **)&slot_of, n_pos * 4, "window slots"));
+    TK_TRY(sc.get((void **)&head, n_words * 4, "node bits"));
+    TK_TRY(sc.get((void **)&heads, n_words * 4, "nodes per word"));
+    TK_TRY(sc.get((void **)&before, n_words * 8, "nodes before"));
+    table_fill_empty(c, slots, n_slots, 0);
+    const unsigned grid = dbg_grid(n_pos, DBG_THREADS);
+    if (g->strand)
+        k_dbg_insert<false><<<grid, DBG_THREADS, 0, c->stream>>>(b->d_codes, b->d_inv, n_pos, k1, b->d_rd_off, n_rec, base,
+                                                                 size, slots, slot_of);
+    else
+        k_dbg_insert<true><<<grid, DBG_THREADS, 0, c->stream>>>(b->d_codes, b->d_inv, n_pos, k1, b->d_rd_off, n_rec, base,
+                                                                size, slots, slot_of);
+    k_dbg_heads<<<grid, DBG_THREADS, 0, c->stream>>>(n_pos, b->d_rd_off, n_rec, base, slots, slot_of, head, heads);
+    c->launches += 2;
     TK_TRY(check_launch(c, "de Bruijn windows"));
-    uint64_t M = 0;
-    TK_TRY(scan_excl_u32_to_u64(c, valid, off, n_win_pos, &M));
-    if (M == 0) {
+    TK_TRY(scan_excl_u32_to_u64(c, heads, before, n_words, &G));
+    if (G == 0) {
         prof_end(c, TK_KID_DBG, ev, 0);
         return TK_OK;
     }
-    if (M >= NO_NODE) return set_err(c, TK_E_RANGE, "FastaToDeBruijn: more than 2^32 - 1 windows in one bundle");
-    uint64_t *wk = nullptr, *wk2 = nullptr;
-    uint32_t *wp = nullptr, *wp2 = nullptr;
-    TK_TRY(sc.get((void **)&wk, M * 8, "windows"));
-    TK_TRY(sc.get((void **)&wk2, M * 8, "windows (sort)"));
-    TK_TRY(sc.get((void **)&wp, M * 4, "window positions"));
-    TK_TRY(sc.get((void **)&wp2, M * 4, "window positions (sort)"));
-    k_dbg_compact<<<dbg_grid(n_win_pos, 256), 256, 0, c->stream>>>(valid, keys, off, n_win_pos, wk, wp);
-    c->launches++;
-    TK_TRY(check_launch(c, "de Bruijn compact"));
-    // 2. by key, then by record (both stable: positions stay ascending)
-    bool in_tmp = false;
-    TK_TRY(radix_sort_pairs(c, wk, wp, M, 2 * k1, wk2, wp2, &in_tmp));
-    uint64_t *sk = in_tmp ? wk2 : wk;
-    uint32_t *sp = in_tmp ? wp2 : wp;
-    uint64_t *rec = keys, *rec2 = off;   // reuse: n_pos >= M
-    uint32_t *idx = valid, *idx2 = in_tmp ? wp : wp2;
-    k_dbg_rec_keys<<<dbg_grid(M, 256), 256, 0, c->stream>>>(sp, M, b->d_rd_off, n_rec, rec, idx);
-    c->launches++;
-    TK_TRY(check_launch(c, "de Bruijn records"));
-    int rbits = 1;
-    while ((1ULL << rbits) < n_rec) rbits++;
-    TK_TRY(radix_sort_pairs(c, rec, idx, M, rbits, rec2, idx2, &in_tmp));
-    TK_CUDA(c, cudaStreamSynchronize(c->stream));
-    TK_TRY(wait_status(c));   // the sorted values index arrays below
-    const uint64_t *srec = in_tmp ? rec2 : rec;
-    const uint32_t *sidx = in_tmp ? idx2 : idx;
-    uint32_t *head = nullptr;
-    uint64_t *hoff = nullptr;
-    TK_TRY(sc.get((void **)&head, M * 4, "node heads"));
-    TK_TRY(sc.get((void **)&hoff, (M + 1) * 8, "node offsets"));
-    k_dbg_heads<<<dbg_grid(M, 256), 256, 0, c->stream>>>(srec, sidx, sk, M, head);
-    c->launches++;
-    TK_TRY(check_launch(c, "de Bruijn heads"));
-    uint64_t G = 0;
-    TK_TRY(scan_excl_u32_to_u64(c, head, hoff, M, &G));
-    uint32_t *node_start = nullptr, *node_g = nullptr, *node_g2 = nullptr, *pos_node = nullptr;
-    uint64_t *node_first = nullptr, *node_first2 = nullptr;
-    TK_TRY(sc.get((void **)&node_start, (G + 1) * 4, "node starts"));
-    TK_TRY(sc.get((void **)&node_first, G * 8, "node first positions"));
-    TK_TRY(sc.get((void **)&node_first2, G * 8, "node first positions (sort)"));
-    TK_TRY(sc.get((void **)&node_g, G * 4, "node ids"));
-    TK_TRY(sc.get((void **)&node_g2, G * 4, "node ids (sort)"));
-    TK_TRY(sc.get((void **)&pos_node, n_pos * 4, "position map"));
-    TK_CUDA(c, cudaMemsetAsync(pos_node, 0xFF, n_pos * 4, c->stream));
-    k_dbg_nodes<<<dbg_grid(M + 1, 256), 256, 0, c->stream>>>(head, hoff, sidx, sp, M, G, node_start, node_first, node_g,
-                                                            pos_node);
-    c->launches++;
-    TK_TRY(check_launch(c, "de Bruijn nodes"));
-    // 3. nodes in first-position order
-    int pbits = 1;
-    while ((1ULL << pbits) < n_pos) pbits++;
-    TK_TRY(radix_sort_pairs(c, node_first, node_g, G, pbits, node_first2, node_g2, &in_tmp));
-    TK_CUDA(c, cudaStreamSynchronize(c->stream));
-    TK_TRY(wait_status(c));
-    const uint64_t *ofirst = in_tmp ? node_first2 : node_first;
-    const uint32_t *og = in_tmp ? node_g2 : node_g;
-    uint32_t *rank_of = nullptr, *rec_first = nullptr;
-    uint64_t *d_comp = nullptr, *len = nullptr, *loff = nullptr;
+    uint64_t *d_comp = nullptr, *ofirst = nullptr, *loff = nullptr;
+    uint32_t *len = nullptr;
     unsigned long long *d_ncomp = nullptr;
     DbgLine *line = nullptr;
     TK_TRY(sc.get((void **)&d_ncomp, 8, "component count"));
     TK_CUDA(c, cudaMemsetAsync(d_ncomp, 0, 8, c->stream));
-    TK_TRY(sc.get((void **)&rank_of, G * 4, "node ranks"));
-    TK_TRY(sc.get((void **)&rec_first, n_rec * 4, "record first ranks"));
     TK_TRY(sc.get((void **)&d_comp, n_rec * 8, "component ids"));
+    TK_TRY(sc.get((void **)&ofirst, G * 8, "node first positions"));
     TK_TRY(sc.get((void **)&line, G * sizeof(DbgLine), "node lines"));
-    TK_TRY(sc.get((void **)&len, G * 8, "line lengths"));
+    TK_TRY(sc.get((void **)&len, G * 4, "line lengths"));
     TK_TRY(sc.get((void **)&loff, (G + 1) * 8, "line offsets"));
     TK_CUDA(c, cudaMemcpyAsync(d_comp, comp_id.data(), n_rec * 8, cudaMemcpyHostToDevice, c->stream));
-    k_dbg_ranks<<<dbg_grid(G, 256), 256, 0, c->stream>>>(ofirst, og, G, b->d_rd_off, n_rec, rank_of, rec_first,
-                                                         d_ncomp);
-    c->launches++;
-    TK_TRY(check_launch(c, "de Bruijn ranks"));
-    k_dbg_lines<<<dbg_grid(G, 256), 256, 0, c->stream>>>(ofirst, og, G, b->d_rd_off, n_rec, rank_of, rec_first,
-                                                         node_start, pos_node, d_comp, k1, line, len);
+    k_dbg_lines<<<grid, DBG_THREADS, 0, c->stream>>>(n_pos, b->d_rd_off, n_rec, base, slots, slot_of, head, before, d_comp,
+                                                     k1, line, ofirst, len, d_ncomp);
     c->launches++;
     TK_TRY(check_launch(c, "de Bruijn lines"));
     uint64_t total = 0;
-    TK_TRY(scan_excl_u64(c, len, loff, G, &total));
+    TK_TRY(scan_excl_u32_to_u64(c, len, loff, G, &total));
     char *text = nullptr;
     TK_TRY(dmalloc(c, (void **)&text, total + 1, "de Bruijn text"));
     k_dbg_write<<<dbg_grid(G, DBG_THREADS), DBG_THREADS, 0, c->stream>>>(line, ofirst, loff, G, total, d_comp, b->d_codes, k1, text);
@@ -372,11 +321,10 @@ int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id
         dfree(c, text);
         return e;
     }
-    prof_end(c, TK_KID_DBG, ev, M);
+    prof_end(c, TK_KID_DBG, ev, n_pos);
     g->d_text = text;
     g->text_len = total;
     g->n_nodes = G;
-    g->n_windows = M;
     g->n_components = n_comp;
     return TK_OK;
 }

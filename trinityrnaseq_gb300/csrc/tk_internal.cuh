@@ -412,7 +412,7 @@ struct tk_dbg {
     int strand = 0;
     char *d_text = nullptr;
     uint64_t text_len = 0;
-    uint64_t n_records = 0, n_components = 0, n_nodes = 0, n_windows = 0;
+    uint64_t n_records = 0, n_components = 0, n_nodes = 0;
 };
 
 namespace tk {
@@ -485,6 +485,7 @@ int wait_status(tk_ctx *c);
 int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits,
                      uint64_t *tmp_keys, uint32_t *tmp_vals, bool *result_in_tmp, int first_bit = 0);
 int table_alloc(tk_table *t, uint64_t capacity);
+void table_fill_empty(tk_ctx *c, Slot *slots, uint64_t n, uint64_t init_val);
 int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val);
 int table_rehash(tk_table *t, uint64_t new_capacity);
 int table_count_seq(tk_table *t, const tk_reads *r);

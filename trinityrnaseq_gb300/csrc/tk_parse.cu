@@ -18,6 +18,8 @@
 // 4-line record checks of util/support_scripts/fastQ_to_fastA.pl:80-92.
 #include "tk_text.cuh"
 
+#include <algorithm>
+
 namespace tk {
 
 constexpr int PT_THREADS = 256;
@@ -193,20 +195,26 @@ __global__ void k_fastq_records(uint64_t *__restrict__ line_rec, uint64_t n_line
 // loads line l's metadata (coalesced), header lines record their read's start,
 // and then the warp copies the group's sequence lines in aligned 16-byte
 // output words (copy_group), upper-casing into seq.  A sequence line holding
-// whitespace sets *ws_seen and the byte-wise path redoes the emit.
+// whitespace sets *ws_seen and the byte-wise path redoes the emit.  A warp takes
+// `per` lines, fewer than 32 when there are not 32 for every warp the GPU
+// holds: 10,000 bundle records of 1.4 KB kept 625 warps busy at 32 lines each
+// (0.30 ms).
+static uint32_t lines_per_warp(const tk_ctx *c, uint64_t n) {
+    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(32, n / ((uint64_t)c->sm_count * 64)));
+}
 
 __global__ void k_copy_lines(ParseGeom g, const uint64_t *__restrict__ line_end, const uint8_t *__restrict__ kind,
                              const uint64_t *__restrict__ line_rec, const uint64_t *__restrict__ line_out,
-                             uint64_t n_lines, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
+                             uint64_t n_lines, uint32_t per, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
                              uint32_t *__restrict__ ws_seen) {
     const unsigned lane = lane_id();
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     bool ws = false;
-    for (uint64_t j0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; j0 < n_lines; j0 += warps * 32) {
+    for (uint64_t j0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; j0 < n_lines; j0 += warps * per) {
         const uint64_t j = j0 + lane;
         uint64_t src = 0, dst = 0;
         uint32_t len = 0;
-        if (j < n_lines) {
+        if (lane < per && j < n_lines) {
             const uint8_t kd = kind[j];
             const uint64_t rec = line_rec[j];
             if (rec != ~0ULL) {
@@ -244,16 +252,16 @@ __global__ void k_fq_check(ParseGeom g, const uint64_t *__restrict__ line_end, u
 // A warp takes 32 consecutive records: lane l records read r0 + l's start and
 // holds its sequence line, then the warp copies them as k_copy_lines does.
 __global__ void k_fq_copy(ParseGeom g, const uint64_t *__restrict__ line_end, const uint64_t *__restrict__ seq_off,
-                          uint64_t n_reads, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
+                          uint64_t n_reads, uint32_t per, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
                           uint32_t *__restrict__ ws_seen) {
     const unsigned lane = lane_id();
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     bool ws = false;
-    for (uint64_t r0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32; r0 < n_reads; r0 += warps * 32) {
+    for (uint64_t r0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; r0 < n_reads; r0 += warps * per) {
         const uint64_t r = r0 + lane;
         uint64_t src = 0, dst = 0;
         uint32_t len = 0;
-        if (r < n_reads) {
+        if (lane < per && r < n_reads) {
             src = line_end[4 * r] + 1;
             len = (uint32_t)(line_end[4 * r + 1] - src);
             dst = seq_off[r] + r;
@@ -551,17 +559,16 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
         uint32_t ws_seen = 0;
         if (n_tiles && n_reads) {
             cudaMemsetAsync(c->d_err + DE_WS, 0, 4, c->stream);
-            if (fastq) {
-                const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n_reads + 255) / 256,
-                                                                                       (uint64_t)c->sm_count * 32));
-                k_fq_copy<<<grid, 256, 0, c->stream>>>(g, line_end, line_out, n_reads, r->d_seq, r->d_rd_off,
+            const uint64_t n = fastq ? n_reads : n_lines;
+            const uint32_t per = lines_per_warp(c, n);
+            const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 8ull * per - 1) / (8ull * per),
+                                                                                     (uint64_t)c->sm_count * 32));
+            if (fastq)
+                k_fq_copy<<<grid, 256, 0, c->stream>>>(g, line_end, line_out, n_reads, per, r->d_seq, r->d_rd_off,
                                                        c->d_err + DE_WS);
-            } else {
-                const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n_lines + 7) / 8,
-                                                                                       (uint64_t)c->sm_count * 32));
-                k_copy_lines<<<grid, 256, 0, c->stream>>>(g, line_end, kind, line_rec, line_out, n_lines, r->d_seq,
+            else
+                k_copy_lines<<<grid, 256, 0, c->stream>>>(g, line_end, kind, line_rec, line_out, n_lines, per, r->d_seq,
                                                           r->d_rd_off, c->d_err + DE_WS);
-            }
             c->launches++;
             e = cuda_check(c, cudaMemcpyAsync(&ws_seen, c->d_err + DE_WS, 4, cudaMemcpyDeviceToHost, c->stream), "ws flag");
             if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "copy sync");

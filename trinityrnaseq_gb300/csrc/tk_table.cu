@@ -767,6 +767,12 @@ static int table_alloc_geom(tk_table *t, uint64_t capacity, uint64_t init_val, b
     return check_launch(c, "table fill");
 }
 
+// n empty slots whose value words are init_val
+void table_fill_empty(tk_ctx *c, Slot *slots, uint64_t n, uint64_t init_val) {
+    k_fill_empty<<<stream_grid(c, n, 256), 256, 0, c->stream>>>(slots, n, init_val);
+    c->launches++;
+}
+
 int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val) {
     return table_alloc_geom(t, capacity, init_val, true);
 }
