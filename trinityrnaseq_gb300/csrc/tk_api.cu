@@ -14,6 +14,7 @@
 
 namespace tk {
 int parse_reads(tk_ctx *c, tk_reads *r);
+int component_ids(tk_ctx *c, const tk_reads *b, uint64_t *d_ids);
 int table_info(tk_table *t, uint64_t *distinct, uint64_t *total, uint64_t *capacity);
 int table_histo(tk_table *t, uint64_t low, uint64_t high, uint64_t *hist);
 int table_sorted_pairs(tk_table *t, uint32_t min_count, uint64_t **keys, uint32_t **cnt, uint64_t *n);
@@ -989,34 +990,6 @@ int tk_coverage_stats(tk_table *t, const tk_reads *r, int where, uint32_t *media
 
 // ------------------------------------------------------------------ R2T
 
-// Component id of every bundle record: the integer after "s_" in its
-// accession, else the record ordinal.
-static int bundle_component_ids(tk_ctx *c, const tk_reads *b, const char *bundle, uint64_t len, int where,
-                                std::vector<uint64_t> *ids) {
-    ids->assign(b->n_reads, 0);
-    std::vector<uint64_t> off(b->n_reads);
-    std::vector<uint32_t> nl(b->n_reads);
-    TK_TRY(tk_reads_names(b, off.data(), nl.data()));
-    std::vector<char> host_text;
-    const char *ht = bundle;
-    if (where == TK_DEVICE) {
-        host_text.resize(len);
-        TK_CUDA(c, cudaMemcpy(host_text.data(), bundle, len, cudaMemcpyDeviceToHost));
-        ht = host_text.data();
-    }
-    for (uint64_t i = 0; i < b->n_reads; i++) {
-        const char *h = ht + off[i];
-        const uint32_t L = nl[i];
-        uint64_t id = i;
-        if (L > 2 && h[0] == 's' && h[1] == '_' && h[2] >= '0' && h[2] <= '9') {
-            id = 0;
-            for (uint32_t j = 2; j < L && h[j] >= '0' && h[j] <= '9'; j++) id = id * 10 + (uint64_t)(h[j] - '0');
-        }
-        (*ids)[i] = id;
-    }
-    return TK_OK;
-}
-
 int tk_r2t_create(tk_ctx *c, const char *bundle, uint64_t len, int where, int k, int strand, tk_r2t **out) {
     CHECK_CTX(c);
     if (!out) return TK_E_INVAL;
@@ -1035,7 +1008,15 @@ int tk_r2t_create(tk_ctx *c, const char *bundle, uint64_t len, int where, int k,
     if (!e) e = r2t_build(z, b);
     if (!e) {
         z->n_records = b->n_reads;
-        e = bundle_component_ids(c, b, bundle, len, where, &z->comp_id);
+        z->comp_id.assign(b->n_reads, 0);
+        uint64_t *ids = nullptr;
+        e = dmalloc(c, (void **)&ids, b->n_reads * 8, "component ids");
+        if (!e) e = component_ids(c, b, ids);
+        if (!e && b->n_reads)
+            e = cuda_check(c, cudaMemcpyAsync(z->comp_id.data(), ids, b->n_reads * 8, cudaMemcpyDeviceToHost, c->stream),
+                           "component ids");
+        if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "component ids sync");
+        if (ids) dfree(c, ids);
     }
     if (b) tk_reads_free(b);
     if (e) {
@@ -1118,12 +1099,10 @@ int tk_dbg_create(tk_ctx *c, const char *bundle, uint64_t len, int where, int K,
     tk_reads *b = nullptr;
     int e = tk_reads_parse(c, bundle, len, where, &b);
     if (!e && b->format == TK_FMT_FASTQ) e = set_err(c, TK_E_PARSE, "bundle must be FASTA");
-    std::vector<uint64_t> ids;
     if (!e) {
         g->n_records = b->n_reads;
-        e = bundle_component_ids(c, b, bundle, len, where, &ids);
+        e = dbg_build(g, b);
     }
-    if (!e) e = dbg_build(g, b, ids);
     if (b) tk_reads_free(b);
     if (e) {
         tk_dbg_free(g);

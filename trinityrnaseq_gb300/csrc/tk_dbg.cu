@@ -245,7 +245,9 @@ struct DbgScratch {
     }
 };
 
-int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id) {
+int component_ids(tk_ctx *c, const tk_reads *b, uint64_t *d_ids);
+
+int dbg_build(tk_dbg *g, const tk_reads *b) {
     tk_ctx *c = g->ctx;
     const int k1 = g->k + 1;
     const uint64_t n_rec = b->n_reads, n_pos = b->seq_len;
@@ -298,7 +300,7 @@ int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id
     TK_TRY(sc.get((void **)&line, G * sizeof(DbgLine), "node lines"));
     TK_TRY(sc.get((void **)&len, G * 4, "line lengths"));
     TK_TRY(sc.get((void **)&loff, (G + 1) * 8, "line offsets"));
-    TK_CUDA(c, cudaMemcpyAsync(d_comp, comp_id.data(), n_rec * 8, cudaMemcpyHostToDevice, c->stream));
+    TK_TRY(component_ids(c, b, d_comp));
     k_dbg_lines<<<grid, DBG_THREADS, 0, c->stream>>>(n_pos, b->d_rd_off, n_rec, base, slots, slot_of, head, before, d_comp,
                                                      k1, line, ofirst, len, d_ncomp);
     c->launches++;

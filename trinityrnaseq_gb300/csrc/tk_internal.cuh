@@ -512,7 +512,7 @@ int norm_select(tk_norm *nm, const tk_reads *const *const sets[2], const uint32_
 int norm_table(tk_norm *nm);
 int norm_extract(tk_norm *nm, const tk_reads *const *sets, uint32_t nsets);
 void norm_release(tk_norm *nm);
-int dbg_build(tk_dbg *g, const tk_reads *b, const std::vector<uint64_t> &comp_id);
+int dbg_build(tk_dbg *g, const tk_reads *b);
 }  // namespace tk
 
 #define TK_TRY(x) do { int _e = (x); if (_e) return _e; } while (0)
