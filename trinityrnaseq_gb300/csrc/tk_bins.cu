@@ -25,7 +25,7 @@
 //
 // Each bin's dump equals a separate plain `jellyfish count` + `dump -L m` of
 // that bin (sorted by key).
-#include "tk_internal.cuh"
+#include "tk_warp.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -36,7 +36,6 @@ namespace tk {
 
 constexpr int BIN_HLL_P = 5;
 constexpr int BIN_HLL_M = 1 << BIN_HLL_P;
-constexpr int BC_SPAN = 32;
 
 struct BinGeom {
     const uint64_t *seq0;      // n_bins + 1 packed-read offsets of the bin starts
@@ -68,55 +67,58 @@ __global__ void k_bin_starts(const uint64_t *__restrict__ name_off, uint64_t n_r
     seq0[b] = rd_off[lo];
 }
 
-// Calls f(bin, key) for every valid window ending in [p0, p0 + 32).
-template <bool CANON, typename F>
-__device__ __forceinline__ void bin_windows(const uint8_t *__restrict__ seq, uint64_t p0, uint64_t n, int k,
-                                            const uint64_t *__restrict__ seq0, uint32_t n_bins, F &&f) {
-    const uint64_t kmask = (1ULL << (2 * k)) - 1;
-    const int shift = 2 * (k - 1);
-    uint32_t bin = bin_of(seq0, n_bins, p0);
-    uint64_t next = seq0[bin + 1];
-    const uint8_t *p = seq + p0 - 32;
-    uint64_t fw = 0, rc = 0;
-    int run = 0;
-    for (int j = 0; j < 64; j++) {
-        uint32_t c = base_code(p[j]);
-        if (c > 3) {
-            run = 0;
-        } else {
-            fw = ((fw << 2) | c) & kmask;
-            rc = (rc >> 2) | ((uint64_t)(3u - c) << shift);
-            run++;
-        }
-        if (j >= 32 && run >= k) {
-            const uint64_t e = p0 - 32 + j;
-            while (e >= next && bin + 1 < n_bins) { bin++; next = seq0[bin + 1]; }
-            f(bin, (CANON && rc < fw) ? rc : fw);
-        }
-    }
+// A block takes BC_STEPS stretches of blockDim.x window end positions, one
+// after another; the bin of its first position is searched once, and every
+// thread walks on from the bin of its last position.  2000 bins, 71M windows,
+// sketch + count: 32 consecutive positions per thread, rolled byte by byte, 0.55 +
+// 1.14 ms; one stretch per block 1.15 + 1.25 (the search, 11 dependent loads,
+// takes longer than its work); 8, 16 and 32 stretches 0.38 + 1.03, 0.36 + 1.00,
+// 0.35 + 1.04.  The count is bound by L2 atomics (a CAS and an add per window,
+// 82 G pairs/s on GB300); claiming with a 128-bit CAS is 7% slower here, where
+// three windows in four find their key.
+constexpr int BC_STEPS = 16;
+__device__ __forceinline__ uint32_t block_bin(const uint64_t *__restrict__ seq0, uint32_t n_bins, uint64_t p0) {
+    __shared__ uint32_t s_bin;
+    if (threadIdx.x == 0) s_bin = bin_of(seq0, n_bins, p0);
+    __syncthreads();
+    return s_bin;
 }
 
+// Sketch and window count of every bin (a window lies in the bin its end lies
+// in: reads do not cross bins).
 template <bool CANON>
-__global__ void k_bin_sketch(const uint8_t *__restrict__ seq, uint64_t n, int k, const uint64_t *__restrict__ seq0,
-                             uint32_t n_bins, uint32_t *__restrict__ regs, unsigned long long *__restrict__ windows) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * BC_SPAN;
-    for (uint64_t p0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * BC_SPAN; p0 < n; p0 += stride) {
-        uint32_t cur = 0xFFFFFFFFu, cnt = 0;
-        bin_windows<CANON>(seq, p0, n, k, seq0, n_bins, [&](uint32_t bin, uint64_t key) {
-            if (bin != cur) {
-                if (cnt) atomicAdd(&windows[cur], (unsigned long long)cnt);
-                cur = bin;
-                cnt = 0;
-            }
-            cnt++;
-            uint64_t h = mix64(key ^ 0x2545F4914F6CDD1DULL);
-            uint32_t idx = (uint32_t)(h >> (64 - BIN_HLL_P));
-            uint32_t rank = (uint32_t)__clzll((long long)(h << BIN_HLL_P)) + 1u;
-            if (rank > 64 - BIN_HLL_P) rank = 64 - BIN_HLL_P + 1;
-            uint32_t *r = &regs[(uint64_t)bin * BIN_HLL_M + idx];
-            if (rank > *r) atomicMax(r, rank);
-        });
-        if (cnt) atomicAdd(&windows[cur], (unsigned long long)cnt);
+__global__ void __launch_bounds__(256) k_bin_sketch(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv,
+                                                    uint64_t n, int k, const uint64_t *__restrict__ seq0, uint32_t n_bins,
+                                                    uint32_t *__restrict__ regs, unsigned long long *__restrict__ windows) {
+    const uint64_t p0 = (uint64_t)blockIdx.x * 256 * BC_STEPS;
+    uint32_t bin = block_bin(seq0, n_bins, p0), cnt = 0;
+    uint64_t next = __ldg(seq0 + bin + 1);
+#pragma unroll 2
+    for (int st = 0; st < BC_STEPS; st++) {
+        const uint64_t e = p0 + st * 256 + threadIdx.x;
+        if (e >= n) break;
+        if (e >= next) {
+            if (cnt) atomicAdd(&windows[bin], (unsigned long long)cnt);
+            cnt = 0;
+            while (bin + 1 < n_bins && e >= next) next = __ldg(seq0 + ++bin + 1);
+        }
+        uint64_t key;
+        if (!window_at<CANON>(codes, inv, e, k, key)) continue;
+        cnt++;
+        const uint64_t h = mix64(key ^ 0x2545F4914F6CDD1DULL);
+        const uint32_t idx = (uint32_t)(h >> (64 - BIN_HLL_P));
+        uint32_t rank = (uint32_t)__clzll((long long)(h << BIN_HLL_P)) + 1u;
+        if (rank > 64 - BIN_HLL_P) rank = 64 - BIN_HLL_P + 1;
+        uint32_t *r = &regs[(uint64_t)bin * BIN_HLL_M + idx];
+        if (rank > *r) atomicMax(r, rank);
+    }
+    // the warp's windows, one add when they are of one bin
+    const uint32_t b0 = __shfl_sync(0xffffffffu, bin, 0);
+    if (__all_sync(0xffffffffu, bin == b0)) {
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane_id() == 0 && cnt) atomicAdd(&windows[b0], (unsigned long long)cnt);
+    } else if (cnt) {
+        atomicAdd(&windows[bin], (unsigned long long)cnt);
     }
 }
 
@@ -129,25 +131,31 @@ __global__ void k_bin_fill(Slot *slots, uint64_t n) {
     }
 }
 
-// The counting launch: all bins, each k-mer into its bin's slice (a block per
-// chunk of BC_SPAN positions per thread; the loop also serves smaller grids).
+// The counting launch: all bins, each k-mer into its bin's slice.  The
+// positions in flight are those of a short stretch of the text, so the slices
+// in use stay in L2.
 template <bool CANON>
-__global__ void k_bin_count(const uint8_t *__restrict__ seq, uint64_t n, int k, BinGeom g, Slot *__restrict__ slots,
-                            int max_probes, uint32_t *__restrict__ overflow) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x * BC_SPAN;
-    for (uint64_t p0 = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) * BC_SPAN; p0 < n; p0 += stride) {
-        uint32_t cur = 0xFFFFFFFFu;
-        DevTable t;
-        t.pbits = 0;
-        bin_windows<CANON>(seq, p0, n, k, g.seq0, g.n_bins, [&](uint32_t bin, uint64_t key) {
-            if (bin != cur) {
-                cur = bin;
-                t.slots = slots + g.base[bin];
-                t.lbits = g.lbits[bin];
-                t.lmask = (1ULL << t.lbits) - 1;
-            }
-            if (!tbl_add(t, key, 1u, max_probes)) overflow[bin] = 1u;
-        });
+__global__ void k_bin_count(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv, uint64_t n, int k,
+                            BinGeom g, Slot *__restrict__ slots, int max_probes, uint32_t *__restrict__ overflow) {
+    const uint64_t p0 = (uint64_t)blockIdx.x * blockDim.x * BC_STEPS;
+    uint32_t bin = block_bin(g.seq0, g.n_bins, p0);
+    uint64_t next = __ldg(g.seq0 + bin + 1);
+    DevTable t;
+    t.pbits = 0;
+    t.slots = slots + g.base[bin];
+    t.lbits = g.lbits[bin];
+    t.lmask = (1ULL << t.lbits) - 1;
+    for (int st = 0; st < BC_STEPS; st++) {
+        const uint64_t e = p0 + (uint64_t)st * blockDim.x + threadIdx.x;
+        if (e >= n) break;
+        if (e >= next) {
+            while (bin + 1 < g.n_bins && e >= next) next = __ldg(g.seq0 + ++bin + 1);
+            t.slots = slots + g.base[bin];
+            t.lbits = g.lbits[bin];
+            t.lmask = (1ULL << t.lbits) - 1;
+        }
+        uint64_t key;
+        if (window_at<CANON>(codes, inv, e, k, key) && !tbl_add(t, key, 1u, max_probes)) overflow[bin] = 1u;
     }
 }
 
@@ -320,15 +328,13 @@ static std::atomic<int> g_tuned_load[64];
 constexpr uint64_t BIN_TUNE_MIN = 50ull << 20;
 
 template <bool CANON>
-static void launch_count(tk_ctx *c, int block, const uint8_t *seq, uint64_t n, int k, BinGeom g, Slot *slots,
-                         uint32_t *ovf) {
-    // one block per chunk of block x 32 positions: the blocks start in index
-    // order as earlier ones finish, so the bins being counted at any moment
-    // are those of a short stretch of the text and their slices stay in L2
-    // (a persistent grid's warps drift apart over the text)
-    const uint64_t span = (uint64_t)block * BC_SPAN;
-    const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + span - 1) / span, 0x7FFFFFFFull));
-    k_bin_count<CANON><<<grid, block, 0, c->stream>>>(seq, n, k, g, slots, c->max_probes, ovf);
+static void launch_count(tk_ctx *c, int block, const tk_reads &r, int k, BinGeom g, Slot *slots, uint32_t *ovf) {
+    // the blocks start in index order as earlier ones finish, so the bins being
+    // counted at any moment are those of a short stretch of the text (a
+    // persistent grid's warps drift apart over the text)
+    const uint64_t n = r.seq_len, span = (uint64_t)block * BC_STEPS;
+    k_bin_count<CANON><<<(unsigned)((n + span - 1) / span), block, 0, c->stream>>>(r.d_codes, r.d_inv, n, k, g, slots,
+                                                                                  c->max_probes, ovf);
     c->launches++;
 }
 
@@ -390,12 +396,11 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
         cudaMemsetAsync(d_regs, 0, regs.size() * 4, c->stream);
         cudaMemsetAsync(d_win, 0, n_bins * 8, c->stream);
         if (n) {
-            const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 256 * BC_SPAN - 1) / (256 * BC_SPAN),
-                                                                                     (uint64_t)c->sm_count * 8));
+            const unsigned grid = (unsigned)((n + 256 * BC_STEPS - 1) / (256 * BC_STEPS));
             cudaEvent_t ev;
             prof_begin(c, TK_KID_HLL, &ev);
-            if (canonical) k_bin_sketch<true><<<grid, 256, 0, c->stream>>>(r.d_seq, n, k, d_seq0, n_bins, d_regs, d_win);
-            else k_bin_sketch<false><<<grid, 256, 0, c->stream>>>(r.d_seq, n, k, d_seq0, n_bins, d_regs, d_win);
+            if (canonical) k_bin_sketch<true><<<grid, 256, 0, c->stream>>>(r.d_codes, r.d_inv, n, k, d_seq0, n_bins, d_regs, d_win);
+            else k_bin_sketch<false><<<grid, 256, 0, c->stream>>>(r.d_codes, r.d_inv, n, k, d_seq0, n_bins, d_regs, d_win);
             c->launches++;
             prof_end(c, TK_KID_HLL, ev, n);
         }
@@ -452,8 +457,8 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
             cudaEventCreate(&b2);
             cudaEventRecord(a, c->stream);
             k_bin_fill<<<(unsigned)c->sm_count * 8, 256, 0, c->stream>>>(ts, total);
-            if (canonical) launch_count<true>(c, tb, r.d_seq, n, k, g, ts, d_ovf);
-            else launch_count<false>(c, tb, r.d_seq, n, k, g, ts, d_ovf);
+            if (canonical) launch_count<true>(c, tb, r, k, g, ts, d_ovf);
+            else launch_count<false>(c, tb, r, k, g, ts, d_ovf);
             cudaEventRecord(b2, c->stream);
             e = cuda_check(c, cudaEventSynchronize(b2), "load tuning");
             float ms = 0;
@@ -490,8 +495,8 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
                 cudaEventCreate(&a);
                 cudaEventCreate(&b2);
                 cudaEventRecord(a, c->stream);
-                if (canonical) launch_count<true>(c, cand, r.d_seq, n, k, g, slots, d_ovf);
-                else launch_count<false>(c, cand, r.d_seq, n, k, g, slots, d_ovf);
+                if (canonical) launch_count<true>(c, cand, r, k, g, slots, d_ovf);
+                else launch_count<false>(c, cand, r, k, g, slots, d_ovf);
                 cudaEventRecord(b2, c->stream);
                 cudaEventSynchronize(b2);
                 float ms = 0;
@@ -512,8 +517,8 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
         k_bin_fill<<<(unsigned)c->sm_count * 8, 256, 0, c->stream>>>(slots, total);
         c->launches++;
         if (n) {
-            if (canonical) launch_count<true>(c, block, r.d_seq, n, k, g, slots, d_ovf);
-            else launch_count<false>(c, block, r.d_seq, n, k, g, slots, d_ovf);
+            if (canonical) launch_count<true>(c, block, r, k, g, slots, d_ovf);
+            else launch_count<false>(c, block, r, k, g, slots, d_ovf);
         }
         e = cuda_check(c, cudaStreamEndCapture(c->stream, &graph), "capture end");
         // the context's executable graph takes this batch's parameters in
