@@ -11,8 +11,9 @@ namespace tk {
 // use (k <= 31).  Each window is cut out of the 128-bit code pair with one
 // funnel shift, its reverse complement out of the pair's reverse complement,
 // and it is valid when none of its k positions has its invalid bit set.
-// Calls f(key, i) for every valid window, in order of its end position 32w + i.
-template <bool CANON, typename F>
+// Calls f(key, i) for every valid window, in order of its end position 32w + i;
+// i from I0 up to I1.
+template <bool CANON, int I0 = 0, int I1 = 32, typename F>
 __device__ __forceinline__ void thread_windows(const uint64_t *__restrict__ codes, const uint32_t *__restrict__ inv,
                                                uint64_t w, bool active, int k, F &&f) {
     uint64_t hi = 0, lo = 0, m = ~0ULL;
@@ -40,7 +41,7 @@ __device__ __forceinline__ void thread_windows(const uint64_t *__restrict__ code
     rlo = ((rlo >> 1) & 0x5555555555555555ULL) | ((rlo & 0x5555555555555555ULL) << 1);
     const uint64_t kmask = (1ULL << (2 * k)) - 1;
 #pragma unroll
-    for (int i = 0; i < 32; i++) {
+    for (int i = I0; i < I1; i++) {
         if ((bad >> (31 - i)) & 1ULL) continue;
         // forward: the window ends at position 32 + i of the 64
         const int s = 62 - 2 * i;
