@@ -606,21 +606,23 @@ __global__ void k_occupied(const Slot *__restrict__ slots, uint64_t cap, unsigne
 // per thread, ranks its selected slots with a block scan and reserves their
 // output range with one atomicAdd per chunk (a per-warp counter atomic on one
 // address serialises in L2 on a 2G-slot table).  Output order is fixed by the
-// sort that follows.
-constexpr int CP_ITEMS = 16;
+// sort that follows.  Bound by memory: 8.6 GB 1.35 ms (256 threads with 16 slots
+// each, 32 of an SM's warps, 1.53).
+constexpr int CP_THREADS = 512;
+constexpr int CP_ITEMS = 4;
 
-__global__ void __launch_bounds__(256) k_compact(const Slot *__restrict__ slots, uint64_t cap, uint32_t min_count,
+__global__ void __launch_bounds__(CP_THREADS) k_compact(const Slot *__restrict__ slots, uint64_t cap, uint32_t min_count,
                                                  uint64_t *__restrict__ okeys, uint32_t *__restrict__ ovals,
                                                  unsigned long long *__restrict__ n_out) {
-    __shared__ uint32_t sm[256 / 32 + 1];
+    __shared__ uint32_t sm[CP_THREADS / 32 + 1];
     __shared__ unsigned long long s_base;
-    const uint64_t chunk = (uint64_t)blockDim.x * CP_ITEMS;
+    constexpr uint64_t chunk = (uint64_t)CP_THREADS * CP_ITEMS;
     for (uint64_t base = (uint64_t)blockIdx.x * chunk; base < cap; base += (uint64_t)gridDim.x * chunk) {
         ulonglong2 v[CP_ITEMS];
         uint32_t nsel = 0;
 #pragma unroll
         for (int j = 0; j < CP_ITEMS; j++) {
-            const uint64_t i = base + (uint64_t)j * blockDim.x + threadIdx.x;   // coalesced, striped
+            const uint64_t i = base + (uint64_t)j * CP_THREADS + threadIdx.x;   // coalesced, striped
             v[j].x = EMPTY_KEY;
             v[j].y = 0;
             if (i < cap) v[j] = __ldcs(reinterpret_cast<const ulonglong2 *>(&slots[i]));
@@ -644,26 +646,49 @@ __global__ void __launch_bounds__(256) k_compact(const Slot *__restrict__ slots,
     }
 }
 
-// jellyfish histo bins: [0] below low, [1 + c - low], [nb - 1] above high
-__global__ void k_histo(const Slot *__restrict__ slots, uint64_t cap, uint64_t low, uint64_t high,
-                        unsigned long long *__restrict__ hist, int use_smem) {
+// jellyfish histo bins: [0] below low, [1 + c - low], [nb - 1] above high.  A
+// thread takes HS_ITEMS slots at a time (their loads together) and counts the
+// k-mers seen once, most of a table's, in a register.  Bound by memory: one
+// read of the table.  8.6 GB: 1.18 ms (a slot at a time, 512 threads, 1.90; 512
+// threads with 8 slots 1.87, 512 with 4 in four blocks 1.54).
+constexpr int HS_THREADS = 1024;
+constexpr int HS_ITEMS = 4;
+__global__ void __launch_bounds__(HS_THREADS) k_histo(const Slot *__restrict__ slots, uint64_t cap, uint64_t low, uint64_t high,
+                                                      unsigned long long *__restrict__ hist, int use_smem) {
     extern __shared__ uint32_t sh[];
     const uint64_t nb = high - low + 3;
+    auto bin_of_count = [&](uint64_t c) { return c < low ? 0 : (c > high ? nb - 1 : 1 + c - low); };
     if (use_smem) {
-        for (uint64_t i = threadIdx.x; i < nb; i += blockDim.x) sh[i] = 0;
+        for (uint64_t i = threadIdx.x; i < nb; i += HS_THREADS) sh[i] = 0;
         __syncthreads();
     }
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (uint64_t)gridDim.x * blockDim.x) {
-        ulonglong2 v = __ldcs(reinterpret_cast<const ulonglong2 *>(&slots[i]));
-        if (v.x == EMPTY_KEY) continue;
-        uint64_t c = (uint32_t)v.y;
-        uint64_t bin = c < low ? 0 : (c > high ? nb - 1 : 1 + c - low);
-        if (use_smem) atomicAdd(&sh[bin], 1u);
-        else atomicAdd(&hist[bin], 1ULL);
+    uint32_t once = 0;
+    const uint64_t chunk = (uint64_t)HS_THREADS * HS_ITEMS;
+    for (uint64_t base = (uint64_t)blockIdx.x * chunk; base < cap; base += (uint64_t)gridDim.x * chunk) {
+        ulonglong2 v[HS_ITEMS];
+#pragma unroll
+        for (int j = 0; j < HS_ITEMS; j++) {
+            const uint64_t i = base + (uint64_t)j * HS_THREADS + threadIdx.x;
+            v[j].x = EMPTY_KEY;
+            if (i < cap) v[j] = __ldcs(reinterpret_cast<const ulonglong2 *>(&slots[i]));
+        }
+#pragma unroll
+        for (int j = 0; j < HS_ITEMS; j++) {
+            if (v[j].x == EMPTY_KEY) continue;
+            const uint32_t c = (uint32_t)v[j].y;
+            if (c == 1) once++;
+            else if (use_smem) atomicAdd(&sh[bin_of_count(c)], 1u);
+            else atomicAdd(&hist[bin_of_count(c)], 1ULL);
+        }
+    }
+    once = warp_sum(once);
+    if (lane_id() == 0 && once) {
+        if (use_smem) atomicAdd(&sh[bin_of_count(1)], once);
+        else atomicAdd(&hist[bin_of_count(1)], (unsigned long long)once);
     }
     if (use_smem) {
         __syncthreads();
-        for (uint64_t i = threadIdx.x; i < nb; i += blockDim.x)
+        for (uint64_t i = threadIdx.x; i < nb; i += HS_THREADS)
             if (sh[i]) atomicAdd(&hist[i], (unsigned long long)sh[i]);
     }
 }
@@ -1228,7 +1253,7 @@ int table_histo(tk_table *t, uint64_t low, uint64_t high, uint64_t *hist) {
         int use_smem = smem <= 96 * 1024;
         if (use_smem && smem > 48 * 1024)
             cudaFuncSetAttribute(k_histo, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        k_histo<<<(unsigned)c->sm_count * 2, 512, use_smem ? smem : 0, c->stream>>>(t->t.slots, t->capacity, low, high, d,
+        k_histo<<<(unsigned)c->sm_count * 2, HS_THREADS, use_smem ? smem : 0, c->stream>>>(t->t.slots, t->capacity, low, high, d,
                                                                                     use_smem);
         c->launches++;
         prof_end(c, TK_KID_COMPACT, ev, t->capacity);
@@ -1269,7 +1294,8 @@ int table_sorted_pairs(tk_table *t, uint32_t min_count, uint64_t **keys_out, uin
         cudaMemsetAsync(d_n, 0, 8, c->stream);
         cudaEvent_t ev;
         prof_begin(c, TK_KID_COMPACT, &ev);
-        k_compact<<<stream_grid(c, (t->capacity + CP_ITEMS - 1) / CP_ITEMS, 256), 256, 0, c->stream>>>(
+        k_compact<<<(unsigned)std::min<uint64_t>((t->capacity + CP_THREADS * CP_ITEMS - 1) / (CP_THREADS * CP_ITEMS),
+                                                   (uint64_t)c->sm_count * 4), CP_THREADS, 0, c->stream>>>(
             t->t.slots, t->capacity, min_count, k0, v0, d_n);
         c->launches++;
         prof_end(c, TK_KID_COMPACT, ev, t->capacity);
