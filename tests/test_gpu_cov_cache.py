@@ -112,3 +112,21 @@ def test_default_cache_serves_large_tables(ctx, oracle):
     assert builds == (1 if cap * 16 >= 256 << 20 else 0)
     keys, counts = oracle.count(text, 25, True)
     assert_stats(got, oracle.cov_values(text, keys, counts, 25, True))
+
+
+@pytest.mark.parametrize("capacity", [1 << 24, 1 << 29, 1 << 30])
+def test_counts_of_zero_one_and_absent_keys(ctx, oracle, small_cache, capacity):
+    """The filter beside the cache (tables of up to 2^29 slots) answers for keys seen once and for absent ones only:
+    keys loaded with count 0 are read from the table, with the filter and without."""
+    text = mixed_reads(25, seed=9)
+    keys, _ = oracle.count(text, 25, True)
+    rnd = np.random.default_rng(3)
+    keys = keys[rnd.random(keys.size) < 0.7]
+    counts = rnd.choice(np.array([0, 1, 1, 1, 2, 3, 50, 70_000], np.uint32), keys.size)
+    t = KmerTable(ctx, 25, True, capacity)
+    t.load_pairs(keys, counts)
+    assert t.info()[2] == capacity
+    got = coverage_stats(t, ReadSet(ctx, text))
+    want = oracle.cov_values(text, keys, counts, 25, True)
+    for g, w in zip(got, want):
+        assert np.array_equal(g.view(np.uint32), w.view(np.uint32))

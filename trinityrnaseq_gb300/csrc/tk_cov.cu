@@ -28,11 +28,15 @@
 // do not depend on what the cache holds.  Random lookups into HBM run at
 // ~40 G/s on GB300 whatever the table size above 1 GB, and into an
 // L2-resident table at ~300 G/s; at the plain path's scale the 6-7M k-mers
-// the cache holds answer ~70% of the lookups.  (Most lookups the cache
-// misses are k-mers seen once, whose answer is 1.  A 32 or 64 MB bit filter
-// of the keys whose count is not 1, consulted before the table, made the pass
-// ~8% slower on GB300: its lines share L2 with the cache's, and a lookup that
-// passes it pays two dependent loads.)
+// the cache holds answer ~70% of the lookups.
+//
+// Most lookups the cache misses are k-mers seen once, whose answer is 1.  Beside
+// the cache of a table of at most 2^29 slots lies a 16 MB filter of the keys
+// whose count is not 1 (two bits in a 32-bit word): a k-mer it does not hold
+// needs no table access.  5M pairs 14.1 -> 13.4 ms, 1.5M 4.29 -> 3.83, 0.6M 1.52 ->
+// 1.44; with 32 MB 13.5, 3.86 and 1.45, with 8 MB 14.2, 3.91 and 1.46.  For larger
+// tables the filter passes most keys while its lines share L2 with the
+// cache's (20M pairs: 8% slower with 32 or 64 MB).
 #include "tk_warp.cuh"
 
 #include <algorithm>
@@ -52,6 +56,7 @@ struct CovCache {
     uint64_t *ent;     // 4 entries per bucket; nullptr = no cache
     int n;             // key bits (2k)
     int rbits;         // hash bits below the bucket index (<= 32): an entry is (those bits << 32) | count
+    uint32_t *seen2;   // filter of the keys whose count is not 1 (nullptr: none)
 };
 
 // A bijection of [0, 2^n) (n <= 62): a three-round Feistel network over the
@@ -98,6 +103,22 @@ __device__ __forceinline__ uint32_t cache_match(const uint64_t *b, uint32_t tag)
     return c;
 }
 
+constexpr int SEEN2_BITS = 22;                        // 2^22 words, 16 MB
+constexpr uint64_t SEEN2_MAX_CAPACITY = 1ULL << 29;   // slots of the table
+__device__ __forceinline__ uint32_t seen2_word(uint64_t h) { return (uint32_t)(h >> 20) & ((1u << SEEN2_BITS) - 1); }
+__device__ __forceinline__ uint32_t seen2_bits(uint64_t h) { return (1u << (h >> 5 & 31)) | (1u << (h & 31)); }
+
+// false: the filter says that key's count in the table is 1, or that it is absent
+__device__ __forceinline__ bool seen_twice(const CovCache &cc, uint64_t key) {
+    const uint64_t h = mix64(key);
+    const uint32_t b = seen2_bits(h);
+    uint32_t w;
+    uint64_t pol;
+    asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+    asm("ld.global.L2::cache_hint.u32 %0, [%1], %2;" : "=r"(w) : "l"(cc.seen2 + seen2_word(h)), "l"(pol));
+    return (w & b) == b;
+}
+
 // the count of `key` for the statistics: the cache, else the table (1 when absent)
 __device__ __forceinline__ uint32_t cov_lookup(const CovCache &cc, DevTable t, uint64_t key) {
     if (cc.ent) {
@@ -141,8 +162,12 @@ __global__ void __launch_bounds__(256) k_cache_build(const Slot *__restrict__ sl
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += stride) {
         const ulonglong2 s = __ldcs(reinterpret_cast<const ulonglong2 *>(slots + i));
         const uint32_t c = (uint32_t)s.y;
-        if (s.x == EMPTY_KEY || c < 2) continue;
-        cache_offer(cc, s.x, c);
+        if (s.x == EMPTY_KEY || c == 1) continue;
+        if (cc.seen2) {
+            const uint64_t h = mix64(s.x);
+            atomicOr(cc.seen2 + seen2_word(h), seen2_bits(h));
+        }
+        if (c) cache_offer(cc, s.x, c);
     }
 }
 
@@ -156,6 +181,7 @@ static uint64_t cache_bytes_wanted() {
 // the table is small enough for L2 to hold it whole, or k is too small.
 static int cache_get_or_build(tk_table *t, CovCache *cc) {
     cc->ent = nullptr;
+    cc->seen2 = nullptr;
     tk_ctx *c = t->ctx;
     const uint64_t want = cache_bytes_wanted();
     if (want < 32 || t->capacity * sizeof(Slot) < 4 * want) return TK_OK;
@@ -166,15 +192,18 @@ static int cache_get_or_build(tk_table *t, CovCache *cc) {
     const uint64_t bytes = 32ULL << hbits;
     cc->n = n;
     cc->rbits = n - hbits;
+    const bool filter = t->capacity <= SEEN2_MAX_CAPACITY;   // its 16 MB lie behind the cache
+    const uint64_t all = bytes + (4ULL << SEEN2_BITS);
     if (!t->hot_valid || t->hot_bytes != bytes) {
         if (t->d_hot && t->hot_bytes != bytes) {
             dfree(c, t->d_hot);
             t->d_hot = nullptr;
         }
-        if (!t->d_hot) TK_TRY(dmalloc(c, (void **)&t->d_hot, bytes, "coverage cache"));
+        if (!t->d_hot) TK_TRY(dmalloc(c, (void **)&t->d_hot, all, "coverage cache"));
         t->hot_bytes = bytes;
-        TK_CUDA(c, cudaMemsetAsync(t->d_hot, 0, bytes, c->stream));
+        TK_CUDA(c, cudaMemsetAsync(t->d_hot, 0, all, c->stream));
         cc->ent = t->d_hot;
+        if (filter) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
         cudaEvent_t ev;
         prof_begin(c, TK_KID_COV_CACHE, &ev);
         const uint64_t blocks = std::min<uint64_t>((t->capacity + 255) / 256, (uint64_t)c->sm_count * 16);
@@ -185,6 +214,7 @@ static int cache_get_or_build(tk_table *t, CovCache *cc) {
         t->hot_valid = true;
     }
     cc->ent = t->d_hot;
+    if (filter) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
     return TK_OK;
 }
 
@@ -196,7 +226,8 @@ struct ReadSums {
 constexpr uint32_t LONG_READ = 0xFFFFFFFFu;   // cnt of a read left to the long-read pass
 
 // A read's windows in three stages.  Stage 1: the lane's keys and their
-// validity, and the cache's count for each (0 = not in the cache).  Stage 2:
+// validity, and the cache's (FILTER: and then the filter's) count for each (0 =
+// the table has to be asked).  Stage 2:
 // the table for the windows the cache did not answer.  Stage 3: the read's
 // statistics.  The lookups of a stage are independent loads issued together.
 // (Pipelining two reads -- the next read's cache answers and table prefetches
@@ -207,7 +238,7 @@ constexpr uint32_t LONG_READ = 0xFFFFFFFFu;   // cnt of a read left to the long-
 // probe of a sector per step instead of a slot, the sectors first to leave L2,
 // took them from 15.6 ms: random sectors come from HBM at 38 G/s on GB300
 // whatever their size up to 128 bytes, so what counts is their number.)
-template <int S, bool CANON>
+template <int S, bool CANON, bool FILTER>
 __device__ __forceinline__ void cov_stage1(const CovCache &cc, const uint64_t *__restrict__ codes,
                                            const uint32_t *__restrict__ inv, uint64_t start, uint32_t nwin, int k,
                                            uint64_t (&key)[S], uint32_t (&v)[S], uint32_t &vm) {
@@ -225,6 +256,11 @@ __device__ __forceinline__ void cov_stage1(const CovCache &cc, const uint64_t *_
             const uint64_t *b = cache_bucket(cc, key[j], &tag);
             v[j] = cache_match(b, tag);
         }
+    }
+    if (FILTER) {
+#pragma unroll
+        for (int j = 0; j < S; j++)
+            if (((vm >> j) & 1u) && v[j] == 0 && !seen_twice(cc, key[j])) v[j] = 1;
     }
 }
 
@@ -283,13 +319,13 @@ __device__ __forceinline__ ReadSums cov_stage3(const uint32_t (&v)[S], uint32_t 
     return rs;
 }
 
-template <int S, bool CANON>
+template <int S, bool CANON, bool FILTER>
 __device__ __forceinline__ ReadSums cov_warp_read(const CovCache &cc, DevTable t, const uint64_t *__restrict__ codes,
                                                   const uint32_t *__restrict__ inv, uint64_t start, uint32_t nwin,
                                                   int k) {
     uint64_t key[S];
     uint32_t v[S], vm;
-    cov_stage1<S, CANON>(cc, codes, inv, start, nwin, k, key, v, vm);
+    cov_stage1<S, CANON, FILTER>(cc, codes, inv, start, nwin, k, key, v, vm);
     cov_stage2<S>(t, cc.ent != nullptr, key, v, vm);
     return cov_stage3<S>(v, vm);
 }
@@ -303,7 +339,7 @@ __device__ __forceinline__ ReadSums cov_warp_read(const CovCache &cc, DevTable t
 // separate pass) and not written here.  MAXS = the largest window class
 // compiled in (windows per lane); a read set whose reads all have at most
 // 32 * MAXS windows needs no larger one.
-template <bool CANON, int MAXS = 8>
+template <bool CANON, int MAXS = 8, bool FILTER = false>
 __device__ __forceinline__ void cov_warp_chunk(const CovCache &cc, DevTable t, const uint64_t *__restrict__ codes,
                                                const uint32_t *__restrict__ inv,
                                                const uint64_t *__restrict__ rd_off, uint64_t n_reads, uint32_t per, int k,
@@ -324,12 +360,12 @@ __device__ __forceinline__ void cov_warp_chunk(const CovCache &cc, DevTable t, c
         const uint32_t nwin = L >= (uint64_t)k ? (uint32_t)(L - k + 1) : 0u;
         ReadSums rs;
         bool is_long = false;
-        if (nwin <= 32) rs = cov_warp_read<1, CANON>(cc, t, codes, inv, start, nwin, k);
-        else if (nwin <= 64) rs = cov_warp_read<2, CANON>(cc, t, codes, inv, start, nwin, k);
-        else if (nwin <= 96) rs = cov_warp_read<3, CANON>(cc, t, codes, inv, start, nwin, k);
-        else if (MAXS >= 4 && nwin <= 128) rs = cov_warp_read<(MAXS >= 4 ? 4 : 1), CANON>(cc, t, codes, inv, start, nwin, k);
-        else if (MAXS >= 6 && nwin <= 192) rs = cov_warp_read<(MAXS >= 6 ? 6 : 1), CANON>(cc, t, codes, inv, start, nwin, k);
-        else if (MAXS >= 8 && nwin <= CV_WARP_MAX) rs = cov_warp_read<(MAXS >= 8 ? 8 : 1), CANON>(cc, t, codes, inv, start, nwin, k);
+        if (nwin <= 32) rs = cov_warp_read<1, CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
+        else if (nwin <= 64) rs = cov_warp_read<2, CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
+        else if (nwin <= 96) rs = cov_warp_read<3, CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
+        else if (MAXS >= 4 && nwin <= 128) rs = cov_warp_read<(MAXS >= 4 ? 4 : 1), CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
+        else if (MAXS >= 6 && nwin <= 192) rs = cov_warp_read<(MAXS >= 6 ? 6 : 1), CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
+        else if (MAXS >= 8 && nwin <= CV_WARP_MAX) rs = cov_warp_read<(MAXS >= 8 ? 8 : 1), CANON, FILTER>(cc, t, codes, inv, start, nwin, k);
         else {
             is_long = true;
             if (long_list && lane == 0) long_list[atomicAdd(long_n, 1ULL)] = (uint32_t)r;
@@ -353,7 +389,7 @@ __device__ __forceinline__ void cov_warp_chunk(const CovCache &cc, DevTable t, c
 
 // MAXS 3 / 4: read sets whose reads have at most 96 / 128 windows (up to 120 /
 // 152 nt at k = 25), 8 blocks per SM; MAXS 8: every read, 6 blocks per SM.
-template <bool CANON, int MAXS>
+template <bool CANON, int MAXS, bool FILTER>
 __global__ void __launch_bounds__(CV_THREADS, MAXS <= 4 ? 8 : 6) k_coverage(CovCache cc, DevTable t, const uint64_t *__restrict__ codes,
                                                         const uint32_t *__restrict__ inv,
                                                         const uint64_t *__restrict__ rd_off, uint64_t n_reads,
@@ -365,7 +401,7 @@ __global__ void __launch_bounds__(CV_THREADS, MAXS <= 4 ? 8 : 6) k_coverage(CovC
     const uint64_t warps = (uint64_t)gridDim.x * (CV_THREADS / 32);
     const uint64_t chunks = (n_reads + per - 1) / per;
     for (uint64_t ch = (uint64_t)blockIdx.x * (CV_THREADS / 32) + (threadIdx.x >> 5); ch < chunks; ch += warps)
-        cov_warp_chunk<CANON, MAXS>(cc, t, codes, inv, rd_off, n_reads, per, k, ch * per, median, mean, stdev, long_list,
+        cov_warp_chunk<CANON, MAXS, FILTER>(cc, t, codes, inv, rd_off, n_reads, per, k, ch * per, median, mean, stdev, long_list,
                                     long_n, held + (threadIdx.x & ~31u));
 }
 
@@ -606,40 +642,24 @@ int coverage_stats(tk_table *t, const tk_reads *rd, uint32_t *d_median, float *d
         // one wave of resident blocks, each warp striding over the chunks of
         // `per` reads (a grid of several partial waves leaves SMs idle at its end);
         // the narrowest kernel that holds the longest read's windows
-        static int per_sm[6] = {0, 0, 0, 0, 0, 0};
         const uint64_t max_win = rd->max_len >= (uint32_t)k ? rd->max_len - k + 1 : 0;
-        const int ci = (t->canonical ? 1 : 0) + (max_win <= 96 ? 4 : max_win <= 128 ? 2 : 0);
-        if (!per_sm[ci]) {
-            int b = 0;
-            switch (ci) {
-            case 0: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<false, 8>, CV_THREADS, 0); break;
-            case 1: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<true, 8>, CV_THREADS, 0); break;
-            case 2: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<false, 4>, CV_THREADS, 0); break;
-            case 3: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<true, 4>, CV_THREADS, 0); break;
-            case 4: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<false, 3>, CV_THREADS, 0); break;
-            default: cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_coverage<true, 3>, CV_THREADS, 0); break;
-            }
-            per_sm[ci] = std::max(1, b);
-        }
+        const int ci = (t->canonical ? 1 : 0) + (max_win <= 96 ? 4 : max_win <= 128 ? 2 : 0) + (cc.seen2 ? 6 : 0);
+        using Kernel = void (*)(CovCache, DevTable, const uint64_t *, const uint32_t *, const uint64_t *, uint64_t, uint32_t,
+                                int, uint32_t *, float *, float *, uint32_t *, unsigned long long *);
+        static const Kernel kernels[12] = {
+            k_coverage<false, 8, false>, k_coverage<true, 8, false>, k_coverage<false, 4, false>, k_coverage<true, 4, false>,
+            k_coverage<false, 3, false>, k_coverage<true, 3, false>, k_coverage<false, 8, true>,  k_coverage<true, 8, true>,
+            k_coverage<false, 4, true>,  k_coverage<true, 4, true>,  k_coverage<false, 3, true>,  k_coverage<true, 3, true>};
+        const uint64_t per_sm = ci % 6 < 2 ? 6 : 8;   // the kernels' launch bounds
         const uint32_t per = reads_per_turn(n);
         const uint64_t chunks = (n + per - 1) / per;
         const unsigned grid = (unsigned)std::max<uint64_t>(
             1, std::min<uint64_t>((chunks + CV_THREADS / 32 - 1) / (CV_THREADS / 32),
-                                  (uint64_t)c->sm_count * (uint64_t)per_sm[ci]));
+                                  (uint64_t)c->sm_count * per_sm));
         cudaEvent_t ev;
         prof_begin(c, TK_KID_COVERAGE, &ev);
-#define TK_COV_LAUNCH(C, M)                                                                                   \
-    k_coverage<C, M><<<grid, CV_THREADS, 0, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, n, per, k, d_median, \
-                                                         d_mean, d_stdev, long_list, long_n)
-        switch (ci) {
-        case 0: TK_COV_LAUNCH(false, 8); break;
-        case 1: TK_COV_LAUNCH(true, 8); break;
-        case 2: TK_COV_LAUNCH(false, 4); break;
-        case 3: TK_COV_LAUNCH(true, 4); break;
-        case 4: TK_COV_LAUNCH(false, 3); break;
-        default: TK_COV_LAUNCH(true, 3); break;
-        }
-#undef TK_COV_LAUNCH
+        kernels[ci]<<<grid, CV_THREADS, 0, c->stream>>>(cc, dt, rd->d_codes, rd->d_inv, rd->d_rd_off, n, per, k, d_median, d_mean,
+                                                        d_stdev, long_list, long_n);
         c->launches++;
         prof_end(c, TK_KID_COVERAGE, ev, rd->n_bases);
         e = check_launch(c, "coverage");
