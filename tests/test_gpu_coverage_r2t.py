@@ -200,6 +200,10 @@ def r2t_shapes(seed, k, n_reads):
         s = bytearray(c[a:a + L])
         if rnd.random() < 0.2:
             s += contigs[rnd.integers(len(contigs))][:L - len(s)]
+        if i % 7 == 0:   # on past the end of one record, over one base, into the next
+            j = int(rnd.integers(len(recs) - 1))
+            one, two = (recs[q].split(b"\n")[1] for q in (j, j + 1))
+            s = bytearray(one[-int(rnd.integers(k, 60)):] + b"A" + two[:int(rnd.integers(k, 60))])
         for _ in range(rnd.integers(0, 4)):
             if s:
                 s[rnd.integers(len(s))] = rnd.choice(np.frombuffer(b"ACGTN", dtype=np.uint8))

@@ -8,17 +8,19 @@
 // a k-mer held by several records belongs to the first of them whatever the
 // insertion order, and the table also says where it first occurs.
 //
-// Assign, by alignment (k_r2t_align): one thread per read.  A lookup of the
-// read's first open window gives the place of its k-mer in the bundle; from
-// there read and bundle are compared 32 bases at a time, and every window up
-// to the first difference has the same owner, as long as no earlier record
-// owns the bundle's k-mer there (a bit per bundle position).  Windows over a
-// sequencing error mostly hold k-mers the bundle does not have: a small filter
-// of the bundle's k-mers that stays in L2 answers for them.  A read of 100
-// bases then costs two or three random table accesses instead of 76.  Reads
-// whose windows belong to more than one record, or with more than 128
-// windows, are left to the per-window kernel.  The bits and the filter are
-// built by the first read set that has as many bases as the bundle.
+// Assign, by alignment (k_r2t_align): one thread per read.  The first of a few
+// windows that the bundle holds (they share no base) gives a place in the
+// bundle; the whole read is compared with the bundle there, 32 bases at a time,
+// and every window without a difference has the same owner, as long as no
+// earlier record owns the bundle's k-mer there (a bit per bundle position).
+// What is left are mostly windows over a sequencing error, whose k-mers the
+// bundle does not have: a warp takes the left windows of its 32 reads one per
+// lane, and a small filter of the bundle's k-mers that stays in L2 answers for
+// most of them.  A read of 100 bases then costs one or two random table
+// accesses instead of 76.  Reads whose windows belong to more than one record,
+// or with more than 128 windows, are left to the per-window kernel.  The bits
+// and the filter are built by the first read set that has as many bases as
+// the bundle.
 //
 // Assign, per window (k_r2t_assign): one warp per read packs the read's bases
 // 2 bits each into shared memory, cuts each lane's windows out of it, looks
@@ -126,133 +128,198 @@ struct R2tIndex {
     const uint32_t *inv, *foreign;
     const unsigned long long *filter;
     uint64_t filter_mask;
+    const uint64_t *rd_off;  // the bundle's records
+    uint64_t len;            // positions of the bundle
 };
 constexpr uint32_t RT_ALIGN_MAX = 128;   // windows of a read the alignment path takes (two 64-bit masks)
 
-// A read's open windows as a bit mask.
-struct WinMask {
-    uint64_t a, b;
-    __device__ __forceinline__ uint32_t first() const { return a ? (uint32_t)__ffsll((long long)a) - 1 : 63u + (uint32_t)__ffsll((long long)b); }
-    // drops windows [lo, hi]; how many of them were open
-    __device__ __forceinline__ uint32_t drop(uint32_t lo, uint32_t hi) {
-        const uint64_t ma = lo < 64 ? (~0ULL << lo) & (~0ULL >> (63 - min(hi, 63u))) : 0ULL;
-        const uint64_t mb = hi >= 64 ? (~0ULL >> (127 - hi)) & (lo > 64 ? ~0ULL << (lo - 64) : ~0ULL) : 0ULL;
-        const uint32_t c = __popcll(a & ma) + __popcll(b & mb);
-        a &= ~ma;
-        b &= ~mb;
-        return c;
-    }
+// A mask over a read's windows or positions, bit j of (a, b, c) = number j.
+struct Bits192 {
+    uint64_t a, b, c;
 };
 
-// The windows [0, nwin) of the read at `start` that hold A/C/G/T only.
-__device__ __forceinline__ WinMask read_windows(const uint32_t *__restrict__ inv, uint64_t start, uint32_t nwin, int k) {
-    // invalid positions of the read, position j at bit j of m0, m1, m2
-    uint64_t m0, m1, m2;
-    {
-        const int64_t p = (int64_t)start;
-        m0 = (uint64_t)__brev(bits_at(inv, p));
-        m1 = m2 = 0;
-        const uint32_t L = nwin + (uint32_t)k - 1;   // nothing past the read is asked for
-        if (L > 32) m0 |= (uint64_t)__brev(bits_at(inv, p + 32)) << 32;
-        if (L > 64) m1 = (uint64_t)__brev(bits_at(inv, p + 64));
-        if (L > 96) m1 |= (uint64_t)__brev(bits_at(inv, p + 96)) << 32;
-        if (L > 128) m2 = (uint64_t)__brev(bits_at(inv, p + 128));
-    }
-    uint64_t b0 = 0, b1 = 0;   // window w covers an invalid position
+__device__ __forceinline__ Bits192 low_bits(uint32_t n) {   // n <= 128
+    return {n >= 64 ? ~0ULL : (1ULL << n) - 1, n > 64 ? ~0ULL >> (128 - n) : 0ULL, 0ULL};
+}
+
+// Windows (bit w: positions w .. w+k-1) that hold a marked position.
+__device__ __forceinline__ Bits192 windows_over(Bits192 m, int k) {
+    Bits192 r{0, 0, 0};
     int sh = 0;
 #pragma unroll
     for (int l = 0; l < 5; l++) {
         if (k & (1 << l)) {
-            b0 |= sh ? (m0 >> sh) | (m1 << (64 - sh)) : m0;
-            b1 |= sh ? (m1 >> sh) | (m2 << (64 - sh)) : m1;
+            r.a |= sh ? (m.a >> sh) | (m.b << (64 - sh)) : m.a;
+            r.b |= sh ? (m.b >> sh) | (m.c << (64 - sh)) : m.b;
             sh += 1 << l;
         }
         const int d = 1 << l;
-        m0 |= (m0 >> d) | (m1 << (64 - d));
-        m1 |= (m1 >> d) | (m2 << (64 - d));
-        m2 |= m2 >> d;
+        m.a |= (m.a >> d) | (m.b << (64 - d));
+        m.b |= (m.b >> d) | (m.c << (64 - d));
+        m.c |= m.c >> d;
     }
-    WinMask u;
-    u.a = ~b0 & (nwin >= 64 ? ~0ULL : (1ULL << nwin) - 1);
-    u.b = nwin > 64 ? ~b1 & (~0ULL >> (128 - nwin)) : 0ULL;
-    return u;
+    return r;
 }
 
-// A thread per read (see the head of the file).  3M reads of 100 nt against
-// 13.6M bundle k-mers: 1.44 ms (ALU 90% busy: a lane whose read has errors keeps
-// its warp), and 0.10 for the reads left over; the per-window kernel takes
-// 7.68 ms, bound by its 76 random accesses per read at 38-44 G/s.
+// Word i (numbers 32i .. 32i+31) of a mask
+__device__ __forceinline__ void set_word(Bits192 &m, int i, uint32_t w) {
+    const uint64_t v = (uint64_t)w << (32 * (i & 1));
+    if (i < 2) m.a |= v;
+    else if (i < 4) m.b |= v;
+    else m.c |= v;
+}
+
+// bit j: base j (of 32, the first in the top two bits) of x is not zero
+__device__ __forceinline__ uint32_t base_mask(uint64_t x) {
+    x = (x | x >> 1) & 0x5555555555555555ULL;
+    x = (x | x >> 1) & 0x3333333333333333ULL;
+    x = (x | x >> 2) & 0x0F0F0F0F0F0F0F0FULL;
+    x = (x | x >> 4) & 0x00FF00FF00FF00FFULL;
+    x = (x | x >> 8) & 0x0000FFFF0000FFFFULL;
+    return __brev((uint32_t)(x | x >> 16));
+}
+
+// What the table says of the window starting at p: (end position << 32) |
+// record, ~0 when the bundle does not have it.  The filter is asked first.
 template <bool CANON>
-__global__ void __launch_bounds__(RT_THREADS) k_r2t_align(R2tIndex ix, DevTable t, const uint64_t *__restrict__ codes,
-                                                         const uint32_t *__restrict__ inv,
-                                                         const uint64_t *__restrict__ rd_off, uint64_t n_reads, int k,
-                                                         int32_t *__restrict__ rec, uint32_t *__restrict__ hits,
-                                                         uint32_t *__restrict__ nwin_out, uint32_t *__restrict__ rest,
-                                                         unsigned long long *__restrict__ rest_n) {
-    const uint64_t r = (uint64_t)blockIdx.x * RT_THREADS + threadIdx.x;
-    if (r >= n_reads) return;
-    const uint64_t start = rd_off[r];
-    const uint64_t L = rd_off[r + 1] - start - 1;
-    const uint64_t nw = L >= (uint64_t)k ? L - k + 1 : 0;
-    nwin_out[r] = (uint32_t)nw;
-    if (nw > RT_ALIGN_MAX) {
-        rest[atomicAdd(rest_n, 1ULL)] = (uint32_t)r;
-        return;
+__device__ __forceinline__ uint64_t bundle_lookup(const R2tIndex &ix, const DevTable &t, uint64_t fw, int k) {
+    uint64_t key = fw;
+    if (CANON) {
+        const uint64_t rc = kmer_revcomp(fw, k);
+        key = rc < fw ? rc : fw;
     }
-    const uint32_t nwin = (uint32_t)nw;
+    const uint64_t h = mix64(key);
+    const unsigned long long fb = filter_bits(h);
+    if ((__ldg(ix.filter + filter_word(h, ix.filter_mask)) & fb) != fb) return ~0ULL;
+    return tbl_get2<uint64_t>(t, key, true, ~0ULL);
+}
+
+constexpr uint32_t RT_LEFT = 1024;   // left windows a warp lists at a time (32 of each read)
+
+// A thread per read (see the head of the file).  3M reads of 100 nt against
+// 13.6M bundle k-mers: 1.02 ms (ALU 74% busy), and 0.12 for the reads left over;
+// with every thread walking its own open windows, extending to the first
+// difference, 1.44 (a lane whose read has errors kept its warp); the per-window
+// kernel takes 7.68, bound by its 76 random accesses per read at 38-44 G/s.
+template <bool CANON>
+__global__ void __launch_bounds__(RT_THREADS, 4) k_r2t_align(R2tIndex ix, DevTable t, const uint64_t *__restrict__ codes,
+                                                            const uint32_t *__restrict__ inv,
+                                                            const uint64_t *__restrict__ rd_off, uint64_t n_reads, int k,
+                                                            int32_t *__restrict__ rec, uint32_t *__restrict__ hits,
+                                                            uint32_t *__restrict__ nwin_out, uint32_t *__restrict__ rest,
+                                                            unsigned long long *__restrict__ rest_n) {
+    __shared__ uint16_t s_left[RT_THREADS / 32][RT_LEFT];   // (lane << 7) | window
+    __shared__ uint32_t s_votes[RT_THREADS], s_other[RT_THREADS];
+    const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+    const uint64_t r = (uint64_t)blockIdx.x * RT_THREADS + threadIdx.x;
+    uint64_t start = 0, nw = 0;
+    if (r < n_reads) {
+        start = rd_off[r];
+        const uint64_t L = rd_off[r + 1] - start - 1;
+        nw = L >= (uint64_t)k ? L - k + 1 : 0;
+        nwin_out[r] = (uint32_t)nw;
+    }
+    const bool too_long = nw > RT_ALIGN_MAX;
+    const uint32_t nwin = too_long ? 0u : (uint32_t)nw;
     uint32_t owner = PAD_VAL, votes = 0;
+    uint64_t left_a = 0, left_b = 0;
     if (nwin) {
-        WinMask open = read_windows(inv, start, nwin, k);
-        const uint64_t kmask = (1ULL << (2 * k)) - 1;
-        while (open.a | open.b) {
-            const uint32_t w = open.first();
-            const uint64_t fw = codes_at(codes, (int64_t)(start + w)) >> (64 - 2 * k);
-            uint64_t key = fw;
-            if (CANON) {
-                const uint64_t rc = kmer_revcomp(fw, k);
-                key = rc < fw ? rc : fw;
+        const int words = (int)((nwin + k - 1 + 31) / 32);   // of the read's bases, 1 .. 5
+        Bits192 bad{0, 0, 0};                                // positions that are not A/C/G/T
+        for (int i = 0; i < words; i++) set_word(bad, i, __brev(bits_at(inv, (int64_t)start + 32 * i)));
+        const Bits192 all = low_bits(nwin);
+        const Bits192 nb = windows_over(bad, k);
+        left_a = all.a & ~nb.a;
+        left_b = all.b & ~nb.b;
+        // the first window among 0, k, 2k, ... and the last that the bundle holds
+        uint64_t hit = ~0ULL, fw = 0;
+        uint32_t w = 0;
+        for (;;) {
+            if (((w < 64 ? left_a >> w : left_b >> (w - 64)) & 1ULL)) {
+                fw = codes_at(codes, (int64_t)(start + w)) >> (64 - 2 * k);
+                hit = bundle_lookup<CANON>(ix, t, fw, k);
+                if (hit != ~0ULL) break;
             }
-            const uint64_t h = mix64(key);
-            const unsigned long long fb = filter_bits(h);
-            uint64_t hit = ~0ULL;
-            if ((__ldg(ix.filter + filter_word(h, ix.filter_mask)) & fb) == fb) hit = tbl_get2<uint64_t>(t, key, true, ~0ULL);
-            if (hit == ~0ULL) {
-                open.drop(w, w);
-                continue;
-            }
-            const uint32_t own = (uint32_t)hit;
-            const int64_t e = (int64_t)(hit >> 32), s0 = e - k + 1;   // the bundle's window: positions s0 .. e
-            const bool forward = !CANON || (codes_at(ix.codes, s0) >> (64 - 2 * k) & kmask) == fw;
-            // t further windows: the read's bases after this window against the
-            // bundle's after e, or the complements of those before s0
-            const uint32_t most = nwin - 1 - w;
-            uint32_t ext = 0;
-            while (ext < most) {
-                const uint64_t rw = codes_at(codes, (int64_t)(start + w + k) + ext);
-                uint64_t bw;
-                uint32_t stop;
-                if (forward) {
-                    bw = codes_at(ix.codes, e + 1 + ext);
-                    stop = bits_at(ix.inv, e + 1 + ext) | bits_at(ix.foreign, e + 1 + ext);
-                } else {
-                    bw = kmer_revcomp(codes_at(ix.codes, s0 - 32 - (int64_t)ext), 32);
-                    stop = __brev(bits_at(ix.inv, s0 - 32 - (int64_t)ext) | bits_at(ix.foreign, e - 32 - (int64_t)ext));
-                }
-                const uint64_t x = rw ^ bw;
-                const uint32_t same = min(x ? (uint32_t)__clzll((long long)x) >> 1 : 32u, (uint32_t)__clz((int)stop));
-                ext += same;
-                if (same < 32) break;
-            }
-            ext = min(ext, most);
-            const uint32_t c = open.drop(w, w + ext);
-            if (owner == PAD_VAL) {
-                owner = own;
-            } else if (owner != own) {
-                rest[atomicAdd(rest_n, 1ULL)] = (uint32_t)r;   // more than one record: votes are counted per window
-                return;
-            }
-            votes += c;
+            if (w == nwin - 1) break;
+            w = min(w + (uint32_t)k, nwin - 1);
         }
+        if (hit != ~0ULL) {
+            owner = (uint32_t)hit;
+            const int64_t e = (int64_t)(hit >> 32), s0 = e - k + 1;   // the bundle's window: positions s0 .. e
+            const bool forward = !CANON || codes_at(ix.codes, s0) >> (64 - 2 * k) == fw;
+            Bits192 diff = bad, foreign{0, 0, 0};
+            for (int i = 0; i < words; i++) {
+                // the bundle's 32 positions against the read's bases 32i ..: from p up, or p + 31 down
+                const int64_t p = forward ? s0 - (int64_t)w + 32 * i : e + (int64_t)w - 32 * i - 31;
+                uint32_t d = ~0u;
+                if (p >= -32 && p < (int64_t)ix.len) {
+                    uint64_t bw = codes_at(ix.codes, p);
+                    uint32_t bi = bits_at(ix.inv, p);
+                    if (forward) bi = __brev(bi);
+                    else bw = kmer_revcomp(bw, 32);
+                    d = bi | base_mask(bw ^ codes_at(codes, (int64_t)start + 32 * i));
+                }
+                set_word(diff, i, d);
+                // windows 32i .. end at the bundle's positions from f up, or f + 31 down
+                const int64_t f = forward ? p + k - 1 : p;
+                if (i < 4 && f >= -32 && f < (int64_t)ix.len) {
+                    const uint32_t b = bits_at(ix.foreign, f);
+                    set_word(foreign, i, forward ? __brev(b) : b);
+                }
+            }
+            // only the windows whose place lies in the owner's record (the next
+            // record may go on where the read does)
+            const int64_t r_lo = (int64_t)ix.rd_off[owner], r_hi = (int64_t)ix.rd_off[owner + 1] - 2;   // its first and last position
+            const int64_t w_lo = forward ? r_lo - s0 + (int64_t)w : e + (int64_t)w - r_hi;
+            const int64_t w_hi = forward ? r_hi - e + (int64_t)w : s0 + (int64_t)w - r_lo;
+            const Bits192 upto = low_bits((uint32_t)min(w_hi + 1, (int64_t)RT_ALIGN_MAX));
+            const Bits192 below = low_bits((uint32_t)max(w_lo, (int64_t)0));
+            const Bits192 over = windows_over(diff, k);
+            const uint64_t ma = all.a & upto.a & ~below.a & ~over.a & ~foreign.a;
+            const uint64_t mb = all.b & upto.b & ~below.b & ~over.b & ~foreign.b;
+            votes = __popcll(ma) + __popcll(mb);
+            left_a &= ~ma;
+            left_b &= ~mb;
+        }
+    }
+    s_votes[threadIdx.x] = 0;
+    s_other[threadIdx.x] = 0;
+    __syncwarp();
+    // the left windows of the warp's reads, listed and taken one per lane
+    uint16_t *list = s_left[warp];
+    while (__any_sync(0xffffffffu, (left_a | left_b) != 0)) {
+        const uint32_t mine = min(32u, (uint32_t)(__popcll(left_a) + __popcll(left_b)));
+        const uint32_t incl = warp_incl_scan(mine), total = __shfl_sync(0xffffffffu, incl, 31);
+        uint32_t at = incl - mine;
+        for (uint32_t j = 0; j < mine; j++) {
+            uint32_t w;
+            if (left_a) {
+                w = (uint32_t)__ffsll((long long)left_a) - 1;
+                left_a &= left_a - 1;
+            } else {
+                w = 63u + (uint32_t)__ffsll((long long)left_b);
+                left_b &= left_b - 1;
+            }
+            list[at++] = (uint16_t)(lane << 7 | w);
+        }
+        __syncwarp();
+        for (uint32_t i = lane; i < ((total + 31) & ~31u); i += 32) {
+            const uint32_t item = i < total ? list[i] : 0u, l = item >> 7;
+            const uint64_t st = __shfl_sync(0xffffffffu, start, (int)l);
+            const uint32_t own = __shfl_sync(0xffffffffu, owner, (int)l);
+            if (i >= total) continue;
+            const uint64_t hit = bundle_lookup<CANON>(ix, t, codes_at(codes, (int64_t)(st + (item & 127u))) >> (64 - 2 * k), k);
+            if (hit == ~0ULL) continue;
+            if ((uint32_t)hit == own) atomicAdd(&s_votes[warp * 32 + l], 1u);
+            else s_other[warp * 32 + l] = 1u;
+        }
+        __syncwarp();
+    }
+    if (r >= n_reads) return;
+    votes += s_votes[threadIdx.x];
+    if (too_long || s_other[threadIdx.x]) {
+        rest[atomicAdd(rest_n, 1ULL)] = (uint32_t)r;   // votes are counted per window
+        return;
     }
     rec[r] = votes ? (int32_t)owner : -1;
     hits[r] = votes;
@@ -480,7 +547,7 @@ int r2t_assign(tk_r2t *z, const tk_reads *rd, int32_t *d_rec, uint32_t *d_hits, 
     if (!e) e = cuda_check(c, cudaMemsetAsync(long_n, 0, 8, c->stream), "long reset");
     // The alignment path, for reads of at most 128 windows on average: from as
     // many read bases as the bundle has on, building its index costs less than
-    // it saves (0.29 ms for 13.6M bundle bases against 7.7 -> 1.5 ms for 228M
+    // it saves (0.3 ms for 13.6M bundle bases against 7.7 -> 1.1 ms for 228M
     // windows); once built, every such read set takes it.
     bool align = rd->n_bases <= n * (uint64_t)(RT_ALIGN_MAX + k - 1);
     uint32_t *rest = nullptr;
@@ -491,7 +558,7 @@ int r2t_assign(tk_r2t *z, const tk_reads *rd, int32_t *d_rec, uint32_t *d_hits, 
         if (!e && align && dmalloc(c, (void **)&rest, n * 4, "reads left to the per-window vote")) align = false;
     }
     if (!e && align) {
-        const R2tIndex ix{z->d_codes, z->d_inv, z->d_foreign + 1, z->d_filter, z->filter_mask};
+        const R2tIndex ix{z->d_codes, z->d_inv, z->d_foreign + 1, z->d_filter, z->filter_mask, z->d_rd_off, z->seq_len};
         const unsigned grid = (unsigned)((n + RT_THREADS - 1) / RT_THREADS);
         cudaEvent_t ev;
         prof_begin(c, TK_KID_R2T_ASSIGN, &ev);
