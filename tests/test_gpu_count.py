@@ -299,3 +299,27 @@ def test_count_texts_error_leaves_the_context_usable(ctx, oracle):
     sets = t2.count_texts([np.frombuffer(good, dtype=np.uint8)])
     assert sets[0].n_reads == 20000
     assert_pairs(t2.dump(1), oracle.count(good, 25, True))
+
+
+@pytest.mark.parametrize("n", [3, 1 << 21, (1 << 21) + 1])
+@pytest.mark.parametrize("dirty", [False, True])
+def test_sizes_read_back_or_bounded(ctx, oracle, n, dirty):
+    """Small FASTA inputs and small sets get buffers of the largest size they
+    can need, larger ones (above 2^22 lines, 2^24 positions) of the size read
+    back: n records of seven bases lie below, at and above both lines.  A space
+    in one sequence line has the codes packed a second time."""
+    rng = np.random.default_rng(71)
+    rec = np.empty((n, 11), dtype=np.uint8)
+    rec[:, :] = np.frombuffer(b">r\n.......\n", dtype=np.uint8)
+    rec[:, 3:10] = np.frombuffer(b"ACGT", dtype=np.uint8)[rng.integers(0, 4, (n, 7), dtype=np.uint8)]
+    if dirty:
+        rec[n // 2, 6] = ord(" ")
+    text = rec.tobytes()
+    rs = ReadSet(ctx, text)
+    assert rs.n_reads == n
+    t = KmerTable(ctx, 5, True)
+    t.add(rs)
+    clean = text.replace(b" ", b"")
+    assert_pairs(t.dump(1), oracle.count(clean, 5, True))
+    if n < 10:
+        assert rs.sequences() == [clean.split(b"\n")[2 * i + 1] for i in range(n)]

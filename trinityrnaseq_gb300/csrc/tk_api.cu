@@ -328,14 +328,15 @@ int tk_ctx_create(int device, tk_ctx **out) {
         uint64_t thr = UINT64_MAX;
         cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr);
     }
-    if (cudaHostAlloc((void **)&c->h_wait_err, sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&c->h_stage, STAGE_BYTES + sizeof(uint32_t), cudaHostAllocDefault) != cudaSuccess) {
         cudaStreamDestroy(c->stream);
         delete c;
         return TK_E_OOM;
     }
+    c->h_wait_err = reinterpret_cast<uint32_t *>(c->h_stage + STAGE_BYTES);
     *c->h_wait_err = 0;
     if (cudaMalloc(&c->d_err, (DE_COUNT + 1) * sizeof(uint32_t)) != cudaSuccess) {
-        cudaFreeHost(c->h_wait_err);
+        cudaFreeHost(c->h_stage);
         cudaStreamDestroy(c->stream);
         delete c;
         return TK_E_OOM;
@@ -373,7 +374,7 @@ static void ctx_release_now(tk_ctx *c) {
     for (auto e : c->free_events) cudaEventDestroy(e);
     if (c->bins_exec) cudaGraphExecDestroy(c->bins_exec);
     cudaFree(c->d_err);
-    cudaFreeHost(c->h_wait_err);
+    cudaFreeHost(c->h_stage);
     if (c->own_stream) cudaStreamDestroy(c->stream);
     cudaMemPool_t pool;
     if (cudaDeviceGetDefaultMemPool(&pool, c->device) == cudaSuccess) cudaMemPoolTrimTo(pool, 0);

@@ -58,8 +58,11 @@ enum DevErr : uint32_t {
     DE_PARSE = 0,       // [0] parse error flag, [1] first bad line (low 32 bits)
     DE_OVERFLOW = 2,    // [2] overflow list overrun
     DE_WS = 3,          // [3] parser: whitespace seen inside a sequence line
+    DE_MAXLEN = 4,      // [4] parser: the longest read
     DE_COUNT = 8
 };
+
+constexpr size_t STAGE_BYTES = 64 << 10;
 
 __host__ __device__ inline uint64_t mix64(uint64_t x) {
     x ^= x >> 33; x *= 0xff51afd7ed558ccdULL;
@@ -310,6 +313,7 @@ struct tk_ctx {
     cudaStream_t copy_stream = nullptr;
     uint32_t *d_err = nullptr;             // tk::DE_COUNT words, then the sorts' wait error
     uint32_t *h_wait_err = nullptr;        // page-locked: set when a sort's bounded wait ran out (wait_status)
+    unsigned char *h_stage = nullptr;      // page-locked, STAGE_BYTES: small results read back at one synchronisation
     std::string last_error;
     // profiling (CUDA events on `stream` around the hot kernels)
     bool prof = false;
@@ -480,6 +484,10 @@ int scan_excl_u32_to_u64(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t 
 // K4 formatting of sorted (key, count) pairs (tk_table.cu)
 int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n, int k, char **text, uint64_t *len,
                 uint64_t **offs_out = nullptr);
+// The scan without waiting for it: the total goes to *d_total on the GPU.  When its bounded wait runs out
+// (wait_status after a synchronisation) out is not written: a kernel that stores by it first
+// looks at the context's word d_err[DE_COUNT].
+int scan_excl_u32_to_u64_async(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *d_total);
 int scan_record_lengths(tk_ctx *c, const uint32_t *counts, uint64_t *out, uint64_t n, int k, uint64_t *total_host);
 int wait_status(tk_ctx *c);
 int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits,
@@ -497,6 +505,7 @@ int table_count_many(tk_table *t, const tk_reads *const *sets, int nsets);
 struct BucketKeys {
     uint64_t *keys = nullptr;   // nullptr: the set has no windows
     uint64_t *offs = nullptr;   // NBUCKETS * cols + 1
+    uint64_t *starts = nullptr; // NBUCKETS + 1: where each bucket begins
     uint64_t cols = 0;
 };
 // Counting in two steps (tk_table.cu): table_count_begin, then pass 1 per

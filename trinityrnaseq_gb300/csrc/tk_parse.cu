@@ -112,8 +112,12 @@ __device__ __forceinline__ uint32_t newline_bits(const ParseGeom &g, const Bytes
 }
 
 // ---- A1: newlines per tile, and each thread's newline bits for A2
-__global__ void k_tile_newlines(ParseGeom g, uint32_t *__restrict__ tile_nl, uint32_t *__restrict__ nl_bits) {
+// (the parsed range still on the GPU, as k_bounds found it)
+__global__ void k_tile_newlines(ParseGeom g, const unsigned long long *__restrict__ bounds, uint32_t *__restrict__ tile_nl,
+                                uint32_t *__restrict__ nl_bits) {
     __shared__ uint32_t sm[PT_THREADS / 32 + 1];
+    g.S = bounds[0];
+    g.E = bounds[1];
     uint64_t p = g.A + (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
     Bytes32 b = load32(g.text, g.len, p, g.vec);
     const uint32_t m = newline_bits(g, b, p);
@@ -174,9 +178,10 @@ __global__ void k_line_kinds(ParseGeom g, const uint64_t *__restrict__ line_end,
 
 // record index per line (~0 before the first header) and header line per record
 __global__ void k_line_records(const uint32_t *__restrict__ is_hdr, uint64_t *__restrict__ line_rec_io, uint64_t n_lines,
-                               uint64_t *__restrict__ hdr_line, uint32_t *__restrict__ len) {
+                               uint64_t *__restrict__ hdr_line, uint32_t *__restrict__ len,
+                               const uint32_t *__restrict__ wait_err) {
     uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n_lines) return;
+    if (j >= n_lines || *wait_err) return;   // (the scan gave up: nothing to store by)
     uint64_t incl = line_rec_io[j] + is_hdr[j];   // exclusive scan + own flag
     if (is_hdr[j]) hdr_line[incl - 1] = j;
     line_rec_io[j] = incl == 0 ? ~0ULL : incl - 1;
@@ -452,6 +457,8 @@ int component_ids(tk_ctx *c, const tk_reads *b, uint64_t *d_ids) {
 }
 
 // Builds r->d_codes / r->d_inv from r->d_seq (after the last write to seq).
+constexpr uint64_t PARSE_FEW_LINES = 1ull << 22;   // 32 MB of header lines; a round trip is 1% of their 1.2 ms
+
 static int pack_reads(tk_ctx *c, tk_reads *r) {
     const int64_t n_words = (int64_t)((r->seq_len + 31) / 32) + 1;
     const uint64_t code_words = (uint64_t)n_words + 1;          // incl. word -1
@@ -470,33 +477,34 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
     const char *text = r->d_text;
     uint64_t len = r->text_len;
     unsigned long long *d_bounds = nullptr;
-    unsigned long long hb[3] = {0, 0, 0};
     cudaEvent_t ev;
     prof_begin(c, TK_KID_PARSE, &ev);
-    TK_TRY(dmalloc(c, (void **)&d_bounds, 3 * sizeof(unsigned long long), "parse bounds"));
+    // What the host has to know comes back at three synchronisations: the
+    // parsed range and the lines; the reads and their bases; whether sequence
+    // lines held whitespace, and the longest read.  (A round trip takes about
+    // 10 us, one bin of 2000 reads 600.)
+    TK_TRY(dmalloc(c, (void **)&d_bounds, 4 * sizeof(unsigned long long), "parse bounds"));   // [3]: records
     k_bounds<<<1, 256, 0, c->stream>>>(text, len, d_bounds);
     c->launches++;
-    int e = cuda_check(c, cudaMemcpyAsync(hb, d_bounds, sizeof(hb), cudaMemcpyDeviceToHost, c->stream), "bounds d2h");
-    if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "bounds sync");
-    dfree(c, d_bounds);
-    if (e) return e;
+    volatile unsigned long long *hb = reinterpret_cast<volatile unsigned long long *>(c->h_stage);
+    int e = TK_OK;
     ParseGeom g;
     g.text = text;
     g.len = len;
-    g.S = hb[0];
-    g.E = hb[1];
+    g.S = g.E = 0;
     g.vec = ((uintptr_t)text & 15u) == 0;
-    g.A = g.vec ? (g.S & ~15ULL) : g.S;
-    r->format = g.S >= g.E ? TK_FMT_NONE : (hb[2] == '@' ? TK_FMT_FASTQ : TK_FMT_FASTA);
-    const int fastq = r->format == TK_FMT_FASTQ;
+    g.A = 0;
+    r->format = TK_FMT_NONE;
+    int fastq = 0;
 
-    uint64_t n_tiles = g.S >= g.E ? 0 : (g.E - g.A + PT_TILE - 1) / PT_TILE;
+    const uint64_t all_tiles = (len + PT_TILE - 1) / PT_TILE;
+    uint64_t n_tiles = 0;
     uint32_t *tile_nl = nullptr, *tile_em = nullptr, *is_hdr = nullptr, *nl_bits = nullptr;
     uint64_t *tile_line0 = nullptr, *tile_emit0 = nullptr, *line_end = nullptr, *line_rec = nullptr, *hdr_line = nullptr;
     uint32_t *line_len = nullptr;
     uint64_t *line_out = nullptr;
     uint8_t *kind = nullptr;
-    uint32_t *d_maxlen = nullptr;
+    uint32_t *d_maxlen = c->d_err + DE_MAXLEN;
     uint64_t n_nl = 0, n_lines = 0, n_reads = 0, n_emit = 0;
     std::vector<void *> tmp;
     auto alloc = [&](void **p, size_t bytes, const char *what) {
@@ -505,13 +513,20 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
         return ee;
     };
     do {
-        if (n_tiles == 0) break;
-        if ((e = alloc((void **)&tile_nl, n_tiles * 4, "tile newlines"))) break;
-        if ((e = alloc((void **)&tile_line0, (n_tiles + 1) * 8, "tile lines"))) break;
-        if ((e = alloc((void **)&nl_bits, n_tiles * PT_THREADS * 4, "newline bits"))) break;
-        k_tile_newlines<<<(unsigned)n_tiles, PT_THREADS, 0, c->stream>>>(g, tile_nl, nl_bits);
+        if (all_tiles == 0) break;
+        if ((e = alloc((void **)&tile_nl, all_tiles * 4, "tile newlines"))) break;
+        if ((e = alloc((void **)&tile_line0, (all_tiles + 1) * 8, "tile lines"))) break;
+        if ((e = alloc((void **)&nl_bits, all_tiles * PT_THREADS * 4, "newline bits"))) break;
+        k_tile_newlines<<<(unsigned)all_tiles, PT_THREADS, 0, c->stream>>>(g, d_bounds, tile_nl, nl_bits);
         c->launches++;
-        if ((e = scan_excl_u32_to_u64(c, tile_nl, tile_line0, n_tiles, &n_nl))) break;
+        if ((e = cuda_check(c, cudaMemcpyAsync(c->h_stage, d_bounds, 24, cudaMemcpyDeviceToHost, c->stream), "bounds d2h"))) break;
+        if ((e = scan_excl_u32_to_u64(c, tile_nl, tile_line0, all_tiles, &n_nl))) break;   // syncs
+        g.S = hb[0];
+        g.E = hb[1];
+        if (g.S >= g.E) break;   // nothing but whitespace
+        n_tiles = all_tiles;
+        r->format = hb[2] == '@' ? TK_FMT_FASTQ : TK_FMT_FASTA;
+        fastq = r->format == TK_FMT_FASTQ;
         n_lines = n_nl + 1;
         if ((e = alloc((void **)&line_end, n_lines * 8, "line ends"))) break;
         k_line_ends<<<(unsigned)n_tiles, PT_THREADS, 0, c->stream>>>(g, nl_bits, tile_line0, line_end);
@@ -548,20 +563,21 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
         k_line_kinds<<<grid_for(n_lines, 256), 256, 0, c->stream>>>(g, line_end, n_lines, fastq, kind, is_hdr, line_len,
                                                                      c->d_err);
         c->launches++;
-        if ((e = cuda_check(c, cudaMemcpyAsync(herr, c->d_err + DE_PARSE, 8, cudaMemcpyDeviceToHost, c->stream), "err d2h"))) break;
-        {
-            if ((e = scan_excl_u32_to_u64(c, is_hdr, line_rec, n_lines, &n_reads))) break;  // syncs
-            if ((e = alloc((void **)&hdr_line, (n_reads + 1) * 8, "header lines"))) break;
-            k_line_records<<<grid_for(n_lines, 256), 256, 0, c->stream>>>(is_hdr, line_rec, n_lines, hdr_line, line_len);
-            c->launches++;
-        }
+        // few lines: room for a record at each instead of a round trip for their number
+        const bool few = n_lines <= PARSE_FEW_LINES;
+        if (few) e = scan_excl_u32_to_u64_async(c, is_hdr, line_rec, n_lines, (uint64_t *)d_bounds + 3);
+        else e = scan_excl_u32_to_u64(c, is_hdr, line_rec, n_lines, &n_reads);   // syncs
+        if (e) break;
+        if ((e = alloc((void **)&hdr_line, ((few ? n_lines : n_reads) + 1) * 8, "header lines"))) break;
+        k_line_records<<<grid_for(n_lines, 256), 256, 0, c->stream>>>(is_hdr, line_rec, n_lines, hdr_line, line_len,
+                                                                      c->d_err + DE_COUNT);
+        c->launches++;
         if ((e = alloc((void **)&line_out, (n_lines + 1) * 8, "line outputs"))) break;
+        if (few && (e = cuda_check(c, cudaMemcpyAsync(c->h_stage, d_bounds + 3, 8, cudaMemcpyDeviceToHost, c->stream), "records d2h"))) break;
         if ((e = scan_excl_u32_to_u64(c, line_len, line_out, n_lines, &n_emit))) break;   // syncs
-        if (herr[0]) {
-            e = set_err(c, TK_E_PARSE, "FASTQ input: malformed record at line " + std::to_string(herr[1]));
-            break;
-        }
+        if (few) n_reads = hb[0];
     } while (0);
+    dfree(c, d_bounds);
     if (e) {
         for (void *p : tmp) dfree(c, p);
         return e;
@@ -574,16 +590,30 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
     if (!e) e = dmalloc(c, (void **)&r->d_rd_off, (n_reads + 1) * 8, "read offsets");
     if (!e) e = dmalloc(c, (void **)&r->d_name_off, (n_reads ? n_reads : 1) * 8, "name offsets");
     if (!e) e = dmalloc(c, (void **)&r->d_name_len, (n_reads ? n_reads : 1) * 4, "name lengths");
-    if (!e) e = dmalloc(c, (void **)&d_maxlen, 4, "max length");
     if (!e) {
         r->d_seq = r->d_seq_alloc + SEQ_PAD;
         cudaMemsetAsync(r->d_seq_alloc, '\n', seq_alloc, c->stream);
-        cudaMemsetAsync(d_maxlen, 0, 4, c->stream);
+        cudaMemsetAsync(c->d_err + DE_WS, 0, 8, c->stream);   // whitespace seen, the longest read
         uint64_t tail = r->seq_len;
         cudaMemcpyAsync(r->d_rd_off + n_reads, &tail, 8, cudaMemcpyHostToDevice, c->stream);
         uint32_t ws_seen = 0;
+        // accessions and read lengths, the 2-bit codes, and what the host reads back
+        auto finish = [&]() -> int {
+            if (n_tiles && n_reads) {
+                k_names<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, hdr_line, fastq, line_end, n_reads, r->d_rd_off,
+                                                                       r->d_name_off, r->d_name_len, d_maxlen);
+                c->launches++;
+            }
+            TK_TRY(pack_reads(c, r));
+            TK_CUDA(c, cudaMemcpyAsync(c->h_stage, c->d_err + DE_WS, 8, cudaMemcpyDeviceToHost, c->stream));
+            TK_CUDA(c, cudaStreamSynchronize(c->stream));
+            TK_TRY(wait_status(c));
+            const volatile uint32_t *h = reinterpret_cast<volatile uint32_t *>(c->h_stage);
+            ws_seen = h[0];
+            r->max_len = h[1];
+            return TK_OK;
+        };
         if (n_tiles && n_reads) {
-            cudaMemsetAsync(c->d_err + DE_WS, 0, 4, c->stream);
             const uint64_t n = fastq ? n_reads : n_lines;
             const uint32_t per = lines_per_warp(c, n);
             const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 8ull * per - 1) / (8ull * per),
@@ -595,9 +625,8 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
                 k_copy_lines<<<grid, 256, 0, c->stream>>>(g, line_end, kind, line_rec, line_out, n_lines, per, r->d_seq,
                                                           r->d_rd_off, c->d_err + DE_WS);
             c->launches++;
-            e = cuda_check(c, cudaMemcpyAsync(&ws_seen, c->d_err + DE_WS, 4, cudaMemcpyDeviceToHost, c->stream), "ws flag");
-            if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "copy sync");
         }
+        e = finish();
         r->plain_seq = fastq && !ws_seen;
         if (!e && ws_seen) {
             // some sequence line holds spaces, tabs or CRs: redo the emit byte by byte
@@ -629,19 +658,14 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
                 k_emit<<<(unsigned)n_tiles, PT_THREADS, 0, c->stream>>>(g, tile_line0, tile_emit0, kind, line_rec, n_lines,
                                                                        r->d_seq, r->d_rd_off);
                 c->launches++;
+                dfree(c, r->d_pack_alloc);   // of the lines as they were
+                r->d_pack_alloc = nullptr;
+                cudaMemsetAsync(d_maxlen, 0, 4, c->stream);
+                e = finish();
             } while (0);
         }
-        if (!e && n_tiles && n_reads) {
-            k_names<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, hdr_line, fastq, line_end, n_reads, r->d_rd_off,
-                                                                   r->d_name_off, r->d_name_len, d_maxlen);
-            c->launches++;
-        }
-        if (!e) e = pack_reads(c, r);
-        if (!e) e = cuda_check(c, cudaMemcpyAsync(&r->max_len, d_maxlen, 4, cudaMemcpyDeviceToHost, c->stream), "maxlen d2h");
-        if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "parse sync");
     }
     for (void *p : tmp) dfree(c, p);
-    if (d_maxlen) dfree(c, d_maxlen);
     prof_end(c, TK_KID_PARSE, ev, r->text_len);
     return e;
 }

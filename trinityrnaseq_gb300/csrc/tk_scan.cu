@@ -64,7 +64,8 @@ struct RecordLength {   // ">COUNT\nKMER\n"
 // and read its input twice.
 template <typename Tin, typename F>
 __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
-                                                    int vec, ScanHead *__restrict__ head, uint64_t *__restrict__ state) {
+                                                    int vec, ScanHead *__restrict__ head, uint64_t *__restrict__ state,
+                                                    uint64_t *__restrict__ total_at, uint32_t *__restrict__ err_at) {
     __shared__ uint64_t s_warp[SN_WARPS], s_before;
     __shared__ uint32_t s_tile, s_fail;
     if (threadIdx.x == 0) {
@@ -125,10 +126,14 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
         if (lane == 0) {
             if (fail) {
                 atomicExch(&head->err, 1u);
+                atomicExch(err_at, 1u);
                 s_fail = 1;
             } else {
                 if (tile) st_write(&state[tile], ST_FULL | (before + sum));
-                if (tile == (n - 1) / SN_TILE) head->total = before + sum;
+                if (tile == (n - 1) / SN_TILE) {
+                    head->total = before + sum;
+                    if (total_at) *total_at = before + sum;
+                }
             }
             s_before = before;
         }
@@ -155,41 +160,61 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
     }
 }
 
-// Whether the wait limit of a sort enqueued earlier ran out (every sort copies
-// the context's error word to its page-locked word; call after a
+// Whether the wait limit of a sort or scan enqueued earlier ran out (each
+// copies the context's error word to its page-locked word; call after a
 // synchronisation).
 int wait_status(tk_ctx *c) {
     if (!c->h_wait_err || *reinterpret_cast<volatile uint32_t *>(c->h_wait_err) == 0) return TK_OK;
     *c->h_wait_err = 0;
     cudaMemsetAsync(c->d_err + DE_COUNT, 0, 4, c->stream);
-    return set_err(c, TK_E_CUDA, "radix sort: the wait for an earlier tile ran out");
+    return set_err(c, TK_E_CUDA, "sort or scan: the wait for an earlier tile ran out");
+}
+
+// The scan enqueued, its head left in *mem (the caller frees it).
+template <typename Tin, typename F>
+static int scan_enqueue(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_at, ScanHead **mem) {
+    const uint64_t nt = (n + SN_TILE - 1) / SN_TILE;
+    const size_t bytes = sizeof(ScanHead) + nt * 8;
+    TK_TRY(dmalloc(c, (void **)mem, bytes, "scan tiles"));
+    int e = cuda_check(c, cudaMemsetAsync(*mem, 0, bytes, c->stream), "scan reset");
+    if (!e) {
+        const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
+        k_scan<Tin, F><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, *mem, reinterpret_cast<uint64_t *>(*mem + 1),
+                                                                  total_at, c->d_err + DE_COUNT);
+        c->launches++;
+        e = check_launch(c, "scan");
+    }
+    return e;
 }
 
 template <typename Tin, typename F>
 static int scan_impl(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
     *total_host = 0;
     if (n == 0) return TK_OK;
-    const uint64_t nt = (n + SN_TILE - 1) / SN_TILE;
-    unsigned char *mem = nullptr;
-    const size_t bytes = sizeof(ScanHead) + nt * 8;
-    TK_TRY(dmalloc(c, (void **)&mem, bytes, "scan tiles"));
-    ScanHead *head = reinterpret_cast<ScanHead *>(mem), h;
-    int e = cuda_check(c, cudaMemsetAsync(mem, 0, bytes, c->stream), "scan reset");
-    if (!e) {
-        const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
-        k_scan<Tin, F><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, head,
-                                                               reinterpret_cast<uint64_t *>(mem + sizeof(ScanHead)));
-        c->launches++;
-        e = check_launch(c, "scan");
-    }
+    ScanHead *head = nullptr, h;
+    int e = scan_enqueue<Tin>(c, f, in, out, n, nullptr, &head);
     if (!e) e = cuda_check(c, cudaMemcpyAsync(&h, head, sizeof h, cudaMemcpyDeviceToHost, c->stream), "scan total");
     if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "scan total sync");
-    dfree(c, mem);
+    if (head) dfree(c, head);
     if (e) return e;
-    if (h.err) return set_err(c, TK_E_CUDA, "scan: the wait for an earlier tile ran out");
+    if (h.err) {
+        *c->h_wait_err = 0;
+        cudaMemsetAsync(c->d_err + DE_COUNT, 0, 4, c->stream);
+        return set_err(c, TK_E_CUDA, "scan: the wait for an earlier tile ran out");
+    }
     TK_TRY(wait_status(c));
     *total_host = h.total;
     return TK_OK;
+}
+
+int scan_excl_u32_to_u64_async(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *d_total) {
+    if (n == 0) return cuda_check(c, cudaMemsetAsync(d_total, 0, 8, c->stream), "scan total");
+    ScanHead *head = nullptr;
+    int e = scan_enqueue<uint32_t>(c, ItemItself{}, in, out, n, d_total, &head);
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(c->h_wait_err, c->d_err + DE_COUNT, 4, cudaMemcpyDeviceToHost, c->stream),
+                           "scan status");
+    if (head) dfree(c, head);
+    return e;
 }
 
 int scan_excl_u64(tk_ctx *c, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_host) {

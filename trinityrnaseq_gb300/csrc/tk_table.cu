@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdlib>
+#include <cstring>
 
 namespace tk {
 
@@ -34,6 +35,11 @@ constexpr int INS_PER_THREAD = 1;
 // memory between flushes.  760M windows: 3.87 ms, with 512 threads 4.35.
 constexpr int SC_THREADS = 1024;
 constexpr int SC_TILE = 16384;                                   // window end positions per tile
+// Positions of a set whose key buffer is not sized exactly: reading the size
+// back is a round trip of about 12 us, 2% of the 600 us of one bin of 2000
+// pairs and below 0.5% of the 3 ms that 2^24 positions take; the buffer is then
+// 134 MB at most.
+constexpr uint64_t SC_SMALL = 1ull << 24;
 constexpr int SC_BUF = 24;                                       // a multiple of 4 (whole 32-byte sectors)
 static_assert(SC_BUF % 4 == 0 && SC_BUF <= 32, "a half-warp flushes a bucket in two 16-key stores");
 constexpr int SC_BUCKETS_PER_WARP = NBUCKETS / (SC_THREADS / 32);
@@ -100,7 +106,9 @@ template <bool CANON>
 __global__ void __launch_bounds__(SC_THREADS, 1) k_part_scatter(const uint64_t *__restrict__ codes,
                                                                const uint32_t *__restrict__ inv, uint64_t n, int k,
                                                                const uint64_t *__restrict__ offs, uint64_t cols,
-                                                               uint64_t col0, uint64_t *__restrict__ keys) {
+                                                               uint64_t col0, uint64_t *__restrict__ keys,
+                                                               const uint32_t *__restrict__ wait_err) {
+    if (*wait_err) return;   // the offsets' scan gave up: they are not to be stored by
     extern __shared__ __align__(16) unsigned char sc_smem[];
     uint64_t *buf = reinterpret_cast<uint64_t *>(sc_smem);                       // [NBUCKETS][SC_BUF]
     unsigned long long *gpos = reinterpret_cast<unsigned long long *>(buf + (size_t)NBUCKETS * SC_BUF);
@@ -568,8 +576,7 @@ __global__ void k_rehash(const Slot *__restrict__ old, uint64_t old_cap, DevTabl
 
 __global__ void k_insert_pairs(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ cnt, uint64_t n, DevTable t,
                                int max_probes, uint64_t *__restrict__ ovf_keys, uint32_t *__restrict__ ovf_cnt,
-                               uint64_t ovf_cap, unsigned long long *__restrict__ counters,
-                               unsigned long long *__restrict__ distinct) {
+                               uint64_t ovf_cap, unsigned long long *__restrict__ counters) {
     uint32_t added = 0;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         uint64_t key = keys[i];
@@ -579,10 +586,24 @@ __global__ void k_insert_pairs(const uint64_t *__restrict__ keys, const uint32_t
             if (j < ovf_cap) { ovf_keys[j] = key; ovf_cnt[j] = c; }
         }
     }
-    if (distinct) {
-        added = warp_sum(added);
-        if (lane_id() == 0 && added) atomicAdd(distinct, (unsigned long long)added);
+}
+
+// The deferred keys of a range build (*n of them; none when they overran cap).
+__global__ void k_insert_deferred(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ cnt,
+                                  const unsigned long long *__restrict__ n, uint64_t cap, DevTable t, int max_probes,
+                                  uint64_t *__restrict__ ovf_keys, uint32_t *__restrict__ ovf_cnt, uint64_t ovf_cap,
+                                  unsigned long long *__restrict__ counters, unsigned long long *__restrict__ distinct) {
+    const uint64_t m = *n;
+    if (m > cap) return;
+    uint32_t added = 0;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (uint64_t)gridDim.x * blockDim.x) {
+        if (!tbl_add_new(t, keys[i], cnt[i], max_probes, &added)) {
+            const unsigned long long j = atomicAdd(&counters[0], 1ULL);
+            if (j < ovf_cap) { ovf_keys[j] = keys[i]; ovf_cnt[j] = cnt[i]; }
+        }
     }
+    added = warp_sum(added);
+    if (lane_id() == 0 && added) atomicAdd(distinct, (unsigned long long)added);
 }
 
 __global__ void k_fill_empty(Slot *slots, uint64_t cap, uint64_t init_val) {
@@ -872,7 +893,7 @@ static int drain_overflow(tk_table *t) {
         if (!e) {
             k_insert_pairs<<<stream_grid(c, ovf, 256), 256, 0, c->stream>>>(pk, pc, ovf, t->t, c->max_probes, t->d_ovf,
                                                                              (uint32_t *)(t->d_ovf + t->ovf_cap), t->ovf_cap,
-                                                                             t->d_counters, nullptr);
+                                                                             t->d_counters);
             c->launches++;
             e = check_launch(c, "overflow insert");
         }
@@ -933,7 +954,8 @@ static int count_by_atomics(tk_table *t, const std::vector<BucketKeys> &bk) {
 // Pass 2 by ranges on a fresh table (see k_sr_build).  *done is false when
 // the deferred list overran its capacity: the table is then emptied again and
 // the caller counts with count_by_atomics instead, so nothing is lost.
-static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool *done) {
+static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, const std::vector<const uint64_t *> &starts_of,
+                           bool *done, bool *overflowed) {
     tk_ctx *c = t->ctx;
     *done = false;
     const int nparts = 1 << t->t.pbits;
@@ -944,15 +966,7 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
     else nsub = (uint32_t)(wave * ((slice + wave * SR_MAX_SLOTS - 1) / (wave * SR_MAX_SLOTS)));
     if (nsub > 0xFFFF) return TK_OK;   // run starts and ranges are 16-bit
     const uint64_t bpp = (uint64_t)(NBUCKETS >> t->t.pbits);
-    // partition boundaries on the host: the first offset of each partition's
-    // buckets in each set's buffer; partition p's keys are one segment of each
     const uint32_t nsets = (uint32_t)bk.size();
-    std::vector<std::vector<uint64_t>> pb(nsets, std::vector<uint64_t>(nparts + 1));
-    for (uint32_t q = 0; q < nsets; q++)
-        if (bk[q].keys)
-            TK_CUDA(c, cudaMemcpy2DAsync(pb[q].data(), 8, bk[q].offs, bpp * bk[q].cols * 8, 8, nparts + 1,
-                                         cudaMemcpyDeviceToHost, c->stream));
-    TK_CUDA(c, cudaStreamSynchronize(c->stream));
     std::vector<KeySeg> segs((size_t)nparts * nsets);
     std::vector<PartGeom> parts(nparts);
     std::vector<int> batch{0};                 // first partition of every batch, then nparts
@@ -961,8 +975,10 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
         uint64_t part = 0;
         for (uint32_t q = 0; q < nsets; q++) {
             KeySeg &g = segs[(size_t)p * nsets + q];
-            g.keys = bk[q].keys ? bk[q].keys + pb[q][p] : nullptr;
-            g.len = bk[q].keys ? pb[q][p + 1] - pb[q][p] : 0;
+            // partition p's keys are one segment of each set's buffer
+            const uint64_t *b = starts_of[q];
+            g.keys = bk[q].keys ? bk[q].keys + b[p * bpp] : nullptr;
+            g.len = bk[q].keys ? b[(p + 1) * bpp] - b[p * bpp] : 0;
             part += g.len;
         }
         if (p > batch.back() && batch_keys + part > SR_BATCH_KEYS) {
@@ -1017,12 +1033,20 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
                                                                           counters + 1);
         c->launches++;
     }
-    unsigned long long h[2] = {0, 0};
-    if (!e) e = check_launch(c, "range build");
-    if (!e) e = cuda_check(c, cudaMemcpyAsync(h, counters, 16, cudaMemcpyDeviceToHost, c->stream), "count counters d2h");
-    if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "defer sync");
-    const unsigned long long nd = h[0];
-    if (!e && nd > defer_cap) {
+    if (!e) {
+        k_insert_deferred<<<(unsigned)c->sm_count * 8, 256, 0, c->stream>>>(defer_keys, defer_cnt, counters, defer_cap, t->t,
+                                                                      c->max_probes, t->d_ovf,
+                                                                      (uint32_t *)(t->d_ovf + t->ovf_cap), t->ovf_cap,
+                                                                      t->d_counters, counters + 1);
+        c->launches++;
+        e = check_launch(c, "range build");
+    }
+    // deferred keys, distinct keys, keys on the overflow list
+    volatile unsigned long long *h = reinterpret_cast<volatile unsigned long long *>(c->h_stage);
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(c->h_stage, counters, 16, cudaMemcpyDeviceToHost, c->stream), "count counters d2h");
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(c->h_stage + 16, t->d_counters, 8, cudaMemcpyDeviceToHost, c->stream), "overflow d2h");
+    if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "count sync");
+    if (!e && h[0] > defer_cap) {
         // the deferred list overran: empty the table again and count with atomics
         k_fill_empty<<<stream_grid(c, t->capacity, 256), 256, 0, c->stream>>>(t->t.slots, t->capacity, 0);
         c->launches++;
@@ -1030,20 +1054,10 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
         e = check_launch(c, "table refill");
     } else if (!e) {
         t->fresh = false;
-        if (nd) {
-            k_insert_pairs<<<stream_grid(c, nd, 256), 256, 0, c->stream>>>(defer_keys, defer_cnt, nd, t->t, c->max_probes,
-                                                                            t->d_ovf, (uint32_t *)(t->d_ovf + t->ovf_cap),
-                                                                            t->ovf_cap, t->d_counters, counters + 1);
-            c->launches++;
-            e = check_launch(c, "deferred insert");
-            if (!e) e = cuda_check(c, cudaMemcpyAsync(h, counters, 16, cudaMemcpyDeviceToHost, c->stream), "count counters d2h");
-            if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "deferred insert sync");
-        }
-        if (!e) {
-            t->distinct = h[1];   // every key of the table was new to it once
-            t->distinct_valid = true;
-            *done = true;
-        }
+        t->distinct = h[1];   // every key of the table was new to it once
+        t->distinct_valid = true;
+        *overflowed = h[2] != 0;
+        *done = true;
     }
     dfree(c, grouped);
     if (starts) dfree(c, starts);
@@ -1053,6 +1067,12 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, bool 
     if (defer_cnt) dfree(c, defer_cnt);
     if (counters) dfree(c, counters);
     return e;
+}
+
+// where each of the NBUCKETS buckets begins, and where the last one ends
+__global__ void k_bucket_starts(const uint64_t *__restrict__ offs, uint64_t cols, uint64_t *__restrict__ starts) {
+    const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b <= NBUCKETS) starts[b] = offs[(uint64_t)b * cols];
 }
 
 // Pass 1 for one read set: the bucket histogram of its windows with the HLL
@@ -1086,12 +1106,22 @@ int table_bucket_pass(tk_table *t, const tk_reads *r, BucketKeys *out) {
         e = check_launch(c, "bucket histogram");
     }
     // key-buffer entries: the windows plus the EMPTY_KEY padding of every
-    // region (0 exactly when the set has no windows)
-    uint64_t padded = 0;
-    if (!e) e = scan_excl_u32_to_u64(c, hist, offs, cells, &padded);   // synchronises
+    // region (0 exactly when the set has no windows).  A set of up to SC_SMALL
+    // positions gets room for a window at each of them instead and is not
+    // waited for, unless that much memory is not to be had.
+    uint64_t padded = len + 3 * cells;
+    uint64_t *starts = nullptr;
+    if (!e) e = dmalloc(c, (void **)&starts, (NBUCKETS + 1) * 8, "bucket starts");
+    if (!e && len <= SC_SMALL && dmalloc(c, (void **)&keys, padded * 8, "bucketed k-mers") == TK_OK) {
+        e = scan_excl_u32_to_u64_async(c, hist, offs, cells, offs + cells);
+    } else if (!e) {
+        e = scan_excl_u32_to_u64(c, hist, offs, cells, &padded);   // synchronises
+        if (!e) e = cuda_check(c, cudaMemcpyAsync(offs + cells, &padded, 8, cudaMemcpyHostToDevice, c->stream), "bucket end");
+        if (!e && padded) e = dmalloc(c, (void **)&keys, padded * 8, "bucketed k-mers");
+    }
     if (!e && padded) {
-        cudaMemcpyAsync(offs + cells, &padded, 8, cudaMemcpyHostToDevice, c->stream);
-        e = dmalloc(c, (void **)&keys, padded * 8, "bucketed k-mers");
+        k_bucket_starts<<<(NBUCKETS + 256) / 256, 256, 0, c->stream>>>(offs, cols, starts);
+        c->launches++;
         static_assert(SC_SMEM <= 227 * 1024, "bucket staging exceeds shared memory");
         if (!e) e = cuda_check(c, cudaFuncSetAttribute(k_part_scatter<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                        (int)SC_SMEM), "scatter smem");
@@ -1101,10 +1131,10 @@ int table_bucket_pass(tk_table *t, const tk_reads *r, BucketKeys *out) {
             prof_begin(c, TK_KID_SCATTER, &ev);
             if (t->canonical)
                 k_part_scatter<true><<<grid, SC_THREADS, SC_SMEM, c->stream>>>(r->d_codes, r->d_inv, len, t->k, offs, cols,
-                                                                              0, keys);
+                                                                              0, keys, c->d_err + DE_COUNT);
             else
                 k_part_scatter<false><<<grid, SC_THREADS, SC_SMEM, c->stream>>>(r->d_codes, r->d_inv, len, t->k, offs, cols,
-                                                                               0, keys);
+                                                                               0, keys, c->d_err + DE_COUNT);
             c->launches++;
             prof_end(c, TK_KID_SCATTER, ev, padded);
             e = check_launch(c, "bucket scatter");
@@ -1114,10 +1144,12 @@ int table_bucket_pass(tk_table *t, const tk_reads *r, BucketKeys *out) {
     if (e || !padded) {
         if (keys) dfree(c, keys);
         if (offs) dfree(c, offs);
+        if (starts) dfree(c, starts);
         return e;
     }
     out->keys = keys;
     out->offs = offs;
+    out->starts = starts;
     out->cols = cols;
     return TK_OK;
 }
@@ -1125,6 +1157,7 @@ int table_bucket_pass(tk_table *t, const tk_reads *r, BucketKeys *out) {
 void table_bucket_free(tk_table *t, BucketKeys *bk) {
     if (bk->keys) dfree(t->ctx, bk->keys);
     if (bk->offs) dfree(t->ctx, bk->offs);
+    if (bk->starts) dfree(t->ctx, bk->starts);
     *bk = BucketKeys();
 }
 
@@ -1133,12 +1166,32 @@ void table_bucket_free(tk_table *t, BucketKeys *bk) {
 // set's keys counted partition by partition; frees the key buffers.
 int table_count_buckets(tk_table *t, std::vector<BucketKeys> &bk) {
     tk_ctx *c = t->ctx;
+    // the sketch, the window count and every set's bucket starts, read back at
+    // one synchronisation through the context's page-locked stage (the starts of
+    // more sets than fit there through pageable memory)
+    constexpr size_t STARTS = (NBUCKETS + 1) * 8, STAGED = (STAGE_BYTES - HLL_M * 4 - 8) / STARTS;
     uint64_t windows = 0;
     std::vector<uint32_t> regs(HLL_M);
-    int e = cuda_check(c, cudaMemcpyAsync(regs.data(), t->d_hll, HLL_M * 4, cudaMemcpyDeviceToHost, c->stream), "hll d2h");
-    if (!e) e = cuda_check(c, cudaMemcpyAsync(&windows, t->d_counters + 1, 8, cudaMemcpyDeviceToHost, c->stream),
+    std::vector<uint64_t> starts(bk.size() * (NBUCKETS + 1));
+    std::vector<const uint64_t *> starts_of(bk.size());
+    int e = cuda_check(c, cudaMemcpyAsync(c->h_stage, t->d_hll, HLL_M * 4, cudaMemcpyDeviceToHost, c->stream), "hll d2h");
+    if (!e) e = cuda_check(c, cudaMemcpyAsync(c->h_stage + HLL_M * 4, t->d_counters + 1, 8, cudaMemcpyDeviceToHost, c->stream),
                            "window count d2h");
+    for (size_t q = 0; q < bk.size() && !e; q++) {
+        void *to = q < STAGED ? (void *)(c->h_stage + HLL_M * 4 + 8 + q * STARTS) : (void *)(starts.data() + q * (NBUCKETS + 1));
+        if (bk[q].keys) e = cuda_check(c, cudaMemcpyAsync(to, bk[q].starts, STARTS, cudaMemcpyDeviceToHost, c->stream), "bucket starts d2h");
+    }
     if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "hll sync");
+    if (!e) e = wait_status(c);
+    if (!e) {
+        memcpy(regs.data(), c->h_stage, HLL_M * 4);
+        memcpy(&windows, c->h_stage + HLL_M * 4, 8);
+        for (size_t q = 0; q < bk.size(); q++) {
+            uint64_t *at = starts.data() + q * (NBUCKETS + 1);
+            if (q < STAGED && bk[q].keys) memcpy(at, c->h_stage + HLL_M * 4 + 8 + q * STARTS, STARTS);
+            starts_of[q] = at;
+        }
+    }
     if (!e) {
         double est = hll_estimate(regs.data());
         uint64_t want = pow2_at_least((uint64_t)(est * 1.08 / t->max_load) + 1);
@@ -1146,16 +1199,18 @@ int table_count_buckets(tk_table *t, std::vector<BucketKeys> &bk) {
         else if (want > t->capacity) e = table_rehash(t, want);
     }
     cudaEvent_t ev;
+    bool settled = false;   // nothing on the overflow list, as read back already
     if (!e && windows) {
         e = overflow_reset(t);
         t->distinct_valid = false;
         prof_begin(c, TK_KID_COUNT, &ev);
-        bool done = false;
-        if (!e && t->fresh && t->t.lbits >= SR_MIN_LBITS) e = count_by_ranges(t, bk, &done);
+        bool done = false, overflowed = true;
+        if (!e && t->fresh && t->t.lbits >= SR_MIN_LBITS) e = count_by_ranges(t, bk, starts_of, &done, &overflowed);
         if (!e && !done) e = count_by_atomics(t, bk);
         prof_end(c, TK_KID_COUNT, ev, windows);
         if (!e) e = check_launch(c, "count insert");
         if (!e) t->fresh = false;
+        settled = done && !overflowed;
     } else if (!e && t->fresh) {
         // nothing to insert: still leave every slot empty
         k_fill_empty<<<stream_grid(c, t->capacity, 256), 256, 0, c->stream>>>(t->t.slots, t->capacity, 0);
@@ -1172,7 +1227,7 @@ int table_count_buckets(tk_table *t, std::vector<BucketKeys> &bk) {
     }
     if (e) return e;
     t->total += windows;
-    return drain_overflow(t);
+    return settled ? TK_OK : drain_overflow(t);
 }
 
 // Resets the window counter before a group of pass-1 calls.
@@ -1373,7 +1428,7 @@ int table_insert_pairs(tk_table *t, const uint64_t *d_keys, const uint32_t *d_cn
     prof_begin(c, TK_KID_LOAD, &ev);
     k_insert_pairs<<<stream_grid(c, n, 256), 256, 0, c->stream>>>(d_keys, d_cnt, n, t->t, c->max_probes, t->d_ovf,
                                                                    (uint32_t *)(t->d_ovf + t->ovf_cap), t->ovf_cap,
-                                                                   t->d_counters, nullptr);
+                                                                   t->d_counters);
     c->launches++;
     prof_end(c, TK_KID_LOAD, ev, n);
     TK_TRY(check_launch(c, "insert pairs"));
