@@ -323,3 +323,47 @@ def test_sizes_read_back_or_bounded(ctx, oracle, n, dirty):
     assert_pairs(t.dump(1), oracle.count(clean, 5, True))
     if n < 10:
         assert rs.sequences() == [clean.split(b"\n")[2 * i + 1] for i in range(n)]
+
+
+def line_mix(seed, n, lens, fastq, blank=0.0, lower=True):
+    """Records of the given sequence-line lengths (FASTA: up to three lines a record, blank lines among them)."""
+    rng = np.random.default_rng(seed)
+    out, seqs = [], []
+    letters = np.frombuffer(b"ACGTACGTACGTNacgtnR" if lower else b"ACGTACGTACGTN", dtype=np.uint8)
+    for i in range(n):
+        rows = [letters[rng.integers(0, len(letters), int(L))].tobytes()
+                for L in rng.choice(lens, 1 if fastq else int(rng.integers(0, 4)))]
+        if fastq and i == n - 1:
+            rows = [b"ACGTA"]   # (an empty last quality line would be trimmed with the text's trailing whitespace)
+        seq = b"".join(rows)
+        seqs.append(seq.upper())
+        if fastq:
+            out.append(b"@r%d x\n%s\n+\n%s\n" % (i, seq, b"I" * len(seq)))
+        else:
+            body = b"".join(r + b"\n" + b"\n" * int(blank * rng.integers(0, 40)) for r in rows)
+            out.append(b">r%d\n%s" % (i, body))
+    return b"".join(out), seqs
+
+
+@pytest.mark.parametrize("shift", [0, 1, 7])
+@pytest.mark.parametrize("fastq", [False, True])
+@pytest.mark.parametrize("case", ["reads", "short", "blank", "long", "clean"])
+def test_copied_lines_and_codes(ctx, oracle, case, fastq, shift):
+    """Sequence lines into the read array and its codes, in tiles of 8192
+    positions and pieces of 32: lines around the size of a piece, more lines in
+    a tile than are held at a time (512), blank lines among them, lines over
+    several tiles, lower-case and N, texts at odd addresses on the GPU."""
+    import torch
+    n, lens, blank = {"reads": (2500, [31, 32, 33, 64, 76, 100], 0), "short": (9000, [0, 1, 2, 5], 0),
+                      "blank": (1500, [0, 3, 40], 1.0), "long": (9, [8191, 8192, 8193, 20000, 70000], 0),
+                      "clean": (2500, [76], 0)}[case]
+    text, seqs = line_mix(81, n, lens, fastq, blank, case != "clean")
+    dev = torch.zeros(len(text) + shift, dtype=torch.uint8, device="cuda:0")
+    dev[shift:] = torch.frombuffer(bytearray(text), dtype=torch.uint8).to("cuda:0")
+    torch.cuda.synchronize()
+    rs = ReadSet(ctx, dev.data_ptr() + shift, len(text), device=True)
+    assert rs.n_reads == n
+    assert rs.sequences() == seqs
+    t = KmerTable(ctx, 5, True)
+    t.add(rs)
+    assert_pairs(t.dump(1), oracle.count(text, 5, True))

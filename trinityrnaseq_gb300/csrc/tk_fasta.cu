@@ -224,9 +224,8 @@ __global__ void __launch_bounds__(FA_THREADS) k_fa_write(FaSet s, ParseGeom g, i
             seq_n = f.seq_len;
             out[o + seq_n] = '\n';
         }
-        bool ws = false;
         uint8_t *ob = reinterpret_cast<uint8_t *>(out);
-        copy_group<false>(g, name_src, name_dst, name_n, ob, ws);
+        copy_group(g, name_src, name_dst, name_n, ob);
         if (flags & TK_FA_REVCOMP) {
             for (int i = 0; i < 32; i++) {
                 const uint32_t n = __shfl_sync(0xffffffffu, seq_n, i);
@@ -234,7 +233,7 @@ __global__ void __launch_bounds__(FA_THREADS) k_fa_write(FaSet s, ParseGeom g, i
                 for (uint32_t j = lane; j < n; j += 32) ob[dst + j] = rc[(uint8_t)s.text[src + n - 1 - j]];
             }
         } else {
-            copy_group<false>(g, seq_src, seq_dst, seq_n, ob, ws);
+            copy_group(g, seq_src, seq_dst, seq_n, ob);
         }
     }
 }

@@ -8,10 +8,13 @@
 //   L   line kinds: FASTA '>' header / sequence; FASTQ line index mod 4,
 //       with the '@' and '+' checks of a 4-line record; header lines are
 //       scanned into a record index per line
+//   C   every 32 positions of seq from the line (or lines) that hold them,
+//       upper-cased, with their 2-bit codes
+//   N   accession (first header token) and read length per record
+// and, when a sequence line holds whitespace, instead of C
 //   B1  emitted bases per tile (sequence-line bytes that are not whitespace)
 //   B2  emit: base -> seq[emit_prefix + record] upper-cased; a header's first
 //       byte records its read's start
-//   N   accession (first header token) and read length per record
 // Semantics follow PerlLib/Fasta_reader.pm:45-73 (records start at '>' lines,
 // sequence = following lines with whitespace removed), Sequence->new at
 // PerlLib/Fasta_reader.pm:107-118 (accession = first whitespace token), and the
@@ -196,47 +199,6 @@ __global__ void k_fastq_records(uint64_t *__restrict__ line_rec, uint64_t n_line
     if ((j & 3) == 0) hdr_line[j >> 2] = j;
 }
 
-// ---- fast path, copy.  A warp takes 32 consecutive lines (or records): lane l
-// loads line l's metadata (coalesced), header lines record their read's start,
-// and then the warp copies the group's sequence lines in aligned 16-byte
-// output words (copy_group), upper-casing into seq.  A sequence line holding
-// whitespace sets *ws_seen and the byte-wise path redoes the emit.  A warp takes
-// `per` lines, fewer than 32 when there are not 32 for every warp the GPU
-// holds: 10,000 bundle records of 1.4 KB kept 625 warps busy at 32 lines each
-// (0.30 ms).
-static uint32_t lines_per_warp(const tk_ctx *c, uint64_t n) {
-    return (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(32, n / ((uint64_t)c->sm_count * 64)));
-}
-
-__global__ void k_copy_lines(ParseGeom g, const uint64_t *__restrict__ line_end, const uint8_t *__restrict__ kind,
-                             const uint64_t *__restrict__ line_rec, const uint64_t *__restrict__ line_out,
-                             uint64_t n_lines, uint32_t per, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
-                             uint32_t *__restrict__ ws_seen) {
-    const unsigned lane = lane_id();
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    bool ws = false;
-    for (uint64_t j0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; j0 < n_lines; j0 += warps * per) {
-        const uint64_t j = j0 + lane;
-        uint64_t src = 0, dst = 0;
-        uint32_t len = 0;
-        if (lane < per && j < n_lines) {
-            const uint8_t kd = kind[j];
-            const uint64_t rec = line_rec[j];
-            if (rec != ~0ULL) {
-                const uint64_t out = line_out[j] + rec;
-                if (kd == LK_HDR) rd_off[rec] = out;
-                else if (kd == LK_SEQ) {
-                    src = j == 0 ? g.S : line_end[j - 1] + 1;
-                    len = (uint32_t)(line_end[j] - src);
-                    dst = out;
-                }
-            }
-        }
-        copy_group<true>(g, src, dst, len, seq, ws);
-    }
-    if (__any_sync(0xffffffffu, ws) && lane == 0) atomicExch(ws_seen, 1u);
-}
-
 // ---- FASTQ: records of four lines, handled per record (no per-line arrays).
 // Check: the header line starts with '@' and the third with '+' (the first
 // offending line is recorded, as k_line_kinds does); seq_len = the sequence
@@ -252,29 +214,6 @@ __global__ void k_fq_check(ParseGeom g, const uint64_t *__restrict__ line_end, u
     if (fh != '@') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 1)); }
     if (fp != '+') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 3)); }
     seq_len[r] = (uint32_t)(line_end[j + 1] - (h1 + 1));
-}
-
-// A warp takes 32 consecutive records: lane l records read r0 + l's start and
-// holds its sequence line, then the warp copies them as k_copy_lines does.
-__global__ void k_fq_copy(ParseGeom g, const uint64_t *__restrict__ line_end, const uint64_t *__restrict__ seq_off,
-                          uint64_t n_reads, uint32_t per, uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off,
-                          uint32_t *__restrict__ ws_seen) {
-    const unsigned lane = lane_id();
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    bool ws = false;
-    for (uint64_t r0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * per; r0 < n_reads; r0 += warps * per) {
-        const uint64_t r = r0 + lane;
-        uint64_t src = 0, dst = 0;
-        uint32_t len = 0;
-        if (lane < per && r < n_reads) {
-            src = line_end[4 * r] + 1;
-            len = (uint32_t)(line_end[4 * r + 1] - src);
-            dst = seq_off[r] + r;
-            rd_off[r] = dst;
-        }
-        copy_group<true>(g, src, dst, len, seq, ws);
-    }
-    if (__any_sync(0xffffffffu, ws) && lane == 0) atomicExch(ws_seen, 1u);
 }
 
 // per-thread walk over its 32 bytes with the line each byte belongs to
@@ -398,11 +337,41 @@ __global__ void k_names(ParseGeom g, const uint64_t *__restrict__ hdr_line, int 
     if (lane_id() == 0 && L32) atomicMax(max_len, L32);
 }
 
-// The packed read array as 2-bit codes and invalid-position bits: thread j
-// converts positions 32j .. 32j+31 (j = -1 .. n_words-1; the 64 '\n' bytes
-// around `seq` make word -1 all invalid).  Per 4-byte group: the code of
-// A/C/G/T is ((c >> 1) & 3) ^ (its bit 1 moved to bit 0); the group is valid
-// where its bytes equal the letters those codes name.
+// 32 positions of the read array as 2-bit codes and invalid-position bits, four
+// bytes at a time.  Bits 1 and 2 of an upper-case A, C, T, G count 0..3 (code:
+// bit 2, then bit 1 ^ bit 2) and the letter is 0x41 with those bits in, but for
+// T (bit 2 without bit 1), 0x11 off: a byte that differs is invalid.  The four
+// codes, and the four invalid bits, are gathered to the top of a word by one
+// multiply each, whose other terms fall on lower bits of their own.
+// Returns whether an invalid byte was none of 'N', 'J', '\n' and 0x0E (the
+// bytes that are 0x0A under the mask 0xBB): only then can a byte be a lower-case
+// letter, or whitespace inside a line.
+__device__ __forceinline__ bool pack32(const uint32_t (&w)[8], uint64_t &code, uint32_t &bad) {
+    uint32_t other = 0, m[8];
+    bad = 0;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const uint32_t s1 = w[q] >> 1, s2 = w[q] >> 2;
+        const uint32_t x = ((s1 ^ s2) & 0x01010101u) | (s1 & 0x02020202u);
+        const uint32_t t = s2 & ~s1 & 0x01010101u;
+        const uint32_t d = ((w[q] & 0xF9F9F9F9u) ^ 0x41414141u) ^ t ^ (t << 4);
+        const uint32_t nz = (d | ((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu)) & 0x80808080u;   // bit 7 of each differing byte
+        const uint32_t dn = (w[q] & 0xBBBBBBBBu) ^ 0x0A0A0A0Au;
+        other |= nz & (dn | ((dn & 0x7F7F7F7Fu) + 0x7F7F7F7Fu));
+        bad = __funnelshift_l((nz >> 7) * 0x80402010u, bad, 4);                      // position 4q at bit 31
+        m[q] = x * 0x40100401u;                                                        // position 4q at bits 31, 30
+    }
+    // the top byte of each product, the first positions at the top
+    const uint32_t hi = __byte_perm(__byte_perm(m[3], m[2], 0x0073), __byte_perm(m[1], m[0], 0x0073), 0x5410);
+    const uint32_t lo = __byte_perm(__byte_perm(m[7], m[6], 0x0073), __byte_perm(m[5], m[4], 0x0073), 0x5410);
+    code = ((uint64_t)hi << 32) | lo;
+    return other != 0u;
+}
+
+// The codes of the whole read array: thread j converts positions 32j .. 32j+31
+// (j = -1 .. n_words-1; the 64 '\n' bytes around `seq` make word -1 all invalid).
+// After the byte-wise emit, and for a text without reads; otherwise
+// k_seq_tiles has the bases in registers and makes their codes itself.
 __global__ void k_pack_codes(const uint8_t *__restrict__ seq, int64_t n_words, uint64_t *__restrict__ codes,
                              uint32_t *__restrict__ inv) {
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x - 1;
@@ -410,23 +379,189 @@ __global__ void k_pack_codes(const uint8_t *__restrict__ seq, int64_t n_words, u
     const uint4 *v = reinterpret_cast<const uint4 *>(seq + 32 * j);
     const uint4 a = v[0], b = v[1];
     const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint64_t code = 0;
-    uint32_t bad = 0;
-#pragma unroll
-    for (int q = 0; q < 8; q++) {
-        uint32_t x = (w[q] >> 1) & 0x03030303u;
-        x ^= (x >> 1) & 0x01010101u;   // byte b: code of position 4q+b
-        // the letter each code names, compared with the byte itself
-        const uint32_t sel = (x & 3u) | ((x >> 4) & 0x30u) | ((x >> 8) & 0x300u) | ((x >> 12) & 0x3000u);
-        const uint32_t d = w[q] ^ __byte_perm(0x54474341u, 0u, sel);
-        const uint32_t nz = (d | ((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu)) & 0x80808080u;   // bit 7 of each differing byte
-        const uint32_t nib = (((nz >> 7) * 0x08040201u) >> 24) & 0xFu;                  // position 4q at bit 3
-        const uint32_t byte = ((x << 6) & 0xC0u) | ((x >> 4) & 0x30u) | ((x >> 14) & 0x0Cu) | ((x >> 24) & 0x03u);
-        code = (code << 8) | byte;
-        bad = (bad << 4) | nib;
-    }
+    uint64_t code;
+    uint32_t bad;
+    pack32(w, code, bad);
     codes[j] = code;
     inv[j] = bad;
+}
+
+// ---- fast path, copy.  The read array is cut into tiles of 8192 positions, a
+// block each, 32 consecutive positions a thread.  The lines (FASTA) or records
+// (FASTQ) that hold the sequence are numbered along it: line j begins at
+// start(j) and holds line_len[j] bases, position start(j+1) - 1 is a separator
+// if it is not a base; k_line_tiles writes which line each tile begins in.
+template <bool FASTQ>
+struct SeqLines {
+    const uint64_t *line_end, *line_rec, *line_out;   // (line_rec: FASTA)
+    const uint32_t *line_len;
+    uint64_t n, S, seq_len;
+    __device__ __forceinline__ uint64_t start(uint64_t j) const {
+        if (j >= n) return seq_len;
+        if (FASTQ) return line_out[j] + j;
+        const uint64_t rec = line_rec[j];
+        return line_out[j] + (rec == ~0ULL ? 0 : rec);   // (lines before the first record are empty)
+    }
+    __device__ __forceinline__ uint64_t src(uint64_t j) const {
+        return FASTQ ? line_end[4 * j] + 1 : j == 0 ? S : line_end[j - 1] + 1;
+    }
+};
+
+constexpr int ST_THREADS = 256;
+constexpr int ST_BLOCKS = 6;         // an SM: 42 registers a thread
+constexpr uint32_t ST_TILE = ST_THREADS * 32;
+constexpr uint32_t ST_LINES = 512;   // lines of a tile held in shared memory at a time
+
+// Per line: its record's start, and the tiles whose first position it holds.
+template <bool FASTQ>
+__global__ void k_line_tiles(SeqLines<FASTQ> L, const uint8_t *__restrict__ kind, uint64_t *__restrict__ rd_off,
+                             uint64_t *__restrict__ tile_line) {
+    const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= L.n) return;
+    const uint64_t s = L.start(j), e = L.start(j + 1);
+    if (FASTQ) rd_off[j] = s;
+    else if (kind[j] == LK_HDR) rd_off[L.line_rec[j]] = s;
+    for (uint64_t t = (s + ST_TILE - 1) / ST_TILE; t * ST_TILE < e; t++) tile_line[t] = j;
+}
+
+// x = v from byte a (0..31) on
+__device__ __forceinline__ void lay_from(uint32_t (&x)[8], const uint32_t (&v)[8], uint32_t a) {
+#pragma unroll
+    for (int w = 0; w < 8; w++) {
+        const uint32_t from = __funnelshift_lc(0u, ~0u, (uint32_t)max((int)(8 * a) - 32 * w, 0));
+        x[w] = (x[w] & ~from) | (v[w] & from);
+    }
+}
+
+// Copies the sequence lines, upper-cased and with a '\n' after every read, and
+// makes their 2-bit codes.  A thread finds the line of its first position by a
+// binary search over the tile's lines in shared memory, loads the 32 text bytes
+// around each stretch of a line (three aligned 16-byte loads and shifts), lays
+// each next stretch over the words from its first position on, and stores
+// whole 32-byte pieces.  A byte that may be a lower-case letter or whitespace
+// (pack32) takes the slower way of upper-casing; whitespace sets *ws_seen and the
+// byte-wise path redoes the emit.  The bytes around seq become '\n' too.
+// Bound by instructions and, for each block, by three dependent
+// loads before its first base: 3M reads of 100 nt took 377 us with 4 blocks to
+// an SM, 287 with 5, 262 with 6, 380 with 7 (spills).  The warps that copied 32
+// lines in aligned 16-byte words, the fill of the array with '\n' and the pass
+// that made the codes took 286 and 118 us for them, and the fill's 330 MB.
+template <bool FASTQ>
+__global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_seq_tiles(const char *__restrict__ text, uint64_t len, SeqLines<FASTQ> L,
+                                                         const uint64_t *__restrict__ tile_line, uint64_t n_words,
+                                                         uint8_t *__restrict__ seq, uint64_t seq_bytes,
+                                                         uint64_t *__restrict__ codes, uint32_t *__restrict__ inv,
+                                                         uint32_t *__restrict__ ws_seen) {
+    __shared__ uint32_t s_start[ST_LINES + 1], s_end[ST_LINES];
+    __shared__ int64_t s_delta[ST_LINES];   // text position of a base less its place in seq
+    const uint64_t T0 = (uint64_t)blockIdx.x * ST_TILE;
+    const uint32_t q0 = threadIdx.x * 32u;
+    const uint32_t sep[8] = {0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au,
+                             0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au, 0x0A0A0A0Au};
+    uint32_t x[8], held = 0;                // held: positions that are bases
+#pragma unroll
+    for (int w = 0; w < 8; w++) x[w] = sep[w];
+    if (T0 < L.seq_len) {
+        const uint32_t lim = (uint32_t)min((uint64_t)ST_TILE, L.seq_len - T0);
+        const uint32_t qe = min(q0 + 32u, lim);
+        const uint64_t first = tile_line[blockIdx.x];
+        const uint64_t last = T0 + ST_TILE < L.seq_len ? tile_line[blockIdx.x + 1] : L.n - 1;
+        uint32_t q = q0;
+        for (uint64_t c0 = first; c0 <= last; c0 += ST_LINES) {
+            const uint32_t m = (uint32_t)min((uint64_t)ST_LINES, last - c0 + 1);
+            if (c0 != first) __syncthreads();
+            for (uint32_t i = threadIdx.x; i <= m; i += ST_THREADS) {
+                const uint64_t j = c0 + i, s = L.start(j);
+                s_start[i] = s <= T0 ? 0u : (uint32_t)min(s - T0, (uint64_t)ST_TILE);
+                if (i < m) {
+                    const uint64_t e = s + L.line_len[j];
+                    s_end[i] = e <= T0 ? 0u : (uint32_t)min(e - T0, (uint64_t)ST_TILE);
+                    s_delta[i] = (int64_t)L.src(j) - (int64_t)s;
+                }
+            }
+            __syncthreads();
+            const uint32_t stop = min(qe, s_start[m]);
+            if (q < stop) {
+                uint32_t i = 0, hi = m;   // the last line that begins at or before q
+                while (hi - i > 1) {
+                    const uint32_t mid = (i + hi) >> 1;
+                    if (s_start[mid] <= q) i = mid;
+                    else hi = mid;
+                }
+                while (q < stop) {
+                    while (s_start[i + 1] <= q) i++;
+                    const uint32_t e = min(s_end[i], qe);
+                    if (e > q) {
+                        // the text byte that would lie at this thread's first position
+                        const int64_t at = (int64_t)(T0 + q0) + s_delta[i];
+                        const uint32_t a = q - q0;
+                        const uintptr_t p = (uintptr_t)text + (uintptr_t)at, p16 = p & ~(uintptr_t)15;
+                        uint32_t v[8];
+                        if (p16 >= (uintptr_t)text && p16 + 48 <= (uintptr_t)text + len) {
+                            const uint4 *u = reinterpret_cast<const uint4 *>(p16);
+                            const uint4 u0 = __ldg(u), u1 = __ldg(u + 1), u2 = __ldg(u + 2);
+                            uint32_t t[12] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.x, u2.y, u2.z, u2.w};
+                            if (p & 8) {
+#pragma unroll
+                                for (int w = 0; w < 10; w++) t[w] = t[w + 2];
+                            }
+                            if (p & 4) {
+#pragma unroll
+                                for (int w = 0; w < 9; w++) t[w] = t[w + 1];
+                            }
+                            const uint32_t sh = 8u * (uint32_t)(p & 3);
+#pragma unroll
+                            for (int w = 0; w < 8; w++) v[w] = __funnelshift_r(t[w], t[w + 1], sh);
+                        } else {   // at an end of the text
+#pragma unroll
+                            for (int w = 0; w < 8; w++) {
+                                v[w] = 0;
+                                for (uint32_t i4 = 0; i4 < 4; i4++) {
+                                    const uint32_t o = 4 * w + i4;
+                                    if (o >= a && q0 + o < e) v[w] |= (uint32_t)(uint8_t)text[at + o] << (8 * i4);
+                                }
+                            }
+                        }
+                        lay_from(x, v, a);
+                        if (e < q0 + 32u) lay_from(x, sep, e - q0);
+                        held |= (e - q0 >= 32u ? ~0u : (1u << (e - q0)) - 1u) & (~0u << a);
+                    }
+                    q = min(s_start[i + 1], stop);
+                }
+            }
+        }
+    }
+    const uint64_t word = T0 / 32 + threadIdx.x;
+    if (word < n_words) {
+        uint64_t code;
+        uint32_t bad;
+        if (pack32(x, code, bad)) {
+            bool ws = false;
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                const uint32_t in = ((((held >> (4 * w)) & 0xFu) * 0x00204081u) & 0x01010101u) * 0xFFu;
+                x[w] = (upcase_word((x[w] & in) | (0x41414141u & ~in), ws) & in) | (0x0A0A0A0Au & ~in);
+            }
+            if (ws) atomicExch(ws_seen, 1u);
+            pack32(x, code, bad);
+        }
+        uint4 *o = reinterpret_cast<uint4 *>(seq + 32 * word);
+        o[0] = make_uint4(x[0], x[1], x[2], x[3]);
+        o[1] = make_uint4(x[4], x[5], x[6], x[7]);
+        codes[word] = code;
+        inv[word] = bad;
+    }
+    if (blockIdx.x == 0) {
+        if (threadIdx.x < SEQ_PAD / 4) reinterpret_cast<uint32_t *>(seq - SEQ_PAD)[threadIdx.x] = 0x0A0A0A0Au;
+        for (uint64_t i = 32 * n_words + threadIdx.x; i < seq_bytes; i += ST_THREADS) seq[i] = (uint8_t)'\n';
+        if (threadIdx.x == 0) {
+            uint64_t code;
+            uint32_t bad;
+            pack32(sep, code, bad);
+            codes[-1] = code;
+            inv[-1] = bad;
+        }
+    }
 }
 
 // Component id of every bundle record: the integer after "s_" in its
@@ -456,21 +591,42 @@ int component_ids(tk_ctx *c, const tk_reads *b, uint64_t *d_ids) {
     return check_launch(c, "component ids");
 }
 
-// Builds r->d_codes / r->d_inv from r->d_seq (after the last write to seq).
 constexpr uint64_t PARSE_FEW_LINES = 1ull << 22;   // 32 MB of header lines; a round trip is 1% of their 1.2 ms
 
+static uint64_t code_words(const tk_reads *r) { return (r->seq_len + 31) / 32 + 1; }   // without word -1
+
+static int alloc_codes(tk_ctx *c, tk_reads *r) {
+    const uint64_t words = code_words(r) + 1;   // incl. word -1
+    const uint64_t inv_words = (words + 1) & ~1ULL;
+    TK_TRY(dmalloc(c, (void **)&r->d_pack_alloc, words * 8 + inv_words * 4, "2-bit codes"));
+    r->d_codes = r->d_pack_alloc + 1;
+    r->d_inv = reinterpret_cast<uint32_t *>(r->d_pack_alloc + words) + 1;
+    return TK_OK;
+}
+
+// r->d_codes / r->d_inv from r->d_seq
 static int pack_reads(tk_ctx *c, tk_reads *r) {
-    const int64_t n_words = (int64_t)((r->seq_len + 31) / 32) + 1;
-    const uint64_t code_words = (uint64_t)n_words + 1;          // incl. word -1
-    const uint64_t inv_words = ((uint64_t)n_words + 1 + 1) & ~1ULL;
-    TK_TRY(dmalloc(c, (void **)&r->d_pack_alloc, code_words * 8 + inv_words * 4, "2-bit codes"));
-    uint64_t *codes = r->d_pack_alloc + 1;
-    uint32_t *inv = reinterpret_cast<uint32_t *>(r->d_pack_alloc + code_words) + 1;
-    k_pack_codes<<<grid_for((uint64_t)n_words + 1, 256), 256, 0, c->stream>>>(r->d_seq, n_words, codes, inv);
+    TK_TRY(alloc_codes(c, r));
+    const uint64_t n = code_words(r);
+    k_pack_codes<<<grid_for(n + 1, 256), 256, 0, c->stream>>>(r->d_seq, (int64_t)n, const_cast<uint64_t *>(r->d_codes),
+                                                              const_cast<uint32_t *>(r->d_inv));
     c->launches++;
-    r->d_codes = codes;
-    r->d_inv = inv;
     return check_launch(c, "2-bit codes");
+}
+
+template <bool FASTQ>
+static int copy_sequences(tk_ctx *c, tk_reads *r, const SeqLines<FASTQ> &L, const uint8_t *kind, uint64_t seq_bytes) {
+    TK_TRY(alloc_codes(c, r));
+    const uint64_t words = code_words(r), tiles = (words * 32 + ST_TILE - 1) / ST_TILE;
+    uint64_t *tile_line = nullptr;
+    TK_TRY(dmalloc(c, (void **)&tile_line, tiles * 8, "sequence tiles"));
+    k_line_tiles<FASTQ><<<grid_for(L.n, 256), 256, 0, c->stream>>>(L, kind, r->d_rd_off, tile_line);
+    k_seq_tiles<FASTQ><<<(unsigned)tiles, ST_THREADS, 0, c->stream>>>(
+        r->d_text, r->text_len, L, tile_line, words, r->d_seq, seq_bytes, const_cast<uint64_t *>(r->d_codes),
+        const_cast<uint32_t *>(r->d_inv), c->d_err + DE_WS);
+    c->launches += 2;
+    dfree(c, tile_line);
+    return check_launch(c, "sequence copy");
 }
 
 int parse_reads(tk_ctx *c, tk_reads *r) {
@@ -592,19 +748,17 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
     if (!e) e = dmalloc(c, (void **)&r->d_name_len, (n_reads ? n_reads : 1) * 4, "name lengths");
     if (!e) {
         r->d_seq = r->d_seq_alloc + SEQ_PAD;
-        cudaMemsetAsync(r->d_seq_alloc, '\n', seq_alloc, c->stream);
         cudaMemsetAsync(c->d_err + DE_WS, 0, 8, c->stream);   // whitespace seen, the longest read
         uint64_t tail = r->seq_len;
         cudaMemcpyAsync(r->d_rd_off + n_reads, &tail, 8, cudaMemcpyHostToDevice, c->stream);
         uint32_t ws_seen = 0;
-        // accessions and read lengths, the 2-bit codes, and what the host reads back
+        // accessions and read lengths, and what the host reads back
         auto finish = [&]() -> int {
             if (n_tiles && n_reads) {
                 k_names<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, hdr_line, fastq, line_end, n_reads, r->d_rd_off,
                                                                        r->d_name_off, r->d_name_len, d_maxlen);
                 c->launches++;
             }
-            TK_TRY(pack_reads(c, r));
             TK_CUDA(c, cudaMemcpyAsync(c->h_stage, c->d_err + DE_WS, 8, cudaMemcpyDeviceToHost, c->stream));
             TK_CUDA(c, cudaStreamSynchronize(c->stream));
             TK_TRY(wait_status(c));
@@ -613,20 +767,16 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
             r->max_len = h[1];
             return TK_OK;
         };
-        if (n_tiles && n_reads) {
-            const uint64_t n = fastq ? n_reads : n_lines;
-            const uint32_t per = lines_per_warp(c, n);
-            const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + 8ull * per - 1) / (8ull * per),
-                                                                                     (uint64_t)c->sm_count * 32));
-            if (fastq)
-                k_fq_copy<<<grid, 256, 0, c->stream>>>(g, line_end, line_out, n_reads, per, r->d_seq, r->d_rd_off,
-                                                       c->d_err + DE_WS);
-            else
-                k_copy_lines<<<grid, 256, 0, c->stream>>>(g, line_end, kind, line_rec, line_out, n_lines, per, r->d_seq,
-                                                          r->d_rd_off, c->d_err + DE_WS);
-            c->launches++;
+        const uint64_t seq_bytes = seq_alloc - SEQ_PAD;
+        if (n_tiles && n_reads && fastq) {
+            e = copy_sequences(c, r, SeqLines<true>{line_end, nullptr, line_out, line_len, n_reads, g.S, r->seq_len}, nullptr, seq_bytes);
+        } else if (n_tiles && n_reads) {
+            e = copy_sequences(c, r, SeqLines<false>{line_end, line_rec, line_out, line_len, n_lines, g.S, r->seq_len}, kind, seq_bytes);
+        } else {
+            cudaMemsetAsync(r->d_seq_alloc, '\n', seq_alloc, c->stream);
+            e = pack_reads(c, r);
         }
-        e = finish();
+        if (!e) e = finish();
         r->plain_seq = fastq && !ws_seen;
         if (!e && ws_seen) {
             // some sequence line holds spaces, tabs or CRs: redo the emit byte by byte
@@ -661,7 +811,7 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
                 dfree(c, r->d_pack_alloc);   // of the lines as they were
                 r->d_pack_alloc = nullptr;
                 cudaMemsetAsync(d_maxlen, 0, 4, c->stream);
-                e = finish();
+                if (!(e = pack_reads(c, r))) e = finish();
             } while (0);
         }
     }

@@ -1,5 +1,5 @@
-// tk_text.cuh -- copying stretches of the input text with whole warps, shared
-// by the parser (sequence lines into the read array) and the FASTA writer.
+// tk_text.cuh -- the parsed text's geometry, upper-casing, and copying
+// stretches of the input text with whole warps (the FASTA writer).
 #pragma once
 #include "tk_internal.cuh"
 
@@ -65,8 +65,7 @@ __device__ __forceinline__ uint32_t upcase_word(uint32_t x, bool &ws) {
 }
 
 // The warp copies the lines its lanes hold (lane l: text[src, src + len) to
-// seq + dst; len 0 = none); with UP it upper-cases them and notes whether a
-// line held whitespace.  The output is cut into the aligned 16-byte words the
+// seq + dst; len 0 = none).  The output is cut into the aligned 16-byte words the
 // lines touch; the warp numbers the words of its 32 lines one after another (a scan
 // of each line's word count) and each lane takes every 32nd, so the lanes stay
 // busy whatever the line lengths; a lane finds its word's line by a binary
@@ -74,9 +73,8 @@ __device__ __forceinline__ uint32_t upcase_word(uint32_t x, bool &ws) {
 // is one 16-byte store; the first and last word of a line (shared with the
 // separator and the neighbouring line) are stored byte by byte.  seq is
 // 16-byte aligned.
-template <bool UP>
 __device__ __forceinline__ void copy_group(const ParseGeom &g, uint64_t src, uint64_t dst, uint32_t len,
-                                           uint8_t *__restrict__ seq, bool &ws) {
+                                           uint8_t *__restrict__ seq) {
     const unsigned lane = lane_id();
     const uint32_t nw = len ? (uint32_t)(((dst + len + 15) >> 4) - (dst >> 4)) : 0u;
     uint32_t incl = nw;
@@ -106,9 +104,6 @@ __device__ __forceinline__ void copy_group(const ParseGeom &g, uint64_t src, uin
         const int64_t so = (int64_t)out - (int64_t)d_i;            // its offset in the line
         uint32_t x[4], in[4];
         line_word16(g, s_i, so, n_i, x, in);
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (UP) x[q] = upcase_word(x[q], ws);
         uint8_t *o = seq + out;
         if (so >= 0 && so + 16 <= (int64_t)n_i) {
             *reinterpret_cast<uint4 *>(o) = make_uint4(x[0], x[1], x[2], x[3]);
