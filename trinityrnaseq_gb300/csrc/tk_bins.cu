@@ -26,6 +26,7 @@
 // Each bin's dump equals a separate plain `jellyfish count` + `dump -L m` of
 // that bin (sorted by key).
 #include "tk_warp.cuh"
+#include "tk_emit.cuh"
 
 #include <algorithm>
 #include <atomic>
@@ -279,11 +280,21 @@ __global__ void k_bin_bounds(const uint64_t *__restrict__ keys, const uint64_t *
     first[b] = lo;
 }
 
-__global__ void k_bin_text_bounds(const uint64_t *__restrict__ first, const uint64_t *__restrict__ off, uint64_t n,
-                                  uint64_t total, uint32_t n_bins, uint64_t *__restrict__ text0) {
-    uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
+// Where every bin's text begins: the place of its first record's block of
+// DUMP_BLOCK records, and the records of that block before it (a warp per bin).
+__global__ void k_bin_text_bounds(const uint64_t *__restrict__ first, const uint64_t *__restrict__ off,
+                                  const uint32_t *__restrict__ cnt, uint64_t n, int k, uint64_t total, uint32_t n_bins,
+                                  uint64_t *__restrict__ text0) {
+    const uint32_t b = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (b > n_bins) return;
-    text0[b] = first[b] < n ? off[first[b]] : total;
+    const uint64_t i = first[b];
+    uint64_t at = total;
+    if (i < n) {
+        uint32_t before = 0;
+        for (uint64_t j = i / DUMP_BLOCK * DUMP_BLOCK + lane_id(); j < i; j += 32) before += 3u + dec_digits(cnt[j]) + (uint32_t)k;
+        at = off[i / DUMP_BLOCK] + warp_sum(before);
+    }
+    if (lane_id() == 0) text0[b] = at;
 }
 
 static double hll32(const uint32_t *r) {
@@ -667,7 +678,7 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
         e = format_dump(c, keys, cnts, hn, k, &d_dump, &text_len, &offs);
     }
     if (!e) {
-        k_bin_text_bounds<<<(n_bins + 256) / 256, 256, 0, c->stream>>>(first, offs, hn, text_len, n_bins, d_text0);
+        k_bin_text_bounds<<<n_bins / 8 + 1, 256, 0, c->stream>>>(first, offs, cnts, hn, k, text_len, n_bins, d_text0);
         c->launches++;
         out->text0.resize(n_bins + 1);
         e = cuda_check(c, cudaMemcpyAsync(out->text0.data(), d_text0, (n_bins + 1) * 8, cudaMemcpyDeviceToHost, c->stream),

@@ -481,7 +481,9 @@ void prof_add_units(tk_ctx *c, int kid, uint64_t units);
 int check_launch(tk_ctx *c, const char *what);
 int scan_excl_u64(tk_ctx *c, const uint64_t *in, uint64_t *out, uint64_t n, uint64_t *total_host);
 int scan_excl_u32_to_u64(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *total_host);
-// K4 formatting of sorted (key, count) pairs (tk_table.cu)
+// K4 formatting of sorted (key, count) pairs (tk_table.cu).  offs_out: the place in the text of every
+// DUMP_BLOCK-th record.
+constexpr int DUMP_BLOCK = 256;
 int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n, int k, char **text, uint64_t *len,
                 uint64_t **offs_out = nullptr);
 // The scan without waiting for it: the total goes to *d_total on the GPU.  When its bounded wait runs out

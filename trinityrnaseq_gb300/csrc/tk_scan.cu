@@ -38,7 +38,8 @@ struct ScanHead {
     unsigned int err, ticket;
 };
 
-__device__ __forceinline__ void load4(const uint32_t *in, uint64_t (&x)[4]) {
+template <typename P>
+__device__ __forceinline__ void load4(const uint32_t *in, P (&x)[4]) {
     const uint4 v = __ldg(reinterpret_cast<const uint4 *>(in));
     x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
 }
@@ -47,13 +48,15 @@ __device__ __forceinline__ void load4(const uint64_t *in, uint64_t (&x)[4]) {
     x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
 }
 
-// what the scan adds up for an input item
+// what the scan adds up for an input item, and the type that holds a tile's sum
 struct ItemItself {
+    using Part = uint64_t;
     __device__ __forceinline__ uint64_t operator()(uint64_t x) const { return x; }
 };
 struct RecordLength {   // ">COUNT\nKMER\n"
+    using Part = uint32_t;
     int k;
-    __device__ __forceinline__ uint64_t operator()(uint64_t count) const { return 3u + dec_digits((uint32_t)count) + (uint32_t)k; }
+    __device__ __forceinline__ uint32_t operator()(uint32_t count) const { return 3u + dec_digits(count) + (uint32_t)k; }
 };
 
 // A warp owns 512 consecutive items, four rounds of four per lane (16-byte
@@ -61,8 +64,9 @@ struct RecordLength {   // ">COUNT\nKMER\n"
 // an item for u32 input.  The three-kernel scan this replaces (reduce, one
 // block over the tile sums, and a pass whose threads each walked 16
 // consecutive items) took 10.5 us of kernels for 12,000 items and 45 us for 17M,
-// and read its input twice.
-template <typename Tin, typename F>
+// and read its input twice.  With EVERY > 1 only every EVERY-th item's sum is
+// stored, at out[i / EVERY].
+template <typename Tin, typename F, int EVERY>
 __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
                                                     int vec, ScanHead *__restrict__ head, uint64_t *__restrict__ state,
                                                     uint64_t *__restrict__ total_at, uint32_t *__restrict__ err_at) {
@@ -76,7 +80,8 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
     const uint64_t tile = s_tile;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
     const uint64_t first = tile * SN_TILE + (uint64_t)warp * (SN_TILE / SN_WARPS) + lane * 4;
-    uint64_t x[SN_ROUNDS][4], pre[SN_ROUNDS], run = 0;
+    using P = typename F::Part;
+    P x[SN_ROUNDS][4], pre[SN_ROUNDS], run = 0;
 #pragma unroll
     for (int r = 0; r < SN_ROUNDS; r++) {
         const uint64_t i = first + (uint64_t)r * 128;
@@ -84,7 +89,7 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
             load4(in + i, x[r]);
         } else {
 #pragma unroll
-            for (int j = 0; j < 4; j++) x[r][j] = i + j < n ? (uint64_t)in[i + j] : 0;
+            for (int j = 0; j < 4; j++) x[r][j] = i + j < n ? (P)in[i + j] : 0;
         }
 #pragma unroll
         for (int j = 0; j < 4; j++)
@@ -92,8 +97,8 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
     }
 #pragma unroll
     for (int r = 0; r < SN_ROUNDS; r++) {
-        const uint64_t s = x[r][0] + x[r][1] + x[r][2] + x[r][3];
-        const uint64_t inc = warp_incl_scan(s);
+        const P s = x[r][0] + x[r][1] + x[r][2] + x[r][3];
+        const P inc = warp_incl_scan(s);
         pre[r] = run + inc - s;
         run += __shfl_sync(0xffffffffu, inc, 31);
     }
@@ -148,7 +153,10 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
         o[0] = base + pre[r];
 #pragma unroll
         for (int j = 1; j < 4; j++) o[j] = o[j - 1] + x[r][j - 1];
-        if (vec && i + 4 <= n) {
+        if (EVERY > 1) {
+            static_assert(EVERY == 1 || EVERY % 4 == 0, "a lane's first item of four");
+            if (i < n && i % EVERY == 0) out[i / EVERY] = o[0];
+        } else if (vec && i + 4 <= n) {
             ulonglong2 *q = reinterpret_cast<ulonglong2 *>(out + i);
             q[0] = make_ulonglong2(o[0], o[1]);
             q[1] = make_ulonglong2(o[2], o[3]);
@@ -171,15 +179,15 @@ int wait_status(tk_ctx *c) {
 }
 
 // The scan enqueued, its head left in *mem (the caller frees it).
-template <typename Tin, typename F>
+template <typename Tin, int EVERY, typename F>
 static int scan_enqueue(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_at, ScanHead **mem) {
     const uint64_t nt = (n + SN_TILE - 1) / SN_TILE;
     const size_t bytes = sizeof(ScanHead) + nt * 8;
     TK_TRY(dmalloc(c, (void **)mem, bytes, "scan tiles"));
     int e = cuda_check(c, cudaMemsetAsync(*mem, 0, bytes, c->stream), "scan reset");
     if (!e) {
-        const int vec = (((uintptr_t)in | (uintptr_t)out) & 15u) == 0;
-        k_scan<Tin, F><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, *mem, reinterpret_cast<uint64_t *>(*mem + 1),
+        const int vec = (((uintptr_t)in | (EVERY > 1 ? 0 : (uintptr_t)out)) & 15u) == 0;
+        k_scan<Tin, F, EVERY><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, *mem, reinterpret_cast<uint64_t *>(*mem + 1),
                                                                   total_at, c->d_err + DE_COUNT);
         c->launches++;
         e = check_launch(c, "scan");
@@ -187,12 +195,12 @@ static int scan_enqueue(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n
     return e;
 }
 
-template <typename Tin, typename F>
+template <typename Tin, int EVERY = 1, typename F>
 static int scan_impl(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, uint64_t *total_host) {
     *total_host = 0;
     if (n == 0) return TK_OK;
     ScanHead *head = nullptr, h;
-    int e = scan_enqueue<Tin>(c, f, in, out, n, nullptr, &head);
+    int e = scan_enqueue<Tin, EVERY>(c, f, in, out, n, nullptr, &head);
     if (!e) e = cuda_check(c, cudaMemcpyAsync(&h, head, sizeof h, cudaMemcpyDeviceToHost, c->stream), "scan total");
     if (!e) e = cuda_check(c, cudaStreamSynchronize(c->stream), "scan total sync");
     if (head) dfree(c, head);
@@ -210,7 +218,7 @@ static int scan_impl(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n, u
 int scan_excl_u32_to_u64_async(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t n, uint64_t *d_total) {
     if (n == 0) return cuda_check(c, cudaMemsetAsync(d_total, 0, 8, c->stream), "scan total");
     ScanHead *head = nullptr;
-    int e = scan_enqueue<uint32_t>(c, ItemItself{}, in, out, n, d_total, &head);
+    int e = scan_enqueue<uint32_t, 1>(c, ItemItself{}, in, out, n, d_total, &head);
     if (!e) e = cuda_check(c, cudaMemcpyAsync(c->h_wait_err, c->d_err + DE_COUNT, 4, cudaMemcpyDeviceToHost, c->stream),
                            "scan status");
     if (head) dfree(c, head);
@@ -227,7 +235,7 @@ int scan_excl_u32_to_u64(tk_ctx *c, const uint32_t *in, uint64_t *out, uint64_t 
 
 // Offsets of the dump records of n counts (k-mers of k bases).
 int scan_record_lengths(tk_ctx *c, const uint32_t *counts, uint64_t *out, uint64_t n, int k, uint64_t *total_host) {
-    return scan_impl<uint32_t>(c, RecordLength{k}, counts, out, n, total_host);
+    return scan_impl<uint32_t, DUMP_BLOCK>(c, RecordLength{k}, counts, out, n, total_host);
 }
 
 // ------------------------------------------------------------------ radix sort

@@ -716,30 +716,34 @@ __global__ void __launch_bounds__(HS_THREADS) k_histo(const Slot *__restrict__ s
 
 // K4: each thread formats one record into the block's shared-memory buffer,
 // then the block stores its records' bytes in aligned 16-byte pieces.  Bound by
-// the formatting's instructions (issue slots 70% busy) and memory (53%): 22M
-// records 0.24 ms; with a lane's letters stored one by one and a warp's text
-// leaving byte by byte 0.38, and 0.06 for a pass over the counts for the record
-// lengths that the scan now takes from the counts itself.
-constexpr int DW_THREADS = 256;
+// the formatting's instructions (issue slots 70% busy) and memory (53%).  The
+// block scans its records' lengths itself, so that only its first record's place
+// comes from memory: 22M records 0.265 ms and 0.066 for the scan of the lengths;
+// with a place for every record 0.243 and 0.137.  (With a lane's letters stored
+// one by one and a warp's text leaving byte by byte 0.38.)
+constexpr int DW_THREADS = DUMP_BLOCK;
 constexpr int DW_BYTES = (DW_THREADS * (3 + 10 + MAX_K) + 16 + 15) & ~15;
 
 __global__ void __launch_bounds__(DW_THREADS) k_dump_write(const uint64_t *__restrict__ keys,
                                                           const uint32_t *__restrict__ cnt,
                                                           const uint64_t *__restrict__ off, uint64_t n, int k,
-                                                          uint64_t total, char *__restrict__ out) {
+                                                          char *__restrict__ out) {
     __shared__ __align__(16) char buf[DW_BYTES];
-    const uint64_t i0 = (uint64_t)blockIdx.x * DW_THREADS, i = i0 + threadIdx.x;
-    const uint64_t w0 = off[i0], w1 = i0 + DW_THREADS < n ? off[i0 + DW_THREADS] : total;
+    __shared__ uint32_t sm[DW_THREADS / 32 + 1];
+    const uint64_t i = (uint64_t)blockIdx.x * DW_THREADS + threadIdx.x;
+    const uint64_t w0 = off[blockIdx.x];
+    const uint32_t c = i < n ? cnt[i] : 0u, d = dec_digits(c);
+    uint32_t bytes;
+    const uint32_t at = block_excl_scan<uint32_t>(i < n ? 3u + d + (uint32_t)k : 0u, sm, &bytes);
     if (i < n) {
-        char *p = buf + (w0 & 15) + (off[i] - w0);
-        const uint32_t c = cnt[i];
+        char *p = buf + (w0 & 15) + at;
         *p++ = '>';
-        p = put_dec(p, c, dec_digits(c));
+        p = put_dec(p, c, d);
         *p++ = '\n';
         put_kmer_line(p, keys[i], k);
     }
     __syncthreads();
-    block_store(buf, out, w0, (uint32_t)(w1 - w0));
+    block_store(buf, out, w0, bytes);
 }
 
 // dump records parsed as reads: name = decimal count, sequence = k-mer
@@ -1382,8 +1386,9 @@ int table_sorted_pairs(tk_table *t, uint32_t min_count, uint64_t **keys_out, uin
 }
 
 // K4: format sorted pairs as ">COUNT\nKMER\n" into a device buffer (the low
-// 2k bits of each key); with offs_out, the n record start offsets are handed
-// to the caller (its device block to free) instead of freed.
+// 2k bits of each key); with offs_out, the places in the text of every
+// DUMP_BLOCK-th record are handed to the caller (its device block to free)
+// instead of freed.
 int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n, int k, char **text_out,
                 uint64_t *len_out, uint64_t **offs_out) {
     *text_out = nullptr;
@@ -1391,7 +1396,7 @@ int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n
     if (offs_out) *offs_out = nullptr;
     if (n == 0) return TK_OK;
     uint64_t *offs = nullptr;
-    TK_TRY(dmalloc(c, (void **)&offs, n * 8, "dump offsets"));
+    TK_TRY(dmalloc(c, (void **)&offs, (n + DUMP_BLOCK - 1) / DUMP_BLOCK * 8, "dump offsets"));
     uint64_t total = 0;
     cudaEvent_t ev;
     prof_begin(c, TK_KID_DUMP, &ev);
@@ -1399,7 +1404,7 @@ int format_dump(tk_ctx *c, const uint64_t *keys, const uint32_t *cnt, uint64_t n
     char *text = nullptr;
     if (!e) e = dmalloc(c, (void **)&text, total, "dump text");
     if (!e) {
-        k_dump_write<<<grid_for(n, DW_THREADS), DW_THREADS, 0, c->stream>>>(keys, cnt, offs, n, k, total, text);
+        k_dump_write<<<grid_for(n, DW_THREADS), DW_THREADS, 0, c->stream>>>(keys, cnt, offs, n, k, text);
         c->launches++;
         e = check_launch(c, "dump write");
     }
