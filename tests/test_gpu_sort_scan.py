@@ -47,3 +47,24 @@ def test_sort_of_keys_with_one_digit_apart(ctx):
     t.load_pairs(keys[::-1].copy(), np.arange(n, 0, -1).astype(np.uint32))
     gk, gc = t.dump(1)
     assert np.array_equal(gk, keys) and np.array_equal(gc, np.arange(1, n + 1))
+
+
+@pytest.mark.parametrize("k,low", [(25, 10), (24, 8), (31, 6), (13, 10), (9, 10), (5, 2)])
+@pytest.mark.parametrize("lens", [[1, 2, 3], [63, 64], [65, 66, 1], [700, 1024, 5], [1024]])
+def test_runs_of_keys_alike_but_for_their_last_bits(ctx, k, low, lens):
+    """Keys that agree in all but the bits no radix pass sorts: runs shorter and
+    longer than those ranked by comparing (64), whole and across the edges of
+    tiles (1024), and tables with every key of the last bits."""
+    rng = np.random.default_rng(k)
+    tops = min(1 << (2 * k - low), 3 * 152 if max(lens) > 64 else 3000)
+    parts = []
+    for i in range(tops):
+        n = min(int(lens[i % len(lens)]), 1 << low)
+        parts.append((np.uint64(i * 7 % (1 << (2 * k - low))) << np.uint64(low)) + rng.choice(1 << low, n, replace=False).astype(np.uint64))
+    keys = rng.permutation(np.unique(np.concatenate(parts)))
+    counts = (np.arange(keys.size, dtype=np.uint32) * 31) % 10_007 + 1
+    t = KmerTable(ctx, k, False)
+    t.load_pairs(keys, counts)
+    gk, gc = t.dump(1)
+    order = np.argsort(keys)
+    assert np.array_equal(gk, keys[order]) and np.array_equal(gc, counts[order])

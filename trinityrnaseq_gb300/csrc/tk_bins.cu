@@ -646,7 +646,7 @@ static int bins_run(tk_ctx *c, const char *text, uint64_t len, int where, const 
             const uint64_t o = goff[g], m = goff[g + 1] - o;
             if (m == 0) continue;
             bool t = false;
-            e = radix_sort_pairs(c, k0 + o, v0 + o, m, bits, k1 + o, v1 + o, &t);
+            e = sort_distinct_pairs(c, k0 + o, v0 + o, m, bits, k1 + o, v1 + o, &t);
             in_tmp[g] = t;
             if (m > 1 && final_tmp < 0) final_tmp = t ? 1 : 0;
         }

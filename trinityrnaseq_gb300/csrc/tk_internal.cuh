@@ -494,6 +494,9 @@ int scan_record_lengths(tk_ctx *c, const uint32_t *counts, uint64_t *out, uint64
 int wait_status(tk_ctx *c);
 int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits,
                      uint64_t *tmp_keys, uint32_t *tmp_vals, bool *result_in_tmp, int first_bit = 0);
+// The same for distinct keys whose bits from `bits` on are 0, with fewer passes.
+int sort_distinct_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits, uint64_t *tmp_keys,
+                        uint32_t *tmp_vals, bool *result_in_tmp);
 int table_alloc(tk_table *t, uint64_t capacity);
 void table_fill_empty(tk_ctx *c, Slot *slots, uint64_t n, uint64_t init_val);
 int table_alloc_init(tk_table *t, uint64_t capacity, uint64_t init_val);

@@ -306,7 +306,8 @@ __global__ void __launch_bounds__(RC_THREADS) k_rs_count(const uint64_t *__restr
 // Bound by the ranking's instructions and the tile's shared-memory gathers
 // (ALU 56%, L1 59% of peak): 3.0 TB/s at 24 bytes a pair and pass.  Seven
 // passes over 50 bits: 22M pairs 1.34 ms (2.05 before, with a histogram, a
-// scan and a scatter kernel per pass), 140M 8.0, 30,000 0.076.  Tiles of 3840
+// scan and a scatter kernel per pass), 140M 8.0, 30,000 0.076 (distinct keys take
+// five, see k_sort_runs).  Tiles of 3840
 // pairs (384 threads, three blocks per SM) from 1024 pairs per SM on (300,000
 // pairs: 0.096 against 0.102 ms); below that tiles of 1024, whose shorter
 // work is what counts (30,000 pairs: 0.076 against 0.089).  512 x 8, 512 x 12,
@@ -517,6 +518,113 @@ int radix_sort_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int 
     if (n >= (uint64_t)c->sm_count * 1024)
         return sort_run<384, 10>(c, keys, vals, tmp_keys, tmp_vals, n, passes, first_bit);
     return sort_run<256, 4>(c, keys, vals, tmp_keys, tmp_vals, n, passes, first_bit);
+}
+
+// ---- the last bits of a sort of distinct keys.  With the pairs in order of all
+// but their r <= 10 lowest bits, the keys that agree in the rest form runs of at
+// most 2^r, short ones mostly (k-mers that differ in their last bases), and every
+// run is put in order in place.  A thread ranks its key among the keys of its
+// run, FX_NEAR or fewer, by comparing; a longer run is ranked by its block
+// through a bitmap of its lowest bits (the keys are distinct).  A run belongs to
+// the block that holds its first pair; a block that reads a neighbour's run while
+// that is reordered sees only its upper bits, which are the same in every order.
+// Bound by instructions (issue slots 81% busy): 22M pairs 92 us, 39M 194 us, where
+// the two passes it saves of seven over 50 bits took 355 and 618 (counting with
+// five digits takes 59 us for 68): 1.31 -> 1.05 ms for the sort of 22M. 10 bits, so
+// that 25-mers save two passes and a run fits one block with four keys a thread.
+constexpr int FX_THREADS = 256, FX_ITEMS = 4, FX_TILE = FX_THREADS * FX_ITEMS;
+constexpr int FX_NEAR = 64;
+constexpr int FX_BITS = 10;
+
+__global__ void __launch_bounds__(FX_THREADS) k_sort_runs(uint64_t *keys, uint32_t *vals, uint64_t n, int r) {
+    static_assert(FX_TILE >= (1 << FX_BITS) && FX_THREADS >= FX_NEAR, "a run fits a block");
+    __shared__ uint64_t s[FX_TILE + FX_NEAR + 1];   // the pair before the tile, the tile, FX_NEAR pairs behind it
+    __shared__ uint32_t s_long[FX_TILE / FX_NEAR + 1], n_long, map[1 << (FX_BITS - 5)], below[1 << (FX_BITS - 5)];
+    const uint64_t t0 = (uint64_t)blockIdx.x * FX_TILE;
+    const int tid = (int)threadIdx.x;
+    const int from = t0 ? 0 : 1;                                                      // valid places: [from, end)
+    const int end = 1 + (int)min(n - t0, (uint64_t)(FX_TILE + FX_NEAR));
+    if (tid == 0) n_long = 0;
+    for (int j = from + tid; j < end; j += FX_THREADS) s[j] = keys[t0 + j - 1];
+    __syncthreads();
+    int to[FX_ITEMS + 1];
+    uint32_t val[FX_ITEMS + 1];
+#pragma unroll
+    for (int u = 0; u <= FX_ITEMS; u++) {
+        to[u] = -1;
+        const int j = 1 + u * FX_THREADS + tid;   // (the last round: the pairs behind the tile)
+        if (j >= end || j > FX_TILE + FX_NEAR) continue;
+        const uint64_t key = s[j], top = key >> r;
+        const bool prev = j > from && s[j - 1] >> r == top, next = j + 1 < end && s[j + 1] >> r == top;
+        if (!prev && !next) continue;
+        int a = j, less = 0;
+        while (a > from && j - a <= FX_NEAR && s[a - 1] >> r == top) less += s[--a] < key;
+        if (a == 0 || a > FX_TILE || j - a > FX_NEAR) continue;   // another block's run, or a long one
+        int b = j + 1;
+        while (b < end && b - a <= FX_NEAR && s[b] >> r == top) less += s[b++] < key;
+        if (b - a > FX_NEAR) {
+            if (a == j) s_long[atomicAdd(&n_long, 1u)] = (uint32_t)j;
+            continue;
+        }
+        if (a + less != j) {
+            to[u] = a + less;
+            val[u] = vals[t0 + j - 1];
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u <= FX_ITEMS; u++) {
+        if (to[u] < 0) continue;
+        keys[t0 + to[u] - 1] = s[1 + u * FX_THREADS + tid];
+        vals[t0 + to[u] - 1] = val[u];
+    }
+    for (uint32_t q = 0; q < n_long; q++) {
+        const uint64_t g0 = t0 + s_long[q] - 1, top = s[s_long[q]] >> r;
+        uint64_t key[FX_ITEMS];
+        bool in[FX_ITEMS];
+        for (int i = tid; i < 1 << (FX_BITS - 5); i += FX_THREADS) map[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < FX_ITEMS; u++) {
+            const uint64_t g = g0 + u * FX_THREADS + tid;
+            in[u] = false;
+            if (g >= n) continue;
+            key[u] = keys[g];
+            in[u] = key[u] >> r == top;
+            if (!in[u]) continue;
+            val[u] = vals[g];
+            const uint32_t low = (uint32_t)key[u] & ((1u << r) - 1u);
+            atomicOr(&map[low >> 5], 1u << (low & 31u));
+        }
+        __syncthreads();
+        if (tid < 32) {
+            const uint32_t c = __popc(map[tid]);
+            below[tid] = warp_incl_scan(c) - c;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int u = 0; u < FX_ITEMS; u++) {
+            if (!in[u]) continue;
+            const uint32_t low = (uint32_t)key[u] & ((1u << r) - 1u);
+            const uint64_t g = g0 + below[low >> 5] + __popc(map[low >> 5] & ((1u << (low & 31u)) - 1u));
+            keys[g] = key[u];
+            vals[g] = val[u];
+        }
+        __syncthreads();
+    }
+}
+
+// Sorts pairs of distinct keys by their lowest `bits` bits (the others are 0):
+// 8-bit passes over the upper bits and k_sort_runs for up to FX_BITS lowest ones.
+int sort_distinct_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, int bits, uint64_t *tmp_keys,
+                        uint32_t *tmp_vals, bool *result_in_tmp) {
+    const int passes = std::max(1, (bits - FX_BITS + 7) / 8), low = std::max(0, bits - 8 * passes);
+    TK_TRY(radix_sort_pairs(c, keys, vals, n, bits - low, tmp_keys, tmp_vals, result_in_tmp, low));
+    if (low == 0 || n <= 1) return TK_OK;
+    k_sort_runs<<<(unsigned)((n + FX_TILE - 1) / FX_TILE), FX_THREADS, 0, c->stream>>>(
+        *result_in_tmp ? tmp_keys : keys, *result_in_tmp ? tmp_vals : vals, n, low);
+    c->launches++;
+    return check_launch(c, "sort runs");
 }
 
 }  // namespace tk

@@ -1365,7 +1365,7 @@ int table_sorted_pairs(tk_table *t, uint32_t min_count, uint64_t **keys_out, uin
     if (!e && hn > 1) {
         cudaEvent_t ev;
         prof_begin(c, TK_KID_SORT, &ev);
-        e = radix_sort_pairs(c, k0, v0, hn, 2 * t->k, k1, v1, &in_tmp);
+        e = sort_distinct_pairs(c, k0, v0, hn, 2 * t->k, k1, v1, &in_tmp);
         prof_end(c, TK_KID_SORT, ev, hn);
     }
     if (d_n) dfree(c, d_n);
