@@ -367,3 +367,31 @@ def test_copied_lines_and_codes(ctx, oracle, case, fastq, shift):
     t = KmerTable(ctx, 5, True)
     t.add(rs)
     assert_pairs(t.dump(1), oracle.count(text, 5, True))
+
+
+@pytest.mark.parametrize("shift", [0, 1, 3, 7])
+@pytest.mark.parametrize("fastq", [False, True])
+def test_accessions_of_every_length(ctx, fastq, shift):
+    """First header tokens of 0 to 40 bytes, ended by each kind of whitespace, by
+    the line's end and by the text's, at every alignment of the text's words."""
+    import torch
+    seps = [b"", b" x", b"\tx", b"\r", b"\x0bx", b"\x0cx", b" ", b"\x0e y", b"\x80\x89\xa0 z"]
+    names, out = [], []
+    for i in range(41 * len(seps)):
+        name = (b"abcdefghijklmnopqrstuvwxyz/123456789_.:-|"[:i % 41])
+        sep = seps[i // 41]
+        cut = name + sep.split(b" ")[0] if sep[:1] in (b"\x0e", b"\x80") else name
+        names.append(cut)
+        out.append((b"@%s%s\nACGT\n+\nIIII\n" if fastq else b">%s%s\nACGT\n") % (name, sep))
+    if not fastq:
+        out.append(b">last_one")
+        names.append(b"last_one")
+    text = b"".join(out)
+    dev = torch.zeros(len(text) + shift, dtype=torch.uint8, device="cuda:0")
+    dev[shift:] = torch.frombuffer(bytearray(text), dtype=torch.uint8).to("cuda:0")
+    torch.cuda.synchronize()
+    rs = ReadSet(ctx, dev.data_ptr() + shift, len(text), device=True)
+    noff, nlen = np.zeros(rs.n_reads, np.uint64), np.zeros(rs.n_reads, np.uint32)
+    ctx.check(rs.lib.tk_reads_names(rs.h, noff.ctypes.data, nlen.ctypes.data), "names")
+    assert [text[int(o):int(o) + int(n)] for o, n in zip(noff, nlen)] == names
+    assert rs.max_len == 4

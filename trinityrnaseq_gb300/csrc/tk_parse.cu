@@ -199,21 +199,70 @@ __global__ void k_fastq_records(uint64_t *__restrict__ line_rec, uint64_t n_line
     if ((j & 3) == 0) hdr_line[j >> 2] = j;
 }
 
+// The accession of the header line [ls, le): where the first whitespace after
+// its first byte is (le if there is none), and that first byte.  Aligned
+// 8-byte words of the text, byte by byte at its ends: every load of a warp
+// touches 32 headers, so that fewer loads are what counts.
+__device__ __forceinline__ uint64_t accession_end(const ParseGeom &g, uint64_t ls, uint64_t le, uint32_t &first) {
+    first = 0;
+    if (ls >= le) return ls + 1;   // an empty line
+    const uintptr_t text = (uintptr_t)g.text, end = text + g.len, at = text + ls;
+    uintptr_t w = at & ~(uintptr_t)7;
+    uint64_t q = ls + 1;
+    if (w >= text) {
+        uint64_t skip = ~0ULL << (8 * (uint32_t)(at & 7)) << 8;   // the bytes after the first
+        if (w + 8 <= end) first = (uint32_t)(__ldg(reinterpret_cast<const unsigned long long *>(w)) >> (8 * (uint32_t)(at & 7))) & 0xFFu;
+        else first = (uint8_t)g.text[ls];
+        while (w + 8 <= end) {
+            const uint64_t v = __ldg(reinterpret_cast<const unsigned long long *>(w));
+            const uint64_t m = (((uint64_t)ws_bytes((uint32_t)(v >> 32)) << 32) | ws_bytes((uint32_t)v)) & skip;
+            if (m) return min((uint64_t)(w - text) + (uint64_t)((__ffsll((long long)m) - 1) >> 3), le);
+            w += 8;
+            skip = ~0ULL;
+            q = w - text;
+            if (q >= le) return le;
+        }
+    } else {
+        first = (uint8_t)g.text[ls];
+    }
+    if (q < ls + 1) q = ls + 1;
+    while (q < le && !is_ws((uint8_t)g.text[q])) q++;
+    return q;
+}
+
 // ---- FASTQ: records of four lines, handled per record (no per-line arrays).
-// Check: the header line starts with '@' and the third with '+' (the first
-// offending line is recorded, as k_line_kinds does); seq_len = the sequence
-// line's length.
-__global__ void k_fq_check(ParseGeom g, const uint64_t *__restrict__ line_end, uint64_t n_reads,
-                           uint32_t *__restrict__ seq_len, uint32_t *__restrict__ err) {
+// The header line starts with '@' and the third with '+' (the first offending
+// line is recorded, as k_line_kinds does); the accession; the sequence line's
+// length, and the longest (the reads' lengths if no line holds whitespace).
+// A record's line ends are two 16-byte loads, the one before them is the
+// neighbouring lane's last.  3M records: 196 us, where a pass over the records for
+// the checks and one after the copy for the accessions, byte by byte, took 107
+// and 188.
+__global__ void k_fq_records(ParseGeom g, const uint64_t *__restrict__ line_end, uint64_t n_reads,
+                             uint32_t *__restrict__ seq_len, uint64_t *__restrict__ name_off,
+                             uint32_t *__restrict__ name_len, uint32_t *__restrict__ err) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_reads) return;
-    const uint64_t j = 4 * r;
-    const uint64_t h0 = j == 0 ? g.S : line_end[j - 1] + 1, h1 = line_end[j];
-    const uint64_t p0 = line_end[j + 1] + 1, p1 = line_end[j + 2];
-    const uint32_t fh = h1 > h0 ? (uint8_t)g.text[h0] : 0u, fp = p1 > p0 ? (uint8_t)g.text[p0] : 0u;
-    if (fh != '@') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 1)); }
-    if (fp != '+') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 3)); }
-    seq_len[r] = (uint32_t)(line_end[j + 1] - (h1 + 1));
+    const uint64_t j = 4 * min(r, n_reads - 1);
+    const ulonglong2 e01 = __ldg(reinterpret_cast<const ulonglong2 *>(line_end + j));
+    const ulonglong2 e23 = __ldg(reinterpret_cast<const ulonglong2 *>(line_end + j + 2));
+    uint64_t before = __shfl_up_sync(0xffffffffu, (unsigned long long)e23.y, 1);
+    if (lane_id() == 0 && j) before = line_end[j - 1];
+    uint32_t L = 0;
+    if (r < n_reads) {
+        const uint64_t h0 = j == 0 ? g.S : before + 1, h1 = e01.x;
+        const uint64_t p0 = e01.y + 1, p1 = e23.x;
+        uint32_t fh;
+        const uint64_t q = accession_end(g, h0, h1, fh);
+        const uint32_t fp = p1 > p0 ? (uint8_t)g.text[p0] : 0u;
+        if (fh != '@') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 1)); }
+        if (fp != '+') { atomicExch(&err[DE_PARSE], 1u); atomicMin(&err[DE_PARSE + 1], (uint32_t)(j + 3)); }
+        name_off[r] = h0 + 1;
+        name_len[r] = (uint32_t)(q - (h0 + 1));
+        L = (uint32_t)(e01.y - (h1 + 1));
+        seq_len[r] = L;
+    }
+    L = __reduce_max_sync(0xffffffffu, L);
+    if (lane_id() == 0 && L) atomicMax(&err[DE_MAXLEN], L);
 }
 
 // per-thread walk over its 32 bytes with the line each byte belongs to
@@ -323,12 +372,9 @@ __global__ void k_names(ParseGeom g, const uint64_t *__restrict__ hdr_line, int 
         const uint64_t j = fastq ? 4 * r : hdr_line[r];   // FASTQ: the header is line 4r
         const uint64_t ls = j == 0 ? g.S : line_end[j - 1] + 1;
         const uint64_t le = line_end[j];
-        uint64_t s = ls + 1, q = s;
-        // byte by byte: a thread's header bytes share sectors, and 16-byte
-        // word loads of unrelated headers per lane were slower
-        while (q < le && !is_ws((uint8_t)g.text[q])) q++;
-        name_off[r] = s;
-        name_len[r] = (uint32_t)(q - s);
+        uint32_t first;
+        name_off[r] = ls + 1;
+        name_len[r] = (uint32_t)(accession_end(g, ls, le, first) - (ls + 1));
         const uint64_t L = rd_off[r + 1] - rd_off[r] - 1;
         L32 = (uint32_t)(L > 0xFFFFFFFFull ? 0xFFFFFFFFull : L);
     }
@@ -701,7 +747,10 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
             // their scan gives every read's place in seq
             n_reads = n_lines / 4;
             if ((e = alloc((void **)&line_len, n_reads * 4, "sequence lengths"))) break;
-            k_fq_check<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, line_end, n_reads, line_len, c->d_err);
+            if ((e = dmalloc(c, (void **)&r->d_name_off, n_reads * 8, "name offsets"))) break;
+            if ((e = dmalloc(c, (void **)&r->d_name_len, n_reads * 4, "name lengths"))) break;
+            k_fq_records<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, line_end, n_reads, line_len, r->d_name_off,
+                                                                        r->d_name_len, c->d_err);
             c->launches++;
             if ((e = cuda_check(c, cudaMemcpyAsync(herr, c->d_err + DE_PARSE, 8, cudaMemcpyDeviceToHost, c->stream), "err d2h"))) break;
             if ((e = alloc((void **)&line_out, (n_reads + 1) * 8, "sequence offsets"))) break;
@@ -744,17 +793,17 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
     uint64_t seq_alloc = ((r->seq_len + 2 * SEQ_PAD + 15) / 16) * 16 + 16;
     e = dmalloc(c, (void **)&r->d_seq_alloc, seq_alloc, "packed reads");
     if (!e) e = dmalloc(c, (void **)&r->d_rd_off, (n_reads + 1) * 8, "read offsets");
-    if (!e) e = dmalloc(c, (void **)&r->d_name_off, (n_reads ? n_reads : 1) * 8, "name offsets");
-    if (!e) e = dmalloc(c, (void **)&r->d_name_len, (n_reads ? n_reads : 1) * 4, "name lengths");
+    if (!e && !r->d_name_off) e = dmalloc(c, (void **)&r->d_name_off, (n_reads ? n_reads : 1) * 8, "name offsets");
+    if (!e && !r->d_name_len) e = dmalloc(c, (void **)&r->d_name_len, (n_reads ? n_reads : 1) * 4, "name lengths");
     if (!e) {
         r->d_seq = r->d_seq_alloc + SEQ_PAD;
-        cudaMemsetAsync(c->d_err + DE_WS, 0, 8, c->stream);   // whitespace seen, the longest read
+        if (!n_tiles) cudaMemsetAsync(c->d_err, 0, DE_COUNT * 4, c->stream);   // whitespace seen, the longest read
         uint64_t tail = r->seq_len;
         cudaMemcpyAsync(r->d_rd_off + n_reads, &tail, 8, cudaMemcpyHostToDevice, c->stream);
         uint32_t ws_seen = 0;
-        // accessions and read lengths, and what the host reads back
-        auto finish = [&]() -> int {
-            if (n_tiles && n_reads) {
+        // accessions and read lengths (unless k_fq_records had them), and what the host reads back
+        auto finish = [&](bool names) -> int {
+            if (n_tiles && n_reads && names) {
                 k_names<<<grid_for(n_reads, 256), 256, 0, c->stream>>>(g, hdr_line, fastq, line_end, n_reads, r->d_rd_off,
                                                                        r->d_name_off, r->d_name_len, d_maxlen);
                 c->launches++;
@@ -776,7 +825,7 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
             cudaMemsetAsync(r->d_seq_alloc, '\n', seq_alloc, c->stream);
             e = pack_reads(c, r);
         }
-        if (!e) e = finish();
+        if (!e) e = finish(!fastq);
         r->plain_seq = fastq && !ws_seen;
         if (!e && ws_seen) {
             // some sequence line holds spaces, tabs or CRs: redo the emit byte by byte
@@ -811,7 +860,7 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
                 dfree(c, r->d_pack_alloc);   // of the lines as they were
                 r->d_pack_alloc = nullptr;
                 cudaMemsetAsync(d_maxlen, 0, 4, c->stream);
-                if (!(e = pack_reads(c, r))) e = finish();
+                if (!(e = pack_reads(c, r))) e = finish(true);
             } while (0);
         }
     }

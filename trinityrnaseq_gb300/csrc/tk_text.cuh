@@ -52,15 +52,20 @@ __device__ __forceinline__ void line_word16(const ParseGeom &g, uint64_t S, int6
     }
 }
 
-// Upper-cases a word of bases; notes whether it held whitespace (' ' or 9..13).
+// Bit 7 of each byte of a word that is whitespace (' ' or 9..13).
+__device__ __forceinline__ uint32_t ws_bytes(uint32_t x) {
+    const uint32_t t = x & 0x7F7F7F7Fu, sp = x ^ 0x20202020u;
+    const uint32_t zsp = ~(((sp & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | sp);
+    const uint32_t rng = (t + 0x77777777u) & ~(t + 0x72727272u) & ~x;
+    return (zsp | rng) & 0x80808080u;
+}
+
+// Upper-cases a word of bases; notes whether it held whitespace.
 __device__ __forceinline__ uint32_t upcase_word(uint32_t x, bool &ws) {
     const uint32_t t = x & 0x7F7F7F7Fu;
-    // bit 7 of each byte that is a-z, then of each byte that is ' ' or 9..13
+    // bit 7 of each byte that is a-z
     const uint32_t lower = (t + 0x1F1F1F1Fu) & ~(t + 0x05050505u) & ~x & 0x80808080u;
-    const uint32_t sp = x ^ 0x20202020u;
-    const uint32_t zsp = ~(((sp & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | sp) & 0x80808080u;
-    const uint32_t rng = (t + 0x77777777u) & ~(t + 0x72727272u) & ~x & 0x80808080u;
-    ws |= (zsp | rng) != 0u;
+    ws |= ws_bytes(x) != 0u;
     return x ^ (lower >> 2);
 }
 
