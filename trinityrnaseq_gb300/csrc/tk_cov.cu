@@ -192,18 +192,21 @@ static int cache_get_or_build(tk_table *t, CovCache *cc) {
     const uint64_t bytes = 32ULL << hbits;
     cc->n = n;
     cc->rbits = n - hbits;
-    const bool filter = t->capacity <= SEEN2_MAX_CAPACITY;   // its 16 MB lie behind the cache
-    const uint64_t all = bytes + (4ULL << SEEN2_BITS);
+    const bool filter = t->capacity <= SEEN2_MAX_CAPACITY;   // its 16 MB lie behind the cache, if they are to be had
+    constexpr uint64_t seen2_bytes = 4ULL << SEEN2_BITS;
     if (!t->hot_valid || t->hot_bytes != bytes) {
         if (t->d_hot && t->hot_bytes != bytes) {
             dfree(c, t->d_hot);
             t->d_hot = nullptr;
         }
-        if (!t->d_hot) TK_TRY(dmalloc(c, (void **)&t->d_hot, all, "coverage cache"));
+        if (!t->d_hot) {
+            t->hot_seen2 = filter && dmalloc(c, (void **)&t->d_hot, bytes + seen2_bytes, "coverage cache") == TK_OK;
+            if (!t->hot_seen2) TK_TRY(dmalloc(c, (void **)&t->d_hot, bytes, "coverage cache"));
+        }
         t->hot_bytes = bytes;
-        TK_CUDA(c, cudaMemsetAsync(t->d_hot, 0, all, c->stream));
+        TK_CUDA(c, cudaMemsetAsync(t->d_hot, 0, bytes + (t->hot_seen2 ? seen2_bytes : 0), c->stream));
         cc->ent = t->d_hot;
-        if (filter) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
+        if (filter && t->hot_seen2) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
         cudaEvent_t ev;
         prof_begin(c, TK_KID_COV_CACHE, &ev);
         const uint64_t blocks = std::min<uint64_t>((t->capacity + 255) / 256, (uint64_t)c->sm_count * 16);
@@ -214,7 +217,7 @@ static int cache_get_or_build(tk_table *t, CovCache *cc) {
         t->hot_valid = true;
     }
     cc->ent = t->d_hot;
-    if (filter) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
+    if (filter && t->hot_seen2) cc->seen2 = reinterpret_cast<uint32_t *>(t->d_hot + bytes / 8);
     return TK_OK;
 }
 

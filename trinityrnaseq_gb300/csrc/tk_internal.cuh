@@ -387,6 +387,7 @@ struct tk_table {
     // L2-sized table, built on the first coverage pass after a change
     uint64_t *d_hot = nullptr;
     uint64_t hot_bytes = 0;
+    bool hot_seen2 = false;                   // d_hot has room for the filter behind the cache
     bool hot_valid = false;
 };
 

@@ -1014,6 +1014,15 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, const
     if (!e) e = dmalloc(c, (void **)&defer_keys, defer_cap * 8, "deferred keys");
     if (!e) e = dmalloc(c, (void **)&defer_cnt, defer_cap * 4, "deferred counts");
     if (!e) e = dmalloc(c, (void **)&counters, 16, "count counters");
+    if (e == TK_E_OOM) {   // no room for the batches: the caller counts with atomics, which need none
+        if (grouped) dfree(c, grouped);
+        if (starts) dfree(c, starts);
+        if (d_segs) dfree(c, d_segs);
+        if (d_parts) dfree(c, d_parts);
+        if (defer_keys) dfree(c, defer_keys);
+        if (defer_cnt) dfree(c, defer_cnt);
+        return TK_OK;
+    }
     if (!e) e = cuda_check(c, cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(KeySeg), cudaMemcpyHostToDevice,
                                               c->stream), "partition segments h2d");
     if (!e) e = cuda_check(c, cudaMemcpyAsync(d_parts, parts.data(), parts.size() * sizeof(PartGeom), cudaMemcpyHostToDevice,
@@ -1063,7 +1072,7 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, const
         *overflowed = h[2] != 0;
         *done = true;
     }
-    dfree(c, grouped);
+    if (grouped) dfree(c, grouped);
     if (starts) dfree(c, starts);
     if (d_segs) dfree(c, d_segs);
     if (d_parts) dfree(c, d_parts);
