@@ -47,12 +47,12 @@ L2_BYTES = 129 * 2**20
 E2E_PIECES = 2          # record-aligned pieces per mate file on the end-to-end path
 NORM_ARGS = (200, 1, 10000)   # normalization: Trinity's --max_cov 200 --min_cov 1 --max_CV 10000
 # ncu (--cache-control none), one k_coverage launch at 20M pairs (one mate:
-# 1,516,211,092 lookups): dram__bytes_read.sum 121.66 GB + dram__bytes_write.sum 2.11 GB
-COV_DRAM_BYTES_PER_LOOKUP = (121.66e9 + 2.11e9) / (3_032_422_183 / 2)
-# ncu (--cache-control none), the 1537 count launches of one step at 20M pairs
-# (512 x k_sr_hist, k_sr_scatter, k_sr_build + k_insert_pairs): 48.68 GB read +
-# 38.22 GB written, for 3,032,422,183 occurrences
-COUNT_DRAM_BYTES_PER_OCCURRENCE = (48.68e9 + 38.22e9) / 3_032_422_183
+# 1,516,211,092 lookups): dram__bytes_read.sum 76.36 GB + dram__bytes_write.sum 0.82 GB
+COV_DRAM_BYTES_PER_LOOKUP = (76.36e9 + 0.82e9) / (3_032_422_183 / 2)
+# ncu (--cache-control none), the 207 count launches of one step at 20M pairs
+# (103 x k_sr_group, k_sr_build + k_insert_deferred): 48.86 GB read + 41.59 GB
+# written, for 3,032,422,183 occurrences
+COUNT_DRAM_BYTES_PER_OCCURRENCE = (48.86e9 + 41.59e9) / 3_032_422_183
 
 
 def log(*a):
@@ -478,7 +478,7 @@ def run_gpu(args, dist, world, rank, local):
             "coverage": kernel_roofline("k_coverage (per-read k-mer coverage stats)", "coverage",
                                         packed + 32.0 * windows + 12.0 * reads, windows, ceil_lookup,
                                         "random 16-byte slot lookups vs random 8-byte loads into a table of this size"),
-            "insert": kernel_roofline("k_sr_hist + k_sr_scatter + k_sr_build (count by table ranges)", "count",
+            "insert": kernel_roofline("k_sr_group + k_sr_build (count by table ranges)", "count",
                                       40.0 * windows, windows, ceil_insert,
                                       "k-mer occurrences counted vs random CAS+red.add pairs into a table of this size"),
             "scatter": kernel_roofline("k_part_scatter (k-mers into hash buckets)", "scatter",
@@ -491,14 +491,14 @@ def run_gpu(args, dist, world, rank, local):
         cov_launches = max(per_step["coverage"][1], 1)
         kernels["coverage"]["traffic"] = COV_DRAM_BYTES_PER_LOOKUP * windows / cov_launches
         kernels["coverage"]["traffic_source"] = (
-            "ncu capture (--cache-control none) of one k_coverage launch at 20M pairs (121.66 GB read + 2.11 GB "
+            "ncu capture (--cache-control none) of one k_coverage launch at 20M pairs (76.36 GB read + 0.82 GB "
             "written), " + ("this workload" if args.pairs == FULL_PAIRS else
                             f"scaled by lookups: {COV_DRAM_BYTES_PER_LOOKUP:.0f} DRAM bytes per lookup"))
         ins_launches = max(per_step["count"][1], 1)
         kernels["insert"]["traffic"] = COUNT_DRAM_BYTES_PER_OCCURRENCE * windows / ins_launches
         kernels["insert"]["traffic_source"] = (
-            "ncu capture (--cache-control none) of one step's 1537 count launches at 20M pairs (48.68 GB read + "
-            "38.22 GB written), per launch" + ("" if args.pairs == FULL_PAIRS else
+            "ncu capture (--cache-control none) of one step's 207 count launches at 20M pairs (48.86 GB read + "
+            "41.59 GB written), per launch" + ("" if args.pairs == FULL_PAIRS else
                                                f", scaled by occurrences: {COUNT_DRAM_BYTES_PER_OCCURRENCE:.1f} B each"))
         # the dominant kernel: k_coverage, one kernel with ~29% of the step in
         # the launch list; the count's ~28% is spread over three kernels

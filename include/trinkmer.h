@@ -373,7 +373,7 @@ void tk_norm_free(tk_norm *norm);
  * FASTA back to back; bin b is the records whose header starts in
  * [bin_off[b], bin_off[b+1]) (n_bins + 1 offsets).  Each bin is counted in its
  * own table slice (sized per bin from a sketch, block shape autotuned) by one
- * persistent, CUDA-graph-captured launch, and its ">COUNT\nKMER\n" dump
+ * CUDA-graph-captured launch, and its ">COUNT\nKMER\n" dump
  * (count >= min_count, sorted by key) is bytes [off[b], off[b+1]) of the
  * result text -- the same bytes as a separate tk_table_dump_fasta of that bin. */
 typedef struct tk_bins tk_bins;

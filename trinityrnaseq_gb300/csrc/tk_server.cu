@@ -111,7 +111,7 @@ char text_format(const tk_job_spec &s) {
 }
 
 // Several count jobs as the bins of one batched pass (tk_count_bins_ex): one
-// parse, one persistent counting launch, one dump formatting for all of them.
+// parse, one counting launch, one dump formatting for all of them.
 // The texts are copied straight into one device buffer, a newline between
 // jobs whose text does not end with one.
 int run_count_batch(tk_ctx *c, std::vector<Job *> &batch) {
