@@ -395,3 +395,28 @@ def test_accessions_of_every_length(ctx, fastq, shift):
     ctx.check(rs.lib.tk_reads_names(rs.h, noff.ctypes.data, nlen.ctypes.data), "names")
     assert [text[int(o):int(o) + int(n)] for o, n in zip(noff, nlen)] == names
     assert rs.max_len == 4
+
+
+@pytest.mark.parametrize("k", [1, 2, 15, 16, 25, 31])
+@pytest.mark.parametrize("canonical", [True, False])
+def test_loaded_kmers_at_every_offset_of_the_codes(ctx, k, canonical):
+    """A catalogue's k-mers are cut from the codes at records' starts, k + 1
+    positions apart; a letter that is no base is refused wherever it stands."""
+    rng = np.random.default_rng(k)
+    n = min(4 ** k, 300)
+    mers = sorted({"".join(rng.choice(list("ACGT"), k)) for _ in range(n)})
+    lines = [">%d\n%s\n" % (i + 1, m if i % 3 else m.lower()) for i, m in enumerate(mers)]
+    want = {}
+    for i, m in enumerate(mers):
+        rc = m[::-1].translate(str.maketrans("ACGT", "TGCA"))
+        key = min(m, rc) if canonical else m
+        want[key] = want.get(key, 0) + i + 1
+    t = KmerTable(ctx, k, canonical)
+    t.load_dump_fasta("".join(lines).encode())
+    got = t.dump(1)
+    code = lambda m: sum("ACGT".index(c) << (2 * (k - 1 - i)) for i, c in enumerate(m))
+    assert dict(zip(got[0].tolist(), got[1].tolist())) == {code(m): c for m, c in want.items()}
+    for at in {0, k // 2, k - 1}:
+        m = mers[-1][:at] + "N" + mers[-1][at + 1:]
+        with pytest.raises(native.TrinkmerError):
+            KmerTable(ctx, k, canonical).load_dump_fasta(("".join(lines) + ">1\n%s\n>2\n%s\n" % (m, mers[0])).encode())

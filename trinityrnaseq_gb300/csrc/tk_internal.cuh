@@ -80,6 +80,14 @@ __device__ __forceinline__ uint32_t base_code(uint32_t c) {
     return ok ? b : 4u;
 }
 
+// Reverse complement of a k-mer in 2-bit A<C<G<T code (the low 2k bits):
+// complement every base, then reverse the order of the 2-bit groups.
+__device__ __forceinline__ uint64_t kmer_revcomp(uint64_t fw, int k) {
+    uint64_t x = __brevll(~fw);   // group order reversed, the two bits of each group swapped
+    x = ((x >> 1) & 0x5555555555555555ULL) | ((x & 0x5555555555555555ULL) << 1);
+    return x >> (64 - 2 * k);
+}
+
 __device__ __forceinline__ unsigned lane_id() { return threadIdx.x & 31u; }
 
 // ------------------------------------------------------------------ table ops

@@ -58,14 +58,6 @@ __device__ __forceinline__ void lane_windows(const uint8_t *__restrict__ seq, ui
     }
 }
 
-// Reverse complement of a k-mer in 2-bit A<C<G<T code (the low 2k bits):
-// complement every base, then reverse the order of the 2-bit groups.
-__device__ __forceinline__ uint64_t kmer_revcomp(uint64_t fw, int k) {
-    uint64_t x = __brevll(~fw);   // group order reversed, the two bits of each group swapped
-    x = ((x >> 1) & 0x5555555555555555ULL) | ((x & 0x5555555555555555ULL) << 1);
-    return x >> (64 - 2 * k);
-}
-
 // Packed form of lane_windows for reads made of A/C/G/T only (the common
 // case): the warp first writes the read as a 2-bit, first-base-most-
 // significant bit string into `words` (per-warp shared memory, 12 words),
