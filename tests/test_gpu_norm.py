@@ -311,3 +311,39 @@ def test_extract_copy_async_overlaps_the_next_extraction(ctx):
     ctx.synchronize()
     for i, (b, n) in enumerate(zip(more, lens)):
         assert b.numpy()[:n].tobytes() == want[i % 2]
+
+
+@pytest.mark.parametrize("device_shift", [0, 3])
+def test_extract_names_of_every_length(ctx, oracle, device_shift):
+    """Names of 1 to 40 bytes at every alignment, looked up in words; with "_forward" or "_reverse" at their start,
+    middle and end, one after the other and as halves of one another, looked up in pieces."""
+    import torch
+    rnd = random.Random(3)
+    cores = list(dict.fromkeys("".join(rnd.choice("abXY01_:") for _ in range(1 + i % 40)) for i in range(2000)))
+    marks = ["", "", "", "_forward", "_reverse", "_forward_reverse", "_for_forwardward", "_rev", "_"]
+    recs, names = [], []
+    for i, c in enumerate(cores):
+        m = rnd.choice(marks)
+        at = rnd.randint(0, len(c))
+        names.append(c[:at] + m + c[at:] + rnd.choice(["", "/1", "/2", "/3"]))
+        recs.append("@%s\nACGTACGT\n+\nIIIIIIII\n" % names[-1])
+    text = "".join(recs).encode()
+    # the selection by the plain core names, and by the records' own
+    for rows in (cores, names):
+        fa = "".join(">%s\nACGT\n" % c for c in rows).encode()
+        lrs = ReadSet(ctx, fa)
+        n = len(rows)
+        nm = Normalization(ctx, lrs, (np.full(n, 5, np.uint32), np.full(n, 5, np.float32), np.zeros(n, np.float32)),
+                           max_cov=20, min_cov=1, max_cv=10000)
+        dev = torch.zeros(len(text) + device_shift, dtype=torch.uint8, device="cuda:0")
+        dev[device_shift:] = torch.frombuffer(bytearray(text), dtype=torch.uint8).to("cuda:0")
+        torch.cuda.synchronize()
+        fq = ReadSet(ctx, dev.data_ptr() + device_shift, len(text), device=True)
+        accs = nm.accs()
+        try:
+            want = oracle.norm_extract(text, accs)
+        except Exception:
+            with pytest.raises(native.TrinkmerError):
+                nm.extract(fq)
+        else:
+            assert nm.extract(fq) == want

@@ -825,7 +825,68 @@ __global__ void k_table_write(RowArgs a, SNames L, SNames R, const uint64_t *__r
 
 // ---------------------------------------------------------------- extraction
 
-__device__ __forceinline__ uint64_t fnv_step(uint64_t h, uint8_t c) { return (h ^ c) * 0x100000001b3ULL; }
+// A name's hash, eight of its bytes at a time (the last word's missing bytes 0).
+struct NameHash {
+    uint64_t h = 0xcbf29ce484222325ULL, w = 0;
+    uint32_t n = 0;
+    __device__ __forceinline__ void word(uint64_t v) {
+        h = (h ^ v) * 0x9E3779B97F4A7C15ULL;
+        h ^= h >> 29;
+    }
+    __device__ __forceinline__ void byte(uint8_t c) {
+        w |= (uint64_t)c << (8 * (n & 7u));
+        if ((++n & 7u) == 0) {
+            word(w);
+            w = 0;
+        }
+    }
+    __device__ __forceinline__ uint64_t of_bytes() {
+        if (n & 7u) word(w);
+        return mix64(h ^ n);
+    }
+};
+
+// A stretch of bytes in GPU memory, read in aligned words inside it.
+struct Bytes {
+    const char *lo, *hi;
+    // the n (1 to 8) bytes at p, the first in the low byte
+    __device__ __forceinline__ uint64_t at(const char *p, uint32_t n) const {
+        const uintptr_t a = (uintptr_t)p & ~(uintptr_t)7;
+        const uint32_t o = (uint32_t)((uintptr_t)p & 7);
+        const bool two = o + n > 8;
+        uint64_t v;
+        if (a >= (uintptr_t)lo && a + (two ? 16 : 8) <= (uintptr_t)hi) {
+            const uint64_t *q = reinterpret_cast<const uint64_t *>(a);
+            v = q[0] >> (8 * o);
+            if (two) v |= q[1] << (64 - 8 * o);
+        } else {
+            v = 0;
+            for (uint32_t i = 0; i < n; i++) v |= (uint64_t)(uint8_t)p[i] << (8 * i);
+        }
+        return n < 8 ? v & ((1ULL << (8 * n)) - 1) : v;
+    }
+    // the hash of the n bytes at p; *low whether one of them is '_'
+    __device__ __forceinline__ uint64_t hash(const char *p, uint32_t n, bool *low) const {
+        NameHash x;
+        uint64_t z = 0;
+        for (uint32_t i = 0; i < n; i += 8) {
+            const uint64_t v = at(p + i, min(8u, n - i)), u = v ^ 0x5F5F5F5F5F5F5F5FULL;
+            z |= (u - 0x0101010101010101ULL) & ~u & 0x8080808080808080ULL;
+            x.word(v);
+        }
+        *low = z != 0;
+        return mix64(x.h ^ n);
+    }
+};
+
+// whether the n bytes at p (in a) are the n at q (in b)
+__device__ __forceinline__ bool same_bytes(const Bytes &a, const char *p, const Bytes &b, const char *q, uint32_t n) {
+    for (uint32_t i = 0; i < n; i += 8) {
+        const uint32_t m = min(8u, n - i);
+        if (a.at(p + i, m) != b.at(q + i, m)) return false;
+    }
+    return true;
+}
 
 // A name as up to three pieces of device text (the FASTQ core name after its
 // "_forward" and "_reverse" were cut out).
@@ -880,10 +941,10 @@ __device__ void pieces_cut(Pieces &s, const char *pat) {
 }
 
 __device__ __forceinline__ uint64_t pieces_hash(const Pieces &s) {
-    uint64_t h = 0xcbf29ce484222325ULL;
+    NameHash h;
     for (int q = 0; q < s.k; q++)
-        for (uint32_t i = 0; i < s.n[q]; i++) h = fnv_step(h, (uint8_t)s.p[q][i]);
-    return mix64(h);
+        for (uint32_t i = 0; i < s.n[q]; i++) h.byte((uint8_t)s.p[q][i]);
+    return h.of_bytes();
 }
 
 __device__ __forceinline__ bool pieces_eq(const Pieces &s, const char *b, uint32_t bn) {
@@ -917,17 +978,15 @@ __global__ void k_hash_insert(const char *__restrict__ accs, const uint64_t *__r
         return;
     }
     const uint32_t n = key_len(accs, o, (uint32_t)(acc_off[p + 1] - o - 1));
-    Pieces s;
-    s.k = 1;
-    s.p[0] = accs + o;
-    s.n[0] = n;
-    uint64_t h = pieces_hash(s) & mask;
+    const Bytes text{accs, accs + acc_off[n_rows]};
+    bool low;
+    uint64_t h = text.hash(accs + o, n, &low) & mask;
     for (uint64_t probe = 0; probe <= mask; probe++) {
         const uint32_t cur = atomicCAS(&slots[h], ~0u, (uint32_t)p);
         if (cur == ~0u) return;
         const uint64_t co = acc_off[cur];
         const uint32_t cn = key_len(accs, co, (uint32_t)(acc_off[cur + 1] - co - 1));
-        if (pieces_eq(s, accs + co, cn)) {
+        if (cn == n && same_bytes(text, accs + o, text, accs + co, n)) {
             dup[p] = 1;
             return;
         }
@@ -936,30 +995,40 @@ __global__ void k_hash_insert(const char *__restrict__ accs, const uint64_t *__r
     flag_err(err, NE_HASH);
 }
 
-// per FASTQ record: its core name looked up in the selection
+// Per FASTQ record: its core name looked up in the selection.  The name is read
+// in words once for its hash and once against the name found; only a name with
+// a '_' in it can hold a "_forward" or "_reverse" to be cut out, and is taken
+// in pieces, byte by byte.  Bound by three dependent random loads (slot, offset,
+// name): 2M records 162 us; all names in pieces 189.
 __global__ void k_extract_find(const char *__restrict__ text, uint64_t text_len, const uint64_t *__restrict__ name_off,
                                const uint32_t *__restrict__ name_len, uint64_t n, const char *__restrict__ accs,
-                               const uint64_t *__restrict__ acc_off, const uint32_t *__restrict__ slots, uint64_t mask,
-                               uint8_t *__restrict__ found, uint32_t *__restrict__ rec_len) {
+                               const uint64_t *__restrict__ acc_off, uint64_t n_rows, const uint32_t *__restrict__ slots,
+                               uint64_t mask, uint8_t *__restrict__ found, uint32_t *__restrict__ rec_len) {
     const uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n) return;
     const uint64_t o = name_off[r];
     uint32_t l = name_len[r];
     if (l >= 3 && text[o + l - 2] == '/' && (text[o + l - 1] == '1' || text[o + l - 1] == '2')) l -= 2;
+    const Bytes in{text, text + text_len};
+    bool cut;
+    uint64_t h = in.hash(text + o, l, &cut) & mask;
     Pieces s;
-    s.k = 1;
-    s.p[0] = text + o;
-    s.n[0] = l;
-    pieces_cut(s, "_forward");
-    pieces_cut(s, "_reverse");
-    uint64_t h = pieces_hash(s) & mask;
+    if (cut) {
+        s.k = 1;
+        s.p[0] = text + o;
+        s.n[0] = l;
+        pieces_cut(s, "_forward");
+        pieces_cut(s, "_reverse");
+        h = pieces_hash(s) & mask;
+    }
     bool hit = false;
     for (uint64_t probe = 0; probe <= mask; probe++) {
         const uint32_t cur = slots[h];
         if (cur == ~0u) break;
         const uint64_t co = acc_off[cur];
         const uint32_t cn = key_len(accs, co, (uint32_t)(acc_off[cur + 1] - co - 1));
-        if (pieces_eq(s, accs + co, cn)) {
+        const Bytes sel{accs, accs + acc_off[n_rows]};
+        if (cut ? pieces_eq(s, accs + co, cn) : cn == l && same_bytes(in, text + o, sel, accs + co, l)) {
             found[cur] = 1;
             hit = true;
             break;
@@ -1688,7 +1757,7 @@ int norm_extract(tk_norm *nm, const tk_reads *const *sets, uint32_t nsets) {
                                                                              nm->hash_mask, found, rl, d_err);
             else
                 k_extract_find<<<nm_grid(n), NM_THREADS, 0, c->stream>>>(fq->d_text, fq->text_len, fq->d_name_off,
-                                                                          fq->d_name_len, n, nm->d_accs, nm->acc_off,
+                                                                          fq->d_name_len, n, nm->d_accs, nm->acc_off, P,
                                                                           nm->d_hash, nm->hash_mask, found, rl);
             c->launches++;
             TK_TRY(check_launch(c, "extract find"));
