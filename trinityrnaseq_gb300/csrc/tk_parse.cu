@@ -121,7 +121,7 @@ __global__ void k_tile_newlines(ParseGeom g, const unsigned long long *__restric
     __shared__ uint32_t sm[PT_THREADS / 32 + 1];
     g.S = bounds[0];
     g.E = bounds[1];
-    uint64_t p = g.A + (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
+    uint64_t p = (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
     Bytes32 b = load32(g.text, g.len, p, g.vec);
     const uint32_t m = newline_bits(g, b, p);
     nl_bits[(uint64_t)blockIdx.x * PT_THREADS + threadIdx.x] = m;
@@ -134,7 +134,7 @@ __global__ void k_tile_newlines(ParseGeom g, const unsigned long long *__restric
 __global__ void k_line_ends(ParseGeom g, const uint32_t *__restrict__ nl_bits, const uint64_t *__restrict__ tile_line0,
                             uint64_t *__restrict__ line_end) {
     __shared__ uint32_t sm[PT_THREADS / 32 + 1];
-    const uint64_t p = g.A + (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
+    const uint64_t p = (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
     uint32_t m = nl_bits[(uint64_t)blockIdx.x * PT_THREADS + threadIdx.x];
     uint32_t tot;
     uint64_t line = tile_line0[blockIdx.x] + block_excl_scan<uint32_t>(__popc(m), sm, &tot);
@@ -288,7 +288,7 @@ __device__ __forceinline__ void line_info(const uint8_t *__restrict__ kind, cons
 __global__ void k_tile_emits(ParseGeom g, const uint64_t *__restrict__ tile_line0, const uint8_t *__restrict__ kind,
                              const uint64_t *__restrict__ line_rec, uint64_t n_lines, uint32_t *__restrict__ tile_emit) {
     __shared__ uint32_t sm[PT_THREADS / 32 + 1];
-    uint64_t p = g.A + (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
+    uint64_t p = (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
     Bytes32 b = load32(g.text, g.len, p, g.vec);
     uint32_t nl = 0;
 #pragma unroll
@@ -320,7 +320,7 @@ __global__ void k_emit(ParseGeom g, const uint64_t *__restrict__ tile_line0, con
                        const uint8_t *__restrict__ kind, const uint64_t *__restrict__ line_rec, uint64_t n_lines,
                        uint8_t *__restrict__ seq, uint64_t *__restrict__ rd_off) {
     __shared__ uint32_t sm[PT_THREADS / 32 + 1];
-    uint64_t p = g.A + (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
+    uint64_t p = (uint64_t)blockIdx.x * PT_TILE + (uint64_t)threadIdx.x * PT_BYTES;
     Bytes32 b = load32(g.text, g.len, p, g.vec);
     uint32_t nl = 0;
 #pragma unroll
@@ -695,7 +695,6 @@ int parse_reads(tk_ctx *c, tk_reads *r) {
     g.len = len;
     g.S = g.E = 0;
     g.vec = ((uintptr_t)text & 15u) == 0;
-    g.A = 0;
     r->format = TK_FMT_NONE;
     int fastq = 0;
 

@@ -5,15 +5,14 @@
 // Replaces `jellyfish count/histo/dump` as Trinity drives them
 // (Trinity:2612-2638, util/insilico_read_normalization.pl:617-643).
 //
-// K2 walks the packed read array as one flat stream: each thread owns 32
-// window end positions, reads the 64 bytes [p0-32, p0+32) as four 16-byte
-// vectors, and rolls the forward and reverse-complement 2-bit words in
-// registers; a window is valid after k consecutive A/C/G/T, so read
-// separators and N bases break k-mers with no per-read bookkeeping.  Lanes of
-// a warp that hold the same key in the same step are merged (match.any) and
-// the leader adds the multiplicity with one atomic.  A key that finds no slot
-// within max_probes goes to an overflow list; the host then doubles the table
-// and re-inserts it, so no k-mer is ever dropped silently.
+// K2 walks the read array's 2-bit codes as one flat stream (thread_windows: 32
+// window end positions a thread; a window is valid when no position in it is
+// marked invalid, so read separators and N break k-mers with no per-read
+// bookkeeping), buckets every window by its hash, and builds the table range
+// by range in shared memory; a table that already holds keys is added to with
+// atomics.  A key that finds no slot within max_probes goes to an overflow
+// list; the host then doubles the table and re-inserts it, so no k-mer is ever
+// dropped silently.
 #include "tk_emit.cuh"
 #include "tk_windows.cuh"
 

@@ -9,7 +9,6 @@ struct ParseGeom {
     const char *text;
     uint64_t len;
     uint64_t S, E;        // parsed byte range (leading/trailing whitespace trimmed)
-    uint64_t A;           // first tile start (S rounded down to 16)
     bool vec;
 };
 
