@@ -342,6 +342,11 @@ int tk_ctx_create(int device, tk_ctx **out) {
         return TK_E_OOM;
     }
     cudaMemset(c->d_err, 0, (DE_COUNT + 1) * sizeof(uint32_t));
+    if (const char *v = getenv("TRINKMER_WAIT_TEST")) {
+        char *rest = nullptr;
+        c->wait_test = (uint32_t)strtoul(v, &rest, 10);
+        c->wait_test_polls = std::min<uint32_t>((uint32_t)strtoul(rest, nullptr, 10), 1u << 20);
+    }
     *out = c;
     return TK_OK;
 }

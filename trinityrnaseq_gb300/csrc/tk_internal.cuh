@@ -321,6 +321,9 @@ struct tk_ctx {
     cudaStream_t copy_stream = nullptr;
     uint32_t *d_err = nullptr;             // tk::DE_COUNT words, then the sorts' wait error
     uint32_t *h_wait_err = nullptr;        // page-locked: set when a sort's bounded wait ran out (wait_status)
+    // tests (TRINKMER_WAIT_TEST="<which> <polls>", read when the context is made): the which-th scan or sort
+    // pass of several tiles leaves its first tile out and gives up after so many polls
+    uint32_t wait_test = 0, wait_test_polls = 0;
     unsigned char *h_stage = nullptr;      // page-locked, STAGE_BYTES: small results read back at one synchronisation
     std::string last_error;
     // profiling (CUDA events on `stream` around the hot kernels)

@@ -1406,8 +1406,9 @@ static int sort_side(tk_ctx *c, NormSide &s) {
         TK_TRY(pass(2, 0));
         for (int ch = (int)nch - 1; ch >= 0; ch--) TK_TRY(pass(0, (uint32_t)ch));
         TK_TRY(gather());
+        TK_CUDA(c, cudaStreamSynchronize(c->stream));
     }
-    TK_TRY(wait_status(c));   // the sorts before the last synchronisation
+    TK_TRY(wait_status(c));   // of every sort: each lies before the last synchronisation
     if (perm != s.perm) {
         TK_CUDA(c, cudaMemcpyAsync(s.perm, perm, n * 4, cudaMemcpyDeviceToDevice, c->stream));
     }

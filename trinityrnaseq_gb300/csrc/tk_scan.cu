@@ -10,8 +10,12 @@
 // A published word is 64 bits, written and read whole, so it needs no fence:
 // bits 62-63 say what it holds (0 nothing yet, 1 the tile alone, 2 the tile
 // and all before it) and, in the sort, bits 58-61 the pass it belongs to.
-// Every wait is bounded: past WAIT_POLLS polls the block sets the error word
-// and returns without storing, and the host reports it (wait_status).
+// Every wait is bounded: past WAIT_POLLS polls the block sets the context's
+// error word and returns without storing, and the host reports it
+// (wait_status).  The others that wait look at the word too and give up with
+// it, so that one limit's time is all that is lost; and what is enqueued behind
+// a sort pass that gave up stores nothing: its input is not whole, and places
+// taken from the counts of the true keys could lie outside the arrays.
 #include "tk_emit.cuh"
 
 #include <algorithm>
@@ -20,11 +24,25 @@ namespace tk {
 
 constexpr uint64_t ST_PART = 1ULL << 62, ST_FULL = 2ULL << 62, ST_VALUE = (1ULL << 58) - 1;
 constexpr uint32_t WAIT_POLLS = 1u << 20;   // of about a microsecond each
+constexpr uint32_t WAIT_LOOK = 256;         // polls between two looks at the error word
 
 __device__ __forceinline__ uint64_t st_read(const uint64_t *p) {
     return *reinterpret_cast<const volatile uint64_t *>(p);
 }
 __device__ __forceinline__ void st_write(uint64_t *p, uint64_t v) { *reinterpret_cast<volatile uint64_t *>(p) = v; }
+__device__ __forceinline__ bool gave_up(const uint32_t *wait_err) {
+    return *reinterpret_cast<const volatile uint32_t *>(wait_err) != 0;
+}
+
+// The polls a launch over `tiles` tiles may wait.  A test can have one such
+// launch of a context leave out its first tile (*skip 1: the tickets start
+// there, with a block fewer), so that every later tile's wait runs out.
+static uint32_t wait_limit(tk_ctx *c, uint64_t tiles, uint32_t *skip) {
+    *skip = 0;
+    if (c->wait_test == 0 || tiles < 2 || --c->wait_test != 0) return WAIT_POLLS;
+    *skip = 1;
+    return c->wait_test_polls;
+}
 
 // ------------------------------------------------------------------ scan
 
@@ -69,7 +87,8 @@ struct RecordLength {   // ">COUNT\nKMER\n"
 template <typename Tin, typename F, int EVERY>
 __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict__ in, uint64_t *__restrict__ out, uint64_t n,
                                                     int vec, ScanHead *__restrict__ head, uint64_t *__restrict__ state,
-                                                    uint64_t *__restrict__ total_at, uint32_t *__restrict__ err_at) {
+                                                    uint64_t *__restrict__ total_at, uint32_t *__restrict__ err_at,
+                                                    uint32_t max_polls) {
     __shared__ uint64_t s_warp[SN_WARPS], s_before;
     __shared__ uint32_t s_tile, s_fail;
     if (threadIdx.x == 0) {
@@ -118,10 +137,8 @@ __global__ void __launch_bounds__(SN_THREADS) k_scan(F f, const Tin *__restrict_
             uint64_t v = mine >= 0 ? 0 : ST_FULL;
             for (uint32_t polls = 0; __any_sync(0xffffffffu, v < ST_PART); polls++) {
                 if (v < ST_PART) v = st_read(&state[mine]);
-                if (polls > WAIT_POLLS) {   // uniform over the warp
-                    fail = true;
-                    break;
-                }
+                fail = polls > max_polls || (polls % WAIT_LOOK == WAIT_LOOK - 1 && __any_sync(0xffffffffu, gave_up(err_at)));
+                if (fail) break;   // uniform over the warp
             }
             const unsigned full = __ballot_sync(0xffffffffu, v >= ST_FULL);
             const int stop = full ? __ffs((int)full) - 1 : 31;
@@ -185,10 +202,13 @@ static int scan_enqueue(tk_ctx *c, F f, const Tin *in, uint64_t *out, uint64_t n
     const size_t bytes = sizeof(ScanHead) + nt * 8;
     TK_TRY(dmalloc(c, (void **)mem, bytes, "scan tiles"));
     int e = cuda_check(c, cudaMemsetAsync(*mem, 0, bytes, c->stream), "scan reset");
+    uint32_t skip;
+    const uint32_t polls = wait_limit(c, nt, &skip);
+    if (!e && skip) e = cuda_check(c, cudaMemsetAsync(&(*mem)->ticket, 1, 1, c->stream), "scan ticket");
     if (!e) {
         const int vec = (((uintptr_t)in | (EVERY > 1 ? 0 : (uintptr_t)out)) & 15u) == 0;
-        k_scan<Tin, F, EVERY><<<(unsigned)nt, SN_THREADS, 0, c->stream>>>(f, in, out, n, vec, *mem, reinterpret_cast<uint64_t *>(*mem + 1),
-                                                                  total_at, c->d_err + DE_COUNT);
+        k_scan<Tin, F, EVERY><<<(unsigned)nt - skip, SN_THREADS, 0, c->stream>>>(
+            f, in, out, n, vec, *mem, reinterpret_cast<uint64_t *>(*mem + 1), total_at, c->d_err + DE_COUNT, polls);
         c->launches++;
         e = check_launch(c, "scan");
     }
@@ -335,7 +355,7 @@ template <int THREADS, int ITEMS>
 __global__ void __launch_bounds__(THREADS, THREADS == 384 ? 3 : 4)
     k_rs_pass(const uint64_t *__restrict__ keys, const uint32_t *__restrict__ vals, uint64_t *__restrict__ okeys,
               uint32_t *__restrict__ ovals, uint64_t n, int shift, int pass, SortHead *__restrict__ head,
-              uint64_t *__restrict__ state, uint32_t *__restrict__ wait_err) {
+              uint64_t *__restrict__ state, uint32_t *__restrict__ wait_err, uint32_t max_polls) {
     constexpr uint32_t TILE = THREADS * ITEMS;
     static_assert(THREADS >= RS_BINS && TILE <= 65536, "one digit per thread, 16-bit places");
     extern __shared__ __align__(16) unsigned char rs_mem[];
@@ -343,12 +363,13 @@ __global__ void __launch_bounds__(THREADS, THREADS == 384 ? 3 : 4)
     __shared__ uint32_t s_warp[RS_BINS / 32];
     __shared__ uint32_t s_tile, s_fail;
     if (threadIdx.x == 0) {
+        s_fail = gave_up(wait_err);
         s_tile = atomicAdd(&head->ticket[pass], 1u);
-        s_fail = 0;
     }
     for (uint32_t i = threadIdx.x; i < THREADS / 32 * RS_BINS / 2; i += THREADS)
         reinterpret_cast<uint32_t *>(&sm.wcnt[0][0])[i] = 0;
     __syncthreads();
+    if (s_fail) return;   // an earlier pass or tile gave up
     const uint64_t tile = s_tile, t0 = tile * TILE;
     const uint32_t m = n - t0 < (uint64_t)TILE ? (uint32_t)(n - t0) : TILE;
     const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -431,7 +452,8 @@ __global__ void __launch_bounds__(THREADS, THREADS == 384 ? 3 : 4)
         uint64_t before = 0;
         bool found = tile == 0;
         const uint64_t *q = words + tile * RS_BINS;   // the words of the tile last taken
-        for (uint32_t polls = 0; !found && polls <= WAIT_POLLS; polls++) {
+        for (uint32_t polls = 0; !found && polls <= max_polls; polls++) {
+            if (polls % WAIT_LOOK == WAIT_LOOK - 1 && gave_up(wait_err)) break;
             uint64_t w[LOOK];
 #pragma unroll
             for (int i = 0; i < LOOK; i++) {
@@ -492,8 +514,11 @@ static int sort_run(tk_ctx *c, uint64_t *ka, uint32_t *va, uint64_t *kb, uint32_
             ka, n, first_bit, passes, head);
         c->launches++;
         for (int p = 0; p < passes; p++) {
-            k_rs_pass<THREADS, ITEMS><<<(unsigned)nt, THREADS, smem, c->stream>>>(
-                ka, va, kb, vb, n, first_bit + p * RS_BITS, p, head, state, c->d_err + DE_COUNT);
+            uint32_t skip;
+            const uint32_t polls = wait_limit(c, nt, &skip);
+            if (skip) cudaMemsetAsync(&head->ticket[p], 1, 1, c->stream);
+            k_rs_pass<THREADS, ITEMS><<<(unsigned)nt - skip, THREADS, smem, c->stream>>>(
+                ka, va, kb, vb, n, first_bit + p * RS_BITS, p, head, state, c->d_err + DE_COUNT, polls);
             c->launches++;
             std::swap(ka, kb);
             std::swap(va, vb);
@@ -536,7 +561,9 @@ constexpr int FX_THREADS = 256, FX_ITEMS = 4, FX_TILE = FX_THREADS * FX_ITEMS;
 constexpr int FX_NEAR = 64;
 constexpr int FX_BITS = 10;
 
-__global__ void __launch_bounds__(FX_THREADS) k_sort_runs(uint64_t *keys, uint32_t *vals, uint64_t n, int r) {
+__global__ void __launch_bounds__(FX_THREADS) k_sort_runs(uint64_t *keys, uint32_t *vals, uint64_t n, int r,
+                                                          const uint32_t *__restrict__ wait_err) {
+    if (*wait_err) return;   // a pass gave up: the pairs are not in order
     static_assert(FX_TILE >= (1 << FX_BITS) && FX_THREADS >= FX_NEAR, "a run fits a block");
     __shared__ uint64_t s[FX_TILE + FX_NEAR + 1];   // the pair before the tile, the tile, FX_NEAR pairs behind it
     __shared__ uint32_t s_long[FX_TILE / FX_NEAR + 1], n_long, map[1 << (FX_BITS - 5)], below[1 << (FX_BITS - 5)];
@@ -622,7 +649,7 @@ int sort_distinct_pairs(tk_ctx *c, uint64_t *keys, uint32_t *vals, uint64_t n, i
     TK_TRY(radix_sort_pairs(c, keys, vals, n, bits - low, tmp_keys, tmp_vals, result_in_tmp, low));
     if (low == 0 || n <= 1) return TK_OK;
     k_sort_runs<<<(unsigned)((n + FX_TILE - 1) / FX_TILE), FX_THREADS, 0, c->stream>>>(
-        *result_in_tmp ? tmp_keys : keys, *result_in_tmp ? tmp_vals : vals, n, low);
+        *result_in_tmp ? tmp_keys : keys, *result_in_tmp ? tmp_vals : vals, n, low, c->d_err + DE_COUNT);
     c->launches++;
     return check_launch(c, "sort runs");
 }
