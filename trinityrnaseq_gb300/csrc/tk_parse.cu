@@ -588,7 +588,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_seq_tiles(const char 
                 const uint32_t in = ((((held >> (4 * w)) & 0xFu) * 0x00204081u) & 0x01010101u) * 0xFFu;
                 x[w] = (upcase_word((x[w] & in) | (0x41414141u & ~in), ws) & in) | (0x0A0A0A0Au & ~in);
             }
-            if (ws) atomicExch(ws_seen, 1u);
+            if (ws) *ws_seen = 1u;   // (an atomic per line of a CRLF text took four times the copy)
             pack32(x, code, bad);
         }
         uint4 *o = reinterpret_cast<uint4 *>(seq + 32 * word);
