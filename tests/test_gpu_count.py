@@ -420,3 +420,63 @@ def test_loaded_kmers_at_every_offset_of_the_codes(ctx, k, canonical):
         m = mers[-1][:at] + "N" + mers[-1][at + 1:]
         with pytest.raises(native.TrinkmerError):
             KmerTable(ctx, k, canonical).load_dump_fasta(("".join(lines) + ">1\n%s\n>2\n%s\n" % (m, mers[0])).encode())
+
+
+def fasta_of(seqs, gap):
+    """Records of seqs with gap(i) blank lines after record i."""
+    return b"".join(b">r%d x\n%s\n%s" % (i, s, b"\n" * gap(i)) for i, s in enumerate(seqs))
+
+
+@pytest.mark.parametrize("gap", [4090, 4094, 4095, 4096, 4097, 9000, 40_000])
+@pytest.mark.parametrize("at", [0, 1, 70, 119])
+def test_parse_many_blank_lines_at_one_place(ctx, gap, at):
+    """Lines without positions: a tile of the read array may hold any number of them."""
+    rng = np.random.default_rng(gap + at)
+    seqs = [bytes(rng.choice(np.frombuffer(b"ACGTacgtN", np.uint8), int(n))) for n in rng.integers(0, 400, 120)]
+    rs = ReadSet(ctx, fasta_of(seqs, lambda i: gap if i == at else 0))
+    assert rs.sequences() == [s.upper() for s in seqs]
+    assert rs.accessions() == [b"r%d" % i for i in range(120)]
+
+
+@pytest.mark.parametrize("n", [2047, 2048, 2049, 12_289])
+@pytest.mark.parametrize("lens", [(0,), (1,), (0, 1, 0, 40), (3, 0, 0, 0, 9000), (2, 0, 0, 0, 0, 0, 0, 1)])
+@pytest.mark.parametrize("fastq", [False, True])
+def test_parse_short_and_empty_records(ctx, n, lens, fastq):
+    rng = np.random.default_rng(n)
+    letters = rng.choice(np.frombuffer(b"ACGTN", np.uint8), 20_000).tobytes()
+    seqs = [letters[i % 7000:i % 7000 + lens[i % len(lens)]] for i in range(n)] + [b"ACGTACGTAC"]
+    if fastq:
+        text = b"".join(b"@r%d/1\n%s\n+\n%s\n" % (i, s, b"I" * len(s)) for i, s in enumerate(seqs))
+    else:
+        text = b"".join(b">r%d/1\n%s\n" % (i, s) for i, s in enumerate(seqs))
+    rs = ReadSet(ctx, text)
+    assert rs.sequences() == seqs
+    k = KmerTable(ctx, 5, False)
+    k.add(rs)   # the 2-bit codes made beside the letters
+    want = {}
+    for s in seqs:
+        for j in range(len(s) - 4):
+            w = s[j:j + 5]
+            if b"N" not in w:
+                want[w.decode()] = want.get(w.decode(), 0) + 1
+    assert_pairs(k.dump(1), dict_to_arrays(want))
+
+
+def test_blank_lines_do_not_hold_up_the_parser(ctx):
+    """3M blank lines in one place cost about what their bytes cost (one block
+    that walked them took 80 times the parse without them)."""
+    import time
+    rng = np.random.default_rng(3)
+    seqs = [s.tobytes() for s in rng.choice(np.frombuffer(b"ACGT", np.uint8), (100_000, 100))]
+
+    def best(text):
+        out = []
+        for _ in range(6):
+            t0 = time.perf_counter()
+            ReadSet(ctx, text).free()
+            out.append(time.perf_counter() - t0)
+        return min(out)
+
+    plain = best(fasta_of(seqs, lambda i: 0))
+    blank = best(fasta_of(seqs, lambda i: 3_000_000 if i == 50_000 else 0))
+    assert blank < 6 * plain, (blank, plain)

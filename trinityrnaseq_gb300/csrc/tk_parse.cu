@@ -457,6 +457,13 @@ constexpr int ST_THREADS = 256;
 constexpr int ST_BLOCKS = 6;         // an SM: 42 registers a thread
 constexpr uint32_t ST_TILE = ST_THREADS * 32;
 constexpr uint32_t ST_LINES = 512;   // lines of a tile held in shared memory at a time
+// Lines of a tile from which each thread looks its lines up in memory instead:
+// blank lines and empty records take few positions or none, so there is no
+// bound to a tile's lines, and one block would go through all of them (2.4 us for
+// 512: 400,000 reads with 300,000 blank lines in one place 1.69 ms against 0.25
+// this way, with 100,000 empty records among them 0.49 against 0.30).  Reads of four
+// bases have 3300 lines a tile; from 1024 to 8192 lines the time is the same.
+constexpr uint32_t ST_DENSE = 8 * ST_LINES;
 
 // Per line: its record's start, and the tiles whose first position it holds.
 template <bool FASTQ>
@@ -507,13 +514,70 @@ __global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_seq_tiles(const char 
     uint32_t x[8], held = 0;                // held: positions that are bases
 #pragma unroll
     for (int w = 0; w < 8; w++) x[w] = sep[w];
+    // lays the bases of a line on [q, e) of the tile (e past the thread's last position: cut there)
+    auto lay_line = [&](uint32_t q, uint32_t e, int64_t delta) {
+        // the text byte that would lie at this thread's first position
+        const int64_t at = (int64_t)(T0 + q0) + delta;
+        const uint32_t a = q - q0;
+        const uintptr_t p = (uintptr_t)text + (uintptr_t)at, p16 = p & ~(uintptr_t)15;
+        uint32_t v[8];
+        if (p16 >= (uintptr_t)text && p16 + 48 <= (uintptr_t)text + len) {
+            const uint4 *u = reinterpret_cast<const uint4 *>(p16);
+            const uint4 u0 = __ldg(u), u1 = __ldg(u + 1), u2 = __ldg(u + 2);
+            uint32_t t[12] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.x, u2.y, u2.z, u2.w};
+            if (p & 8) {
+#pragma unroll
+                for (int w = 0; w < 10; w++) t[w] = t[w + 2];
+            }
+            if (p & 4) {
+#pragma unroll
+                for (int w = 0; w < 9; w++) t[w] = t[w + 1];
+            }
+            const uint32_t sh = 8u * (uint32_t)(p & 3);
+#pragma unroll
+            for (int w = 0; w < 8; w++) v[w] = __funnelshift_r(t[w], t[w + 1], sh);
+        } else {   // at an end of the text
+#pragma unroll
+            for (int w = 0; w < 8; w++) {
+                v[w] = 0;
+                for (uint32_t i4 = 0; i4 < 4; i4++) {
+                    const uint32_t o = 4 * w + i4;
+                    if (o >= a && q0 + o < e) v[w] |= (uint32_t)(uint8_t)text[at + o] << (8 * i4);
+                }
+            }
+        }
+        lay_from(x, v, a);
+        if (e < q0 + 32u) lay_from(x, sep, e - q0);
+        held |= (e - q0 >= 32u ? ~0u : (1u << (e - q0)) - 1u) & (~0u << a);
+    };
     if (T0 < L.seq_len) {
         const uint32_t lim = (uint32_t)min((uint64_t)ST_TILE, L.seq_len - T0);
         const uint32_t qe = min(q0 + 32u, lim);
         const uint64_t first = tile_line[blockIdx.x];
         const uint64_t last = T0 + ST_TILE < L.seq_len ? tile_line[blockIdx.x + 1] : L.n - 1;
         uint32_t q = q0;
-        for (uint64_t c0 = first; c0 <= last; c0 += ST_LINES) {
+        if (last - first >= ST_DENSE) {
+            // a line at a time from memory: the last line that begins at or before q
+            uint64_t i = first, hi = last + 1;
+            while (hi - i > 1) {
+                const uint64_t mid = (i + hi) >> 1;
+                if (L.start(mid) <= T0 + q) i = mid;
+                else hi = mid;
+            }
+            while (q < qe) {
+                const uint64_t s = L.start(i), e = s + L.line_len[i];
+                if (e > T0 + q) lay_line(q, (uint32_t)min(e - T0, (uint64_t)qe), (int64_t)L.src(i) - (int64_t)s);
+                q = (uint32_t)min(L.start(i + 1) - T0, (uint64_t)qe);
+                uint64_t step = 1;   // on to the line of the new q, in doubling steps and back
+                while (i + step <= last && L.start(i + step) <= T0 + q) {
+                    i += step;
+                    step *= 2;
+                }
+                for (; step; step >>= 1)
+                    if (i + step <= last && L.start(i + step) <= T0 + q) i += step;
+            }
+        }
+        for (uint64_t c0 = first; last - first < ST_DENSE && c0 <= last; c0 += ST_LINES) {
             const uint32_t m = (uint32_t)min((uint64_t)ST_LINES, last - c0 + 1);
             if (c0 != first) __syncthreads();
             for (uint32_t i = threadIdx.x; i <= m; i += ST_THREADS) {
@@ -537,41 +601,7 @@ __global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_seq_tiles(const char 
                 while (q < stop) {
                     while (s_start[i + 1] <= q) i++;
                     const uint32_t e = min(s_end[i], qe);
-                    if (e > q) {
-                        // the text byte that would lie at this thread's first position
-                        const int64_t at = (int64_t)(T0 + q0) + s_delta[i];
-                        const uint32_t a = q - q0;
-                        const uintptr_t p = (uintptr_t)text + (uintptr_t)at, p16 = p & ~(uintptr_t)15;
-                        uint32_t v[8];
-                        if (p16 >= (uintptr_t)text && p16 + 48 <= (uintptr_t)text + len) {
-                            const uint4 *u = reinterpret_cast<const uint4 *>(p16);
-                            const uint4 u0 = __ldg(u), u1 = __ldg(u + 1), u2 = __ldg(u + 2);
-                            uint32_t t[12] = {u0.x, u0.y, u0.z, u0.w, u1.x, u1.y, u1.z, u1.w, u2.x, u2.y, u2.z, u2.w};
-                            if (p & 8) {
-#pragma unroll
-                                for (int w = 0; w < 10; w++) t[w] = t[w + 2];
-                            }
-                            if (p & 4) {
-#pragma unroll
-                                for (int w = 0; w < 9; w++) t[w] = t[w + 1];
-                            }
-                            const uint32_t sh = 8u * (uint32_t)(p & 3);
-#pragma unroll
-                            for (int w = 0; w < 8; w++) v[w] = __funnelshift_r(t[w], t[w + 1], sh);
-                        } else {   // at an end of the text
-#pragma unroll
-                            for (int w = 0; w < 8; w++) {
-                                v[w] = 0;
-                                for (uint32_t i4 = 0; i4 < 4; i4++) {
-                                    const uint32_t o = 4 * w + i4;
-                                    if (o >= a && q0 + o < e) v[w] |= (uint32_t)(uint8_t)text[at + o] << (8 * i4);
-                                }
-                            }
-                        }
-                        lay_from(x, v, a);
-                        if (e < q0 + 32u) lay_from(x, sep, e - q0);
-                        held |= (e - q0 >= 32u ? ~0u : (1u << (e - q0)) - 1u) & (~0u << a);
-                    }
+                    if (e > q) lay_line(q, e, s_delta[i]);
                     q = min(s_start[i + 1], stop);
                 }
             }
