@@ -439,7 +439,7 @@ def test_parse_many_blank_lines_at_one_place(ctx, gap, at):
 
 
 @pytest.mark.parametrize("n", [2047, 2048, 2049, 12_289])
-@pytest.mark.parametrize("lens", [(0,), (1,), (0, 1, 0, 40), (3, 0, 0, 0, 9000), (2, 0, 0, 0, 0, 0, 0, 1)])
+@pytest.mark.parametrize("lens", [(0,), (1,), (0, 1, 0, 40), (3, 0, 0, 0, 900), (2, 0, 0, 0, 0, 0, 0, 1)])
 @pytest.mark.parametrize("fastq", [False, True])
 def test_parse_short_and_empty_records(ctx, n, lens, fastq):
     rng = np.random.default_rng(n)
@@ -480,3 +480,40 @@ def test_blank_lines_do_not_hold_up_the_parser(ctx):
     plain = best(fasta_of(seqs, lambda i: 0))
     blank = best(fasta_of(seqs, lambda i: 3_000_000 if i == 50_000 else 0))
     assert blank < 6 * plain, (blank, plain)
+
+
+def test_count_a_partition_of_more_than_2_32_keys(ctx):
+    """Deep reads over few k-mers: one table slice, 4.6G windows in one call.
+    Counted by ranges like any other call (the same launches per read set and
+    three more), every count a multiple of the one set's."""
+    import torch
+    if torch.cuda.mem_get_info()[0] < 150 << 30:
+        pytest.skip("needs 150 GB of GPU memory")
+    g = torch.Generator().manual_seed(4)
+    letters = torch.tensor(list(b"ACGT"), dtype=torch.uint8)
+    genome = letters[torch.randint(0, 4, (60_000,), generator=g)].cuda()
+    at = torch.randint(0, 60_000 - 100, (3_000_000,), generator=g).cuda()
+    reads = genome[at[:, None] + torch.arange(100, device="cuda")]
+    n = at.numel()
+    text = torch.cat([torch.tensor(list(b">r\n"), dtype=torch.uint8, device="cuda").expand(n, 3), reads,
+                      torch.full((n, 1), 10, dtype=torch.uint8, device="cuda")], 1).reshape(-1)
+    torch.cuda.synchronize()
+    rs = ReadSet(ctx, text.data_ptr(), text.numel(), device=True)
+    launches, pairs = [], []
+    for times in (2, 3, 20):
+        t = KmerTable(ctx, 25, True)
+        before = ctx.kernel_launches
+        t.add_many([rs] * times)
+        launches.append(ctx.kernel_launches - before)
+        keys, counts = t.dump(1)
+        pairs.append((keys, counts // times))
+        assert not (counts % times).any()
+        assert t.info()[1] == times * n * 76
+        t.free()
+    assert 20 * n * 76 > 1 << 32 and launches[2] - launches[0] == 18 * (launches[1] - launches[0])
+    for p in pairs[1:]:
+        assert_pairs(p, pairs[0])
+    rs.free()
+    del text, reads
+    torch.cuda.empty_cache()
+    ctx.trim()

@@ -454,8 +454,9 @@ __device__ __forceinline__ bool smem_add(unsigned long long *keys, uint32_t *val
 struct __align__(16) BuildSmem {
     unsigned long long tkey[SR_MAX_SLOTS], mkey[SR_MINI];   // 16-byte aligned pairs
     uint32_t tval[SR_MAX_SLOTS], mval[SR_MINI];
+    uint64_t run[SR_BUILD_THREADS];          // where the chunk's run begins in the grouped keys, less cum (64-bit: a
+                                             // partition of deep reads over few k-mers may be more than 2^32 keys)
     uint32_t cum[SR_BUILD_THREADS + 1];      // keys of the range in the chunks before
-    uint32_t run[SR_BUILD_THREADS];          // where the chunk's run begins in the grouped keys
     uint32_t scan[SR_BUILD_THREADS / 32 + 1];
 };
 
@@ -486,16 +487,18 @@ __global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *_
     for (uint32_t t0 = 0; t0 < part.chunks; t0 += SR_BUILD_THREADS) {
         // the runs of up to SR_BUILD_THREADS chunks, taken as one sequence
         const uint32_t c = t0 + threadIdx.x;
-        uint32_t n = 0, first = 0;
+        uint32_t n = 0;
+        uint64_t first = 0;
         if (c < part.chunks) {
             const uint16_t *st = starts + (uint64_t)(part.chunk0 + c) * (nsub + 1) + r;
             const uint32_t a = st[0];
             n = st[1] - a;
-            first = (part.chunk0 + c) * SG_CHUNK + a;
+            first = (uint64_t)(part.chunk0 + c) * SG_CHUNK + a;
         }
         uint32_t total;
-        sm.cum[threadIdx.x] = block_excl_scan<uint32_t>(n, sm.scan, &total);
-        sm.run[threadIdx.x] = first;
+        const uint32_t before = block_excl_scan<uint32_t>(n, sm.scan, &total);
+        sm.cum[threadIdx.x] = before;
+        sm.run[threadIdx.x] = first - before;
         if (threadIdx.x == 0) sm.cum[SR_BUILD_THREADS] = total;
         __syncthreads();
         // a warp takes a stretch of the sequence; a lane walks its runs forward
@@ -517,7 +520,7 @@ __global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *_
                 k4[u] = EMPTY_KEY;
                 if (i < hi) {
                     while (sm.cum[q + 1] <= i) q++;
-                    k4[u] = __ldcg(grouped + sm.run[q] + (i - sm.cum[q]));
+                    k4[u] = __ldcg(grouped + (sm.run[q] + i));
                 }
             }
 #pragma unroll
@@ -999,7 +1002,6 @@ static int count_by_ranges(tk_table *t, const std::vector<BucketKeys> &bk, const
         all_keys += part;
     }
     batch.push_back(nparts);
-    if (max_chunks * SG_CHUNK > 0xFFFFFFFFull) return TK_OK;   // places in the grouped keys are 32-bit
     uint64_t defer_cap = std::max<uint64_t>(1u << 16, std::min<uint64_t>(all_keys / 64, 1u << 24));
     if (const char *v = getenv("TRINKMER_DEFER_CAP")) defer_cap = std::max<uint64_t>(1, strtoull(v, nullptr, 10));   // tests: force the fallback
     uint64_t *grouped = nullptr, *defer_keys = nullptr;
