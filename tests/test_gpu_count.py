@@ -517,3 +517,33 @@ def test_count_a_partition_of_more_than_2_32_keys(ctx):
     del text, reads
     torch.cuda.empty_cache()
     ctx.trim()
+
+
+def test_count_runs_of_equal_keys(ctx):
+    """One-window reads, every k-mer many times in a row, in table slices short
+    enough that some runs lie at the end of a range: whole warps add one key."""
+    rng = np.random.default_rng(12)
+    kmers = np.unique(rng.choice(np.frombuffer(b"ACGT", np.uint8), (20_000, 25)), axis=0)
+    times = rng.choice([1, 31, 127, 128, 129, 200, 700], kmers.shape[0])
+    at = np.repeat(np.arange(kmers.shape[0]), times)
+    rows = np.concatenate([np.full((at.size, 1), ord(">"), np.uint8), np.full((at.size, 1), 10, np.uint8), kmers[at],
+                           np.full((at.size, 1), 10, np.uint8)], axis=1)
+    t = gpu_count(ctx, rows.tobytes(), canonical=False)
+    code = np.zeros(kmers.shape[0], np.uint64)
+    for j in range(25):
+        code = code * np.uint64(4) + np.searchsorted(np.frombuffer(b"ACGT", np.uint8), kmers[:, j]).astype(np.uint64)
+    order = np.argsort(code)
+    assert_pairs(t.dump(1), (code[order], times[order].astype(np.uint32)))
+    assert t.info()[:2] == (kmers.shape[0], int(times.sum()))
+
+
+@pytest.mark.parametrize("unit", [b"A", b"AC", b"ACGT", b"ACGTTGCAAC"])
+def test_count_repeats_beside_ordinary_reads(ctx, oracle, unit):
+    rng = np.random.default_rng(len(unit))
+    genome = rng.choice(np.frombuffer(b"ACGT", np.uint8), 30_000)
+    recs = [b">a\n" + (unit * 100)[i % len(unit):][:100] + b"\n" for i in range(20_000)]
+    for p in rng.integers(0, 29_900, 20_000):
+        recs.append(b">b\n" + genome[p:p + 100].tobytes() + b"\n")
+    for mixed in (False, True):
+        text = b"".join([recs[i] for i in rng.permutation(len(recs))] if mixed else recs)
+        assert_pairs(gpu_count(ctx, text).dump(1), oracle.count(text, 25, True))

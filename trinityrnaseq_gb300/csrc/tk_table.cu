@@ -512,7 +512,20 @@ __global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *_
                 if (sm.cum[mid] <= lo) q = mid; else e = mid;
             }
         }
-        for (uint32_t i0 = lo + lane; i0 < hi; i0 += 128) {
+        auto put = [&](uint64_t key, uint32_t inc) {
+            if (smem_add(sm.tkey, sm.tval, (uint32_t)((mix64(key) & t.lmask) - r0), len, key, inc, added)) return;
+            // the probe left the range: count it in the per-block table, or defer it
+            const uint32_t m = (uint32_t)(mix64(key ^ 0x5851F42D4C957F2DULL) & (SR_MINI - 1));
+            if (smem_add(sm.mkey, sm.mval, m, SR_MINI, key, inc, unused) ||
+                (m && smem_add(sm.mkey, sm.mval, 0, m, key, inc, unused)))
+                return;
+            const unsigned long long j = atomicAdd(defer_n, 1ULL);
+            if (j < defer_cap) {
+                defer_keys[j] = key;
+                defer_cnt[j] = inc;
+            }
+        };
+        for (uint32_t i0 = lo + lane; i0 - lane < hi; i0 += 128) {
             uint64_t k4[4];
 #pragma unroll
             for (int u = 0; u < 4; u++) {
@@ -523,22 +536,20 @@ __global__ void __launch_bounds__(SR_BUILD_THREADS) k_sr_build(const uint64_t *_
                     k4[u] = __ldcg(grouped + (sm.run[q] + i));
                 }
             }
-#pragma unroll
-            for (int u = 0; u < 4; u++) {
-                const uint64_t key = k4[u];
-                if (key == EMPTY_KEY || smem_add(sm.tkey, sm.tval, (uint32_t)((mix64(key) & t.lmask) - r0), len, key, 1u, added))
-                    continue;
-                // the probe left the range: count it in the per-block table, or defer it singly
-                const uint32_t m = (uint32_t)(mix64(key ^ 0x5851F42D4C957F2DULL) & (SR_MINI - 1));
-                if (smem_add(sm.mkey, sm.mval, m, SR_MINI, key, 1u, unused) ||
-                    (m && smem_add(sm.mkey, sm.mval, 0, m, key, 1u, unused)))
-                    continue;
-                const unsigned long long j = atomicAdd(defer_n, 1ULL);
-                if (j < defer_cap) {
-                    defer_keys[j] = key;
-                    defer_cnt[j] = 1u;
-                }
+            // A repeat's key: one add for the warp's 128 (without it the one block
+            // that holds poly-A is what the call waits for: 400,000 reads, half of them
+            // poly-A, 7.5 ms for 4.5).  The loop is uniform over the warp, and the vote
+            // brings its lanes together before the probes: 3M reads of a 40 Mb genome
+            // 2.83 -> 2.69 ms, of 20 kb over and over 5.7 -> 4.0.
+            const uint64_t k0 = __shfl_sync(0xffffffffu, k4[0], 0);   // (every lane takes it)
+            const bool alike = (k4[0] == k0) & (k4[1] == k0) & (k4[2] == k0) & (k4[3] == k0);
+            if (__all_sync(0xffffffffu, alike)) {
+                if (lane == 0 && k0 != EMPTY_KEY) put(k0, 128u);
+                continue;
             }
+#pragma unroll
+            for (int u = 0; u < 4; u++)
+                if (k4[u] != EMPTY_KEY) put(k4[u], 1u);
         }
         __syncthreads();
     }
