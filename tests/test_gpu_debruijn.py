@@ -93,3 +93,17 @@ def test_tool_writes_the_graphs(native_built, oracle, golden, tmp_path):
     assert ss == oracle.debruijn(b.read_bytes(), 24, True)
     bad = subprocess.run([str(exe), "--fasta", str(b), "-K", "24"], stdout=subprocess.PIPE, stderr=subprocess.PIPE)
     assert bad.returncode != 0
+
+
+@pytest.mark.parametrize("n", [23, 24, 25, 55, 56, 57, 300, 2047, 2048, 9000])
+def test_stretches_of_one_letter(ctx, oracle, n):
+    """Whole warps of one k-mer, cut by other letters, joins and record ends, and met again in the next record."""
+    rnd = np.random.default_rng(n)
+    recs = []
+    for i in range(40):
+        s = rnd.choice(np.frombuffer(b"ACGT", dtype=np.uint8), int(rnd.integers(1, 90))).tobytes()
+        recs.append(b">s_%d\n%s%sX%s%sNN%s\n" % (i, s, b"A" * n, b"T" * (n // 2), s, b"G" * n))
+    b = b"".join(recs)
+    for K in (4, 24):
+        for ss in (False, True):
+            assert gpu_text(ctx, b, K, ss) == oracle.debruijn(b, K, ss), (K, ss)
