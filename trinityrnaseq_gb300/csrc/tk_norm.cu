@@ -1327,7 +1327,6 @@ static int sort_side(tk_ctx *c, NormSide &s) {
     TK_TRY(sc.get((void **)&d_stats, sizeof(NameStats), "name statistics"));
     TK_TRY(sc.get((void **)&orand, 16, "sort key bits"));
     TK_CUDA(c, cudaMemsetAsync(tperm, 0, n * 4, c->stream));   // whatever a sort leaves there indexes a read
-    TK_CUDA(c, cudaMemsetAsync(tperm, 0, n * 4, c->stream));   // whatever a sort leaves there indexes a read
     TK_CUDA(c, cudaMemsetAsync(d_stats, 0, sizeof(NameStats), c->stream));
     TK_CUDA(c, cudaMemsetAsync(d_stats->all, 0xFF, sizeof stats.all, c->stream));
     k_name_stats<<<(unsigned)std::min<uint64_t>(nm_grid(n), (uint64_t)c->sm_count * 8), NM_THREADS, 0, c->stream>>>(
