@@ -46,13 +46,14 @@ MIN_COUNT = 2           # the catalogue fastaToKmerCoverageStats reads (util/ins
 L2_BYTES = 129 * 2**20
 E2E_PIECES = 2          # record-aligned pieces per mate file on the end-to-end path
 NORM_ARGS = (200, 1, 10000)   # normalization: Trinity's --max_cov 200 --min_cov 1 --max_CV 10000
-# ncu (--cache-control none), one k_coverage launch at 20M pairs (one mate:
-# 1,516,211,092 lookups): dram__bytes_read.sum 76.36 GB + dram__bytes_write.sum 0.82 GB
-COV_DRAM_BYTES_PER_LOOKUP = (76.36e9 + 0.82e9) / (3_032_422_183 / 2)
-# ncu (--cache-control none), the 207 count launches of one step at 20M pairs
-# (103 x k_sr_group, k_sr_build + k_insert_deferred): 48.86 GB read + 41.59 GB
-# written, for 3,032,422,183 occurrences
-COUNT_DRAM_BYTES_PER_OCCURRENCE = (48.86e9 + 41.59e9) / 3_032_422_183
+# ncu (--cache-control none), one k_coverage launch at 1M pairs (one mate: 75,812,258
+# lookups): dram__bytes_read.sum 3.035 GB + dram__bytes_write.sum 0.094 GB
+COV_DRAM_BYTES_PER_LOOKUP = (3.035e9 + 0.094e9) / (151_624_516 / 2)
+# ncu (--cache-control none), one k_sr_group and one k_sr_build launch at 200K pairs
+# (30,325,297 occurrences, one batch): keys read and written by the group, read
+# again by the build, 0.232 + 0.232 + 0.246 GB; the build also writes the
+# table's slots, 16 B each
+COUNT_DRAM_BYTES_PER_OCCURRENCE = (0.232e9 + 0.232e9 + 0.246e9) / 30_325_297
 
 
 def log(*a):
@@ -485,24 +486,21 @@ def run_gpu(args, dist, world, rank, local):
                                        packed + 8.0 * windows, 0, None, None),
         }
         kernels["insert"]["random_access"]["l2_slice_ceiling_per_s"] = ceil_slice
-        # DRAM traffic of the coverage kernel: one ncu capture (1 pass) of the
-        # same kernel on the 20M-pair workload, per lookup, times this run's
-        # lookups per launch (random 16-byte loads fetch whole DRAM bursts)
+        # DRAM traffic per launch, from captures of one launch on small cases: the
+        # coverage's per lookup (a larger table is missed more often: an estimate
+        # from below), the count's per occurrence plus the table written once
         cov_launches = max(per_step["coverage"][1], 1)
         kernels["coverage"]["traffic"] = COV_DRAM_BYTES_PER_LOOKUP * windows / cov_launches
         kernels["coverage"]["traffic_source"] = (
-            "ncu capture (--cache-control none) of one k_coverage launch at 20M pairs (76.36 GB read + 0.82 GB "
-            "written), " + ("this workload" if args.pairs == FULL_PAIRS else
-                            f"scaled by lookups: {COV_DRAM_BYTES_PER_LOOKUP:.0f} DRAM bytes per lookup"))
+            "ncu capture (--cache-control none) of one k_coverage launch at 1M pairs (3.035 GB read + 0.094 GB "
+            f"written), scaled by lookups: {COV_DRAM_BYTES_PER_LOOKUP:.0f} DRAM bytes per lookup")
         ins_launches = max(per_step["count"][1], 1)
-        kernels["insert"]["traffic"] = COUNT_DRAM_BYTES_PER_OCCURRENCE * windows / ins_launches
+        kernels["insert"]["traffic"] = (COUNT_DRAM_BYTES_PER_OCCURRENCE * windows + 16.0 * capacity) / ins_launches
         kernels["insert"]["traffic_source"] = (
-            "ncu capture (--cache-control none) of one step's 207 count launches at 20M pairs (48.86 GB read + "
-            "41.59 GB written), per launch" + ("" if args.pairs == FULL_PAIRS else
-                                               f", scaled by occurrences: {COUNT_DRAM_BYTES_PER_OCCURRENCE:.1f} B each"))
-        # the dominant kernel: k_coverage, one kernel with ~29% of the step in
-        # the launch list; the count's ~28% is spread over three kernels
-        # (k_sr_build, the largest, ~12%), reported under roofline_kernels
+            "ncu captures (--cache-control none) of one k_sr_group and one k_sr_build launch at 200K pairs, scaled by "
+            f"occurrences: {COUNT_DRAM_BYTES_PER_OCCURRENCE:.1f} B each, and 16 B per slot of the table; per launch")
+        # the dominant kernel: k_coverage, one kernel with 32% of the step (CUDA
+        # events of the default run); the count's 21% are two kernels
         top = "coverage"
         out = {
             "metric": METRIC, "value": tot_windows / t_step, "unit": UNIT, "n_gpus": world, "steps": args.steps,

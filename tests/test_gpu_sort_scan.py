@@ -68,3 +68,16 @@ def test_runs_of_keys_alike_but_for_their_last_bits(ctx, k, low, lens):
     gk, gc = t.dump(1)
     order = np.argsort(keys)
     assert np.array_equal(gk, keys[order]) and np.array_equal(gc, counts[order])
+
+
+@pytest.mark.parametrize("off", [-1, 0, 1])
+def test_dump_order_where_the_tiles_change(ctx, off):
+    """1024 pairs per SM of this device."""
+    import torch
+    n = torch.cuda.get_device_properties(ctx.device).multi_processor_count * 1024 + off
+    keys = distinct_keys(n, 25, n)
+    t = KmerTable(ctx, 25, False)
+    t.load_pairs(keys, np.arange(1, n + 1, dtype=np.uint32))
+    gk, gc = t.dump(1)
+    order = np.argsort(keys)
+    assert np.array_equal(gk, keys[order]) and np.array_equal(gc, np.arange(1, n + 1, dtype=np.uint32)[order])

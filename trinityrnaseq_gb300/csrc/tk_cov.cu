@@ -33,10 +33,12 @@
 // Most lookups the cache misses are k-mers seen once, whose answer is 1.  Beside
 // the cache of a table of at most 2^29 slots lies a 16 MB filter of the keys
 // whose count is not 1 (two bits in a 32-bit word): a k-mer it does not hold
-// needs no table access.  5M pairs 14.1 -> 13.4 ms, 1.5M 4.29 -> 3.83, 0.6M 1.52 ->
-// 1.44; with 32 MB 13.5, 3.86 and 1.45, with 8 MB 14.2, 3.91 and 1.46.  For larger
-// tables the filter passes most keys while its lines share L2 with the
-// cache's (20M pairs: 8% slower with 32 or 64 MB).
+// needs no table access.  Without and with it, both mates: 0.3M pairs 0.75 and
+// 0.66 ms, 1M 2.32 and 2.36, 2M 5.45 and 4.94, 5M 14.0 and 13.0, 9M (2^29 slots,
+// nearly full) 26.6 and 25.2; 10M (2^30 slots) 27.7 both, 12M 33.6 and 33.9, 16M
+// 45.5 and 47.9: the fuller filter passes most keys while its lines share L2
+// with the cache's.  With 32 MB 5M pairs 13.5 and 1.5M 3.86, with 8 MB 14.2
+// and 3.91 (16 MB: 13.4 and 3.83 then).
 #include "tk_warp.cuh"
 
 #include <algorithm>

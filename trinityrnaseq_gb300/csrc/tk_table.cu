@@ -37,7 +37,8 @@ constexpr int SC_TILE = 16384;                                   // window end p
 // Positions of a set whose key buffer is not sized exactly: reading the size
 // back is a round trip of about 12 us, 2% of the 600 us of one bin of 2000
 // pairs and below 0.5% of the 3 ms that 2^24 positions take; the buffer is then
-// 134 MB at most.
+// at most a window at each position and three keys of padding per bucket and
+// block, 138 MB with 152 blocks.
 constexpr uint64_t SC_SMALL = 1ull << 24;
 constexpr int SC_BUF = 24;                                       // a multiple of 4 (whole 32-byte sectors)
 static_assert(SC_BUF % 4 == 0 && SC_BUF <= 32, "a half-warp flushes a bucket in two 16-key stores");
